@@ -5,9 +5,10 @@
 // Semantics follow the reference's per-point arithmetic in src/TD.jl:
 //   frame + TDCS coordinates       CalculateLocalTriCoords! :712-732, GlobalToTDECoords :870-908
 //   interior angles, side vectors  CalcTDVectsAndAngles :962-1008
-//   configuration selection        trimodefinder :1010-1079
-//   full-space strain / disp       TDstrainFS :1499-1620 + TDSetupS :1623-1750,
-//                                  TDdispFS :735-867 + TDSetupD :1081-1173
+//   points on a side               trimodefinder :1010-1079
+//   full-space strain / disp       TDstrainFS :1499-1620, TDdispFS :735-867 (the reference sums
+//                                  three angular dislocations; here the same closed loop is
+//                                  summed as three straight segments, see seg_integrals)
 //   free-surface correction        AngSetupStrainFSC :1867-2081, AngSetupDispFSC :1258-1409
 //   image dislocation              ComputeStrainInfluences :670-708, ComputeDispInfluences :631-668
 // The closed-form angular-dislocation terms come from tde_closed_form.cuh.
@@ -31,22 +32,13 @@ namespace cad {
 // array of T: the FP32 copy used for far-field pairs is an element-wise
 // conversion of the FP64 record (flags are stored as 0 / 1 values).
 template <typename T>
-struct AngDisT {         // one angular dislocation of a TD frame (configuration I)
-    T cosT, sinT;        // side-vector z and y components; configuration II negates both
-    T tv1, tv2;          // vertex y, z in TDCS
-    T sinADE1;           // sin(alpha - pi) / (8 pi (1 - nu))
-    ang_dis_strain_k<T> ks;
-    ang_dis_disp_k<T> kd;
-};
-
-template <typename T>
 struct FrameT {          // a TD (real or image) in its own coordinate system
     T P2[3];
     T P2lo[3];           // FP32 records: P2 - (double)(float)P2 (0 in FP64 records)
     T Vn[3], Vs[3], Vd[3];
     T p1y, p1z, p3y, p3z;           // TDCS (y, z) of P1 and P3; P2 is the origin
-    T t23y, t32x, t31y, t13x, base; // configuration-test constants
-    AngDisT<T> v[3];                // at P1 (side -e13), P2 (e12), P3 (e23)
+    T t23y, t32x, t31y, t13x, base; // on-a-side test constants
+    T sy[3], sz[3];                 // unit vectors (TDCS y, z) of the sides P1-P2, P2-P3, P3-P1
     T flat;                         // 1: all vertex z exactly 0
 };
 
@@ -73,7 +65,6 @@ struct TriDevT {
     FscSideT<T> side[3];
 };
 
-using AngDis = AngDisT<double>;
 using Frame = FrameT<double>;
 using FscSide = FscSideT<double>;
 using TriDev = TriDevT<double>;
@@ -201,20 +192,6 @@ CAD_HD void tensor_rot(R t[6], const R* A)
            (A[5] * A[7] + A[4] * A[8]) * Tyz + A[4] * A[5] * Tyy + A[7] * A[8] * Tzz;
 }
 
-// Rotation of a tensor about the TDCS x axis by the side angle (the B matrix
-// [1 0 0; 0 c -s; 0 s c] of TDSetupS, stored column-major), written out.
-template <typename R>
-CAD_HD void tensor_rot_x(R t[6], R c, R s)
-{
-    const R Tyy = t[1], Tzz = t[2], Txy = t[3], Txz = t[4], Tyz = t[5];
-    const R cc = c * c, ss = s * s, cs = c * s;
-    t[1] = R(2.0) * cs * Tyz + cc * Tyy + ss * Tzz;
-    t[2] = R(-2.0) * cs * Tyz + ss * Tyy + cc * Tzz;
-    t[3] = c * Txy + s * Txz;
-    t[4] = -s * Txy + c * Txz;
-    t[5] = (cc - ss) * Tyz + cs * (Tzz - Tyy);
-}
-
 // Observation point -> TDCS of frame f.
 template <typename R>
 CAD_HD void to_tdcs(const FrameT<R>& f, double X, double Y, double Z, R& x, R& y, R& z)
@@ -226,226 +203,266 @@ CAD_HD void to_tdcs(const FrameT<R>& f, double X, double Y, double Z, R& x, R& y
     z = dot3_rn(f.Vd[0], f.Vd[1], f.Vd[2], dX, dY, dZ);
 }
 
-// Artefact-free configuration: +1 (I), -1 (II), 0 (on a side, in the TD plane).
+// Whether the point (TDCS) lies on a side of the triangle, in its plane: the
+// reference's trimodefinder returning 0.  Its other two values select which
+// way the angular dislocations run; segments need no such choice.
 template <typename R>
-CAD_HD int trimode(const FrameT<R>& f, R x, R y, R z)
+CAD_HD bool on_side(const FrameT<R>& f, R x, R y, R z)
 {
+    if (x != 0.0) return false;
     const R dy = sub_rn(y, f.p3y), dz = sub_rn(z, f.p3z);
     const R a = add_rn(mul_rn(f.t23y, dy), mul_rn(f.t32x, dz)) / f.base;
     const R b = add_rn(mul_rn(f.t31y, dy), mul_rn(f.t13x, dz)) / f.base;
     const R c = sub_rn(sub_rn(R(1.0), a), b);
-    bool casen = false, casez = false;
-    if (a <= 0.0 && b > c && c > a) casen = true;
-    else if (b <= 0.0 && c > a && a > b) casen = true;
-    else if (c <= 0.0 && a > b && b > c) casen = true;
-    else if (a == 0.0 && b >= 0.0 && c >= 0.0) casez = true;
-    else if (a >= 0.0 && b == 0.0 && c >= 0.0) casez = true;
-    else if (a >= 0.0 && b >= 0.0 && c == 0.0) casez = true;
-    if (casez && x != 0.0) casez = false;
-    return casez ? 0 : (casen ? -1 : 1);
+    if (a <= 0.0 && b > c && c > a) return false;
+    if (b <= 0.0 && c > a && a > b) return false;
+    if (c <= 0.0 && a > b && b > c) return false;
+    return (a == 0.0 && b >= 0.0 && c >= 0.0) || (a >= 0.0 && b == 0.0 && c >= 0.0) ||
+           (a >= 0.0 && b >= 0.0 && c == 0.0);
 }
 
-// ------------------------------------------------------ full-space strain
-// One angular dislocation's contribution for all three unit modes, added to
-// E[m][k] (TDCS).  sgn = +1 for configuration I, -1 for II.
+// ------------------------------------------------- full-space dislocation
+// The field of a triangular dislocation depends on its boundary alone (the
+// displacement also on the solid angle the triangle subtends), so it is the
+// sum over the three sides of the line integrals of a straight dislocation
+// segment (de Wit 1960; Hirth and Lothe, Theory of Dislocations, ch. 4).
+// With d the offset of the point from the side's line, s the coordinate along
+// it and R the distance, a side contributes
+//   V = int ds / R    K = int ds / R^3    T = int s ds / R^3
+//   I = 3 int ds / R^5                    Q = -3 int s ds / R^5
+// One segment costs about a third of the angular dislocation it replaces, and
+// the vertex distances serve two sides each.
 template <typename R>
-CAD_HD void ad_strain(const AngDisT<R>& v, R sgn, R x, R y, R z, R Dss, R Dds, R Dn, R K8, R E[3][6])
+struct SegInt {
+    R K, I, T, Q, V;
+};
+
+// Integrals of one side from its end distances (R, 1 / R) and the coordinates
+// sA, sB of the ends along it, rho2 = |d|^2.  The side is taken in the
+// direction in which the nearer end has the smaller coordinate, so R + s of
+// the farther end cannot cancel; the nearer end's is rho2 / (R - s) when its
+// coordinate is negative.
+template <bool LOG, typename R>
+CAD_HD SegInt<R> seg_integrals(R RA, R iA, R RB, R iB, R sA, R sB, R rho2)
 {
-    const R CosT = sgn * v.cosT, SinT = sgn * v.sinT;
-    const R dy = y - v.tv1, dz = z - v.tv2;
-    const R Yr = CosT * dy - SinT * dz;
-    const R Zr = SinT * dy + CosT * dz;
-    R o[21];
-    ang_dis_strain(v.ks, x, Yr, Zr, o);
-    const R exxBx = o[0], exxBy = o[1], exxBz = o[2];
-    const R eyyBx = o[3], eyyBy = o[4], eyyBz = o[5];
-    const R ezzBx = o[6], ezzBy = o[7], ezzBz = o[8];
-    const R exyBx = o[9], exyBy = o[10], exyBz = o[11];
-    const R exzBx = o[12], exzBy = o[13], exzBz = o[14];
-    const R eyzBx = o[15], eyzBy = o[16], eyzBz = o[17];
-    const R rFx = o[18], rFy = o[19], rFz = o[20];
-    const R sinADE1 = v.sinADE1;
-    if (Dn != 0.0) {
-        const R E3 = Dn * K8;
-        R t[6];
-        t[0] = Dn * rFx + E3 * exxBx;
-        t[1] = E3 * eyyBx;
-        t[2] = E3 * ezzBx;
-        t[3] = R(0.5) * Dn * rFy - E3 * exyBx;
-        t[4] = R(0.5) * Dn * rFz - E3 * exzBx;
-        t[5] = E3 * eyzBx;
-        tensor_rot_x(t, CosT, SinT);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) E[0][k] += t[k];
-    }
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const R slip = q == 0 ? Dss : Dds;
-        if (!(slip != 0.0)) continue;
-        // in-plane slip (strike, dip) of this mode in ADCS
-        const R Ds = q == 0 ? CosT * Dss : -SinT * Dds;
-        const R Dd = q == 0 ? SinT * Dss : CosT * Dds;
-        const R E5 = Ds * K8;
-        const R E4 = E5 * x;
-        const R dsa = Dd * sinADE1;
-        const R dsax = dsa * x;
-        R t[6];
-        t[0] = -E4 * exxBy + dsax * exxBz;
-        t[1] = Ds * rFy - E4 * eyyBy + dsax * eyyBz;
-        t[2] = -E4 * ezzBy + Dd * rFz + dsax * ezzBz;
-        t[3] = R(0.5) * Ds * rFx + E5 * exyBy - dsa * exyBz;
-        t[4] = E5 * exzBy + R(0.5) * Dd * rFx - dsa * exzBz;
-        t[5] = R(0.5) * Ds * rFz - E4 * eyzBy + R(0.5) * Dd * rFy - dsax * eyzBz;
-        tensor_rot_x(t, CosT, SinT);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) E[1 + q][k] += t[k];
-    }
+    const bool fwd = sA + sB >= R(0.0);
+    const R a = fwd ? sA : -sB, b = fwd ? sB : -sA;
+    const R Ra = fwd ? RA : RB, Rb = fwd ? RB : RA;
+    const R ia = fwd ? iA : iB, ib = fwd ? iB : iA;
+    const bool out = a >= R(0.0);
+    const R den = out ? Ra + a : rho2, num = out ? R(1.0) : Ra - a;
+    const R wb = Rb + b;
+    const R inv = R(1.0) / (den * wb);
+    const R iwa = inv * wb * num, iwb = inv * den;   // 1 / (R + s) at both ends
+    const R ua = ia * iwa, ub = ib * iwb;
+    SegInt<R> g;
+    g.K = ua - ub;
+    g.I = ua * ua * (R(2.0) * Ra + a) * ia - ub * ub * (R(2.0) * Rb + b) * ib;
+    g.T = iA - iB;
+    g.Q = iA * iA * iA - iB * iB * iB;
+    g.V = LOG ? cad_log(wb * iwa) : R(0.0);
+    return g;
 }
 
-// Full-space strain of frame f at one point, added into E (EFCS).  For the
-// image frame the accumulated value is first carried into the image TDCS and
-// the result carried back, as the reference does; a flat (z = 0) image
-// triangle keeps the reference's detached xz / yz components.
-template <bool IMAGE, typename R>
-CAD_HD void strain_fs(const FrameT<R>& f, double X, double Y, double Z, R Dss, R Dds, R Dn, R K8, R E[3][6])
+constexpr double kInv4Pi = 0.079577471545947667884;   // 1 / (4 pi)
+
+// Strain of unit slip n, strike, dip (TDCS xx, yy, zz, xy, xz, yz) and the
+// displacement (its solid-angle part included) of frame f at TDCS (x, y, z).
+// K8 = 1 / (8 pi (1 - nu)).  In the segment's own axes (n = TD normal,
+// m = t x n in the plane, t along the side) the offset is (x, e, 0), the
+// Hessian of V is H, and a unit Burgers vector b gives
+//   strain -1/(4 pi) sym(b w) K + (1/(4 pi) - 2 K8) sym((b x t) grad V) - K8 (b.w) H
+//   displacement 1/(4 pi) (b x t) V - K8 ((b x t) V + (b.w) grad V)
+// with w = (-e, x, 0) and grad V = (-x K, -e K, T).
+template <bool STRAIN, bool DISP, typename R>
+CAD_HD void td_unit(const FrameT<R>& f, R x, R y, R z, R K8, R E[3][6], R U[3][3])
 {
-    R x, y, z;
-    to_tdcs(f, X, Y, Z, x, y, z);
-    const int mode = trimode(f, x, y, z);
-    R keep_xz[3], keep_yz[3];
-    const bool detach = IMAGE && f.flat != R(0);
-    if (IMAGE) {
-        const R RotInv[9] = {f.Vn[0], f.Vs[0], f.Vd[0], f.Vn[1], f.Vs[1], f.Vd[1], f.Vn[2], f.Vs[2], f.Vd[2]};
+    const R k1 = R(kInv4Pi), ka = k1 - R(2.0) * K8;
+    const R h = R(-1.0) * K8;   // (ka - k1) / 2
+    const R dy[3] = {y - f.p1y, y, y - f.p3y}, dz[3] = {z - f.p1z, z, z - f.p3z};
+    const R x2 = x * x;
+    R Rv[3], iR[3];
 #pragma unroll
-        for (int m = 0; m < 3; ++m) tensor_rot(E[m], RotInv);
-        if (detach) {
-#pragma unroll
-            for (int m = 0; m < 3; ++m) {
-                keep_xz[m] = E[m][4];
-                keep_yz[m] = E[m][5];
-                E[m][4] = -E[m][4];
-                E[m][5] = -E[m][5];
-            }
-        }
+    for (int v = 0; v < 3; ++v) {
+        const R q = x2 + dy[v] * dy[v] + dz[v] * dz[v];
+        iR[v] = cad_rsqrt(q);
+        Rv[v] = q * iR[v];
     }
-    const R sgn = mode == -1 ? R(-1.0) : R(1.0);
-#pragma unroll 1
-    for (int a = 0; a < 3; ++a) ad_strain(f.v[a], sgn, x, y, z, Dss, Dds, Dn, K8, E);
-    if (mode == 0) {
+    if (STRAIN) {
 #pragma unroll
         for (int m = 0; m < 3; ++m)
 #pragma unroll
-            for (int k = 0; k < 6; ++k) E[m][k] = qnan<R>();
+            for (int k = 0; k < 6; ++k) E[m][k] = R(0.0);
     }
-    const R Rot[9] = {f.Vn[0], f.Vn[1], f.Vn[2], f.Vs[0], f.Vs[1], f.Vs[2], f.Vd[0], f.Vd[1], f.Vd[2]};
+    if (DISP) {
+        // solid angle of the triangle seen from the point
+        const R one = -x * ((dy[1] - dy[0]) * (dz[2] - dz[0]) - (dz[1] - dz[0]) * (dy[2] - dy[0]));
+        const R ab = x2 + dy[0] * dy[1] + dz[0] * dz[1];
+        const R ac = x2 + dy[0] * dy[2] + dz[0] * dz[2];
+        const R bc = x2 + dy[1] * dy[2] + dz[1] * dz[2];
+        const R two = Rv[0] * Rv[1] * Rv[2] + ab * Rv[2] + ac * Rv[1] + bc * Rv[0];
+        const R Fi = R(-2.0) * k1 * cad_atan2(one, two);
 #pragma unroll
-    for (int m = 0; m < 3; ++m) tensor_rot(E[m], Rot);
-    if (detach) {
+        for (int m = 0; m < 3; ++m)
 #pragma unroll
-        for (int m = 0; m < 3; ++m) {
-            E[m][4] = keep_xz[m];
-            E[m][5] = keep_yz[m];
+            for (int c = 0; c < 3; ++c) U[m][c] = m == c ? Fi : R(0.0);
+    }
+#pragma unroll
+    for (int sd = 0; sd < 3; ++sd) {
+        const int A = sd, B = sd == 2 ? 0 : sd + 1;
+        const R ty = f.sy[sd], tz = f.sz[sd];
+        const R sA = -(dy[A] * ty + dz[A] * tz), sB = -(dy[B] * ty + dz[B] * tz);
+        const R e = dy[A] * tz - dz[A] * ty;
+        const R e2 = e * e;
+        const SegInt<R> g = seg_integrals<DISP>(Rv[A], iR[A], Rv[B], iR[B], sA, sB, x2 + e2);
+        if (STRAIN) {
+            const R Hnn = x2 * g.I - g.K, Hmm = e2 * g.I - g.K;
+            const R Htt = -(Hnn + Hmm);
+            const R hT = R(0.5) * ka * g.T;
+            // b = n
+            const R nnn = e * (k1 * g.K + K8 * Hnn), nmm = e * (ka * g.K + K8 * Hmm), ntt = K8 * e * Htt;
+            const R nnm = x * (h * g.K + K8 * e2 * g.I), nmt = -hT - K8 * e2 * g.Q, nnt = -K8 * e * x * g.Q;
+            // b = m
+            const R mmm = x * (-k1 * g.K - K8 * Hmm), mnn = x * (-ka * g.K - K8 * Hnn), mtt = -K8 * x * Htt;
+            const R mnm = -e * (h * g.K + K8 * x2 * g.I), mnt = hT + K8 * x2 * g.Q, mmt = K8 * x * e * g.Q;
+            // b = t: only nt and mt
+            const R tnt = R(0.5) * k1 * g.K * e, tmt = R(-0.5) * k1 * g.K * x;
+            const R yy = ty * ty, zz = tz * tz, yz = ty * tz, dd = zz - yy;
+            E[0][0] += nnn;
+            E[0][1] += nmm * zz + ntt * yy + R(2.0) * nmt * yz;
+            E[0][2] += nmm * yy + ntt * zz - R(2.0) * nmt * yz;
+            E[0][3] += nnm * tz + nnt * ty;
+            E[0][4] += nnt * tz - nnm * ty;
+            E[0][5] += (ntt - nmm) * yz + nmt * dd;
+            // b = m and b = t in TDCS, then unit strike = (tz m + ty t), unit dip = (-ty m + tz t)
+            const R r1 = mmm * zz + mtt * yy + R(2.0) * mmt * yz, r2 = mmm * yy + mtt * zz - R(2.0) * mmt * yz;
+            const R r3 = mnm * tz + mnt * ty, r4 = mnt * tz - mnm * ty, r5 = (mtt - mmm) * yz + mmt * dd;
+            const R q1 = R(2.0) * tmt * yz, q3 = tnt * ty, q4 = tnt * tz, q5 = tmt * dd;
+            E[1][0] += tz * mnn;
+            E[1][1] += tz * r1 + ty * q1;
+            E[1][2] += tz * r2 - ty * q1;
+            E[1][3] += tz * r3 + ty * q3;
+            E[1][4] += tz * r4 + ty * q4;
+            E[1][5] += tz * r5 + ty * q5;
+            E[2][0] += -ty * mnn;
+            E[2][1] += tz * q1 - ty * r1;
+            E[2][2] += -tz * q1 - ty * r2;
+            E[2][3] += tz * q3 - ty * r3;
+            E[2][4] += tz * q4 - ty * r4;
+            E[2][5] += tz * q5 - ty * r5;
+        }
+        if (DISP) {
+            const R cV = k1 - K8;
+            // b = n: -cV V m + K8 e grad V;  b = m: cV V n - K8 x grad V;  b = t: none
+            const R xK = x * g.K, eK = e * g.K;
+            const R vm = -cV * g.V - K8 * e * eK, vt = K8 * e * g.T;
+            const R um = -K8 * x * g.T, un = cV * g.V + K8 * x * xK, uw = K8 * x * eK;
+            U[0][0] -= K8 * e * xK;
+            U[0][1] += vm * tz + vt * ty;
+            U[0][2] += vt * tz - vm * ty;
+            const R a1 = uw * tz + um * ty, a2 = um * tz - uw * ty;
+            U[1][0] += tz * un;
+            U[1][1] += tz * a1;
+            U[1][2] += tz * a2;
+            U[2][0] -= ty * un;
+            U[2][1] -= ty * a1;
+            U[2][2] -= ty * a2;
         }
     }
 }
 
-// -------------------------------------------------- full-space displacement
-template <typename R>
-CAD_HD void ad_disp(const AngDisT<R>& v, R sgn, R x, R y, R z, R Dss, R Dds, R Dn, R K8, R U[3][3])
+// Adds the strain (EFCS) of frame f's slip modes into E.  A flat (z = 0) image
+// triangle keeps the reference's detached xz / yz components: there the
+// accumulated value is carried into the image TDCS, its xz and yz negated,
+// and those two returned as they stood in the TDCS (src/TD.jl:1518-1525,
+// :1610-1617).
+template <bool IMAGE, typename R>
+CAD_HD void add_strain(const FrameT<R>& f, bool nan, const R slip[3], R T[3][6], R E[3][6])
 {
-    const R CosT = sgn * v.cosT, SinT = sgn * v.sinT;
-    const R dy = y - v.tv1, dz = z - v.tv2;
-    const R Yr = CosT * dy - SinT * dz;
-    const R Zr = SinT * dy + CosT * dz;
-    R o[9];
-    ang_dis_disp(v.kd, x, Yr, Zr, o);
-    const R ux = o[0], uy = o[1], uz = o[2], vx = o[3], vy = o[4], vz = o[5], wx = o[6], wy = o[7], wz = o[8];
-    const R sinADE1 = v.sinADE1;
-    // back-rotation of (y, z) components: (c u + s w, -s u + c w)
-    if (Dn != 0.0) {
-        const R c = Dn * K8;
-        const R a = c * vx, b = c * wx;
-        U[0][0] += c * ux;
-        U[0][1] += CosT * a + SinT * b;
-        U[0][2] += -SinT * a + CosT * b;
+    const R Rot[9] = {f.Vn[0], f.Vn[1], f.Vn[2], f.Vs[0], f.Vs[1], f.Vs[2], f.Vd[0], f.Vd[1], f.Vd[2]};
+    if (IMAGE && f.flat != R(0)) {
+        const R RotInv[9] = {f.Vn[0], f.Vs[0], f.Vd[0], f.Vn[1], f.Vs[1], f.Vd[1], f.Vn[2], f.Vs[2], f.Vd[2]};
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            tensor_rot(E[m], RotInv);
+            const R kx = E[m][4], ky = E[m][5];
+            E[m][4] = -kx;
+            E[m][5] = -ky;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                if (slip[m] != R(0.0)) E[m][k] += slip[m] * T[m][k];
+                if (nan) E[m][k] = qnan<R>();
+            }
+            tensor_rot(E[m], Rot);
+            E[m][4] = kx;
+            E[m][5] = ky;
+        }
+        return;
     }
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const R slip = q == 0 ? Dss : Dds;
-        if (!(slip != 0.0)) continue;
-        const R Ds = q == 0 ? CosT * Dss : -SinT * Dds;
-        const R Dd = q == 0 ? SinT * Dss : CosT * Dds;
-        const R cs = Ds * K8, cd = Dd * sinADE1;
-        const R a = x * (cs * vy + cd * vz);
-        const R b = x * (cs * wy + cd * wz);
-        U[1 + q][0] += cs * uy + cd * uz;
-        U[1 + q][1] += CosT * a + SinT * b;
-        U[1 + q][2] += -SinT * a + CosT * b;
+    for (int m = 0; m < 3; ++m) {
+        tensor_rot(T[m], Rot);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            if (slip[m] != R(0.0)) E[m][k] += slip[m] * T[m][k];
+            if (nan) E[m][k] = qnan<R>();
+        }
     }
+}
+
+// The same for the displacement (flat image: the detached z component).
+template <bool IMAGE, typename R>
+CAD_HD void add_disp(const FrameT<R>& f, bool nan, const R slip[3], R T[3][3], R U[3][3])
+{
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+        R keep = R(0.0);
+        const bool flat = IMAGE && f.flat != R(0);
+        if (flat) {
+            const R a = U[m][0], b = U[m][1], c = U[m][2];
+            U[m][0] = f.Vn[0] * a + f.Vn[1] * b + f.Vn[2] * c;
+            U[m][1] = f.Vs[0] * a + f.Vs[1] * b + f.Vs[2] * c;
+            keep = f.Vd[0] * a + f.Vd[1] * b + f.Vd[2] * c;
+            U[m][2] = -keep;
+#pragma unroll
+            for (int c2 = 0; c2 < 3; ++c2)
+                if (slip[m] != R(0.0)) U[m][c2] += slip[m] * T[m][c2];
+            const R p = U[m][0], q = U[m][1], r = U[m][2];
+#pragma unroll
+            for (int c2 = 0; c2 < 3; ++c2) U[m][c2] = f.Vn[c2] * p + f.Vs[c2] * q + f.Vd[c2] * r;
+        } else if (slip[m] != R(0.0)) {
+#pragma unroll
+            for (int c2 = 0; c2 < 3; ++c2)
+                U[m][c2] += slip[m] * (f.Vn[c2] * T[m][0] + f.Vs[c2] * T[m][1] + f.Vd[c2] * T[m][2]);
+        }
+        if (nan) U[m][0] = U[m][1] = U[m][2] = qnan<R>();
+        if (flat) U[m][2] = keep;
+    }
+}
+
+template <bool IMAGE, bool STRAIN, bool DISP, typename R>
+CAD_HD void td_fs(const FrameT<R>& f, double X, double Y, double Z, R Dss, R Dds, R Dn, R K8, R E[3][6], R U[3][3])
+{
+    R x, y, z;
+    to_tdcs(f, X, Y, Z, x, y, z);
+    const bool nan = on_side(f, x, y, z);
+    const R slip[3] = {Dn, Dss, Dds};
+    R T[3][6], V[3][3];
+    td_unit<STRAIN, DISP>(f, x, y, z, K8, T, V);
+    if (STRAIN) add_strain<IMAGE>(f, nan, slip, T, E);
+    if (DISP) add_disp<IMAGE>(f, nan, slip, V, U);
+}
+
+template <bool IMAGE, typename R>
+CAD_HD void strain_fs(const FrameT<R>& f, double X, double Y, double Z, R Dss, R Dds, R Dn, R K8, R E[3][6])
+{
+    td_fs<IMAGE, true, false>(f, X, Y, Z, Dss, Dds, Dn, K8, E, (R(*)[3]) nullptr);
 }
 
 template <bool IMAGE, typename R>
 CAD_HD void disp_fs(const FrameT<R>& f, double X, double Y, double Z, R Dss, R Dds, R Dn, R K8, R U[3][3])
 {
-    R x, y, z;
-    to_tdcs(f, X, Y, Z, x, y, z);
-    const int mode = trimode(f, x, y, z);
-    const bool detach = IMAGE && f.flat != R(0);
-    R keep_z[3];
-    if (IMAGE) {
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-            const R a = U[m][0], b = U[m][1], c = U[m][2];
-            U[m][0] = f.Vn[0] * a + f.Vn[1] * b + f.Vn[2] * c;
-            U[m][1] = f.Vs[0] * a + f.Vs[1] * b + f.Vs[2] * c;
-            U[m][2] = f.Vd[0] * a + f.Vd[1] * b + f.Vd[2] * c;
-        }
-        if (detach) {
-#pragma unroll
-            for (int m = 0; m < 3; ++m) {
-                keep_z[m] = U[m][2];
-                U[m][2] = -U[m][2];
-            }
-        }
-    }
-    const R sgn = mode == -1 ? R(-1.0) : R(1.0);
-#pragma unroll 1
-    for (int a = 0; a < 3; ++a) ad_disp(f.v[a], sgn, x, y, z, Dss, Dds, Dn, K8, U);
-    if (mode == 0) {
-#pragma unroll
-        for (int m = 0; m < 3; ++m)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) U[m][c] = qnan<R>();
-    }
-    {   // Burgers' function (solid angle of the TD seen from the point)
-        const R a1 = -x, a2 = f.p1y - y, a3 = f.p1z - z;
-        const R b2 = -y, b3 = -z;
-        const R c2 = f.p3y - y, c3 = f.p3z - z;
-        const R a12 = a1 * a1;
-        const R na = cad_sqrt(a12 + a2 * a2 + a3 * a3);
-        const R nb = cad_sqrt(a12 + b2 * b2 + b3 * b3);
-        const R nc = cad_sqrt(a12 + c2 * c2 + c3 * c3);
-        const R one = a1 * (b2 * c3 - b3 * c2) - a2 * (a1 * c3 - b3 * a1) + a3 * (a1 * c2 - b2 * a1);
-        const R ab = a1 * a1 + a2 * b2 + a3 * b3;
-        const R ac = a1 * a1 + a2 * c2 + a3 * c3;
-        const R bc = a1 * a1 + b2 * c2 + b3 * c3;
-        const R two = na * nb * nc + ab * nc + ac * nb + bc * na;
-        const R Fi = R(-0.5) * R(M_1_PI) * cad_atan2(one, two);
-        U[0][0] += Dn * Fi;
-        U[1][1] += Dss * Fi;
-        U[2][2] += Dds * Fi;
-    }
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-        const R a = U[m][0], b = U[m][1], c = U[m][2];
-        U[m][0] = f.Vn[0] * a + f.Vs[0] * b + f.Vd[0] * c;
-        U[m][1] = f.Vn[1] * a + f.Vs[1] * b + f.Vd[1] * c;
-        U[m][2] = f.Vn[2] * a + f.Vs[2] * b + f.Vd[2] * c;
-    }
-    if (detach) {
-#pragma unroll
-        for (int m = 0; m < 3; ++m) U[m][2] = keep_z[m];
-    }
+    td_fs<IMAGE, false, true>(f, X, Y, Z, Dss, Dds, Dn, K8, (R(*)[6]) nullptr, U);
 }
 
 // --------------------------------------------------- free-surface correction
@@ -681,7 +698,7 @@ CAD_HD void cross3_rn(const double a[3], const double b[3], double c[3])
     c[2] = sub_rn(mul_rn(a[0], b[1]), mul_rn(a[1], b[0]));
 }
 
-CAD_HD void build_frame(const double P1[3], const double P2[3], const double P3[3], double nu, Frame& f)
+CAD_HD void build_frame(const double P1[3], const double P2[3], const double P3[3], Frame& f)
 {
     double a[3], b[3], Vn[3], Vs[3], Vd[3];
     for (int i = 0; i < 3; ++i) { a[i] = sub_rn(P2[i], P1[i]); b[i] = sub_rn(P3[i], P1[i]); }
@@ -718,11 +735,7 @@ CAD_HD void build_frame(const double P1[3], const double P2[3], const double P3[
     const double n13 = norm3_rn(e13[0], e13[1], e13[2]);
     const double n23 = norm3_rn(e23[0], e23[1], e23[2]);
     for (int i = 0; i < 3; ++i) { e12[i] /= n12; e13[i] /= n13; e23[i] /= n23; }
-    const double A = acos(dot3_rn(e12[0], e12[1], e12[2], e13[0], e13[1], e13[2]));
-    const double B = acos(dot3_rn(-e12[0], -e12[1], -e12[2], e23[0], e23[1], e23[2]));
-    const double C = acos(dot3_rn(e23[0], e23[1], e23[2], e13[0], e13[1], e13[2]));
-
-    // configuration test constants (trimodefinder on the TDCS (y, z) plane)
+    // on-a-side test constants (trimodefinder on the TDCS (y, z) plane)
     f.t23y = sub_rn(0.0, p3[2]);
     f.t32x = sub_rn(p3[1], 0.0);
     f.t13x = sub_rn(p1[1], p3[1]);
@@ -730,23 +743,10 @@ CAD_HD void build_frame(const double P1[3], const double P2[3], const double P3[
     f.t31y = sub_rn(p3[2], p1[2]);
     f.base = add_rn(mul_rn(f.t23y, f.t13x), mul_rn(f.t32x, t13y));
 
-    const double alpha[3] = {A, B, C};
-    const double side_y[3] = {-e13[1], e12[1], e23[1]};
-    const double side_z[3] = {-e13[2], e12[2], e23[2]};
-    const double tv1[3] = {p1[1], 0.0, p3[1]};
-    const double tv2[3] = {p1[2], 0.0, p3[2]};
+    const double* side[3] = {e12, e23, e13};
     for (int v = 0; v < 3; ++v) {
-        AngDis& d = f.v[v];
-        d.cosT = side_z[v];
-        d.sinT = side_y[v];
-        d.tv1 = tv1[v];
-        d.tv2 = tv2[v];
-        const double Ang = -M_PI + alpha[v];
-        const double cosA = cos(Ang), sinA = sin(Ang);
-        d.sinADE1 = sinA / 8.0 / M_PI / sub_rn(1.0, nu);
-        ang_dis_strain_setup(cosA, sinA, nu, add_rn(mul_rn(2.0, nu), 1.0), d.sinADE1, d.ks);
-        ang_dis_disp_setup(cosA, sinA, sub_rn(1.0, nu), sub_rn(1.0, mul_rn(2.0, nu)), mul_rn(cosA, cosA), d.sinADE1,
-                           d.kd);
+        f.sy[v] = v == 2 ? -side[v][1] : side[v][1];
+        f.sz[v] = v == 2 ? -side[v][2] : side[v][2];
     }
     f.flat = (P1[2] == 0.0 && P2[2] == 0.0 && P3[2] == 0.0) ? 1.0 : 0.0;
     for (int i = 0; i < 3; ++i) f.P2lo[i] = 0.0;
@@ -929,10 +929,10 @@ CAD_HD void build_triangle(const double a[3], const double b[3], const double c[
     t.Dds = Dds;
     t.Dn = Dn;
     t.K8 = 1.0 / (8.0 * M_PI * (1.0 - nu));
-    build_frame(a, b, c, nu, t.real);
+    build_frame(a, b, c, t.real);
     if (!hs) return;
     const double ai[3] = {a[0], a[1], -a[2]}, bi[3] = {b[0], b[1], -b[2]}, ci[3] = {c[0], c[1], -c[2]};
-    build_frame(ai, bi, ci, nu, t.image);
+    build_frame(ai, bi, ci, t.image);
     build_side(a, b, t.real, t.Dss, t.Dds, t.Dn, nu, t.side[0]);
     build_side(b, c, t.real, t.Dss, t.Dds, t.Dn, nu, t.side[1]);
     build_side(c, a, t.real, t.Dss, t.Dds, t.Dn, nu, t.side[2]);
