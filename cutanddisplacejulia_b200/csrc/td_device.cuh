@@ -11,7 +11,7 @@
 //                                  summed as three straight segments, see seg_integrals)
 //   free-surface correction        AngSetupStrainFSC :1867-2081, AngSetupDispFSC :1258-1409
 //   image dislocation              ComputeStrainInfluences :670-708, ComputeDispInfluences :631-668
-// The closed-form angular-dislocation terms come from tde_closed_form.cuh.
+// The free-surface rows come from fsc_rows.cuh (generated by gen/gen_fsc.py).
 //
 // Data layout: everything that depends only on the triangle (frames, angles,
 // per-dislocation constants of every closed-form term, slip rotations) is
@@ -23,7 +23,47 @@
 #include <cstddef>
 #include <cstdint>
 
-#include "tde_closed_form.cuh"
+#include <math.h>
+#ifdef __CUDACC__
+#include <cuda_runtime.h>
+#define CAD_HD __host__ __device__ __forceinline__
+#else
+#define CAD_HD inline
+#endif
+
+namespace cad {
+
+#ifndef __CUDACC__
+// plain C++ build of the device code (used only to test it on a CPU)
+inline double rsqrt(double x) { return 1.0 / sqrt(x); }
+inline float rsqrtf(float x) { return 1.0f / sqrtf(x); }
+#endif
+
+// math functions in the pair bodies' arithmetic type
+CAD_HD double cad_rsqrt(double x) { return rsqrt(x); }
+CAD_HD float cad_rsqrt(float x) { return rsqrtf(x); }
+CAD_HD double cad_log(double x) { return log(x); }
+CAD_HD float cad_log(float x) { return logf(x); }
+
+// Accumulators of the free-surface correction, end B minus end A (fsc_end and
+// fsc_disp_end fill them; fsc_rows.cuh combines them).
+template <typename R>
+struct FscAcc {
+    R h0, h1r, h1i, Mr, Mi, Sr, Si, Yr, Yi;   // powers of zeta over r
+    R g1r, g1i, Or, Oi, w2r, w2i, Nr, Ni;     // powers of eta over r
+    R t1, t2, tq, At1, At2, Atq;              // (y1, y2, q) / r^3, and times the end's depth a
+    R s11, s12, s1q, s22, s2q;                // a x second derivatives of 1 / r
+};
+template <typename R>
+struct FscDispAcc {
+    R F, phi, chi, Br, Bi, B3r, B3i, B4r, B4i;
+    R O1r, O1i, O2r, O2i, zg1r, zg1i;
+    R ah0, zh0, azt1, azt2, aztq;
+};
+
+}  // namespace cad
+
+#include "fsc_rows.cuh"
 
 namespace cad {
 
@@ -45,15 +85,18 @@ struct FrameT {          // a TD (real or image) in its own coordinate system
 template <typename T>
 struct FscSideT {        // one TD side PA -> PB of the free-surface correction
     T skip;              // 1: the side adds nothing (beta test)
-    T ey1[3], ey2[3], ey3[3];
+    T ea, eb;            // horizontal direction of the side: ADCS y1 = ea X + eb Y, y2 = eb X - ea Y, y3 = -Z
     T PA[3];
     T PAlo[3];           // as P2lo
-    T y1B, y2B, y3B;
-    T beta;
-    T cs[3][3];          // ADCS slip of each unit mode m (Dn, Dss, Dds), component g
-    T cd[3][3];          // the same scaled by 1 / (4 pi (1 - nu)) for displacements
-    ang_dis_strain_fsc_k<T> ks[2][2];   // [0: beta, 1: pi - beta][0: at PA, 1: at PB]
-    ang_dis_disp_fsc_k<T> kd[2][2];     // [0: beta, 1: beta - pi][0: at PA, 1: at PB]
+    T y1B, y2B;          // PB in ADCS
+    T aA, aB;            // depths of the ends
+    T s, c, nu;          // sine and cosine of the inclination beta, Poisson's ratio
+    T cM, B1;            // -(1 - 2 nu) cot(beta) / 2, (1 - 2 nu) cot(beta)
+    T ct2, tn2;          // cot and tan of beta / 2
+    T K4;                // 1 / (4 pi (1 - nu))
+    T cs[3][3];          // ADCS slip of each unit mode m (Dn, Dss, Dds), component g, times K4
+    FscRows<T> ks;
+    FscDispRows<T> kd;
 };
 
 template <typename T>
@@ -466,95 +509,131 @@ CAD_HD void disp_fs(const FrameT<R>& f, double X, double Y, double Z, R Dss, R D
 }
 
 // --------------------------------------------------- free-surface correction
-// Observation point -> ADCS of a side, relative to PA.
+// Observation point -> horizontal ADCS coordinates of a side, relative to PA,
+// and its depth.
 template <typename R>
-CAD_HD void to_adcs(const FscSideT<R>& s, double X, double Y, double Z, R& x, R& y, R& z)
+CAD_HD void to_adcs(const FscSideT<R>& s, double X, double Y, double Z, R& y1, R& y2, R& z)
 {
     R dX, dY, dZ;
     rel_origin(s.PA, s.PAlo, X, Y, Z, dX, dY, dZ);
-    x = add_rn(add_rn(mul_rn(s.ey1[0], dX), mul_rn(s.ey2[0], dY)), mul_rn(s.ey3[0], dZ));
-    y = add_rn(add_rn(mul_rn(s.ey1[1], dX), mul_rn(s.ey2[1], dY)), mul_rn(s.ey3[1], dZ));
-    z = add_rn(add_rn(mul_rn(s.ey1[2], dX), mul_rn(s.ey2[2], dY)), mul_rn(s.ey3[2], dZ));
+    y1 = s.ea * dX + s.eb * dY;
+    y2 = s.eb * dX - s.ea * dY;
+    z = (R)(-Z);
 }
 
-// The FP64 free-surface strain groups are called out of line: each then gets
-// the whole register file, which spills far less than one inlined body (the
-// FP32 groups fit inline).
-#ifdef __CUDACC__
-#define CAD_OUTLINE static __host__ __device__ __noinline__
-#else
-#define CAD_OUTLINE static inline
-#endif
-CAD_OUTLINE void fsc_strain_g0_f64(const ang_dis_strain_fsc_k<double>& k, double y1, double y2, double y3, double* v)
+// Adds sg x the values of one end of a side (depth a, point at (y1, y2) from
+// it and at depth z) to the accumulators.  f = +-1 takes the inclined leg's
+// functions along +z3 or -z3 (both ends alike); w = r + f z3 is rho^2 / (r - f
+// z3) where f z3 < 0, so it never cancels.
+template <bool FIRST, typename R>
+CAD_HD void fsc_end(const FscSideT<R>& k, R y1, R y2, R a, R z, R f, R z1, R z3, FscAcc<R>& v)
 {
-    ang_dis_strain_fsc_g0(k, y1, y2, y3, v);
-}
-CAD_OUTLINE void fsc_strain_g1_f64(const ang_dis_strain_fsc_k<double>& k, double y1, double y2, double y3, double* v)
-{
-    ang_dis_strain_fsc_g1(k, y1, y2, y3, v);
-}
-CAD_OUTLINE void fsc_strain_g2_f64(const ang_dis_strain_fsc_k<double>& k, double y1, double y2, double y3, double* v)
-{
-    ang_dis_strain_fsc_g2(k, y1, y2, y3, v);
+    const R sg = FIRST ? R(-1.0) : R(1.0);
+    const R q = z + a;
+    const R r2 = y1 * y1 + y2 * y2 + q * q;
+    const R ir = cad_rsqrt(r2), r = r2 * ir, ir2 = ir * ir, ir3 = ir2 * ir;
+    const R zf = f * z3, p = r + q;
+    const bool out = zf >= R(0.0);
+    const R den = out ? r + zf : z1 * z1 + y2 * y2, num = out ? R(1.0) : r - zf;
+    const R inv = R(1.0) / (p * den);
+    const R ip = inv * den, iw = inv * p * num;
+    const R N1 = R(1.0) - R(2.0) * k.nu, hN = R(0.5) * N1;
+    const R c1r = y1 * ip, c1i = y2 * ip;                                    // zeta
+    const R c2r = c1r * c1r - c1i * c1i, c2i = R(2.0) * c1r * c1i;
+    const R c3r = c2r * c1r - c2i * c1i, c3i = c2r * c1i + c2i * c1r;
+    const R n1r = z1 * iw, n1i = y2 * iw;                                    // f eta
+    const R n2r = n1r * n1r - n1i * n1i, n2i = R(2.0) * n1r * n1i;
+    const R n3r = n2r * n1r - n2i * n1i, n3i = n2r * n1i + n2i * n1r;
+    const R kq = q * ir, kz = zf * ir, az = a * z;
+    const R d2 = -(R(2.0) + kq) * ir2, d3 = -(R(3.0) + kq) * ir2;            // D h_m / zeta^m
+    const R dd3 = (R(8.0) + kq * (R(9.0) + R(3.0) * kq)) * ir3;              // D^2 h_3 / zeta^3
+    const R e2 = -(R(2.0) + kz) * ir2, e3 = (R(3.0) + kz) * ir2;
+    const R ee3 = (R(8.0) + kz * (R(9.0) + R(3.0) * kz)) * ir3;
+    const R m2 = sg * k.cM * (N1 * ir + (a + z) * d2);
+    const R m3 = sg * (hN * k.nu * ir + R(0.5) * (k.nu * z - hN * a) * d3 - R(0.25) * az * dd3);
+    const R ms = sg * (R(0.5) * (N1 * a - z) * d2 - hN * ir);
+    const R my = sg * k.nu * z * d2;
+    const R sir = sg * ir, sf = sg * f;
+    v.h0 = (FIRST ? R(0.0) : v.h0) + sir;
+    v.h1r = (FIRST ? R(0.0) : v.h1r) + sir * c1r;
+    v.h1i = (FIRST ? R(0.0) : v.h1i) + sir * c1i;
+    v.Mr = (FIRST ? R(0.0) : v.Mr) + m2 * c2r + m3 * c3r;
+    v.Mi = (FIRST ? R(0.0) : v.Mi) + m2 * c2i + m3 * c3i;
+    v.Sr = (FIRST ? R(0.0) : v.Sr) + ms * c2r;
+    v.Si = (FIRST ? R(0.0) : v.Si) + ms * c2i;
+    v.Yr = (FIRST ? R(0.0) : v.Yr) + my * c2r;
+    v.Yi = (FIRST ? R(0.0) : v.Yi) + my * c2i;
+    const R g1 = sf * ir, w2 = sf * e2;
+    const R o2 = a * w2 - sg * k.c * ir, n3 = sg * R(0.25) * z * (f * a * ee3 + k.c * e3);
+    v.g1r = (FIRST ? R(0.0) : v.g1r) + g1 * n1r;
+    v.g1i = (FIRST ? R(0.0) : v.g1i) + g1 * n1i;
+    v.Or = (FIRST ? R(0.0) : v.Or) + o2 * n2r;
+    v.Oi = (FIRST ? R(0.0) : v.Oi) + o2 * n2i;
+    v.w2r = (FIRST ? R(0.0) : v.w2r) + w2 * n2r;
+    v.w2i = (FIRST ? R(0.0) : v.w2i) + w2 * n2i;
+    v.Nr = (FIRST ? R(0.0) : v.Nr) + n3 * n3r;
+    v.Ni = (FIRST ? R(0.0) : v.Ni) + n3 * n3i;
+    const R s3 = sg * ir3, u1 = y1 * s3, u2 = y2 * s3, uq = q * s3, a3 = R(3.0) * a * ir2;
+    v.t1 = (FIRST ? R(0.0) : v.t1) + u1;
+    v.t2 = (FIRST ? R(0.0) : v.t2) + u2;
+    v.tq = (FIRST ? R(0.0) : v.tq) + uq;
+    v.At1 = (FIRST ? R(0.0) : v.At1) + a * u1;
+    v.At2 = (FIRST ? R(0.0) : v.At2) + a * u2;
+    v.Atq = (FIRST ? R(0.0) : v.Atq) + a * uq;
+    v.s11 = (FIRST ? R(0.0) : v.s11) + (a3 * y1 * u1 - a * s3);
+    v.s12 = (FIRST ? R(0.0) : v.s12) + a3 * y1 * u2;
+    v.s1q = (FIRST ? R(0.0) : v.s1q) + a3 * y1 * uq;
+    v.s22 = (FIRST ? R(0.0) : v.s22) + (a3 * y2 * u2 - a * s3);
+    v.s2q = (FIRST ? R(0.0) : v.s2q) + a3 * y2 * uq;
 }
 
+// Strain of a side's correction in ADCS for a unit ADCS slip along each axis
+// (without K4).  The functions of the two ends are differenced before any
+// coefficient multiplies them: far from the side the ends nearly cancel.
 template <typename R>
-CAD_HD void fsc_strain_eval(const ang_dis_strain_fsc_k<R>& k, R y1, R y2, R y3, R v[18])
+CAD_HD void fsc_strain_adcs(const FscSideT<R>& s, double X, double Y, double Z, R e[3][6])
 {
-    if constexpr (sizeof(R) == sizeof(double)) {
-        fsc_strain_g0_f64(k, y1, y2, y3, v);
-        fsc_strain_g1_f64(k, y1, y2, y3, v + 6);
-        fsc_strain_g2_f64(k, y1, y2, y3, v + 12);
-    } else {
-        ang_dis_strain_fsc_g0(k, y1, y2, y3, v);
-        ang_dis_strain_fsc_g1(k, y1, y2, y3, v + 6);
-        ang_dis_strain_fsc_g2(k, y1, y2, y3, v + 12);
-    }
+    R y1, y2, z;
+    to_adcs(s, X, Y, Z, y1, y2, z);
+    const R qA = z + s.aA, qB = z + s.aB;
+    const R y1b = y1 - s.y1B, y2b = y2 - s.y2B;
+    const R z3A = s.c * qA - s.s * y1, z3B = s.c * qB - s.s * y1b;
+    const R f = z3A + z3B >= R(0.0) ? R(1.0) : R(-1.0);
+    FscAcc<R> v;
+    fsc_end<true>(s, y1, y2, s.aA, z, f, s.c * y1 + s.s * qA, z3A, v);
+    fsc_end<false>(s, y1b, y2b, s.aB, z, f, s.c * y1b + s.s * qB, z3B, v);
+    fsc_rows(s.ks, v, z, e);
+}
+
+// Tensor in ADCS -> EFCS (a rotation about the vertical axis).
+template <typename R>
+CAD_HD void adcs_to_efcs(R t[6], R a, R b)
+{
+    const R aa = a * a, bb = b * b, ab = a * b;
+    const R t11 = t[0], t22 = t[1], t12 = t[3], t13 = t[4], t23 = t[5];
+    t[0] = aa * t11 + bb * t22 + R(2.0) * ab * t12;
+    t[1] = bb * t11 + aa * t22 - R(2.0) * ab * t12;
+    t[3] = ab * (t11 - t22) + (bb - aa) * t12;
+    t[4] = -(a * t13 + b * t23);
+    t[5] = a * t23 - b * t13;
 }
 
 // One side's harmonic correction to the strain, added into E (EFCS).
 template <typename R>
 CAD_HD void fsc_strain(const FscSideT<R>& s, double X, double Y, double Z, R Dss, R Dds, R Dn, R E[3][6])
 {
-    R x, y, z;
-    to_adcs(s, X, Y, Z, x, y, z);
-    const bool flip = mul_rn(s.beta, x) >= 0.0;
-    const int c = flip ? 1 : 0;
-    const R f = flip ? R(-1.0) : R(1.0);
-    // d = (term at PB) - (term at PA), formed before any slip product: far
-    // from the side the two terms nearly cancel, and differencing them first
-    // keeps the products from rounding the two halves differently.
-    R d[18];
-    fsc_strain_eval(s.ks[c][0], f * x, f * y, z, d);
-#pragma unroll
-    for (int q = 0; q < 18; ++q) d[q] = -d[q];
-    {
-        R v[18];
-        fsc_strain_eval(s.ks[c][1], f * (x - s.y1B), f * (y - s.y2B), z - s.y3B, v);
-#pragma unroll
-        for (int q = 0; q < 18; ++q) d[q] += v[q];
-    }
-    R T[3][6];
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-        // configuration flip negates the first two ADCS slip components and
-        // the 13 / 23 strain components
-        const R c0 = f * s.cs[m][0], c1 = f * s.cs[m][1], c2 = s.cs[m][2];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            const R fk = (k >= 4) ? f : R(1.0);
-            const R h = (k >= 3) ? R(0.5) : R(1.0);
-            T[m][k] = h * fk * (c0 * d[k] + c1 * d[6 + k] + c2 * d[12 + k]);
-        }
-    }
-    const R AFlip[9] = {s.ey1[0], s.ey1[1], s.ey1[2], s.ey2[0], s.ey2[1], s.ey2[2], s.ey3[0], s.ey3[1], s.ey3[2]};
+    R e[3][6];
+    fsc_strain_adcs(s, X, Y, Z, e);
     const R slip[3] = {Dn, Dss, Dds};
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
         if (!(slip[m] != 0.0)) continue;
-        tensor_rot(T[m], AFlip);
+        R T[6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) E[m][k] += T[m][k];
+        for (int k = 0; k < 6; ++k) T[k] = s.cs[m][0] * e[0][k] + s.cs[m][1] * e[1][k] + s.cs[m][2] * e[2][k];
+        adcs_to_efcs(T, s.ea, s.eb);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) E[m][k] += T[k];
     }
 }
 
@@ -566,35 +645,17 @@ CAD_HD void fsc_strain(const FscSideT<R>& s, double X, double Y, double Z, R Dss
 template <typename R>
 CAD_HD void fsc_strain_map(const FscSideT<R>& s, double X, double Y, double Z, R G[3][6])
 {
-    R x, y, z;
-    to_adcs(s, X, Y, Z, x, y, z);
-    const bool flip = mul_rn(s.beta, x) >= 0.0;
-    const int c = flip ? 1 : 0;
-    const R f = flip ? R(-1.0) : R(1.0);
-    R d[18];
-    fsc_strain_eval(s.ks[c][0], f * x, f * y, z, d);
+    R e[3][6];
+    fsc_strain_adcs(s, X, Y, Z, e);
+    const R ca = s.K4 * s.ea, cb = s.K4 * s.eb;
 #pragma unroll
-    for (int q = 0; q < 18; ++q) d[q] = -d[q];
-    {
-        R v[18];
-        fsc_strain_eval(s.ks[c][1], f * (x - s.y1B), f * (y - s.y2B), z - s.y3B, v);
-#pragma unroll
-        for (int q = 0; q < 18; ++q) d[q] += v[q];
+    for (int k = 0; k < 6; ++k) {
+        G[0][k] = ca * e[0][k] + cb * e[1][k];
+        G[1][k] = cb * e[0][k] - ca * e[1][k];
+        G[2][k] = -s.K4 * e[2][k];
     }
-    const R AFlip[9] = {s.ey1[0], s.ey1[1], s.ey1[2], s.ey2[0], s.ey2[1], s.ey2[2], s.ey3[0], s.ey3[1], s.ey3[2]};
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        // ADCS slip components of a unit Burgers vector along EFCS axis j (as
-        // build_side forms them: the j-th frame vector ey(j+1))
-        const R c0 = f * AFlip[3 * j], c1 = f * AFlip[3 * j + 1], c2 = AFlip[3 * j + 2];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            const R fk = (k >= 4) ? f : R(1.0);
-            const R h = (k >= 3) ? R(0.5) : R(1.0);
-            G[j][k] = h * fk * (c0 * d[k] + c1 * d[6 + k] + c2 * d[12 + k]);
-        }
-        tensor_rot(G[j], AFlip);
-    }
+    for (int j = 0; j < 3; ++j) adcs_to_efcs(G[j], s.ea, s.eb);
 }
 
 // E[m] += sign * (the map G applied to the EFCS Burgers vector of unit mode m
@@ -613,56 +674,111 @@ CAD_HD void fsc_apply_map(const R G[3][6], R sign, const FrameT<R>& real, R Dss,
     }
 }
 
+// Adds sg x one end's values to the displacement accumulators; returns r + q
+// and r + f z3 (for the logarithms) and the numerator and denominator of the
+// Burgers function's tangent.
+template <bool FIRST, typename R>
+CAD_HD void fsc_disp_end(const FscSideT<R>& k, R y1, R y2, R a, R z, R f, FscDispAcc<R>& v, R& p, R& w, R& fn, R& fd)
+{
+    const R sg = FIRST ? R(-1.0) : R(1.0);
+    const R q = z + a;
+    const R r2 = y1 * y1 + y2 * y2 + q * q;
+    const R ir = cad_rsqrt(r2), r = r2 * ir, ir2 = ir * ir, ir3 = ir2 * ir;
+    const R z1 = k.c * y1 + k.s * q, zf = f * (k.c * q - k.s * y1);
+    p = r + q;
+    w = r + zf;
+    fn = f * y2;
+    fd = f > R(0.0) ? p * k.ct2 - y1 : y1 + p * k.tn2;
+    const R inv = R(1.0) / (p * w);
+    const R ip = inv * w, iw = inv * p;
+    const R N1 = R(1.0) - R(2.0) * k.nu, N2 = R(2.0) * (R(1.0) - k.nu);
+    const R c1r = y1 * ip, c1i = y2 * ip;
+    const R c2r = c1r * c1r - c1i * c1i, c2i = R(2.0) * c1r * c1i;
+    const R n1r = z1 * iw, n1i = y2 * iw;
+    const R n2r = n1r * n1r - n1i * n1i, n2i = R(2.0) * n1r * n1i;
+    const R az = a * z, sir = sg * ir;
+    const R b1 = sg * k.B1 * (N1 - (a + z) * ir);
+    const R b2 = sg * (R(0.5) * (az * (R(2.0) + q * ir) * ir2 - N1 * (k.nu + a * ir)) + k.nu * z * ir);
+    const R b3 = sg * (N1 + (N1 * a - z) * ir);
+    const R b4 = sg * (R(2.0) * N2 * k.nu + (N2 * a + R(2.0) * k.nu * z) * ir);
+    v.Br = (FIRST ? R(0.0) : v.Br) + b1 * c1r + b2 * c2r;
+    v.Bi = (FIRST ? R(0.0) : v.Bi) + b1 * c1i + b2 * c2i;
+    v.B3r = (FIRST ? R(0.0) : v.B3r) + b3 * c1r;
+    v.B3i = (FIRST ? R(0.0) : v.B3i) + b3 * c1i;
+    v.B4r = (FIRST ? R(0.0) : v.B4r) + b4 * c1r;
+    v.B4i = (FIRST ? R(0.0) : v.B4i) + b4 * c1i;
+    const R g1 = f * sir, o1 = sg * k.c + a * g1, o2 = -z * (a * f * sg * (R(2.0) + zf * ir) * ir2 + k.c * sir), zg = z * g1;
+    v.O1r = (FIRST ? R(0.0) : v.O1r) + o1 * n1r;
+    v.O1i = (FIRST ? R(0.0) : v.O1i) + o1 * n1i;
+    v.O2r = (FIRST ? R(0.0) : v.O2r) + o2 * n2r;
+    v.O2i = (FIRST ? R(0.0) : v.O2i) + o2 * n2i;
+    v.zg1r = (FIRST ? R(0.0) : v.zg1r) + zg * n1r;
+    v.zg1i = (FIRST ? R(0.0) : v.zg1i) + zg * n1i;
+    const R t = sg * az * ir3;
+    v.ah0 = (FIRST ? R(0.0) : v.ah0) + a * sir;
+    v.zh0 = (FIRST ? R(0.0) : v.zh0) + z * sir;
+    v.azt1 = (FIRST ? R(0.0) : v.azt1) + t * y1;
+    v.azt2 = (FIRST ? R(0.0) : v.azt2) + t * y2;
+    v.aztq = (FIRST ? R(0.0) : v.aztq) + t * q;
+}
+
+// Displacement of a side's correction in ADCS, d[3 component + slip], for a
+// unit ADCS slip along each axis (without K4).  f follows the side of the
+// vertical plane through PA the point lies on, as the reference's choice
+// between beta and beta - pi does: the Burgers function then stays on one
+// branch at both ends, and their difference is one arctangent.
+template <typename R>
+CAD_HD void fsc_disp_adcs(const FscSideT<R>& s, double X, double Y, double Z, R d[9])
+{
+    R y1, y2, z;
+    to_adcs(s, X, Y, Z, y1, y2, z);
+    const R f = y1 >= R(0.0) ? R(-1.0) : R(1.0);
+    FscDispAcc<R> v;
+    R pA, wA, nA, dA, pB, wB, nB, dB;
+    fsc_disp_end<true>(s, y1, y2, s.aA, z, f, v, pA, wA, nA, dA);
+    fsc_disp_end<false>(s, y1 - s.y1B, y2 - s.y2B, s.aB, z, f, v, pB, wB, nB, dB);
+    v.phi = cad_log(pB / pA);
+    v.chi = f * cad_log(wB / wA);
+    v.F = R(2.0) * cad_atan2(nB * dA - nA * dB, dA * dB + nA * nB);
+    fsc_disp_rows(s.kd, v, d);
+}
+
 // One side's harmonic correction to the displacement, added into U (EFCS).
 template <typename R>
 CAD_HD void fsc_disp(const FscSideT<R>& s, double X, double Y, double Z, R Dss, R Dds, R Dn, R U[3][3])
 {
-    R x, y, z;
-    to_adcs(s, X, Y, Z, x, y, z);
-    const int c = mul_rn(s.beta, x) >= 0.0 ? 1 : 0;
-    R uA[9], uB[9];
-    ang_dis_disp_fsc(s.kd[c][0], x, y, z, uA);
-    ang_dis_disp_fsc(s.kd[c][1], x - s.y1B, y - s.y2B, z - s.y3B, uB);
+    R d[9];
+    fsc_disp_adcs(s, X, Y, Z, d);
     const R slip[3] = {Dn, Dss, Dds};
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
         if (!(slip[m] != 0.0)) continue;
         R u[3];
 #pragma unroll
-        for (int d = 0; d < 3; ++d)
-            u[d] = s.cd[m][0] * (uB[3 * d] - uA[3 * d]) + s.cd[m][1] * (uB[3 * d + 1] - uA[3 * d + 1]) +
-                   s.cd[m][2] * (uB[3 * d + 2] - uA[3 * d + 2]);
-        // ADCS -> EFCS: rows (ey1, ey2, ey3) as in the reference's VxR, VyR, VzR
-        U[m][0] += s.ey1[0] * u[0] + s.ey1[1] * u[1] + s.ey1[2] * u[2];
-        U[m][1] += s.ey2[0] * u[0] + s.ey2[1] * u[1] + s.ey2[2] * u[2];
-        U[m][2] += s.ey3[0] * u[0] + s.ey3[1] * u[1] + s.ey3[2] * u[2];
+        for (int i = 0; i < 3; ++i) u[i] = s.cs[m][0] * d[3 * i] + s.cs[m][1] * d[3 * i + 1] + s.cs[m][2] * d[3 * i + 2];
+        U[m][0] += s.ea * u[0] + s.eb * u[1];
+        U[m][1] += s.eb * u[0] - s.ea * u[1];
+        U[m][2] -= u[2];
     }
 }
 
 // The free-surface displacement of side s at (X, Y, Z) for a unit Burgers
-// vector along EFCS axis j, without the factor 1 / (4 pi (1 - nu)):
-// Gu[j][c] = sum_d ey_c[d] sum_g ey_j[g] (uB - uA)[3 d + g] (fsc_disp with
-// cs = ey_j).  As for the strain map, the reversed side's map is the
-// negative of this one.
+// vector along EFCS axis j, without the factor 1 / (4 pi (1 - nu)).  As for
+// the strain map, the reversed side's map is the negative of this one.
 template <typename R>
 CAD_HD void fsc_disp_map(const FscSideT<R>& s, double X, double Y, double Z, R Gu[3][3])
 {
-    R x, y, z;
-    to_adcs(s, X, Y, Z, x, y, z);
-    const int c = mul_rn(s.beta, x) >= 0.0 ? 1 : 0;
-    R uA[9], uB[9];
-    ang_dis_disp_fsc(s.kd[c][0], x, y, z, uA);
-    ang_dis_disp_fsc(s.kd[c][1], x - s.y1B, y - s.y2B, z - s.y3B, uB);
-    const R* ey[3] = {s.ey1, s.ey2, s.ey3};
+    R d[9];
+    fsc_disp_adcs(s, X, Y, Z, d);
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
         R u[3];
 #pragma unroll
-        for (int d = 0; d < 3; ++d)
-            u[d] = ey[j][0] * (uB[3 * d] - uA[3 * d]) + ey[j][1] * (uB[3 * d + 1] - uA[3 * d + 1]) +
-                   ey[j][2] * (uB[3 * d + 2] - uA[3 * d + 2]);
-#pragma unroll
-        for (int cc = 0; cc < 3; ++cc) Gu[j][cc] = ey[cc][0] * u[0] + ey[cc][1] * u[1] + ey[cc][2] * u[2];
+        for (int i = 0; i < 3; ++i)
+            u[i] = j == 0 ? s.ea * d[3 * i] + s.eb * d[3 * i + 1] : j == 1 ? s.eb * d[3 * i] - s.ea * d[3 * i + 1] : -d[3 * i + 2];
+        Gu[j][0] = s.ea * u[0] + s.eb * u[1];
+        Gu[j][1] = s.eb * u[0] - s.ea * u[1];
+        Gu[j][2] = -u[2];
     }
 }
 
@@ -752,38 +868,48 @@ CAD_HD void build_frame(const double P1[3], const double P2[3], const double P3[
     for (int i = 0; i < 3; ++i) f.P2lo[i] = 0.0;
 }
 
-// The geometry of side PA -> PB (frame, beta test, closed-form constants);
-// its slip coefficients cs, cd are left zero.
+// The geometry of side PA -> PB (frame, beta test, row coefficients); its
+// slip coefficients cs are left zero.
 CAD_HD void build_side_geom(const double PA[3], const double PB[3], double nu, FscSide& s)
 {
     for (int m = 0; m < 3; ++m)
-        for (int g = 0; g < 3; ++g) s.cs[m][g] = s.cd[m][g] = 0.0;
+        for (int g = 0; g < 3; ++g) s.cs[m][g] = 0.0;
     const double S[3] = {sub_rn(PB[0], PA[0]), sub_rn(PB[1], PA[1]), sub_rn(PB[2], PA[2])};
     const double Sv = norm3_rn(S[0], S[1], S[2]);
     const double beta = acos(-S[2] / Sv);
-    s.beta = beta;
     s.skip = ((fabs(beta) < DBL_EPSILON) || (fabs(M_PI - beta) < DBL_EPSILON) || (fabs(1.0 / tan(beta)) > 5e3)) ? 1.0 : 0.0;
     for (int i = 0; i < 3; ++i) { s.PA[i] = PA[i]; s.PAlo[i] = 0.0; }
     if (s.skip != 0.0) return;
     const double n1 = norm3_rn(S[0], S[1], 0.0);
-    const double e1[3] = {S[0] / n1, S[1] / n1, 0.0 / n1};
-    const double e3[3] = {-0.0, -0.0, -1.0};
-    double e2[3];
-    cross3_rn(e3, e1, e2);
-    for (int i = 0; i < 3; ++i) { s.ey1[i] = e1[i]; s.ey2[i] = e2[i]; s.ey3[i] = e3[i]; }
-    s.y1B = add_rn(add_rn(mul_rn(e1[0], S[0]), mul_rn(e2[0], S[1])), mul_rn(e3[0], S[2]));
-    s.y2B = add_rn(add_rn(mul_rn(e1[1], S[0]), mul_rn(e2[1], S[1])), mul_rn(e3[1], S[2]));
-    s.y3B = add_rn(add_rn(mul_rn(e1[2], S[0]), mul_rn(e2[2], S[1])), mul_rn(e3[2], S[2]));
-    const double a_end[2] = {-PA[2], -PB[2]};
-    const double pibs = M_PI - beta, pibd = -M_PI + beta;
-    for (int e = 0; e < 2; ++e) {
-        ang_dis_strain_fsc_setup(cos(beta), sin(beta), 1.0 / tan(beta), nu, a_end[e], s.ks[0][e]);
-        ang_dis_strain_fsc_setup(cos(pibs), sin(pibs), 1.0 / tan(pibs), nu, a_end[e], s.ks[1][e]);
-        ang_dis_disp_fsc_setup(cos(beta), sin(beta), 1.0 / tan(beta), 1.0 / tan(beta / 2.0), nu, a_end[e],
-                               s.kd[0][e]);
-        ang_dis_disp_fsc_setup(cos(pibd), sin(pibd), 1.0 / tan(pibd), 1.0 / tan(pibd / 2.0), nu, a_end[e],
-                               s.kd[1][e]);
+    s.ea = S[0] / n1;
+    s.eb = S[1] / n1;
+    s.y1B = add_rn(mul_rn(s.ea, S[0]), mul_rn(s.eb, S[1]));
+    s.y2B = sub_rn(mul_rn(s.eb, S[0]), mul_rn(s.ea, S[1]));
+    s.aA = -PA[2];
+    s.aB = -PB[2];
+    s.s = n1 / Sv;
+    s.c = -S[2] / Sv;
+    s.nu = nu;
+    const double N1 = sub_rn(1.0, mul_rn(2.0, nu));
+    s.B1 = N1 * s.c / s.s;
+    s.cM = -0.5 * s.B1;
+    s.ct2 = (1.0 + s.c) / s.s;   // cot(beta / 2)
+    s.tn2 = s.s / (1.0 + s.c);
+    if (s.c < 0.0) {
+        s.ct2 = s.s / (1.0 - s.c);
+        s.tn2 = (1.0 - s.c) / s.s;
     }
+    s.K4 = 1.0 / (4.0 * M_PI * sub_rn(1.0, nu));
+    fsc_rows_setup(s.s, s.c, nu, s.ks);
+    fsc_rows_setup(s.s, s.c, nu, s.kd);
+}
+
+// EFCS Burgers vector w -> the side's ADCS slip coefficients (times K4).
+CAD_HD void side_slip(const FscSide& s, const double w[3], double cs[3])
+{
+    cs[0] = mul_rn(s.K4, add_rn(mul_rn(s.ea, w[0]), mul_rn(s.eb, w[1])));
+    cs[1] = mul_rn(s.K4, sub_rn(mul_rn(s.eb, w[0]), mul_rn(s.ea, w[1])));
+    cs[2] = -mul_rn(s.K4, w[2]);
 }
 
 CAD_HD void build_side(const double PA[3], const double PB[3], const Frame& real, double Dss, double Dds,
@@ -797,10 +923,7 @@ CAD_HD void build_side(const double PA[3], const double PB[3], const Frame& real
     for (int m = 0; m < 3; ++m) {
         double w[3];
         for (int i = 0; i < 3; ++i) w[i] = mul_rn(axes[m][i], slip[m]);
-        for (int g = 0; g < 3; ++g) {
-            s.cs[m][g] = add_rn(add_rn(mul_rn(s.ey1[g], w[0]), mul_rn(s.ey2[g], w[1])), mul_rn(s.ey3[g], w[2]));
-            s.cd[m][g] = s.cs[m][g] / 4.0 / M_PI / sub_rn(1.0, nu);
-        }
+        side_slip(s, w, s.cs[m]);
     }
 }
 
@@ -811,10 +934,7 @@ CAD_HD void build_side_burgers(const double PA[3], const double PB[3], const dou
 {
     build_side_geom(PA, PB, nu, s);
     if (s.skip != 0.0) return;
-    for (int g = 0; g < 3; ++g) {
-        s.cs[0][g] = add_rn(add_rn(mul_rn(s.ey1[g], B[0]), mul_rn(s.ey2[g], B[1])), mul_rn(s.ey3[g], B[2]));
-        s.cd[0][g] = s.cs[0][g] / 4.0 / M_PI / sub_rn(1.0, nu);
-    }
+    side_slip(s, B, s.cs[0]);
 }
 
 // ------------------------------------------------------------ pair drivers
