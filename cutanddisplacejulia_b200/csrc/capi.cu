@@ -15,10 +15,10 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
-#include <unordered_map>
 #include <vector>
 
 #include "../../include/cad_td.h"
+#include "edges.h"
 #include "gemm.h"
 #include "krylov.h"
 #include "lcp.h"
@@ -43,7 +43,7 @@ enum Slot {
     S_A32, S_DINV, S_KRYLOV, S_VEC32, S_SYNC, S_TRI32, S_NEAR, S_IR, S_IR32, S_NORMS, S_REL, S_BGEOM, S_BTD, S_MLP,
     S_FIX, S_FOBS, S_FDISP, S_ATA, S_LIST, S_CHAIN, S_LCPJ, S_LCPC, S_LCPV, S_LCPP, S_GEMM, S_LPC_NET, S_LPC_WS, S_LPC_GEOM, S_LPC_TNBR, S_LPC_FEAT, S_LPC_OUT,
     S_LPC_NBR, S_LPC_BLK, S_LPC_MAT, S_LPC_PGEOM, S_BJ_NBR, S_BJ_BLK, S_KWORK, S_A32MV, S_TUNE, S_AT, S_G_A32, S_G_INT, S_G_F32, S_G_F64, S_G_MAPS,
-    S_EDGE_PTS, S_EDGE_CODE, S_EDGE_REC, S_EDGE_G, S_EDGE_PTR, S_EDGE_TRIS, S_COUNT
+    S_EDGE_PTS, S_EDGE_INT, S_EDGE_REC, S_EDGE_G, S_COUNT
 };
 
 constexpr int kGmresRestart = 30; // default Krylov dimension of a GMRES cycle
@@ -114,13 +114,6 @@ struct cad_ctx {
     cudaEvent_t side_fork = nullptr, side_join = nullptr;   // work forked onto the side stream
     Tuner tuner;                           // cad_set_autotune
     int shared_edges = 1;                  // cad_set_shared_edges
-    // mesh-edge table of the last half-space assembly: the vertices it was
-    // built from (P1, P2, P3, 3 N each), its edges' endpoints (6 per edge)
-    // and each triangle side's signed edge number (0 for none); per edge, the
-    // signed triangles on it (edge_ptr offsets into edge_tris)
-    std::vector<double> edge_geom, edge_pts;
-    std::vector<int> edge_code, edge_ptr, edge_tris;
-    int64_t edge_n = -1;
     double tol = 1e-10;
     int max_iter = 200;
     bool fric_ready = false;      // cad_friction_prepare: C = inv(A Scl) of fric_N elements in S_LCPC
@@ -212,50 +205,10 @@ int64_t pick_chunk(int64_t M, int64_t N, bool sum_mode)
     return (N + nchunk - 1) / nchunk;
 }
 
-int hs_check(cad_ctx* ctx, const double* Z, int64_t M, const double* P1, const double* P2, const double* P3,
-             int64_t N)
-{
-    void* flag;
-    if (int r = ensure(ctx, S_FLAG, sizeof(int), &flag)) return r;
-    ++ctx->launches;
-    CK(launch_hs_check(Z, M, P1, P2, P3, N, (int*)flag, ctx->stream));
-    int h = 0;
-    CK(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    if (h) return fail(ctx, CAD_ERR_HS_ABOVE_SURFACE, "Half-space solution: Z coordinates must be negative!");
-    return CAD_OK;
-}
-
-// Number the mesh's distinct triangle sides (edges).  Side s of triangle j
-// runs P1->P2, P2->P3, P3->P1; its code is e + 1 when it runs the way edge e
-// was first seen, -(e + 1) when it runs the other way.  Endpoints match when
-// their coordinates are equal (-0.0 taken as 0.0).  The table is rebuilt only
-// when the vertices differ from the last call's; the device copies of the
-// edge endpoints and codes are uploaded with it.
-struct EdgeKey {
-    double v[6];
-    bool operator==(const EdgeKey& o) const { return std::memcmp(v, o.v, sizeof v) == 0; }
-};
-struct EdgeKeyHash {
-    size_t operator()(const EdgeKey& k) const
-    {
-        uint64_t h = 1469598103934665603ull;
-        for (double d : k.v) {
-            uint64_t u;
-            std::memcpy(&u, &d, sizeof u);
-            h = (h ^ u) * 1099511628211ull;
-            h ^= h >> 29;
-        }
-        return (size_t)h;
-    }
-};
-
 struct EdgeTable {
     int64_t E = 0;
-    double* pts = nullptr;   // device: 6 doubles per edge
-    int* code = nullptr;     // device: 3 per triangle
-    int* ptr = nullptr;      // device: E + 1 offsets into tris
-    int* tris = nullptr;     // device: +-(triangle + 1) per side, by edge
+    EdgeArrays a{};
+    bool use = false;   // the mesh's sides share edges (edges_pay)
 };
 
 // Shared-edge work pays when the mesh's edges are clearly fewer than its
@@ -263,84 +216,33 @@ struct EdgeTable {
 // triangles stays on the per-side kernels.
 bool edges_pay(int64_t E, int64_t N) { return 10 * E < 9 * 3 * N; }
 
-int edge_table(cad_ctx* ctx, const double* P1, const double* P2, const double* P3, int64_t N, EdgeTable* out)
+// The half-space argument check and, with et set and shared edges on, the
+// mesh-edge table (lists: with each edge's sides); one read-back for both.
+int hs_check(cad_ctx* ctx, const double* Z, int64_t M, const double* P1, const double* P2, const double* P3,
+             int64_t N, EdgeTable* et = nullptr, bool lists = false)
 {
-    if (3 * N > INT32_MAX) {   // side codes are ints: such meshes stay on the per-side path
-        out->E = 3 * N;
-        return CAD_OK;
+    void* flag;
+    if (int r = ensure(ctx, S_FLAG, 2 * sizeof(int), &flag)) return r;
+    ++ctx->launches;
+    CK(launch_hs_check(Z, M, P1, P2, P3, N, (int*)flag, ctx->stream));
+    // side codes are ints: larger meshes stay on the per-side path
+    const bool edges = et && ctx->shared_edges && N > 0 && 3 * N <= INT32_MAX;
+    if (edges) {
+        void *pts, *ints;
+        if (int r = ensure(ctx, S_EDGE_PTS, (size_t)18 * N * sizeof(double), &pts)) return r;
+        if (int r = ensure(ctx, S_EDGE_INT, ((size_t)12 * N + edge_work_ints(N)) * sizeof(int), &ints)) return r;
+        int* i = (int*)ints;
+        et->a = EdgeArrays{(double*)pts, i, i + 3 * N, i + 6 * N, i + 9 * N, i + 12 * N, (int*)flag + 1};
+        CK(launch_edge_table(P1, P2, P3, N, et->a, lists, ctx->stream, &ctx->launches));
     }
-    std::vector<double> geom((size_t)9 * N);
-    CK(cudaMemcpyAsync(geom.data(), P1, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(geom.data() + 3 * N, P2, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(geom.data() + 6 * N, P3, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    int h[2] = {0, 0};
+    CK(cudaMemcpyAsync(h, flag, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    void *pts, *code, *eptr, *etris;
-    const bool same = ctx->edge_n == N && ctx->edge_geom == geom;
-    if (!same) {
-        std::unordered_map<EdgeKey, int, EdgeKeyHash> seen;
-        seen.reserve((size_t)3 * N);
-        ctx->edge_pts.clear();
-        ctx->edge_code.assign((size_t)3 * N, 0);
-        for (int64_t j = 0; j < N; ++j)
-            for (int sd = 0; sd < 3; ++sd) {
-                const double* va = geom.data() + 3 * N * sd + j;
-                const double* vb = geom.data() + 3 * N * ((sd + 1) % 3) + j;
-                // + 0.0 turns -0.0 into 0.0
-                const EdgeKey fwd{{va[0] + 0.0, va[N] + 0.0, va[2 * N] + 0.0, vb[0] + 0.0, vb[N] + 0.0, vb[2 * N] + 0.0}};
-                const EdgeKey rev{{fwd.v[3], fwd.v[4], fwd.v[5], fwd.v[0], fwd.v[1], fwd.v[2]}};
-                int c;
-                auto it = seen.find(fwd);
-                if (it != seen.end()) {
-                    c = it->second + 1;
-                } else if ((it = seen.find(rev)) != seen.end()) {
-                    c = -(it->second + 1);
-                } else {
-                    const int e = (int)seen.size();
-                    seen.emplace(fwd, e);
-                    ctx->edge_pts.insert(ctx->edge_pts.end(), fwd.v, fwd.v + 6);
-                    c = e + 1;
-                }
-                ctx->edge_code[(size_t)3 * j + sd] = c;
-            }
-        // edge -> sides, in triangle order (counting sort on the edge number)
-        const size_t E = ctx->edge_pts.size() / 6;
-        ctx->edge_ptr.assign(E + 1, 0);
-        for (int c : ctx->edge_code) ++ctx->edge_ptr[(size_t)(c > 0 ? c : -c)];
-        for (size_t e = 0; e < E; ++e) ctx->edge_ptr[e + 1] += ctx->edge_ptr[e];
-        ctx->edge_tris.assign((size_t)3 * N, 0);
-        std::vector<int> fill(ctx->edge_ptr.begin(), ctx->edge_ptr.end() - 1);
-        for (int64_t k = 0; k < 3 * N; ++k) {
-            const int c = ctx->edge_code[(size_t)k];
-            const int t = (int)(k / 3) + 1;
-            ctx->edge_tris[(size_t)fill[(size_t)((c > 0 ? c : -c) - 1)]++] = c > 0 ? t : -t;
-        }
-        ctx->edge_n = -1;
-        if (int r = ensure(ctx, S_EDGE_PTS, ctx->edge_pts.size() * sizeof(double), &pts)) return r;
-        if (int r = ensure(ctx, S_EDGE_CODE, ctx->edge_code.size() * sizeof(int), &code)) return r;
-        if (int r = ensure(ctx, S_EDGE_PTR, ctx->edge_ptr.size() * sizeof(int), &eptr)) return r;
-        if (int r = ensure(ctx, S_EDGE_TRIS, ctx->edge_tris.size() * sizeof(int), &etris)) return r;
-        CK(cudaMemcpyAsync(eptr, ctx->edge_ptr.data(), ctx->edge_ptr.size() * sizeof(int), cudaMemcpyHostToDevice,
-                           ctx->stream));
-        CK(cudaMemcpyAsync(etris, ctx->edge_tris.data(), ctx->edge_tris.size() * sizeof(int),
-                           cudaMemcpyHostToDevice, ctx->stream));
-        CK(cudaMemcpyAsync(pts, ctx->edge_pts.data(), ctx->edge_pts.size() * sizeof(double),
-                           cudaMemcpyHostToDevice, ctx->stream));
-        CK(cudaMemcpyAsync(code, ctx->edge_code.data(), ctx->edge_code.size() * sizeof(int),
-                           cudaMemcpyHostToDevice, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        ctx->edge_geom.swap(geom);
-        ctx->edge_n = N;
-    } else {
-        pts = ctx->buf[S_EDGE_PTS].p;
-        code = ctx->buf[S_EDGE_CODE].p;
-        eptr = ctx->buf[S_EDGE_PTR].p;
-        etris = ctx->buf[S_EDGE_TRIS].p;
+    if (h[0]) return fail(ctx, CAD_ERR_HS_ABOVE_SURFACE, "Half-space solution: Z coordinates must be negative!");
+    if (edges) {
+        et->E = h[1];
+        et->use = edges_pay(et->E, N);
     }
-    out->E = (int64_t)(ctx->edge_pts.size() / 6);
-    out->pts = (double*)pts;
-    out->code = (int*)code;
-    out->ptr = (int*)eptr;
-    out->tris = (int*)etris;
     return CAD_OK;
 }
 
@@ -350,8 +252,10 @@ int td_device(cad_ctx* ctx, const double* X, const double* Y, const double* Z, i
               double nu, int disp, int strain, int hs, int out_kind, double* strain_out, double* disp_out,
               double* sum_out /* 9 x M for OUT_SUM */)
 {
+    EdgeTable et;
+    const bool edge_kind = (out_kind == OUT_SUM || out_kind == OUT_INF) && (strain == 1 || disp == 1) && M > 0;
     if (hs == 1 && N > 0)
-        if (int r = hs_check(ctx, Z, M, P1, P2, P3, N)) return r;
+        if (int r = hs_check(ctx, Z, M, P1, P2, P3, N, edge_kind ? &et : nullptr, out_kind == OUT_SUM)) return r;
     if (M == 0 || N == 0) {
         if (out_kind == OUT_SUM && sum_out) CK(cudaMemsetAsync(sum_out, 0, 9 * M * sizeof(double), ctx->stream));
         return CAD_OK;
@@ -365,12 +269,7 @@ int td_device(cad_ctx* ctx, const double* X, const double* Y, const double* Z, i
     a.tri_chunk = pick_chunk(M, N, out_kind == OUT_SUM);
     a.strain = strain_out; a.disp = disp_out;
     const int64_t nchunk = (N + a.tri_chunk - 1) / a.tri_chunk;
-    EdgeTable et;
-    const bool edge_kind = (out_kind == OUT_SUM || out_kind == OUT_INF) && hs == 1 && ctx->shared_edges &&
-                           (strain == 1 || disp == 1);
-    if (edge_kind)
-        if (int r = edge_table(ctx, P1, P2, P3, N, &et)) return r;
-    if (edge_kind && out_kind == OUT_INF && edges_pay(et.E, N)) {
+    if (et.use && out_kind == OUT_INF) {
         // per-edge free-surface maps at the points (strain 18, displacement
         // 9 values), read by the triangles that share each edge
         void *rec, *gmap;
@@ -381,13 +280,13 @@ int td_device(cad_ctx* ctx, const double* X, const double* Y, const double* Z, i
         if (Mc > M) Mc = M;
         if (int r = ensure(ctx, S_EDGE_G, (size_t)Mc * per_point, &gmap)) return r;
         CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-        CK(launch_assemble_edges(a, OUT_INF, strain == 1, disp == 1, et.pts, et.E, et.code, rec, (double*)gmap, Mc,
+        CK(launch_assemble_edges(a, OUT_INF, strain == 1, disp == 1, et.a.pts, et.E, et.a.code, rec, (double*)gmap, Mc,
                                  nu, ctx->stream, &ctx->launches));
         CK(cudaEventRecord(ctx->ev[1], ctx->stream));
         ctx->timed[0] = true;
         return CAD_OK;
     }
-    if (edge_kind && out_kind == OUT_SUM && edges_pay(et.E, N)) {
+    if (et.use) {
         // real + image terms per triangle chunk, then each mesh edge's
         // free-surface correction once, for the net Burgers vector of the
         // sides on it; all partials summed in one fixed order
@@ -398,7 +297,7 @@ int td_device(cad_ctx* ctx, const double* X, const double* Y, const double* Z, i
         if (int r = ensure(ctx, S_EDGE_REC, (size_t)et.E * edge_record_bytes(), &rec)) return r;
         a.partial = (double*)part;
         CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-        CK(launch_td_sum_edges(a, strain == 1, disp == 1, et.pts, et.E, et.ptr, et.tris, rec, nu, echunk,
+        CK(launch_td_sum_edges(a, strain == 1, disp == 1, et.a, et.E, rec, nu, echunk,
                                a.partial + (size_t)nchunk * 9 * M, ctx->stream, &ctx->launches));
         CK(cudaEventRecord(ctx->ev[1], ctx->stream));
         ctx->timed[0] = true;
@@ -436,8 +335,10 @@ int assemble_device(cad_ctx* ctx, const double* normals, const double* mid, cons
     double* X = (double*)obs;
     ++ctx->launches;
     CK(launch_colloc(normals, mid, N, X, X + N, X + 2 * N, (double*)dirs, ctx->stream));
+    EdgeTable et;
+    const bool edge_kind = (out_kind == OUT_AMAT && ctx->assembly != CAD_ASSEMBLY_MIXED) || out_kind == OUT_TRAC;
     if (hs == 1 && N > 0)
-        if (int r = hs_check(ctx, X + 2 * N, N, P1, P2, P3, N)) return r;
+        if (int r = hs_check(ctx, X + 2 * N, N, P1, P2, P3, N, edge_kind ? &et : nullptr)) return r;
     if (N == 0) return CAD_OK;
     void* tri;
     if (int r = ensure(ctx, S_TRI, (size_t)N * tri_record_bytes(), &tri)) return r;
@@ -459,16 +360,12 @@ int assemble_device(cad_ctx* ctx, const double* normals, const double* mid, cons
         ctx->timed[0] = true;
         return CAD_OK;
     }
-    EdgeTable et;
-    const bool edge_kind = (out_kind == OUT_AMAT && ctx->assembly != CAD_ASSEMBLY_MIXED) || out_kind == OUT_TRAC;
-    if (edge_kind && hs == 1 && ctx->shared_edges)
-        if (int r = edge_table(ctx, P1, P2, P3, N, &et)) return r;
-    if (edge_kind && hs == 1 && ctx->shared_edges && edges_pay(et.E, N)) {
+    if (et.use) {
         // each mesh edge's free-surface map evaluated once, then read by the
         // (one or two) triangles that share the edge
         const int64_t E = et.E;
-        double* pts = et.pts;
-        int* codes = et.code;
+        double* pts = et.a.pts;
+        int* codes = et.a.code;
         void *rec, *gmap;
         if (int r = ensure(ctx, S_EDGE_REC, (size_t)(E > 0 ? E : 1) * edge_record_bytes(), &rec)) return r;
         const int64_t per_point = 18 * (E > 0 ? E : 1) * (int64_t)sizeof(double);

@@ -614,17 +614,27 @@ cudaError_t launch_assemble_edges(PairArgs a, int out_kind, bool strain, bool di
 }
 
 // Net Burgers vector of each mesh edge: the signed sum over the triangle sides
-// on it (edge_tris[edge_ptr[e] .. edge_ptr[e + 1]) = +-(triangle + 1), in
-// triangle order) of Dn Vn + Dss Vs + Dds Vd, then the edge's record for it.
-__global__ void edge_burgers_kernel(const double* __restrict__ pts, int64_t E, const int* __restrict__ edge_ptr,
-                                    const int* __restrict__ edge_tris, const TriDev* __restrict__ tri, double nu,
-                                    FscSide* __restrict__ out)
+// on it (sides[ptr[e] ..] = +-(triangle + 1), sorted here into triangle order,
+// then side order, so the sum does not depend on how the list was filled) of
+// Dn Vn + Dss Vs + Dds Vd, then the edge's record for it.
+__global__ void edge_burgers_kernel(const double* __restrict__ pts, int64_t E, const int* __restrict__ ptr,
+                                    const int* __restrict__ cnt, int* __restrict__ sides,
+                                    const TriDev* __restrict__ tri, double nu, FscSide* __restrict__ out)
 {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= E) return;
+    int* list = sides + ptr[e];
+    const int n = cnt[e];
+    for (int i = 1; i < n; ++i) {
+        const int v = list[i];
+        int j = i;
+        for (; j > 0 && (abs(list[j - 1]) > abs(v) || (abs(list[j - 1]) == abs(v) && list[j - 1] < v)); --j)
+            list[j] = list[j - 1];
+        list[j] = v;
+    }
     double B[3] = {0.0, 0.0, 0.0};
-    for (int k = edge_ptr[e]; k < edge_ptr[e + 1]; ++k) {
-        const int c = edge_tris[k];
+    for (int k = 0; k < n; ++k) {
+        const int c = list[k];
         const TriDev& t = tri[(c > 0 ? c : -c) - 1];
         const double sg = c > 0 ? 1.0 : -1.0;
         const double slip[3] = {t.Dn, t.Dss, t.Dds};
@@ -673,9 +683,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) fsc_sum_kernel(const FscSide*
     for (int c = 0; c < 3; ++c) p[(6 + c) * M + i] = DISP ? Us[0][c] : 0.0;
 }
 
-cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, const double* edge_pts, int64_t E,
-                                const int* edge_ptr, const int* edge_tris, void* edge_rec, double nu, int64_t echunk,
-                                double* edge_partial, cudaStream_t st, int64_t* launches)
+cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, const EdgeArrays& ed, int64_t E, void* edge_rec,
+                                double nu, int64_t echunk, double* edge_partial, cudaStream_t st, int64_t* launches)
 {
     if (a.M == 0 || a.N == 0 || !(strain || disp)) return cudaSuccess;
     const size_t psmem = (size_t)kTriWordsImg * sizeof(double);
@@ -700,8 +709,8 @@ cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, const double
                     : strain       ? pairs(td_pair_kernel<true, true, false, OUT_SUM, false, false, 1, true>)
                                    : pairs(td_pair_kernel<true, false, true, OUT_SUM, false, false, 1, true>);
     if (e != cudaSuccess || E == 0) return e;
-    edge_burgers_kernel<<<(unsigned)((E + 127) / 128), 128, 0, st>>>(edge_pts, E, edge_ptr, edge_tris, a.tri, nu,
-                                                                      (FscSide*)edge_rec);
+    edge_burgers_kernel<<<(unsigned)((E + 63) / 64), 64, 0, st>>>(ed.pts, E, ed.ptr, ed.cnt, ed.sides, a.tri, nu,
+                                                                   (FscSide*)edge_rec);
     if (launches) ++*launches;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     return strain && disp ? sums(fsc_sum_kernel<true, true>)

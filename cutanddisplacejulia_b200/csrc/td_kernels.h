@@ -4,6 +4,8 @@
 
 #include <cstdint>
 
+#include "edges.h"
+
 namespace cad {
 
 template <typename T>
@@ -73,12 +75,10 @@ size_t edge_record_bytes();
 // per mesh edge for the net Burgers vector of the triangle sides on it:
 // a.partial receives the real + image terms of each triangle chunk (as
 // launch_td_pairs), edge_partial the corrections of each chunk of echunk
-// edges (9 x a.M each).  edge_ptr / edge_tris list each edge's sides as
-// +-(triangle + 1), + for a side running the edge's way.  a.tri must hold the
-// records of launch_td_setup (with the triangles' slip).
-cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, const double* edge_pts, int64_t E,
-                                const int* edge_ptr, const int* edge_tris, void* edge_rec, double nu, int64_t echunk,
-                                double* edge_partial, cudaStream_t st, int64_t* launches);
+// edges (9 x a.M each).  ed: launch_edge_table's arrays with lists.  a.tri must
+// hold the records of launch_td_setup (with the triangles' slip).
+cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, const EdgeArrays& ed, int64_t E, void* edge_rec,
+                                double nu, int64_t echunk, double* edge_partial, cudaStream_t st, int64_t* launches);
 
 // Mixed-precision system matrix: every pair in FP32 (far field), then the
 // pairs of every 128-point tile that has a point within the near radius of

@@ -1,0 +1,64 @@
+"""GPU tests of the device-built mesh-edge table (csrc/edges.cu) through the
+half-space sums and the system matrix, shared edges against the per-side
+path: side counts around the 256-side blocks and the table's powers of two,
+an edge shared by many triangles, repeated triangles, and -0.0 vertices."""
+import numpy as np
+import pytest
+
+from helpers import assert_parity, rel_inf_err
+
+pytestmark = pytest.mark.gpu
+
+
+def _sums(cad, P, sl, pts, shared):
+    from cutanddisplacejulia_b200 import _lib
+    L, ctx = _lib.load(), _lib.context(0)
+    _lib.check(L.cad_set_shared_edges(ctx, int(shared)), ctx)
+    try:
+        S, U = cad.TD(*pts.T, *P, *sl, 0.25, 1.0, 1, 1, 1, cad.Strains(), cad.Disps())
+    finally:
+        _lib.check(L.cad_set_shared_edges(ctx, 1), ctx)
+    return np.stack(list(S)), np.stack(list(U))
+
+
+def _strip(n):
+    """n triangles of a bent strip, neighbours sharing an edge."""
+    k = np.arange(n + 2)
+    node = np.stack([0.3 * (k // 2), 0.4 * (k % 2) + 0.01 * np.sin(k), -0.5 - 0.2 * (k % 2) - 0.02 * np.cos(k)], 1)
+    P1, P2, P3 = node[:-2].copy(), node[1:-1].copy(), node[2:].copy()
+    odd = np.arange(n) % 2 == 1
+    return P1, np.where(odd[:, None], P3, P2), np.where(odd[:, None], P2, P3)
+
+
+@pytest.mark.parametrize("n", [2, 3, 10, 11, 21, 22, 85, 86, 171, 342])
+def test_sums_over_side_counts(cad, n):
+    rng = np.random.default_rng(n)
+    P = _strip(n)
+    sl = rng.uniform(-1e-3, 1e-3, (3, n))
+    pts = np.column_stack([rng.uniform(-1, 0.2 * n, 70), rng.uniform(-1, 1, 70), rng.uniform(-2, -0.05, 70)])
+    a, b = _sums(cad, P, sl, pts, True), _sums(cad, P, sl, pts, False)
+    assert_parity(a[0], b[0])
+    assert_parity(a[1], b[1])
+    # the table is filled in no fixed order; the sums are the same every time
+    c = _sums(cad, P, sl, pts, True)
+    assert np.array_equal(a[0], c[0]) and np.array_equal(a[1], c[1])
+
+
+def test_edge_with_many_triangles_repeats_and_negative_zero(cad):
+    rng = np.random.default_rng(1)
+    k = 9
+    th = np.linspace(0, np.pi, k)
+    A, B = np.array([0.0, 0.0, -0.5]), np.array([1.0, 0.0, -0.7])
+    C = np.stack([0.5 + 0 * th, np.cos(th), -0.6 - 0.5 * np.sin(th)], 1)
+    P1, P2, P3 = np.tile(A, (k, 1)), np.tile(B, (k, 1)), C
+    flip = rng.random(k) < 0.5                    # the common edge run both ways
+    P1, P2 = np.where(flip[:, None], P2, P1), np.where(flip[:, None], P1, P2)
+    P1[0, 1] = P2[0, 1] = -0.0                    # equal to the others' 0.0
+    P = [np.concatenate([p, p[:3]]) for p in (P1, P2, P3)]   # three triangles twice
+    n = len(P[0])
+    sl = rng.uniform(-1e-3, 1e-3, (3, n))
+    pts = rng.uniform([-1, -1, -2], [2, 1, -0.05], (60, 3))
+    a, b = _sums(cad, P, sl, pts, True), _sums(cad, P, sl, pts, False)
+    assert_parity(a[0], b[0])
+    assert_parity(a[1], b[1])
+    assert rel_inf_err(a[0], b[0]) < 1e-12
