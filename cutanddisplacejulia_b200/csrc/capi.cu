@@ -209,6 +209,7 @@ struct EdgeTable {
     int64_t E = 0;
     EdgeArrays a{};
     bool use = false;   // the mesh's sides share edges (edges_pay)
+    bool full = false;  // no triangle is horizontal: the whole strain is a sum over sides
 };
 
 // Shared-edge work pays when the mesh's edges are clearly fewer than its
@@ -222,9 +223,10 @@ int hs_check(cad_ctx* ctx, const double* Z, int64_t M, const double* P1, const d
              int64_t N, EdgeTable* et = nullptr, bool lists = false)
 {
     void* flag;
-    if (int r = ensure(ctx, S_FLAG, 2 * sizeof(int), &flag)) return r;
+    if (int r = ensure(ctx, S_FLAG, 3 * sizeof(int), &flag)) return r;
     ++ctx->launches;
-    CK(launch_hs_check(Z, M, P1, P2, P3, N, (int*)flag, ctx->stream));
+    CK(cudaMemsetAsync(flag, 0, 3 * sizeof(int), ctx->stream));
+    CK(launch_hs_check(Z, M, P1, P2, P3, N, (int*)flag, ctx->stream, nullptr, false, et ? (int*)flag + 2 : nullptr));
     // side codes are ints: larger meshes stay on the per-side path
     const bool edges = et && ctx->shared_edges && N > 0 && 3 * N <= INT32_MAX;
     if (edges) {
@@ -235,13 +237,14 @@ int hs_check(cad_ctx* ctx, const double* Z, int64_t M, const double* P1, const d
         et->a = EdgeArrays{(double*)pts, i, i + 3 * N, i + 6 * N, i + 9 * N, i + 12 * N, (int*)flag + 1};
         CK(launch_edge_table(P1, P2, P3, N, et->a, lists, ctx->stream, &ctx->launches));
     }
-    int h[2] = {0, 0};
+    int h[3] = {0, 0, 0};
     CK(cudaMemcpyAsync(h, flag, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (h[0]) return fail(ctx, CAD_ERR_HS_ABOVE_SURFACE, "Half-space solution: Z coordinates must be negative!");
     if (edges) {
         et->E = h[1];
         et->use = edges_pay(et->E, N);
+        et->full = h[2] == 0;
     }
     return CAD_OK;
 }
@@ -274,13 +277,14 @@ int td_device(cad_ctx* ctx, const double* X, const double* Y, const double* Z, i
         // 9 values), read by the triangles that share each edge
         void *rec, *gmap;
         if (int r = ensure(ctx, S_EDGE_REC, (size_t)et.E * edge_record_bytes(), &rec)) return r;
-        const int64_t per_point = (18 * (strain == 1) + 9 * (disp == 1)) * et.E * (int64_t)sizeof(double);
+        const int64_t per_point =
+            edge_map_values(OUT_INF, strain == 1, disp == 1, et.full) * et.E * (int64_t)sizeof(double);
         int64_t Mc = (int64_t)(kEdgeMapBytes / per_point) / kPairThreads * kPairThreads;
         if (Mc < kPairThreads) Mc = kPairThreads;
         if (Mc > M) Mc = M;
         if (int r = ensure(ctx, S_EDGE_G, (size_t)Mc * per_point, &gmap)) return r;
         CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-        CK(launch_assemble_edges(a, OUT_INF, strain == 1, disp == 1, et.a.pts, et.E, et.a.code, rec, (double*)gmap, Mc,
+        CK(launch_assemble_edges(a, OUT_INF, strain == 1, disp == 1, et.full, et.a.pts, et.E, et.a.code, rec, (double*)gmap, Mc,
                                  nu, ctx->stream, &ctx->launches));
         CK(cudaEventRecord(ctx->ev[1], ctx->stream));
         ctx->timed[0] = true;
@@ -297,7 +301,7 @@ int td_device(cad_ctx* ctx, const double* X, const double* Y, const double* Z, i
         if (int r = ensure(ctx, S_EDGE_REC, (size_t)et.E * edge_record_bytes(), &rec)) return r;
         a.partial = (double*)part;
         CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-        CK(launch_td_sum_edges(a, strain == 1, disp == 1, et.a, et.E, rec, nu, echunk,
+        CK(launch_td_sum_edges(a, strain == 1, disp == 1, et.full, et.a, et.E, rec, nu, echunk,
                                a.partial + (size_t)nchunk * 9 * M, ctx->stream, &ctx->launches));
         CK(cudaEventRecord(ctx->ev[1], ctx->stream));
         ctx->timed[0] = true;
@@ -368,18 +372,19 @@ int assemble_device(cad_ctx* ctx, const double* normals, const double* mid, cons
         int* codes = et.a.code;
         void *rec, *gmap;
         if (int r = ensure(ctx, S_EDGE_REC, (size_t)(E > 0 ? E : 1) * edge_record_bytes(), &rec)) return r;
-        const int64_t per_point = 18 * (E > 0 ? E : 1) * (int64_t)sizeof(double);
+        const int64_t per_point =
+            edge_map_values(out_kind, true, false, et.full) * (E > 0 ? E : 1) * (int64_t)sizeof(double);
         int64_t Mc = (int64_t)(kEdgeMapBytes / per_point) / kPairThreads * kPairThreads;
         if (Mc < kPairThreads) Mc = kPairThreads;
         if (Mc > N) Mc = N;
         if (int r = ensure(ctx, S_EDGE_G, (size_t)Mc * per_point, &gmap)) return r;
         a.min_blocks = kEdgeMinBlocks;
         if (ctx->tuner.mode != TUNE_OFF && out_kind == OUT_AMAT) {
-            // triangles per block of the edge pair kernel, then its build
-            // (resident blocks per SM); each candidate runs the whole path
+            // triangles per block of the edge pair kernel, then edges per
+            // block of the map kernel; each candidate runs the whole path
             char key[96];
             auto run = [&](const PairArgs& t) {
-                return launch_assemble_edges(t, out_kind, true, false, pts, E, codes, rec, (double*)gmap, Mc, nu, ctx->stream,
+                return launch_assemble_edges(t, out_kind, true, false, et.full, pts, E, codes, rec, (double*)gmap, Mc, nu, ctx->stream,
                                              &ctx->launches);
             };
             std::snprintf(key, sizeof key, "pair_amat_f64_hs1_edge_N%lld", (long long)tune_class(N));
@@ -396,7 +401,7 @@ int assemble_device(cad_ctx* ctx, const double* normals, const double* mid, cons
             });
         }
         CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-        CK(launch_assemble_edges(a, out_kind, true, false, pts, E, codes, rec, (double*)gmap, Mc, nu, ctx->stream, &ctx->launches));
+        CK(launch_assemble_edges(a, out_kind, true, false, et.full, pts, E, codes, rec, (double*)gmap, Mc, nu, ctx->stream, &ctx->launches));
         CK(cudaEventRecord(ctx->ev[1], ctx->stream));
         ctx->timed[0] = true;
         return CAD_OK;

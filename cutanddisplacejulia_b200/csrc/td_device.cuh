@@ -53,6 +53,7 @@ struct FscAcc {
     R g1r, g1i, Or, Oi, w2r, w2i, Nr, Ni;     // powers of eta over r
     R t1, t2, tq, At1, At2, Atq;              // (y1, y2, q) / r^3, and times the end's depth a
     R s11, s12, s1q, s22, s2q;                // a x second derivatives of 1 / r
+    R u, v, c3;                               // image segment: 1 / (r w), its I term, 1 / r^3
 };
 template <typename R>
 struct FscDispAcc {
@@ -280,6 +281,12 @@ struct SegInt {
     R K, I, T, Q, V;
 };
 
+template <typename R>
+CAD_HD constexpr R tiny_square()   // its reciprocal's square does not overflow
+{
+    return sizeof(R) == sizeof(double) ? R(1e-140) : R(1e-15);
+}
+
 // Integrals of one side from its end distances (R, 1 / R) and the coordinates
 // sA, sB of the ends along it, rho2 = |d|^2.  The side is taken in the
 // direction in which the nearer end has the smaller coordinate, so R + s of
@@ -293,7 +300,9 @@ CAD_HD SegInt<R> seg_integrals(R RA, R iA, R RB, R iB, R sA, R sB, R rho2)
     const R Ra = fwd ? RA : RB, Rb = fwd ? RB : RA;
     const R ia = fwd ? iA : iB, ib = fwd ? iB : iA;
     const bool out = a >= R(0.0);
-    const R den = out ? Ra + a : rho2, num = out ? R(1.0) : Ra - a;
+    // (a point exactly on the side keeps finite integrals: whether its pair is
+    // NaN is on_side's decision, triangle by triangle)
+    const R den = out ? Ra + a : (rho2 > tiny_square<R>() ? rho2 : tiny_square<R>()), num = out ? R(1.0) : Ra - a;
     const R wb = Rb + b;
     const R inv = R(1.0) / (den * wb);
     const R iwa = inv * wb * num, iwb = inv * den;   // 1 / (R + s) at both ends
@@ -309,19 +318,53 @@ CAD_HD SegInt<R> seg_integrals(R RA, R iA, R RB, R iB, R sA, R sB, R rho2)
 
 constexpr double kInv4Pi = 0.079577471545947667884;   // 1 / (4 pi)
 
+// Strain of a segment for a unit Burgers vector along each of its own axes
+// (n, m = t x n, t the side's direction): the point is offset (x, e) along
+// (n, m).  First letter: the Burgers vector's axis.  k1 = 1 / (4 pi) and K8 =
+// 1 / (8 pi (1 - nu)), or both times a common factor.
+template <typename R>
+struct SegStrain {
+    R nnn, nmm, ntt, nnm, nmt, nnt;
+    R mnn, mmm, mtt, mnm, mmt, mnt;
+    R tnt, tmt;
+};
+template <typename R>
+CAD_HD SegStrain<R> seg_strain(const SegInt<R>& g, R x, R e, R k1, R K8)
+{
+    const R x2 = x * x, e2 = e * e, ka = k1 - R(2.0) * K8;
+    const R Hnn = x2 * g.I - g.K, Hmm = e2 * g.I - g.K, Htt = -(Hnn + Hmm);
+    const R hT = R(0.5) * ka * g.T, kK = K8 * g.K, k1K = k1 * g.K, kaK = ka * g.K, kI = K8 * g.I, kQ = K8 * g.Q;
+    SegStrain<R> s;
+    s.nnn = e * (k1K + K8 * Hnn);
+    s.nmm = e * (kaK + K8 * Hmm);
+    s.ntt = K8 * e * Htt;
+    s.nnm = x * (e2 * kI - kK);
+    s.nmt = -hT - e2 * kQ;
+    s.nnt = -e * x * kQ;
+    s.mmm = -x * (k1K + K8 * Hmm);
+    s.mnn = -x * (kaK + K8 * Hnn);
+    s.mtt = -K8 * x * Htt;
+    s.mnm = e * (kK - x2 * kI);
+    s.mnt = hT + x2 * kQ;
+    s.mmt = e * x * kQ;
+    s.tnt = R(0.5) * e * k1K;
+    s.tmt = R(-0.5) * x * k1K;
+    return s;
+}
+
 // Strain of unit slip n, strike, dip (TDCS xx, yy, zz, xy, xz, yz) and the
 // displacement (its solid-angle part included) of frame f at TDCS (x, y, z).
 // K8 = 1 / (8 pi (1 - nu)).  In the segment's own axes (n = TD normal,
 // m = t x n in the plane, t along the side) the offset is (x, e, 0), the
-// Hessian of V is H, and a unit Burgers vector b gives
+// Hessian of V is H (diagonal entries x^2 I - K, e^2 I - K), and a unit
+// Burgers vector b gives
 //   strain -1/(4 pi) sym(b w) K + (1/(4 pi) - 2 K8) sym((b x t) grad V) - K8 (b.w) H
 //   displacement 1/(4 pi) (b x t) V - K8 ((b x t) V + (b.w) grad V)
 // with w = (-e, x, 0) and grad V = (-x K, -e K, T).
 template <bool STRAIN, bool DISP, typename R>
 CAD_HD void td_unit(const FrameT<R>& f, R x, R y, R z, R K8, R E[3][6], R U[3][3])
 {
-    const R k1 = R(kInv4Pi), ka = k1 - R(2.0) * K8;
-    const R h = R(-1.0) * K8;   // (ka - k1) / 2
+    const R k1 = R(kInv4Pi);
     const R dy[3] = {y - f.p1y, y, y - f.p3y}, dz[3] = {z - f.p1z, z, z - f.p3z};
     const R x2 = x * x;
     R Rv[3], iR[3];
@@ -359,35 +402,27 @@ CAD_HD void td_unit(const FrameT<R>& f, R x, R y, R z, R K8, R E[3][6], R U[3][3
         const R e2 = e * e;
         const SegInt<R> g = seg_integrals<DISP>(Rv[A], iR[A], Rv[B], iR[B], sA, sB, x2 + e2);
         if (STRAIN) {
-            const R Hnn = x2 * g.I - g.K, Hmm = e2 * g.I - g.K;
-            const R Htt = -(Hnn + Hmm);
-            const R hT = R(0.5) * ka * g.T;
-            // b = n
-            const R nnn = e * (k1 * g.K + K8 * Hnn), nmm = e * (ka * g.K + K8 * Hmm), ntt = K8 * e * Htt;
-            const R nnm = x * (h * g.K + K8 * e2 * g.I), nmt = -hT - K8 * e2 * g.Q, nnt = -K8 * e * x * g.Q;
-            // b = m
-            const R mmm = x * (-k1 * g.K - K8 * Hmm), mnn = x * (-ka * g.K - K8 * Hnn), mtt = -K8 * x * Htt;
-            const R mnm = -e * (h * g.K + K8 * x2 * g.I), mnt = hT + K8 * x2 * g.Q, mmt = K8 * x * e * g.Q;
-            // b = t: only nt and mt
-            const R tnt = R(0.5) * k1 * g.K * e, tmt = R(-0.5) * k1 * g.K * x;
+            const SegStrain<R> q = seg_strain(g, x, e, k1, K8);
             const R yy = ty * ty, zz = tz * tz, yz = ty * tz, dd = zz - yy;
-            E[0][0] += nnn;
-            E[0][1] += nmm * zz + ntt * yy + R(2.0) * nmt * yz;
-            E[0][2] += nmm * yy + ntt * zz - R(2.0) * nmt * yz;
-            E[0][3] += nnm * tz + nnt * ty;
-            E[0][4] += nnt * tz - nnm * ty;
-            E[0][5] += (ntt - nmm) * yz + nmt * dd;
+            E[0][0] += q.nnn;
+            E[0][1] += q.nmm * zz + q.ntt * yy + R(2.0) * q.nmt * yz;
+            E[0][2] += q.nmm * yy + q.ntt * zz - R(2.0) * q.nmt * yz;
+            E[0][3] += q.nnm * tz + q.nnt * ty;
+            E[0][4] += q.nnt * tz - q.nnm * ty;
+            E[0][5] += (q.ntt - q.nmm) * yz + q.nmt * dd;
             // b = m and b = t in TDCS, then unit strike = (tz m + ty t), unit dip = (-ty m + tz t)
-            const R r1 = mmm * zz + mtt * yy + R(2.0) * mmt * yz, r2 = mmm * yy + mtt * zz - R(2.0) * mmt * yz;
-            const R r3 = mnm * tz + mnt * ty, r4 = mnt * tz - mnm * ty, r5 = (mtt - mmm) * yz + mmt * dd;
-            const R q1 = R(2.0) * tmt * yz, q3 = tnt * ty, q4 = tnt * tz, q5 = tmt * dd;
-            E[1][0] += tz * mnn;
+            const R r1 = q.mmm * zz + q.mtt * yy + R(2.0) * q.mmt * yz;
+            const R r2 = q.mmm * yy + q.mtt * zz - R(2.0) * q.mmt * yz;
+            const R r3 = q.mnm * tz + q.mnt * ty, r4 = q.mnt * tz - q.mnm * ty;
+            const R r5 = (q.mtt - q.mmm) * yz + q.mmt * dd;
+            const R q1 = R(2.0) * q.tmt * yz, q3 = q.tnt * ty, q4 = q.tnt * tz, q5 = q.tmt * dd;
+            E[1][0] += tz * q.mnn;
             E[1][1] += tz * r1 + ty * q1;
             E[1][2] += tz * r2 - ty * q1;
             E[1][3] += tz * r3 + ty * q3;
             E[1][4] += tz * r4 + ty * q4;
             E[1][5] += tz * r5 + ty * q5;
-            E[2][0] += -ty * mnn;
+            E[2][0] += -ty * q.mnn;
             E[2][1] += tz * q1 - ty * r1;
             E[2][2] += -tz * q1 - ty * r2;
             E[2][3] += tz * q3 - ty * r3;
@@ -585,13 +620,53 @@ CAD_HD void fsc_end(const FscSideT<R>& k, R y1, R y2, R a, R z, R f, R z1, R z3,
     v.s1q = (FIRST ? R(0.0) : v.s1q) + a3 * y1 * uq;
     v.s22 = (FIRST ? R(0.0) : v.s22) + (a3 * y2 * u2 - a * s3);
     v.s2q = (FIRST ? R(0.0) : v.s2q) + a3 * y2 * uq;
+    const R u = ir * iw;
+    v.u = (FIRST ? R(0.0) : v.u) + sg * u;
+    v.v = (FIRST ? R(0.0) : v.v) + sg * u * u * (R(2.0) + kz);
+    v.c3 = (FIRST ? R(0.0) : v.c3) + s3;
+}
+
+// Adds a segment's strain to e[slip][component] (ADCS) for unit slips along the
+// ADCS axes: the segment's axes are n = (c, 0, sg s), m = (0, 1, 0) and t =
+// (-sg s, 0, c); g3 = -1 negates the vertical slip.
+template <typename R>
+CAD_HD void add_segment_adcs(const SegStrain<R>& q, R c, R ss, R g3, R e[3][6])   // ss = sg s
+{
+    const R cc = c * c, s2 = ss * ss, cs = c * ss, dd = cc - s2;
+    const R a0 = cc * q.nnn + s2 * q.ntt - R(2.0) * cs * q.nnt, a2 = s2 * q.nnn + cc * q.ntt + R(2.0) * cs * q.nnt;
+    const R a3 = c * q.nnm - ss * q.nmt, a4 = cs * (q.nnn - q.ntt) + dd * q.nnt, a5 = ss * q.nnm + c * q.nmt;
+    const R b0 = R(2.0) * cs * q.tnt, b3 = ss * q.tmt, b4 = dd * q.tnt, b5 = c * q.tmt;   // -11, 33; -12; 13; 23
+    e[0][0] += c * a0 + ss * b0;
+    e[0][1] += c * q.nmm;
+    e[0][2] += c * a2 - ss * b0;
+    e[0][3] += c * a3 + ss * b3;
+    e[0][4] += c * a4 - ss * b4;
+    e[0][5] += c * a5 - ss * b5;
+    e[1][0] += cc * q.mnn + s2 * q.mtt - R(2.0) * cs * q.mnt;
+    e[1][1] += q.mmm;
+    e[1][2] += s2 * q.mnn + cc * q.mtt + R(2.0) * cs * q.mnt;
+    e[1][3] += c * q.mnm - ss * q.mmt;
+    e[1][4] += cs * (q.mnn - q.mtt) + dd * q.mnt;
+    e[1][5] += ss * q.mnm + c * q.mmt;
+    const R gs = g3 * ss, gc = g3 * c;
+    e[2][0] += gs * a0 - gc * b0;
+    e[2][1] += gs * q.nmm;
+    e[2][2] += gs * a2 + gc * b0;
+    e[2][3] += gs * a3 - gc * b3;
+    e[2][4] += gs * a4 + gc * b4;
+    e[2][5] += gs * a5 + gc * b5;
 }
 
 // Strain of a side's correction in ADCS for a unit ADCS slip along each axis
-// (without K4).  The functions of the two ends are differenced before any
+// (divided by K4).  The functions of the two ends are differenced before any
 // coefficient multiplies them: far from the side the ends nearly cancel.
-template <typename R>
-CAD_HD void fsc_strain_adcs(const FscSideT<R>& s, double X, double Y, double Z, R e[3][6])
+// FULL: with the full-space fields of the side and of its mirror image added
+// (the image segment runs along the same line as the correction's inclined
+// leg and shares its functions; the image dislocation's Burgers vector is the
+// mirrored one, reversed), so that the sum over a triangle's sides is its
+// whole half-space strain.  A near-vertical side (skip) has no correction.
+template <bool FULL, typename R>
+CAD_HD void side_strain_adcs(const FscSideT<R>& s, double X, double Y, double Z, R e[3][6])
 {
     R y1, y2, z;
     to_adcs(s, X, Y, Z, y1, y2, z);
@@ -599,10 +674,34 @@ CAD_HD void fsc_strain_adcs(const FscSideT<R>& s, double X, double Y, double Z, 
     const R y1b = y1 - s.y1B, y2b = y2 - s.y2B;
     const R z3A = s.c * qA - s.s * y1, z3B = s.c * qB - s.s * y1b;
     const R f = z3A + z3B >= R(0.0) ? R(1.0) : R(-1.0);
+    const R z1 = s.c * y1 + s.s * qA;
     FscAcc<R> v;
-    fsc_end<true>(s, y1, y2, s.aA, z, f, s.c * y1 + s.s * qA, z3A, v);
+    fsc_end<true>(s, y1, y2, s.aA, z, f, z1, z3A, v);
     fsc_end<false>(s, y1b, y2b, s.aB, z, f, s.c * y1b + s.s * qB, z3B, v);
-    fsc_rows(s.ks, v, z, e);
+    if (FULL && s.skip != R(0)) {
+#pragma unroll
+        for (int k = 0; k < 18; ++k) e[k / 6][k % 6] = R(0.0);
+    } else {
+        fsc_rows(s.ks, v, z, e);
+    }
+    if (FULL) {
+        const R k1 = R(1.0) - s.nu, K8 = R(0.5);   // 1 / (4 pi) and 1 / (8 pi (1 - nu)) over K4
+        SegInt<R> g;
+        g.K = -f * v.u;
+        g.I = -f * v.v;
+        g.T = v.h0;
+        g.Q = v.c3;
+        g.V = R(0.0);
+        add_segment_adcs(seg_strain(g, z1, y2, k1, K8), s.c, s.s, R(-1.0), e);
+        const R pA = z - s.aA, pB = z - s.aB;   // vertical offsets from the real ends
+        const R x = s.c * y1 - s.s * pA;
+        const R rA2 = fmax(y1 * y1 + y2 * y2 + pA * pA, tiny_square<R>());   // finite at a vertex too
+        const R rB2 = fmax(y1b * y1b + y2b * y2b + pB * pB, tiny_square<R>());
+        const R iA = cad_rsqrt(rA2), iB = cad_rsqrt(rB2);
+        const SegInt<R> h = seg_integrals<false>(rA2 * iA, iA, rB2 * iB, iB, -(s.s * y1 + s.c * pA),
+                                                 -(s.s * y1b + s.c * pB), x * x + y2 * y2);
+        add_segment_adcs(seg_strain(h, x, y2, k1, K8), s.c, -s.s, R(1.0), e);
+    }
 }
 
 // Tensor in ADCS -> EFCS (a rotation about the vertical axis).
@@ -618,12 +717,26 @@ CAD_HD void adcs_to_efcs(R t[6], R a, R b)
     t[5] = a * t23 - b * t13;
 }
 
+// Strain (EFCS) at the point of side s carrying the slip of its mode 0, the
+// real and image segments included, added into E.
+template <typename R>
+CAD_HD void side_strain_sum(const FscSideT<R>& s, double X, double Y, double Z, R E[6])
+{
+    R e[3][6], T[6];
+    side_strain_adcs<true>(s, X, Y, Z, e);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) T[k] = s.cs[0][0] * e[0][k] + s.cs[0][1] * e[1][k] + s.cs[0][2] * e[2][k];
+    adcs_to_efcs(T, s.ea, s.eb);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) E[k] += T[k];
+}
+
 // One side's harmonic correction to the strain, added into E (EFCS).
 template <typename R>
 CAD_HD void fsc_strain(const FscSideT<R>& s, double X, double Y, double Z, R Dss, R Dds, R Dn, R E[3][6])
 {
     R e[3][6];
-    fsc_strain_adcs(s, X, Y, Z, e);
+    side_strain_adcs<false>(s, X, Y, Z, e);
     const R slip[3] = {Dn, Dss, Dds};
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
@@ -642,11 +755,11 @@ CAD_HD void fsc_strain(const FscSideT<R>& s, double X, double Y, double Z, R Dss
 // by two triangles is traversed in opposite directions, and the reversed
 // side's map is the negative of this one (the two dislocation segments
 // cancel), so one evaluation per mesh edge serves both triangles.
-template <typename R>
-CAD_HD void fsc_strain_map(const FscSideT<R>& s, double X, double Y, double Z, R G[3][6])
+template <bool FULL, typename R>
+CAD_HD void side_strain_map(const FscSideT<R>& s, double X, double Y, double Z, R G[3][6])
 {
     R e[3][6];
-    fsc_strain_adcs(s, X, Y, Z, e);
+    side_strain_adcs<FULL>(s, X, Y, Z, e);
     const R ca = s.K4 * s.ea, cb = s.K4 * s.eb;
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
@@ -658,10 +771,48 @@ CAD_HD void fsc_strain_map(const FscSideT<R>& s, double X, double Y, double Z, R
     for (int j = 0; j < 3; ++j) adcs_to_efcs(G[j], s.ea, s.eb);
 }
 
+template <typename R>
+CAD_HD void fsc_strain_map(const FscSideT<R>& s, double X, double Y, double Z, R G[3][6])
+{
+    side_strain_map<false>(s, X, Y, Z, G);
+}
+
+// The whole half-space map of a side as tractions: W[j][r] = traction r
+// (normal, strike, dip) on an element with axes n, ss, ds for a unit Burgers
+// vector along EFCS axis j.  The element's axes are turned into ADCS, where
+// each traction is one weighted sum of the six strains.
+template <typename R>
+CAD_HD void side_traction_map(const FscSideT<R>& s, double X, double Y, double Z, R lam, R G2, const R n[3],
+                              const R ss[3], const R ds[3], R W[3][3])
+{
+    R e[3][6];
+    side_strain_adcs<true>(s, X, Y, Z, e);
+    const R g = s.K4 * G2, l = s.K4 * lam;
+    const R n1 = s.ea * n[0] + s.eb * n[1], n2 = s.eb * n[0] - s.ea * n[1], n3 = -n[2];
+    R t[3][3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const R* d = r == 0 ? n : r == 1 ? ss : ds;
+        const R d1 = s.ea * d[0] + s.eb * d[1], d2 = s.eb * d[0] - s.ea * d[1], d3 = -d[2];
+        const R li = r == 0 ? l * (n1 * n1 + n2 * n2 + n3 * n3) : R(0.0);
+        const R p0 = g * n1 * d1 + li, p1 = g * n2 * d2 + li, p2 = g * n3 * d3 + li;
+        const R p3 = g * (n1 * d2 + n2 * d1), p4 = g * (n1 * d3 + n3 * d1), p5 = g * (n2 * d3 + n3 * d2);
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            t[j][r] = p0 * e[j][0] + p1 * e[j][1] + p2 * e[j][2] + p3 * e[j][3] + p4 * e[j][4] + p5 * e[j][5];
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        W[0][r] = s.ea * t[0][r] + s.eb * t[1][r];
+        W[1][r] = s.eb * t[0][r] - s.ea * t[1][r];
+        W[2][r] = -t[2][r];
+    }
+}
+
 // E[m] += sign * (the map G applied to the EFCS Burgers vector of unit mode m
 // of the triangle with frame `real`), for the modes with non-zero slip.
 template <typename R>
-CAD_HD void fsc_apply_map(const R G[3][6], R sign, const FrameT<R>& real, R Dss, R Dds, R Dn, R E[3][6])
+CAD_HD void fsc_apply_map(const R (*G)[6], R sign, const FrameT<R>& real, R Dss, R Dds, R Dn, R E[3][6])
 {
     const R slip[3] = {Dn, Dss, Dds};
     const R* axes[3] = {real.Vn, real.Vs, real.Vd};
@@ -879,10 +1030,9 @@ CAD_HD void build_side_geom(const double PA[3], const double PB[3], double nu, F
     const double beta = acos(-S[2] / Sv);
     s.skip = ((fabs(beta) < DBL_EPSILON) || (fabs(M_PI - beta) < DBL_EPSILON) || (fabs(1.0 / tan(beta)) > 5e3)) ? 1.0 : 0.0;
     for (int i = 0; i < 3; ++i) { s.PA[i] = PA[i]; s.PAlo[i] = 0.0; }
-    if (s.skip != 0.0) return;
     const double n1 = norm3_rn(S[0], S[1], 0.0);
-    s.ea = S[0] / n1;
-    s.eb = S[1] / n1;
+    s.ea = n1 > 0.0 ? S[0] / n1 : 1.0;
+    s.eb = n1 > 0.0 ? S[1] / n1 : 0.0;
     s.y1B = add_rn(mul_rn(s.ea, S[0]), mul_rn(s.eb, S[1]));
     s.y2B = sub_rn(mul_rn(s.eb, S[0]), mul_rn(s.ea, S[1]));
     s.aA = -PA[2];
@@ -890,6 +1040,10 @@ CAD_HD void build_side_geom(const double PA[3], const double PB[3], double nu, F
     s.s = n1 / Sv;
     s.c = -S[2] / Sv;
     s.nu = nu;
+    s.K4 = 1.0 / (4.0 * M_PI * sub_rn(1.0, nu));
+    s.B1 = s.cM = 0.0;
+    s.ct2 = s.tn2 = 1.0;
+    if (s.skip != 0.0) return;
     const double N1 = sub_rn(1.0, mul_rn(2.0, nu));
     s.B1 = N1 * s.c / s.s;
     s.cM = -0.5 * s.B1;
@@ -899,7 +1053,6 @@ CAD_HD void build_side_geom(const double PA[3], const double PB[3], double nu, F
         s.ct2 = s.s / (1.0 - s.c);
         s.tn2 = (1.0 - s.c) / s.s;
     }
-    s.K4 = 1.0 / (4.0 * M_PI * sub_rn(1.0, nu));
     fsc_rows_setup(s.s, s.c, nu, s.ks);
     fsc_rows_setup(s.s, s.c, nu, s.kd);
 }
@@ -916,7 +1069,6 @@ CAD_HD void build_side(const double PA[3], const double PB[3], const Frame& real
                        double Dn, double nu, FscSide& s)
 {
     build_side_geom(PA, PB, nu, s);
-    if (s.skip != 0.0) return;
     // unit-mode slip vectors: TDCS (n, s, d) -> EFCS -> ADCS
     const double slip[3] = {Dn, Dss, Dds};
     const double* axes[3] = {real.Vn, real.Vs, real.Vd};
@@ -933,11 +1085,24 @@ CAD_HD void build_side(const double PA[3], const double PB[3], const Frame& real
 CAD_HD void build_side_burgers(const double PA[3], const double PB[3], const double B[3], double nu, FscSide& s)
 {
     build_side_geom(PA, PB, nu, s);
-    if (s.skip != 0.0) return;
     side_slip(s, B, s.cs[0]);
 }
 
 // ------------------------------------------------------------ pair drivers
+// Whether the point lies on a side or a vertex of the triangle or of its
+// mirror image, in its plane (the pair is NaN there).
+CAD_HD bool on_side_or_vertex(const Frame& f, double X, double Y, double Z)
+{
+    double x, y, z;
+    to_tdcs(f, X, Y, Z, x, y, z);
+    if (x != 0.0) return false;
+    return on_side(f, x, y, z) || (y == 0.0 && z == 0.0) || (y == f.p1y && z == f.p1z) || (y == f.p3y && z == f.p3z);
+}
+CAD_HD bool pair_on_side(const TriDev& t, double X, double Y, double Z)
+{
+    return on_side_or_vertex(t.real, X, Y, Z) || on_side_or_vertex(t.image, X, Y, Z);
+}
+
 template <bool HS, typename R>
 CAD_HD void pair_strain(const TriDevT<R>& t, double X, double Y, double Z, R E[3][6])
 {
@@ -954,10 +1119,28 @@ CAD_HD void pair_strain(const TriDevT<R>& t, double X, double Y, double Z, R E[3
     }
 }
 
-// Half-space strain with the free-surface corrections of the triangle's sides
-// read from per-edge maps (fsc_strain_map): entry (edge e, value q) of this
-// observation point at G[e * ge + q * gq]; code[sd] = +-(e + 1) for side sd
-// traversed along / against edge e's direction, 0 for no correction.
+// Sum of the three sides' maps of this triangle at a point, signed by the
+// sides' directions: entry (edge e, value q) at G[e * ge + q * gq]; code[sd] =
+// +-(e + 1) for side sd traversed along / against edge e's direction, 0 for
+// none.
+template <int Q>
+CAD_HD void sum_side_maps(const double* G, int64_t gq, int64_t ge, const int* code, double S[Q])
+{
+#pragma unroll
+    for (int q = 0; q < Q; ++q) S[q] = 0.0;
+#pragma unroll
+    for (int sd = 0; sd < 3; ++sd) {
+        const int c = code[sd];
+        if (c == 0) continue;
+        const double* g = G + ((int64_t)(c > 0 ? c : -c) - 1) * ge;
+        const double sg = c > 0 ? 1.0 : -1.0;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) S[q] += sg * g[q * gq];
+    }
+}
+
+// Half-space strain with the sides' corrections read from per-edge maps
+// (fsc_strain_map), real and image full-space terms evaluated here.
 CAD_HD void pair_strain_edges(const TriDev& t, double X, double Y, double Z, const double* G, int64_t gq, int64_t ge,
                               const int* code, double E[3][6])
 {
@@ -966,17 +1149,24 @@ CAD_HD void pair_strain_edges(const TriDev& t, double X, double Y, double Z, con
 #pragma unroll
         for (int k = 0; k < 6; ++k) E[m][k] = 0.0;
     strain_fs<false>(t.real, X, Y, Z, t.Dss, t.Dds, t.Dn, t.K8, E);
-#pragma unroll 1
-    for (int sd = 0; sd < 3; ++sd) {
-        const int c = code[sd];
-        if (c == 0) continue;
-        const int64_t e = (int64_t)(c > 0 ? c : -c) - 1;
-        double Gm[3][6];
-#pragma unroll
-        for (int q = 0; q < 18; ++q) Gm[q / 6][q % 6] = G[e * ge + q * gq];
-        fsc_apply_map(Gm, c > 0 ? 1.0 : -1.0, t.real, t.Dss, t.Dds, t.Dn, E);
-    }
+    double S[18];
+    sum_side_maps<18>(G, gq, ge, code, S);
+    fsc_apply_map((double(*)[6])S, 1.0, t.real, t.Dss, t.Dds, t.Dn, E);
     strain_fs<true>(t.image, X, Y, Z, t.Dss, t.Dds, t.Dn, t.K8, E);
+}
+
+// Half-space strain from maps that hold all of it (side_strain_map<true>).
+CAD_HD void pair_strain_full(const TriDev& t, double X, double Y, double Z, const double* G, int64_t gq, int64_t ge,
+                             const int* code, double E[3][6])
+{
+    double S[18];
+    sum_side_maps<18>(G, gq, ge, code, S);
+    const bool nan = pair_on_side(t, X, Y, Z);
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+#pragma unroll
+        for (int k = 0; k < 6; ++k) E[m][k] = nan ? qnan<double>() : 0.0;
+    fsc_apply_map((double(*)[6])S, 1.0, t.real, t.Dss, t.Dds, t.Dn, E);
 }
 
 // Half-space strain and displacement without the free-surface corrections

@@ -45,20 +45,33 @@ __global__ void td_setup_kernel(const double* __restrict__ P1, const double* __r
 // ------------------------------------------------ half-space argument check
 // flag |= 1 when any vertex or observation z > 0 (src/TD.jl:606-619).
 // With nz set, the observation z is Z - 1e-12 nz (collocation points from
-// midpoints and normals, as SetupCollationPoints forms them).
+// midpoints and normals, as SetupCollationPoints forms them).  horizontal (may
+// be null) |= 1 when a triangle is exactly horizontal.
 __global__ void hs_check_kernel(const double* __restrict__ Z, const double* __restrict__ nz, int64_t M,
                                 const double* __restrict__ P1, const double* __restrict__ P2,
-                                const double* __restrict__ P3, int64_t N, int* __restrict__ flag)
+                                const double* __restrict__ P3, int64_t N, int* __restrict__ flag,
+                                int* __restrict__ horizontal)
 {
-    int bad = 0;
+    int bad = 0, level = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < M + N; i += (int64_t)gridDim.x * blockDim.x) {
         if (i < M) bad |= (nz ? Z[i] - nz[i] * 1e-12 : Z[i]) > 0.0;
         else {
             const int64_t j = i - M;
             bad |= (P1[j + 2 * N] > 0.0) | (P2[j + 2 * N] > 0.0) | (P3[j + 2 * N] > 0.0);
+            if (horizontal) {   // the normal exactly vertical, as build_frame forms it
+                double a[3], b[3], n[3];
+                for (int c = 0; c < 3; ++c) {
+                    a[c] = sub_rn(P2[j + c * N], P1[j + c * N]);
+                    b[c] = sub_rn(P3[j + c * N], P1[j + c * N]);
+                }
+                cross3_rn(a, b, n);
+                const double nn = norm3_rn(n[0], n[1], n[2]);
+                level |= n[0] / nn == 0.0 && n[1] / nn == 0.0;
+            }
         }
     }
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(flag, 1);
+    if (horizontal && __syncthreads_or(level) && threadIdx.x == 0) atomicOr(horizontal, 1);
 }
 
 // ---------------------------------------------------- collocation points
@@ -115,6 +128,12 @@ __device__ __forceinline__ void strain_to_traction(const R e[6], R lam, R G2, co
 }
 
 // ------------------------------------------------------------- pair kernel
+enum EdgeKind { EDGE_NONE = 0, EDGE_FSC = 1, EDGE_FULL = 2 };
+// record values a pair kernel stages per triangle, and triangles staged between
+// two barriers (the small records 8 at a time)
+__host__ __device__ constexpr int pair_words(bool hs, int edge) { return hs ? (edge ? kTriWordsImg : kTriWordsHS) : kTriWordsFS; }
+__host__ __device__ constexpr int pair_stage(bool hs, int edge, bool one) { return one || (hs && !edge) ? 1 : 8; }
+
 // NEAR: rewrite only the triangles whose centroid lies within the near
 // radius of some point of the block (the FP64 pass of the mixed assembly).
 // LIST (OUT_AMAT only): incremental re-assembly through a.tri_list /
@@ -122,24 +141,30 @@ __device__ __forceinline__ void strain_to_traction(const R e[6], R lam, R G2, co
 // MINB > 1: compiled for MINB resident blocks per SM (fewer registers per
 // thread, more warps to hide the FP64 latency, some spilling) -- a launch
 // shape the autotuner may pick for the half-space system matrix.
-// EDGE (half space): the free-surface corrections are left to per-edge work;
-// the staged record is the two frames only.  OUT_AMAT, OUT_TRAC (strain) and
-// OUT_INF: they come from the per-edge maps a.fscG (fsc_edge_kernel).
-// OUT_SUM: they are left out here, and fsc_sum_kernel adds each edge's once.
+// EDGE (half space): the staged record is the two frames only.
+//   EDGE_FSC: the free-surface corrections are left to per-edge work.
+//   OUT_AMAT, OUT_TRAC (strain) and OUT_INF: they come from the per-edge maps
+//   a.fscG (side_map_kernel).  OUT_SUM: they are left out here, and
+//   side_sum_kernel adds each edge's once.
+//   EDGE_FULL: so is the whole strain (real, image and correction), which
+//   depends on the triangles' sides alone; the pair only combines its three
+//   sides' maps (tractions already for OUT_AMAT and OUT_TRAC), or, in
+//   OUT_SUM, marks the points that lie on a side.
 template <bool HS, bool STRAIN, bool DISP, int OUT, bool NEAR = false, bool LIST = false, int MINB = 1,
-          bool EDGE = false>
+          int EDGE = EDGE_NONE>
 __global__ void __launch_bounds__(kPairThreads, MINB) td_pair_kernel(PairArgs a)
 {
-    static_assert(!EDGE || (HS && !LIST && !NEAR &&
+    static_assert(EDGE == EDGE_NONE || (HS && !LIST && !NEAR &&
                             (((OUT == OUT_AMAT || OUT == OUT_TRAC) && STRAIN && !DISP) || OUT == OUT_SUM ||
                              OUT == OUT_INF)),
                   "shared edges: HS system matrix, traction or influence fields, or sums only");
-    constexpr bool EDGE_MAPS = EDGE && OUT != OUT_SUM;
-    // values per (edge, point) in the maps: strain 18, then displacement 9
-    constexpr int64_t kQ = (STRAIN ? 18 : 0) + (DISP ? 9 : 0);
+    constexpr bool EDGE_MAPS = EDGE != EDGE_NONE && OUT != OUT_SUM;
+    constexpr bool EDGE_TRAC = EDGE == EDGE_FULL && (OUT == OUT_AMAT || OUT == OUT_TRAC);
+    // values per (edge, point) in the maps: strain 18 (tractions 9), then displacement 9
+    constexpr int64_t kQ = EDGE_TRAC ? 9 : (STRAIN ? 18 : 0) + (DISP ? 9 : 0);
     extern __shared__ double smem[];
-    constexpr int words = HS ? (EDGE ? kTriWordsImg : kTriWordsHS) : kTriWordsFS;
-    const TriDev& t = *reinterpret_cast<const TriDev*>(smem);
+    constexpr int words = pair_words(HS, EDGE);
+    constexpr int stage = pair_stage(HS, EDGE, NEAR || LIST);
     const int64_t i = (int64_t)blockIdx.x * kPairThreads + threadIdx.x;
     const bool active = i < a.M;
     // LIST: this thread's point (system row) and the full system's size
@@ -165,6 +190,7 @@ __global__ void __launch_bounds__(kPairThreads, MINB) td_pair_kernel(PairArgs a)
     }
     const double near_r2 = NEAR ? a.near[3 * a.N] : 0.0;
     for (int64_t j = j0; j < j1; ++j) {
+        const int slot = (int)(j - j0) % stage;
         if (NEAR) {
             bool nr = false;
             if (active) {
@@ -172,19 +198,47 @@ __global__ void __launch_bounds__(kPairThreads, MINB) td_pair_kernel(PairArgs a)
                 nr = dx * dx + dy * dy + dz * dz < near_r2;
             }
             if (!__syncthreads_or(nr)) continue;   // also the barrier before restaging
-        } else {
+        } else if (slot == 0) {
             __syncthreads();
         }
         const int64_t jt = (LIST && a.tri_list) ? (int64_t)a.tri_list[j] : j;   // system column
-        const double* src = reinterpret_cast<const double*>(a.tri + jt);
-        for (int w = threadIdx.x; w < words; w += kPairThreads) smem[w] = src[w];
-        __syncthreads();
+        if (slot == 0) {   // the next records (`stage` of them, but for lists one) into shared memory
+            const int n = (int)min((int64_t)stage, j1 - j);
+            for (int k = 0; k < n; ++k) {
+                const double* src = reinterpret_cast<const double*>(a.tri + jt + k);
+                for (int w = threadIdx.x; w < words; w += kPairThreads) smem[k * words + w] = src[w];
+            }
+            __syncthreads();
+        }
         if (!active) continue;
-        if (STRAIN) {
+        const TriDev& t = *reinterpret_cast<const TriDev*>(smem + slot * words);
+        if constexpr (EDGE_TRAC) {
+            double S[9];
+            sum_side_maps<9>(a.fscG + i, a.M, 9 * a.M, a.side_edge + 3 * jt, S);
+            const bool nan = pair_on_side(t, X, Y, Z);
+            const double* axes[3] = {t.real.Vn, t.real.Vs, t.real.Vd};
+            const double slip[3] = {t.Dn, t.Dss, t.Dds};
+#pragma unroll
+            for (int m = 0; m < 3; ++m)
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    double tr = slip[m] * (axes[m][0] * S[r] + axes[m][1] * S[3 + r] + axes[m][2] * S[6 + r]);
+                    if (nan) tr = qnan<double>();
+                    if (OUT == OUT_TRAC) a.trac[(3 * m + r) * MN + i + MR * j] = tr;
+                    else a.A[(int64_t)(r * MD + io) + a.lda * (int64_t)(m * NS + jt)] = -tr;
+                }
+            continue;
+        }
+        if constexpr (EDGE == EDGE_FULL && OUT == OUT_SUM && STRAIN) {
+            if (pair_on_side(t, X, Y, Z))
+                for (int k = 0; k < 6; ++k) sumE[k] = qnan<double>();
+        } else if (STRAIN) {
             double E[3][6];
-            if constexpr (EDGE_MAPS)
+            if constexpr (EDGE_MAPS && EDGE == EDGE_FULL)
+                pair_strain_full(t, X, Y, Z, a.fscG + i, a.M, kQ * a.M, a.side_edge + 3 * jt, E);
+            else if constexpr (EDGE_MAPS)
                 pair_strain_edges(t, X, Y, Z, a.fscG + i, a.M, kQ * a.M, a.side_edge + 3 * jt, E);
-            else if constexpr (EDGE)
+            else if constexpr (EDGE != EDGE_NONE)
                 pair_strain_fs_image(t, X, Y, Z, E);
             else
                 pair_strain<HS>(t, X, Y, Z, E);
@@ -217,7 +271,7 @@ __global__ void __launch_bounds__(kPairThreads, MINB) td_pair_kernel(PairArgs a)
             if constexpr (EDGE_MAPS)
                 pair_disp_edges(t, X, Y, Z, a.fscG + i + (STRAIN ? 18 : 0) * a.M, a.M, kQ * a.M, a.side_edge + 3 * jt,
                                 U);
-            else if constexpr (EDGE)
+            else if constexpr (EDGE != EDGE_NONE)
                 pair_disp_fs_image(t, X, Y, Z, U);
             else
                 pair_disp<HS>(t, X, Y, Z, U);
@@ -429,7 +483,7 @@ __global__ void __launch_bounds__(kPairThreads) td_pair_f32_kernel(PairArgs a)
 template <bool HS, bool STRAIN, bool DISP, int OUT, int MINB = 1>
 static cudaError_t launch_pair(const PairArgs& a, cudaStream_t st)
 {
-    const size_t smem = (HS ? kTriWordsHS : kTriWordsFS) * sizeof(double);
+    const size_t smem = (size_t)pair_words(HS, EDGE_NONE) * pair_stage(HS, EDGE_NONE, false) * sizeof(double);
     auto kern = td_pair_kernel<HS, STRAIN, DISP, OUT, false, false, MINB>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -484,63 +538,94 @@ __global__ void edge_setup_kernel(const double* __restrict__ pts, int64_t E, dou
     build_side_geom(PA, PB, nu, out[e]);
 }
 
-// G[(e * Q + q) M + i] = value q of edge e's free-surface maps at point i:
-// the strain map (fsc_strain_map, 18 values) when STRAIN, then the
-// displacement map (fsc_disp_map, 9) when DISP; zero for an edge the beta test
-// drops.  Block = 128 points x a chunk of edges, each edge record staged in
-// shared memory.
-template <bool STRAIN, bool DISP>
-__global__ void __launch_bounds__(kPairThreads, 1) fsc_edge_kernel(const FscSide* __restrict__ edges, int64_t E,
-                                                                 int64_t echunk, const double* __restrict__ X,
-                                                                 const double* __restrict__ Y,
-                                                                 const double* __restrict__ Z, int64_t M,
-                                                                 double* __restrict__ G)
+// G[(e * Q + q) M + i] = value q of edge e's maps at point i: the strain map
+// (18 values, KIND EDGE_FSC the free-surface correction, EDGE_FULL the whole
+// strain) or, TRAC, the whole strain as tractions on the point's element (9),
+// then the correction's displacement map (9) when DISP.  Block = 128 points x
+// a chunk of edges, 8 edge records staged in shared memory at a time.
+constexpr int kEdgeStage = 8;
+struct SideMapArgs {
+    const FscSide* edges;
+    int64_t E, echunk;
+    const double *X, *Y, *Z;
+    int64_t M;
+    double* G;
+    const double* dirs;   // TRAC: the points' element axes (row stride dirs_ld), elastic constants
+    int64_t dirs_ld;
+    double lambda, G2;
+};
+// The whole strain is built for three resident blocks per SM.
+template <int KIND, bool DISP, bool TRAC>
+__global__ void __launch_bounds__(kPairThreads, KIND == EDGE_FULL && !DISP ? 3 : 1) side_map_kernel(const SideMapArgs a)
 {
     extern __shared__ double smem[];
-    const FscSide& s = *reinterpret_cast<const FscSide*>(smem);
     const int64_t i = (int64_t)blockIdx.x * kPairThreads + threadIdx.x;
-    const bool active = i < M;
+    const bool active = i < a.M;
+    const int64_t M = a.M;
+    double* __restrict__ G = a.G + i;
     double x = 0.0, y = 0.0, z = 0.0;
-    if (active) { x = X[i]; y = Y[i]; z = Z[i]; }
-    const int64_t e0 = (int64_t)blockIdx.y * echunk;
-    const int64_t e1 = min(E, e0 + echunk);
-    for (int64_t e = e0; e < e1; ++e) {
+    double n[3] = {0, 0, 0}, ss[3] = {0, 0, 0}, ds[3] = {0, 0, 0};
+    if (active) {
+        x = a.X[i];
+        y = a.Y[i];
+        z = a.Z[i];
+        if (TRAC)
+            for (int k = 0; k < 3; ++k) {
+                n[k] = a.dirs[i + k * a.dirs_ld];
+                ss[k] = a.dirs[i + (3 + k) * a.dirs_ld];
+                ds[k] = a.dirs[i + (6 + k) * a.dirs_ld];
+            }
+    }
+    const int64_t e0 = (int64_t)blockIdx.y * a.echunk;
+    const int64_t e1 = min(a.E, e0 + a.echunk);
+    constexpr int64_t Q = (TRAC ? 9 : KIND != EDGE_NONE ? 18 : 0) + (DISP ? 9 : 0);
+    for (int64_t eb = e0; eb < e1; eb += kEdgeStage) {
+        const int ne = (int)min((int64_t)kEdgeStage, e1 - eb);
         __syncthreads();
-        const double* src = reinterpret_cast<const double*>(edges + e);
-        for (int w = threadIdx.x; w < kSideWords; w += kPairThreads) smem[w] = src[w];
+        const double* src = reinterpret_cast<const double*>(a.edges + eb);
+        for (int w = threadIdx.x; w < ne * kSideWords; w += kPairThreads) smem[w] = src[w];
         __syncthreads();
         if (!active) continue;
-        constexpr int64_t Q = (STRAIN ? 18 : 0) + (DISP ? 9 : 0);
-        if (STRAIN) {
-            double Gm[3][6];
-            if (s.skip != 0.0) {
+#pragma unroll 1
+        for (int k = 0; k < ne; ++k) {
+            const FscSide& s = reinterpret_cast<const FscSide*>(smem)[k];
+            const int64_t e = eb + k;
+            if constexpr (TRAC) {
+                double W[3][3];
+                side_traction_map(s, x, y, z, a.lambda, a.G2, n, ss, ds, W);
 #pragma unroll
-                for (int q = 0; q < 18; ++q) Gm[q / 6][q % 6] = 0.0;
-            } else {
-                fsc_strain_map(s, x, y, z, Gm);
+                for (int q = 0; q < 9; ++q) G[(e * Q + q) * M] = W[q / 3][q % 3];
+            } else if (KIND != EDGE_NONE) {
+                double Gm[3][6];
+                if (KIND == EDGE_FSC && s.skip != 0.0) {
+#pragma unroll
+                    for (int q = 0; q < 18; ++q) Gm[q / 6][q % 6] = 0.0;
+                } else {
+                    side_strain_map<KIND == EDGE_FULL>(s, x, y, z, Gm);
+                }
+#pragma unroll
+                for (int q = 0; q < 18; ++q) G[(e * Q + q) * M] = Gm[q / 6][q % 6];
             }
+            if (DISP) {
+                double Gu[3][3];
+                if (s.skip != 0.0) {
 #pragma unroll
-            for (int q = 0; q < 18; ++q) G[(e * Q + q) * M + i] = Gm[q / 6][q % 6];
-        }
-        if (DISP) {
-            double Gu[3][3];
-            if (s.skip != 0.0) {
+                    for (int q = 0; q < 9; ++q) Gu[q / 3][q % 3] = 0.0;
+                } else {
+                    fsc_disp_map(s, x, y, z, Gu);
+                }
+                constexpr int64_t q0 = Q - 9;
 #pragma unroll
-                for (int q = 0; q < 9; ++q) Gu[q / 3][q % 3] = 0.0;
-            } else {
-                fsc_disp_map(s, x, y, z, Gu);
+                for (int q = 0; q < 9; ++q) G[(e * Q + q0 + q) * M] = Gu[q / 3][q % 3];
             }
-            constexpr int64_t q0 = STRAIN ? 18 : 0;
-#pragma unroll
-            for (int q = 0; q < 9; ++q) G[(e * Q + q0 + q) * M + i] = Gu[q / 3][q % 3];
         }
     }
 }
 
 size_t edge_record_bytes() { return sizeof(FscSide); }
 
-cudaError_t launch_assemble_edges(PairArgs a, int out_kind, bool strain, bool disp, const double* edge_pts,
-                                  int64_t E, const int* side_edge, void* edge_rec, double* G, int64_t Mc, double nu,
+cudaError_t launch_assemble_edges(PairArgs a, int out_kind, bool strain, bool disp, bool full,
+                                  const double* edge_pts, int64_t E, const int* side_edge, void* edge_rec, double* G, int64_t Mc, double nu,
                                   cudaStream_t st, int64_t* launches)
 {
     if (out_kind == OUT_AMAT || out_kind == OUT_TRAC) {
@@ -555,41 +640,44 @@ cudaError_t launch_assemble_edges(PairArgs a, int out_kind, bool strain, bool di
         if (launches) ++*launches;
         if (cudaError_t e = cudaGetLastError()) return e;
     }
-    // a.min_blocks 3: three resident blocks per SM (168 registers, 308 B of
-    // spills), 69.8 ms against 73.9 ms with the full register file (1) at
-    // 10 000 triangles (system matrix; the influence fields keep 1)
     using PairKernel = void (*)(PairArgs);
-    using EdgeKernel = void (*)(const FscSide*, int64_t, int64_t, const double*, const double*, const double*,
-                                int64_t, double*);
+    using MapKernel = void (*)(SideMapArgs);
     PairKernel pk;
-    EdgeKernel ek = fsc_edge_kernel<true, false>;
-    if (out_kind == OUT_TRAC) {
-        pk = a.min_blocks == 1 ? td_pair_kernel<true, true, false, OUT_TRAC, false, false, 1, true>
-                               : td_pair_kernel<true, true, false, OUT_TRAC, false, false, 3, true>;
-    } else if (out_kind == OUT_AMAT) {
-        pk = a.min_blocks == 1 ? td_pair_kernel<true, true, false, OUT_AMAT, false, false, 1, true>
-                               : td_pair_kernel<true, true, false, OUT_AMAT, false, false, 3, true>;
+    MapKernel ek;
+    const bool trac = out_kind != OUT_INF;
+    if (trac && full) {
+        pk = out_kind == OUT_TRAC ? td_pair_kernel<true, true, false, OUT_TRAC, false, false, 1, EDGE_FULL>
+                                  : td_pair_kernel<true, true, false, OUT_AMAT, false, false, 1, EDGE_FULL>;
+        ek = side_map_kernel<EDGE_FULL, false, true>;
+    } else if (trac) {
+        pk = out_kind == OUT_TRAC ? td_pair_kernel<true, true, false, OUT_TRAC, false, false, 1, EDGE_FSC>
+                                  : td_pair_kernel<true, true, false, OUT_AMAT, false, false, 1, EDGE_FSC>;
+        ek = side_map_kernel<EDGE_FSC, false, false>;
     } else if (strain && disp) {
-        pk = td_pair_kernel<true, true, true, OUT_INF, false, false, 1, true>;
-        ek = fsc_edge_kernel<true, true>;
+        pk = full ? td_pair_kernel<true, true, true, OUT_INF, false, false, 1, EDGE_FULL>
+                  : td_pair_kernel<true, true, true, OUT_INF, false, false, 1, EDGE_FSC>;
+        ek = full ? side_map_kernel<EDGE_FULL, true, false> : side_map_kernel<EDGE_FSC, true, false>;
     } else if (strain) {
-        pk = td_pair_kernel<true, true, false, OUT_INF, false, false, 1, true>;
+        pk = full ? td_pair_kernel<true, true, false, OUT_INF, false, false, 1, EDGE_FULL>
+                  : td_pair_kernel<true, true, false, OUT_INF, false, false, 1, EDGE_FSC>;
+        ek = full ? side_map_kernel<EDGE_FULL, false, false> : side_map_kernel<EDGE_FSC, false, false>;
     } else {
-        pk = td_pair_kernel<true, false, true, OUT_INF, false, false, 1, true>;
-        ek = fsc_edge_kernel<false, true>;
+        pk = td_pair_kernel<true, false, true, OUT_INF, false, false, 1, EDGE_FSC>;
+        ek = side_map_kernel<EDGE_NONE, true, false>;
     }
-    const size_t psmem = (size_t)kTriWordsImg * sizeof(double);
-    const size_t esmem = (size_t)kSideWords * sizeof(double);
+    const size_t psmem = (size_t)pair_words(true, EDGE_FSC) * pair_stage(true, EDGE_FSC, false) * sizeof(double);
+    const size_t esmem = (size_t)kSideWords * kEdgeStage * sizeof(double);
     cudaError_t e = cudaFuncSetAttribute(pk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(ek, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)esmem);
     if (e != cudaSuccess) return e;
-    const int64_t echunk = 32;
+    const int64_t echunk = a.min_blocks == 1 ? 96 : 32;
     for (int64_t c0 = 0; c0 < a.M; c0 += Mc) {
         const int64_t mc = a.M - c0 < Mc ? a.M - c0 : Mc;
         const unsigned tiles = (unsigned)((mc + kPairThreads - 1) / kPairThreads);
         if (E > 0) {
-            ek<<<dim3(tiles, (unsigned)((E + echunk - 1) / echunk)), kPairThreads, esmem, st>>>(
-                (const FscSide*)edge_rec, E, echunk, a.X + c0, a.Y + c0, a.Z + c0, mc, G);
+            const SideMapArgs m{(const FscSide*)edge_rec, E, echunk, a.X + c0, a.Y + c0, a.Z + c0, mc, G,
+                                a.dirs ? a.dirs + c0 : nullptr, a.M, a.lambda, 2.0 * a.G};
+            ek<<<dim3(tiles, (unsigned)((E + echunk - 1) / echunk)), kPairThreads, esmem, st>>>(m);
             if (launches) ++*launches;
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
@@ -647,18 +735,18 @@ __global__ void edge_burgers_kernel(const double* __restrict__ pts, int64_t E, c
     build_side_burgers(PA, PB, B, nu, out[e]);
 }
 
-// partial[(blockIdx.y * 9 + f) M + i] = the free-surface strain (f 0-5) and
+// partial[(blockIdx.y * 9 + f) M + i] = the strain (f 0-5; STRAIN EDGE_FSC: the
+// free-surface correction, EDGE_FULL: all of it) and the correction's
 // displacement (f 6-8) at point i of the edges of chunk blockIdx.y, summed in
-// edge order (each edge record staged in shared memory).
-template <bool STRAIN, bool DISP>
-__global__ void __launch_bounds__(kPairThreads, 1) fsc_sum_kernel(const FscSide* __restrict__ edges, int64_t E,
+// edge order (8 edge records staged in shared memory at a time).
+template <int STRAIN, bool DISP>
+__global__ void __launch_bounds__(kPairThreads) side_sum_kernel(const FscSide* __restrict__ edges, int64_t E,
                                                                 int64_t echunk, const double* __restrict__ X,
                                                                 const double* __restrict__ Y,
                                                                 const double* __restrict__ Z, int64_t M,
                                                                 double* __restrict__ partial)
 {
     extern __shared__ double smem[];
-    const FscSide& s = *reinterpret_cast<const FscSide*>(smem);
     const int64_t i = (int64_t)blockIdx.x * kPairThreads + threadIdx.x;
     const bool active = i < M;
     double x = 0.0, y = 0.0, z = 0.0;
@@ -666,14 +754,21 @@ __global__ void __launch_bounds__(kPairThreads, 1) fsc_sum_kernel(const FscSide*
     double Es[3][6] = {}, Us[3][3] = {};
     const int64_t e0 = (int64_t)blockIdx.y * echunk;
     const int64_t e1 = min(E, e0 + echunk);
-    for (int64_t e = e0; e < e1; ++e) {
+    for (int64_t eb = e0; eb < e1; eb += kEdgeStage) {
+        const int ne = (int)min((int64_t)kEdgeStage, e1 - eb);
         __syncthreads();
-        const double* src = reinterpret_cast<const double*>(edges + e);
-        for (int w = threadIdx.x; w < kSideWords; w += kPairThreads) smem[w] = src[w];
+        const double* src = reinterpret_cast<const double*>(edges + eb);
+        for (int w = threadIdx.x; w < ne * kSideWords; w += kPairThreads) smem[w] = src[w];
         __syncthreads();
-        if (!active || s.skip != 0.0) continue;
-        if (STRAIN) fsc_strain(s, x, y, z, 0.0, 0.0, 1.0, Es);
-        if (DISP) fsc_disp(s, x, y, z, 0.0, 0.0, 1.0, Us);
+        if (!active) continue;
+#pragma unroll 1
+        for (int k = 0; k < ne; ++k) {
+            const FscSide& s = reinterpret_cast<const FscSide*>(smem)[k];
+            if (STRAIN == EDGE_FULL) side_strain_sum(s, x, y, z, Es[0]);
+            if (s.skip != 0.0) continue;
+            if (STRAIN == EDGE_FSC) fsc_strain(s, x, y, z, 0.0, 0.0, 1.0, Es);
+            if (DISP) fsc_disp(s, x, y, z, 0.0, 0.0, 1.0, Us);
+        }
     }
     if (!active) return;
     double* p = partial + (int64_t)blockIdx.y * 9 * M;
@@ -683,12 +778,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) fsc_sum_kernel(const FscSide*
     for (int c = 0; c < 3; ++c) p[(6 + c) * M + i] = DISP ? Us[0][c] : 0.0;
 }
 
-cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, const EdgeArrays& ed, int64_t E, void* edge_rec,
-                                double nu, int64_t echunk, double* edge_partial, cudaStream_t st, int64_t* launches)
+cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, bool full, const EdgeArrays& ed, int64_t E,
+                                void* edge_rec, double nu, int64_t echunk, double* edge_partial, cudaStream_t st, int64_t* launches)
 {
     if (a.M == 0 || a.N == 0 || !(strain || disp)) return cudaSuccess;
-    const size_t psmem = (size_t)kTriWordsImg * sizeof(double);
-    const size_t esmem = (size_t)kSideWords * sizeof(double);
+    const size_t psmem = (size_t)pair_words(true, EDGE_FSC) * pair_stage(true, EDGE_FSC, false) * sizeof(double);
+    const size_t esmem = (size_t)kSideWords * kEdgeStage * sizeof(double);
     const unsigned tiles = (unsigned)((a.M + kPairThreads - 1) / kPairThreads);
     auto pairs = [&](auto kern) -> cudaError_t {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem);
@@ -705,17 +800,23 @@ cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, const EdgeAr
         if (launches) ++*launches;
         return cudaGetLastError();
     };
-    cudaError_t e = strain && disp ? pairs(td_pair_kernel<true, true, true, OUT_SUM, false, false, 1, true>)
-                    : strain       ? pairs(td_pair_kernel<true, true, false, OUT_SUM, false, false, 1, true>)
-                                   : pairs(td_pair_kernel<true, false, true, OUT_SUM, false, false, 1, true>);
+    cudaError_t e;
+    if (strain && disp)
+        e = full ? pairs(td_pair_kernel<true, true, true, OUT_SUM, false, false, 1, EDGE_FULL>)
+                 : pairs(td_pair_kernel<true, true, true, OUT_SUM, false, false, 1, EDGE_FSC>);
+    else if (strain)
+        e = full ? pairs(td_pair_kernel<true, true, false, OUT_SUM, false, false, 1, EDGE_FULL>)
+                 : pairs(td_pair_kernel<true, true, false, OUT_SUM, false, false, 1, EDGE_FSC>);
+    else
+        e = pairs(td_pair_kernel<true, false, true, OUT_SUM, false, false, 1, EDGE_FSC>);
     if (e != cudaSuccess || E == 0) return e;
     edge_burgers_kernel<<<(unsigned)((E + 63) / 64), 64, 0, st>>>(ed.pts, E, ed.ptr, ed.cnt, ed.sides, a.tri, nu,
                                                                    (FscSide*)edge_rec);
     if (launches) ++*launches;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    return strain && disp ? sums(fsc_sum_kernel<true, true>)
-           : strain       ? sums(fsc_sum_kernel<true, false>)
-                          : sums(fsc_sum_kernel<false, true>);
+    if (strain && disp) return full ? sums(side_sum_kernel<EDGE_FULL, true>) : sums(side_sum_kernel<EDGE_FSC, true>);
+    if (strain) return full ? sums(side_sum_kernel<EDGE_FULL, false>) : sums(side_sum_kernel<EDGE_FSC, false>);
+    return sums(side_sum_kernel<EDGE_NONE, true>);
 }
 
 cudaError_t launch_splice_fixed(const double* trac, const double* disp, int64_t N, int64_t nfix, const int* fixrow,
@@ -822,14 +923,14 @@ cudaError_t launch_td_setup(const double* P1, const double* P2, const double* P3
 }
 
 cudaError_t launch_hs_check(const double* Z, int64_t M, const double* P1, const double* P2, const double* P3,
-                            int64_t N, int* flag, cudaStream_t st, const double* nz, bool clear)
+                            int64_t N, int* flag, cudaStream_t st, const double* nz, bool clear, int* horizontal)
 {
     cudaError_t e = clear ? cudaMemsetAsync(flag, 0, sizeof(int), st) : cudaSuccess;
     if (e != cudaSuccess || M + N == 0) return e;
     const int bs = 256;
     int64_t nb = (M + N + bs - 1) / bs;
     if (nb > 1184) nb = 1184;
-    hs_check_kernel<<<(unsigned)nb, bs, 0, st>>>(Z, nz, M, P1, P2, P3, N, flag);
+    hs_check_kernel<<<(unsigned)nb, bs, 0, st>>>(Z, nz, M, P1, P2, P3, N, flag, horizontal);
     return cudaGetLastError();
 }
 

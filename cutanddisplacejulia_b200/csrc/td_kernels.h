@@ -13,7 +13,7 @@ struct TriDevT;
 using TriDev = TriDevT<double>;
 
 constexpr int kPairThreads = 128;
-constexpr int kEdgeMinBlocks = 3;   // default build of the shared-edge pair kernel
+constexpr int kEdgeMinBlocks = 3;   // default launch shape of the edge map kernel
 
 enum OutKind { OUT_INF = 0, OUT_SUM = 1, OUT_TRAC = 2, OUT_AMAT = 3 };
 
@@ -57,18 +57,27 @@ struct PairArgs {
 };
 
 // Half-space system matrix (out_kind OUT_AMAT), traction fields (OUT_TRAC) or
-// influence fields (OUT_INF, strain and / or displacement), FP64, with the
-// free-surface correction evaluated once per mesh edge at each point:
-// edge_pts holds E edges (PA, PB: 6 doubles each), side_edge each triangle's
-// three side codes; edge_rec (edge_record_bytes() x E) and G (Q x Mc x E
-// doubles, Q = 18 for strain + 9 for displacement) are workspaces; the points
-// are processed in blocks of Mc.  OUT_AMAT / OUT_TRAC: a.M == a.N (the
-// collocation points).  a.min_blocks selects the system-matrix and traction
-// kernels' build: 1 (the full register file) or anything else for three
-// resident blocks per SM (kEdgeMinBlocks).
-cudaError_t launch_assemble_edges(PairArgs a, int out_kind, bool strain, bool disp, const double* edge_pts,
-                                  int64_t E, const int* side_edge, void* edge_rec, double* G, int64_t Mc, double nu,
-                                  cudaStream_t st, int64_t* launches);
+// influence fields (OUT_INF, strain and / or displacement), FP64, from maps
+// evaluated once per mesh edge at each point: edge_pts holds E edges (PA, PB: 6
+// doubles each), side_edge each triangle's three side codes; edge_rec
+// (edge_record_bytes() x E) and G (edge_map_values() x Mc x E doubles) are
+// workspaces; the points are processed in blocks of Mc.  OUT_AMAT / OUT_TRAC:
+// a.M == a.N (the collocation points).
+// full: the maps hold the whole strain (as tractions for OUT_AMAT, OUT_TRAC);
+// otherwise the free-surface correction only, for meshes with an exactly
+// horizontal triangle, whose image dislocation the reference gives a Burgers
+// vector that is not the mirrored one (src/TD.jl:721-727 keeps the strike
+// axis of both), so that it is no sum over shared sides.  a.min_blocks: 1 takes
+// 96 edges per block of the map kernel (few long blocks per SM), anything else
+// (kEdgeMinBlocks) 32.
+cudaError_t launch_assemble_edges(PairArgs a, int out_kind, bool strain, bool disp, bool full,
+                                  const double* edge_pts, int64_t E, const int* side_edge, void* edge_rec, double* G,
+                                  int64_t Mc, double nu, cudaStream_t st, int64_t* launches);
+inline int64_t edge_map_values(int out_kind, bool strain, bool disp, bool full)
+{
+    if (out_kind != OUT_INF) return full ? 9 : 18;
+    return (strain ? 18 : 0) + (disp ? 9 : 0);
+}
 size_t edge_record_bytes();
 
 // Half-space sums (OUT_SUM) with the free-surface correction evaluated once
@@ -77,8 +86,8 @@ size_t edge_record_bytes();
 // launch_td_pairs), edge_partial the corrections of each chunk of echunk
 // edges (9 x a.M each).  ed: launch_edge_table's arrays with lists.  a.tri must
 // hold the records of launch_td_setup (with the triangles' slip).
-cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, const EdgeArrays& ed, int64_t E, void* edge_rec,
-                                double nu, int64_t echunk, double* edge_partial, cudaStream_t st, int64_t* launches);
+cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, bool full, const EdgeArrays& ed, int64_t E,
+                                void* edge_rec, double nu, int64_t echunk, double* edge_partial, cudaStream_t st, int64_t* launches);
 
 // Mixed-precision system matrix: every pair in FP32 (far field), then the
 // pairs of every 128-point tile that has a point within the near radius of
@@ -108,7 +117,8 @@ cudaError_t launch_td_pairs(const PairArgs& a, int out, bool hs, bool strain, bo
 // flag |= 1 when an observation z or a vertex z is above 0 (nz set: the
 // observation z is Z - 1e-12 nz); clear: zero the flag first.
 cudaError_t launch_hs_check(const double* Z, int64_t M, const double* P1, const double* P2, const double* P3,
-                            int64_t N, int* flag, cudaStream_t st, const double* nz = nullptr, bool clear = true);
+                            int64_t N, int* flag, cudaStream_t st, const double* nz = nullptr, bool clear = true,
+                            int* horizontal = nullptr);
 cudaError_t launch_colloc(const double* normals, const double* mid, int64_t N, double* X, double* Y, double* Z,
                           double* dirs, cudaStream_t st);
 cudaError_t launch_sum_chunks(const double* partial, int64_t nchunk, int64_t M, int fields_mask, double* out,

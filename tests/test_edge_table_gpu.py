@@ -62,3 +62,52 @@ def test_edge_with_many_triangles_repeats_and_negative_zero(cad):
     assert_parity(a[0], b[0])
     assert_parity(a[1], b[1])
     assert rel_inf_err(a[0], b[0]) < 1e-12
+
+
+def _meshes():
+    from cutanddisplacejulia_b200 import workloads
+    dip = workloads.dipping_rect(seed=3, ntri=240, top_depth=0.1)
+    sill = workloads.ellipse_crack(seed=4, ntri=200)
+    sill = tuple(p - [0.0, 0.0, 0.8] for p in sill)          # exactly horizontal
+    wall = workloads.dipping_rect(seed=5, ntri=200, dip=90.0, top_depth=0.3, jitter=0.0)   # vertical sides
+    both = tuple(np.concatenate([a, b - [0.0, 3.0, 0.0]]) for a, b in zip(dip, sill))
+    return {"dip": dip, "sill": sill, "wall": wall, "both": both}
+
+
+@pytest.mark.parametrize("name", ["dip", "sill", "wall", "both"])
+def test_fields_sums_and_tractions_over_meshes(cad, oracle, name):
+    from cutanddisplacejulia_b200 import _lib
+    P = _meshes()[name]
+    n = len(P[0])
+    rng = np.random.default_rng(7)
+    sl = rng.uniform(-1e-3, 1e-3, (3, n))
+    sl[1, ::5] = 0.0
+    pts = rng.uniform([-2, -4, -2.5], [2, 2, -0.01], (131, 3))
+    # points in a triangle's plane and on its sides (NaN there)
+    pts[:5] = [0.5 * (P[0][k] + P[1][k]) for k in range(5)]
+    pts[5:8] = [(P[0][k] + P[1][k] + P[2][k]) / 3 for k in range(3)]
+    pts[8] = P[0][4]
+    L, ctx = _lib.load(), _lib.context(0)
+    nrm, mid = cad.CreateFaceNormalAndMidPoint(*P)
+    _, _, lam, nu, G = cad.ElasticConstantsCheck(1.0, 0.25)
+    got = {}
+    for shared in (1, 0):
+        _lib.check(L.cad_set_shared_edges(ctx, shared), ctx)
+        try:
+            S, U = cad.TD(*pts.T, *P, *sl, nu, G, 1, 1, 1)
+            S1, _ = cad.TD(*pts.T, *P, *sl, nu, G, 0, 1, 1)
+            Ss, Us = cad.TD(*pts.T, *P, *sl, nu, G, 1, 1, 1, cad.Strains(), cad.Disps())
+            Sn, _ = cad.TD(*pts.T, *P, *sl, nu, G, 0, 1, 1, cad.Strains(), cad.Disps())
+            T = cad.CalculateInfluenceMatrices3D(nrm, mid, *P, nu, G, lam, None, 1, n)
+        finally:
+            _lib.check(L.cad_set_shared_edges(ctx, 1), ctx)
+        got[shared] = [np.stack(list(v)) for v in (S, U, S1, Ss, Us, Sn, T)]
+    for a, b in zip(got[1], got[0]):
+        # on a side the pair is NaN or, where rounding puts the point off the
+        # plane, singular: only the NaN masks agree there
+        k = 9 if a.shape[1] == len(pts) else 0
+        assert np.array_equal(np.isnan(a), np.isnan(b)) and np.isfinite(a[:, k:]).all()
+        assert_parity(a[:, k:], b[:, k:])
+    So, Uo = oracle.td_inf(*pts[9:].T, *P, *sl, nu, G, 1, 1, 1)
+    assert_parity(got[1][0][:, 9:], So)
+    assert_parity(got[1][1][:, 9:], Uo)
