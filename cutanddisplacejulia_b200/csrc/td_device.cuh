@@ -352,6 +352,20 @@ CAD_HD SegStrain<R> seg_strain(const SegInt<R>& g, R x, R e, R k1, R K8)
     return s;
 }
 
+// -Omega / (4 pi): the solid-angle part of the displacement (x the TDCS offset
+// from the plane, dy, dz from the three vertices, Rv the vertex distances).
+template <typename R>
+CAD_HD R solid_angle_term(R x, const R dy[3], const R dz[3], const R Rv[3])
+{
+    const R x2 = x * x;
+    const R one = -x * ((dy[1] - dy[0]) * (dz[2] - dz[0]) - (dz[1] - dz[0]) * (dy[2] - dy[0]));
+    const R ab = x2 + dy[0] * dy[1] + dz[0] * dz[1];
+    const R ac = x2 + dy[0] * dy[2] + dz[0] * dz[2];
+    const R bc = x2 + dy[1] * dy[2] + dz[1] * dz[2];
+    const R two = Rv[0] * Rv[1] * Rv[2] + ab * Rv[2] + ac * Rv[1] + bc * Rv[0];
+    return R(-2.0) * R(kInv4Pi) * cad_atan2(one, two);
+}
+
 // Strain of unit slip n, strike, dip (TDCS xx, yy, zz, xy, xz, yz) and the
 // displacement (its solid-angle part included) of frame f at TDCS (x, y, z).
 // K8 = 1 / (8 pi (1 - nu)).  In the segment's own axes (n = TD normal,
@@ -381,13 +395,7 @@ CAD_HD void td_unit(const FrameT<R>& f, R x, R y, R z, R K8, R E[3][6], R U[3][3
             for (int k = 0; k < 6; ++k) E[m][k] = R(0.0);
     }
     if (DISP) {
-        // solid angle of the triangle seen from the point
-        const R one = -x * ((dy[1] - dy[0]) * (dz[2] - dz[0]) - (dz[1] - dz[0]) * (dy[2] - dy[0]));
-        const R ab = x2 + dy[0] * dy[1] + dz[0] * dz[1];
-        const R ac = x2 + dy[0] * dy[2] + dz[0] * dz[2];
-        const R bc = x2 + dy[1] * dy[2] + dz[1] * dz[2];
-        const R two = Rv[0] * Rv[1] * Rv[2] + ab * Rv[2] + ac * Rv[1] + bc * Rv[0];
-        const R Fi = R(-2.0) * k1 * cad_atan2(one, two);
+        const R Fi = solid_angle_term(x, dy, dz, Rv);
 #pragma unroll
         for (int m = 0; m < 3; ++m)
 #pragma unroll
@@ -446,6 +454,74 @@ CAD_HD void td_unit(const FrameT<R>& f, R x, R y, R z, R K8, R E[3][6], R U[3][3
             U[2][1] -= ty * a1;
             U[2][2] -= ty * a2;
         }
+    }
+}
+
+// Strain (6) and displacement (3) at a point of frame f carrying the slip
+// (Dn, Dss, Dds) = b, added into E and U (EFCS): td_unit with the Burgers vector
+// contracted side by side, for sums over modes (6 strains instead of 18, one
+// rotation instead of three).
+template <bool STRAIN, bool DISP, typename R>
+CAD_HD void td_net(const FrameT<R>& f, double X, double Y, double Z, R bn, R bs, R bd, R K8, R E[6], R U[3])
+{
+    R x, y, z;
+    to_tdcs(f, X, Y, Z, x, y, z);
+    const bool nan = on_side(f, x, y, z);
+    const R k1 = R(kInv4Pi);
+    const R dy[3] = {y - f.p1y, y, y - f.p3y}, dz[3] = {z - f.p1z, z, z - f.p3z};
+    const R x2 = x * x;
+    R Rv[3], iR[3];
+#pragma unroll
+    for (int v = 0; v < 3; ++v) {
+        const R q = x2 + dy[v] * dy[v] + dz[v] * dz[v];
+        iR[v] = cad_rsqrt(q);
+        Rv[v] = q * iR[v];
+    }
+    R T[6] = {R(0.0), R(0.0), R(0.0), R(0.0), R(0.0), R(0.0)}, V[3] = {R(0.0), R(0.0), R(0.0)};
+    if (DISP) {
+        const R Fi = solid_angle_term(x, dy, dz, Rv);
+        V[0] = bn * Fi;
+        V[1] = bs * Fi;
+        V[2] = bd * Fi;
+    }
+#pragma unroll
+    for (int sd = 0; sd < 3; ++sd) {
+        const int A = sd, B = sd == 2 ? 0 : sd + 1;
+        const R ty = f.sy[sd], tz = f.sz[sd];
+        const R sA = -(dy[A] * ty + dz[A] * tz), sB = -(dy[B] * ty + dz[B] * tz);
+        const R e = dy[A] * tz - dz[A] * ty;
+        const SegInt<R> g = seg_integrals<DISP>(Rv[A], iR[A], Rv[B], iR[B], sA, sB, x2 + e * e);
+        const R bm = tz * bs - ty * bd, bt = ty * bs + tz * bd;
+        if (STRAIN) {
+            const SegStrain<R> q = seg_strain(g, x, e, k1, K8);
+            const R mm = bn * q.nmm + bm * q.mmm, tt = bn * q.ntt + bm * q.mtt;
+            const R nm = bn * q.nnm + bm * q.mnm, nt = bn * q.nnt + bm * q.mnt + bt * q.tnt;
+            const R mt = bn * q.nmt + bm * q.mmt + bt * q.tmt;
+            const R yy = ty * ty, zz = tz * tz, yz = ty * tz;
+            T[0] += bn * q.nnn + bm * q.mnn;
+            T[1] += mm * zz + tt * yy + R(2.0) * mt * yz;
+            T[2] += mm * yy + tt * zz - R(2.0) * mt * yz;
+            T[3] += nm * tz + nt * ty;
+            T[4] += nt * tz - nm * ty;
+            T[5] += (tt - mm) * yz + mt * (zz - yy);
+        }
+        if (DISP) {
+            const R cV = (k1 - K8) * g.V, w = K8 * (bn * e - bm * x);   // w grad V, and the V terms
+            const R um = -w * e * g.K - bn * cV, ut = w * g.T;
+            V[0] += bm * cV - w * x * g.K;
+            V[1] += um * tz + ut * ty;
+            V[2] += ut * tz - um * ty;
+        }
+    }
+    if (STRAIN) {
+        const R Rot[9] = {f.Vn[0], f.Vn[1], f.Vn[2], f.Vs[0], f.Vs[1], f.Vs[2], f.Vd[0], f.Vd[1], f.Vd[2]};
+        tensor_rot(T, Rot);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) E[k] += nan ? qnan<R>() : T[k];
+    }
+    if (DISP) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) U[c] += nan ? qnan<R>() : f.Vn[c] * V[0] + f.Vs[c] * V[1] + f.Vd[c] * V[2];
     }
 }
 
@@ -544,6 +620,13 @@ CAD_HD void disp_fs(const FrameT<R>& f, double X, double Y, double Z, R Dss, R D
 }
 
 // --------------------------------------------------- free-surface correction
+// out-of-line code that stays out of the callers' register allocation
+#ifdef __CUDACC__
+#define CAD_OUTLINE static __host__ __device__ __noinline__
+#else
+#define CAD_OUTLINE static inline
+#endif
+
 // Observation point -> horizontal ADCS coordinates of a side, relative to PA,
 // and its depth.
 template <typename R>
@@ -1230,6 +1313,47 @@ CAD_HD void pair_disp(const TriDevT<R>& t, double X, double Y, double Z, R U[3][
             if (t.side[sd].skip == R(0)) fsc_disp(t.side[sd], X, Y, Z, t.Dss, t.Dds, t.Dn, U);
         disp_fs<true>(t.image, X, Y, Z, t.Dss, t.Dds, t.Dn, t.K8, U);
     }
+}
+
+// Sums over the modes of the real (HS: and image) full-space terms of a
+// triangle, added into E and U.  A flat image keeps the reference's per-mode
+// order (add_strain, add_disp).
+template <bool STRAIN, bool DISP>
+CAD_OUTLINE void pair_net_flat(const TriDev& t, double X, double Y, double Z, double E[6], double U[3])
+{
+    if (STRAIN) {
+        double M[3][6];
+        pair_strain_fs_image(t, X, Y, Z, M);
+        for (int k = 0; k < 6; ++k) E[k] += (M[0][k] + M[1][k]) + M[2][k];
+    }
+    if (DISP) {
+        double M[3][3];
+        pair_disp_fs_image(t, X, Y, Z, M);
+        for (int c = 0; c < 3; ++c) U[c] += (M[0][c] + M[1][c]) + M[2][c];
+    }
+}
+template <bool HS, bool STRAIN, bool DISP>
+CAD_HD void pair_net(const TriDev& t, double X, double Y, double Z, double E[6], double U[3])
+{
+    if (t.Dn == 0.0 && t.Dss == 0.0 && t.Dds == 0.0) {   // only the NaN of points on a side is left
+        double x, y, z;
+        to_tdcs(t.real, X, Y, Z, x, y, z);
+        bool nan = on_side(t.real, x, y, z);
+        if (HS) nan = nan || pair_on_side(t, X, Y, Z);
+        if (nan) {
+            if (STRAIN)
+                for (int k = 0; k < 6; ++k) E[k] = qnan<double>();
+            if (DISP)
+                for (int c = 0; c < 3; ++c) U[c] = qnan<double>();
+        }
+        return;
+    }
+    if (HS && t.image.flat != 0.0) {
+        pair_net_flat<STRAIN, DISP>(t, X, Y, Z, E, U);
+        return;
+    }
+    td_net<STRAIN, DISP>(t.real, X, Y, Z, t.Dn, t.Dss, t.Dds, t.K8, E, U);
+    if (HS) td_net<STRAIN, DISP>(t.image, X, Y, Z, t.Dn, t.Dss, t.Dds, t.K8, E, U);
 }
 
 CAD_HD void build_triangle(const double a[3], const double b[3], const double c[3], double Dss, double Dds,

@@ -229,17 +229,23 @@ __global__ void __launch_bounds__(kPairThreads, MINB) td_pair_kernel(PairArgs a)
                 }
             continue;
         }
-        if constexpr (EDGE == EDGE_FULL && OUT == OUT_SUM && STRAIN) {
-            if (pair_on_side(t, X, Y, Z))
-                for (int k = 0; k < 6; ++k) sumE[k] = qnan<double>();
-        } else if (STRAIN) {
+        if constexpr (OUT == OUT_SUM && (!HS || EDGE != EDGE_NONE)) {
+            if (EDGE == EDGE_FULL && STRAIN && !DISP) {
+                if (pair_on_side(t, X, Y, Z))
+                    for (int k = 0; k < 6; ++k) sumE[k] = qnan<double>();
+            } else {
+                pair_net<HS, STRAIN && EDGE != EDGE_FULL, DISP>(t, X, Y, Z, sumE, sumU);
+                if (EDGE == EDGE_FULL && STRAIN && sumU[0] != sumU[0])
+                    for (int k = 0; k < 6; ++k) sumE[k] = qnan<double>();
+            }
+            continue;
+        }
+        if (STRAIN) {
             double E[3][6];
             if constexpr (EDGE_MAPS && EDGE == EDGE_FULL)
                 pair_strain_full(t, X, Y, Z, a.fscG + i, a.M, kQ * a.M, a.side_edge + 3 * jt, E);
             else if constexpr (EDGE_MAPS)
                 pair_strain_edges(t, X, Y, Z, a.fscG + i, a.M, kQ * a.M, a.side_edge + 3 * jt, E);
-            else if constexpr (EDGE != EDGE_NONE)
-                pair_strain_fs_image(t, X, Y, Z, E);
             else
                 pair_strain<HS>(t, X, Y, Z, E);
             if (OUT == OUT_INF) {
@@ -271,8 +277,6 @@ __global__ void __launch_bounds__(kPairThreads, MINB) td_pair_kernel(PairArgs a)
             if constexpr (EDGE_MAPS)
                 pair_disp_edges(t, X, Y, Z, a.fscG + i + (STRAIN ? 18 : 0) * a.M, a.M, kQ * a.M, a.side_edge + 3 * jt,
                                 U);
-            else if constexpr (EDGE != EDGE_NONE)
-                pair_disp_fs_image(t, X, Y, Z, U);
             else
                 pair_disp<HS>(t, X, Y, Z, U);
             if (OUT == OUT_INF) {
