@@ -450,7 +450,7 @@ int solve_mixed_device(cad_ctx* ctx, int64_t n, const double* A, int64_t lda, do
     if (int r = ensure(ctx, S_DINV, mixed_dinv_floats(n) * sizeof(float), &dinv)) return r;
     if (int r = ensure(ctx, S_PIV, (size_t)n * sizeof(int), &piv)) return r;
     if (int r = ensure(ctx, S_PERM, (size_t)n * sizeof(int), &perm)) return r;
-    if (int r = ensure(ctx, S_INFO, sizeof(int), &info)) return r;
+    if (int r = ensure(ctx, S_INFO, kLuInfoInts * sizeof(int), &info)) return r;
     const int rs = ctx->gmres_restart;
     if (int r = ensure(ctx, S_KRYLOV, ((size_t)n * (rs + 1) + 3 * (size_t)n + 2 * (rs + 1)) * sizeof(double),
                        &kry))
@@ -459,8 +459,10 @@ int solve_mixed_device(cad_ctx* ctx, int64_t n, const double* A, int64_t lda, do
     if (int r = ensure(ctx, S_SYNC, mixed_sync_ints(n) * sizeof(int), &sync)) return r;
     if (int r = ensure(ctx, S_WORK, (size_t)n * sizeof(double), &work)) return r;
     CK(cudaEventRecord(ctx->ev[2], ctx->stream));
-    const LuStreams ls{ctx->stream, ctx->side_stream, &ctx->launches,
-                        ctx->graphs, ctx->wait_limit};
+    LuStreams ls{ctx->stream, ctx->side_stream, &ctx->launches,
+                 ctx->graphs, ctx->wait_limit};
+    ls.aux = ctx->leaf_aux;
+    ls.naux = kLeafAux;
     ctx->timed[1] = ctx->timed[2] = false;
     int rc = mixed_prepare(ls, A, lda, n, (float*)a32, (float*)dinv, (int*)piv, (int*)perm, (int*)info,
                            lu_nb(ctx, true));
@@ -680,11 +682,13 @@ int solve_device(cad_ctx* ctx, int64_t n, double* A, int64_t lda, double* B, int
     if (int r = ensure(ctx, S_WORK, (size_t)n * nrhs * sizeof(double), &work)) return r;
     if (int r = ensure(ctx, S_PIV, (size_t)n * sizeof(int), &piv)) return r;
     if (int r = ensure(ctx, S_PERM, (size_t)n * sizeof(int), &perm)) return r;
-    if (int r = ensure(ctx, S_INFO, sizeof(int), &info)) return r;
+    if (int r = ensure(ctx, S_INFO, kLuInfoInts * sizeof(int), &info)) return r;
     CK(cudaEventRecord(ctx->ev[2], ctx->stream));
     ctx->timed[1] = ctx->timed[2] = false;
     LuStreams ls{ctx->stream, ctx->side_stream, &ctx->launches,
                  ctx->graphs, ctx->wait_limit};
+    ls.aux = ctx->leaf_aux;
+    ls.naux = kLeafAux;
     if (ctx->tuner.mode != TUNE_OFF) {
         // leaf width of the panel factorisation (rows per leaf thread), timed
         // on a scratch copy of A for systems up to 12288 unknowns
@@ -712,9 +716,8 @@ int solve_device(cad_ctx* ctx, int64_t n, double* A, int64_t lda, double* B, int
         void* chain;
         if (int r = ensure(ctx, S_CHAIN, (size_t)n * sizeof(double) + lu_chain_sync_ints(n) * sizeof(int), &chain))
             return r;
-        int rc = lu_factor_solve<double>(ls, A, n, lda, nullptr, 0, 0, nullptr, 0, (int*)piv, (int*)perm, (int*)info,
+        const int rc = lu_factor_solve<double>(ls, A, n, lda, nullptr, 0, 0, nullptr, 0, (int*)piv, (int*)perm, (int*)info,
                                          lu_nb(ctx, false), true, false);
-        if (rc == LU_OK) rc = lu_pivots_to_perm(ls, (const int*)piv, n, (int*)perm);
         if (rc == LU_TOO_LARGE) return fail(ctx, CAD_ERR_ARG, "matrix too large for the dense LU");
         if (rc != LU_OK) return fail(ctx, CAD_ERR_CUDA, "dense LU failed (CUDA error)");
         double* y = (double*)chain;
@@ -978,7 +981,7 @@ int slip_batched(cad_ctx* ctx, int64_t nbatch, const int64_t* offsets, const dou
         if (int r = lane_ensure(ctx, l, L_A32, mixed_ld(n3) * n3 * sizeof(float), &p)) return r;
         if (int r = lane_ensure(ctx, l, L_PIV, n3 * sizeof(int), &p)) return r;
         if (int r = lane_ensure(ctx, l, L_PERM, n3 * sizeof(int), &p)) return r;
-        if (int r = lane_ensure(ctx, l, L_INFO, sizeof(int), &p)) return r;
+        if (int r = lane_ensure(ctx, l, L_INFO, kLuInfoInts * sizeof(int), &p)) return r;
         if (int r = lane_ensure(ctx, l, L_IR, n3 * sizeof(double), &p)) return r;
         if (int r = lane_ensure(ctx, l, L_IR32, 2 * n3 * sizeof(float), &p)) return r;
         if (int r = lane_ensure(ctx, l, L_NORMS, 2 * sizeof(double), &p)) return r;
@@ -1323,7 +1326,7 @@ int cad_wait_timeout_probe(cad_ctx* ctx, int64_t n)
     if (int r = ensure(ctx, S_B, 3 * (size_t)n * sizeof(double), &vec)) return r;
     if (int r = ensure(ctx, S_PERM, (size_t)n * sizeof(int), &perm)) return r;
     if (int r = ensure(ctx, S_CHAIN, lu_chain_sync_ints(n) * sizeof(int), &chain)) return r;
-    if (int r = ensure(ctx, S_INFO, sizeof(int), &info)) return r;
+    if (int r = ensure(ctx, S_INFO, kLuInfoInts * sizeof(int), &info)) return r;
     CK(cudaMemsetAsync(a, 0, (size_t)n * n * sizeof(double), ctx->stream));
     CK(cudaMemsetAsync(vec, 0, 3 * (size_t)n * sizeof(double), ctx->stream));
     CK(cudaMemsetAsync(perm, 0, (size_t)n * sizeof(int), ctx->stream));

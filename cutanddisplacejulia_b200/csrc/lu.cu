@@ -94,17 +94,20 @@ __device__ __forceinline__ Key key_of(double v, int pos, unsigned who)
     const unsigned long long bits = (unsigned long long)__double_as_longlong(fabs(v));
     return Key{(unsigned)(bits >> 32) + 1u, (unsigned)bits, (unsigned)pos, who};
 }
-// the warp's best key in every lane: three integer warp reductions instead of
-// a shuffle tree of double compares
-__device__ __forceinline__ Key warp_key_max(const Key& k)
+// Lane of the warp's best key.  One integer reduction settles it unless two
+// candidates agree in the upper 32 bits of their magnitude.
+__device__ __forceinline__ int warp_key_lane(const Key& k)
 {
     const unsigned full = 0xffffffffu;
     const unsigned mhi = __reduce_max_sync(full, k.hi);
-    const unsigned mlo = __reduce_max_sync(full, k.hi == mhi ? k.lo : 0u);
-    const bool tie = k.hi == mhi && k.lo == mlo;
-    const unsigned mpos = __reduce_min_sync(full, tie ? k.pos : 0xffffffffu);
-    const unsigned win = __ballot_sync(full, tie && k.pos == mpos);
-    return Key{mhi, mlo, mpos, __shfl_sync(full, k.who, __ffs(win) - 1)};
+    unsigned win = __ballot_sync(full, k.hi == mhi);
+    if (win & (win - 1)) {   // warp-uniform
+        const unsigned mlo = __reduce_max_sync(full, k.hi == mhi ? k.lo : 0u);
+        const bool tie = k.hi == mhi && k.lo == mlo;
+        const unsigned mpos = __reduce_min_sync(full, tie ? k.pos : 0xffffffffu);
+        win = __ballot_sync(full, tie && k.pos == mpos);
+    }
+    return __ffs(win) - 1;
 }
 
 // ------------------------------------------------------------ leaf (cluster)
@@ -118,24 +121,6 @@ __device__ __forceinline__ unsigned cluster_map(unsigned addr, unsigned rank)
     unsigned r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
-}
-__device__ __forceinline__ void st_async_b64(unsigned addr, unsigned long long v, unsigned mbar)
-{
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr), "l"(v), "r"(mbar)
-                 : "memory");
-}
-__device__ __forceinline__ void st_async_b32(unsigned addr, unsigned v, unsigned mbar)
-{
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(mbar)
-                 : "memory");
-}
-__device__ __forceinline__ void st_async_word(unsigned addr, double v, unsigned mbar)
-{
-    st_async_b64(addr, (unsigned long long)__double_as_longlong(v), mbar);
-}
-__device__ __forceinline__ void st_async_word(unsigned addr, float v, unsigned mbar)
-{
-    st_async_b32(addr, __float_as_uint(v), mbar);
 }
 __device__ __forceinline__ void st_async_v4(unsigned addr, unsigned a, unsigned b, unsigned c, unsigned d, unsigned mbar)
 {
@@ -167,26 +152,37 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned mbar, unsigned parity)
 // keeps rows t + 512*k (k < RPT) in registers for the whole leaf and never
 // moves them -- each row carries its current logical position.  Per column j:
 // every warp reduces its candidates, every warp then reduces the 16 warp
-// results, and one warp pushes the CTA's best row, the reciprocal of its pivot
-// entry and its key into slot [j & 1][q] of every CTA of the cluster; each CTA
-// waits on its own barrier for the C payloads, picks the pivot and updates its
-// rows from the pivot row in shared memory.  Two slots suffice: a CTA pushes
+// results, and the warp with the CTA's best row pushes that row, its key and
+// the reciprocal of its pivot entry (staged in shared memory by the winning
+// thread, sent in 16-byte pieces by all lanes) into slot [j & 1][q] of every
+// CTA of the cluster; each CTA waits on its own barrier for the C payloads,
+// picks the pivot and updates its rows from the pivot row in shared memory.  Two slots suffice: a CTA pushes
 // column j + 2 only after every CTA's column j + 1 payload reached it, and a
 // CTA sends that payload only once all its threads are done with column j.
 // Rows are stored to their final positions at the end.  piv[c] = piv_base +
 // position swapped with c (LAPACK order); info: smallest zero-pivot column
-// (1-based, + col_base), or -1 if a wait ran out.
+// (1-based, + col_base), or -1 if a wait ran out.  moved (may be null): the net
+// row movement for leaf_update_kernel, moved[c] = panel row now at position c,
+// moved[W + c] = position of the row that was at c (c < w).
 template <typename T, int W, int RPT>
 __device__ __forceinline__ void leaf_body(T* __restrict__ A, int64_t lda, int m, int w, int* __restrict__ piv,
-                                          int piv_base, int* __restrict__ info, int col_base, long wait_limit)
+                                          int piv_base, int* __restrict__ info, int col_base, long wait_limit,
+                                          int* __restrict__ moved)
 {
     static_assert(W * RPT <= kLeafRegs && W <= 32, "leaf tile exceeds its register budget");
     cg::cluster_group cluster = cg::this_cluster();
     const int crank = (int)cluster.block_rank();
     const int C = (int)cluster.num_blocks();
-    __shared__ __align__(16) T s_row[2][kMaxCluster][W];
-    __shared__ __align__(16) T s_rinv[2][kMaxCluster];
-    __shared__ __align__(16) Key s_ckey[2][kMaxCluster];
+    // one column's payload of one CTA: its best row, the key, the reciprocal
+    struct __align__(16) Payload {
+        T row[W];
+        Key key;
+        T rinv, pad[16 / sizeof(T) - 1];
+    };
+    constexpr int kPieces = (int)sizeof(Payload) / 16;
+    static_assert(sizeof(Payload) == (W + 16 / sizeof(T)) * sizeof(T) + sizeof(Key) && W * sizeof(T) % 16 == 0, "layout");
+    __shared__ Payload s_pay[2][kMaxCluster];
+    __shared__ Payload s_mine;
     __shared__ __align__(8) unsigned long long s_bar[2];
     __shared__ Key s_wkey[2][kLeafWarps];   // by column parity: a fast warp may write column j + 1's
                                             // while a slow one still reads column j's
@@ -194,15 +190,14 @@ __device__ __forceinline__ void leaf_body(T* __restrict__ A, int64_t lda, int m,
     __shared__ int s_fail;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // bytes one column delivers to each CTA: C rows, reciprocals and keys
-    const unsigned col_bytes = (unsigned)C * (unsigned)(W * sizeof(T) + sizeof(T) + sizeof(Key));
+    const unsigned col_bytes = (unsigned)C * (unsigned)sizeof(Payload);   // one column delivers to each CTA
     if (tid == 0) {
         s_fail = 0;
         mbar_init(smem_u32(&s_bar[0]), 1);
         mbar_init(smem_u32(&s_bar[1]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        mbar_arrive_expect(smem_u32(&s_bar[0]), col_bytes);
-        if (w > 1) mbar_arrive_expect(smem_u32(&s_bar[1]), col_bytes);
+        if (C > 1) mbar_arrive_expect(smem_u32(&s_bar[0]), col_bytes);
+        if (C > 1 && w > 1) mbar_arrive_expect(smem_u32(&s_bar[1]), col_bytes);
     }
     T x[RPT][W];
     int pos[RPT];
@@ -216,62 +211,68 @@ __device__ __forceinline__ void leaf_body(T* __restrict__ A, int64_t lda, int m,
     }
     cluster.sync();   // barriers initialised and every CTA running before the first push
 
+    // Columns in groups of GS: the code of one group is unrolled (registers need
+    // static indices) and run W / GS times, the rows turned left by GS after
+    // each, so that it stays in the instruction cache -- unrolled over all W
+    // columns every instruction is fetched once and the fetch bounds the column.
+    // At group g, x[k][c] is column (g GS + c) mod W; the last g GS are done.
+    constexpr int GS = W < 8 ? W : 8;
+    static_assert(GS % 4 == 0 && W % GS == 0, "column parity and barrier phase repeat with the group");
+#pragma unroll 1
+    for (int g0 = 0; g0 < W; g0 += GS) {
+    const int live = W - g0;
 #pragma unroll
-    for (int j = 0; j < W; ++j) {
+    for (int jj = 0; jj < GS; ++jj) {
+        const int j = g0 + jj;
         if (j >= w) break;
-        const int par = j & 1;
+        const int par = jj & 1;
         Key key{0u, 0u, 0xffffffffu, 0u};
         T piv_val = (T)0;
 #pragma unroll
         for (int k = 0; k < RPT; ++k)
             if (pos[k] != INT_MAX && pos[k] >= j) {
-                const Key kk = key_of((double)x[k][j], pos[k], (unsigned)((k << 10) | tid));
+                const Key kk = key_of((double)x[k][jj], pos[k], (unsigned)((k << 10) | tid));
                 if (key_better(kk, key)) {
                     key = kk;
-                    piv_val = x[k][j];
+                    piv_val = x[k][jj];
                 }
             }
-        const T inv_c = piv_val != (T)0 ? (T)1 / piv_val : (T)0;
-        const Key wk = warp_key_max(key);
-        if (lane == 0) s_wkey[par][warp] = wk;
+        const T inv_c = piv_val != (T)0 ? (T)1 / piv_val : (T)0;   // ahead of the reduction, off its chain
+        if (lane == warp_key_lane(key)) s_wkey[par][warp] = key;
         __syncthreads();
-        const Key b = warp_key_max(lane < kLeafWarps ? s_wkey[par][lane] : Key{0u, 0u, 0xffffffffu, 0u});
-        // one warp pushes this CTA's payload for column j to every CTA: the
-        // best row (zeros if none), its reciprocal and its key
-        const int pusher = b.hi != 0u ? (int)((b.who & 1023u) >> 5) : 0;
-        if (warp == pusher) {
-            const int src = (int)(b.who & 31u), kk = (int)(b.who >> 10);
-            T mine = (T)0;
+        const Key cand = lane < kLeafWarps ? s_wkey[par][lane] : Key{0u, 0u, 0xffffffffu, 0u};
+        // the warp of the CTA's best row pushes the payload for column j to
+        // every CTA (zeros if the CTA has no candidate left)
+        if (warp == warp_key_lane(cand)) {
+            const Key b = s_wkey[par][warp];
+            Payload& mine = C == 1 ? s_pay[par][0] : s_mine;
+            if (lane == (int)(b.who & 31u)) {
+                const int kk = (int)((b.who >> 10) & 15u);
 #pragma unroll
-            for (int cc = 0; cc < W; ++cc) {
-                T v = x[0][cc];
+                for (int c = 0; c < W; ++c) {
+                    T v = x[0][c];
 #pragma unroll
-                for (int k = 1; k < RPT; ++k)
-                    if (k == kk) v = x[k][cc];
-                v = __shfl_sync(0xffffffffu, v, src);
-                if (lane == cc) mine = v;
+                    for (int k = 1; k < RPT; ++k)
+                        if (k == kk) v = x[k][c];
+                    mine.row[c] = v;   // any row if no candidate is left: key.hi = 0 is never taken
+                }
+                mine.key = Key{b.hi, b.lo, b.pos, (unsigned)crank};
+                mine.rinv = inv_c;
             }
-            T rinv = __shfl_sync(0xffffffffu, inv_c, src);
-            if (b.hi == 0u) mine = rinv = (T)0;
-            const unsigned bar = smem_u32(&s_bar[par]);
-            const unsigned row_addr = smem_u32(&s_row[par][crank][lane]);
-            const unsigned rinv_addr = smem_u32(&s_rinv[par][crank]);
-            const unsigned key_addr = smem_u32(&s_ckey[par][crank]);
-            for (int q = 0; q < C; ++q) {
-                const unsigned rbar = cluster_map(bar, (unsigned)q);
-                if (lane < W)
-                    st_async_word(cluster_map(row_addr, (unsigned)q), mine, rbar);
-            }
-            if (lane < C) {
-                const unsigned rbar = cluster_map(bar, (unsigned)lane);
-                st_async_word(cluster_map(rinv_addr, (unsigned)lane), rinv, rbar);
-                st_async_v4(cluster_map(key_addr, (unsigned)lane), b.hi, b.lo, b.pos, b.who, rbar);
+            __syncwarp();
+            const unsigned bar = smem_u32(&s_bar[par]), slot = smem_u32(&s_pay[par][crank]);
+            for (int t = lane; C > 1 && t < C * kPieces; t += 32) {
+                const int q = t / kPieces, pc = t - q * kPieces;
+                const uint4 v = reinterpret_cast<const uint4*>(&s_mine)[pc];
+                st_async_v4(cluster_map(slot + 16 * pc, (unsigned)q), v.x, v.y, v.z, v.w, cluster_map(bar, (unsigned)q));
             }
         }
-        // wait for the C payloads of column j
-        {
+        // wait for the C payloads of column j (a single CTA reads its own)
+        if (C == 1) {
+            __syncthreads();
+        } else {
             const unsigned bar = smem_u32(&s_bar[par]);
-            const unsigned parity = (unsigned)((j >> 1) & 1);
+            const unsigned parity = (unsigned)((jj >> 1) & 1);
             long spins = 0;
             while (!mbar_try_wait(bar, parity))
                 if (++spins > (wait_limit >> 2)) {   // a try_wait round may suspend briefly
@@ -280,19 +281,19 @@ __device__ __forceinline__ void leaf_body(T* __restrict__ A, int64_t lda, int m,
                 }
         }
         __syncwarp();
-        if (tid == 0 && j + 2 < w) mbar_arrive_expect(smem_u32(&s_bar[par]), col_bytes);
-        Key g = lane < C ? s_ckey[par][lane] : Key{0u, 0u, 0xffffffffu, 0u};
-        g.who = (unsigned)lane;
-        g = warp_key_max(g);
-        const bool ok = g.hi > 1u || (g.hi == 1u && g.lo != 0u);
-        const int p = ok ? (int)g.pos : j;
+        if (tid == 0 && C > 1 && j + 2 < w) mbar_arrive_expect(smem_u32(&s_bar[par]), col_bytes);
+        const Key g = lane < C ? s_pay[par][lane].key : Key{0u, 0u, 0xffffffffu, 0u};
+        const Payload& best = s_pay[par][warp_key_lane(g)];
+        const Key w_key = best.key;
+        const bool ok = w_key.hi > 1u || (w_key.hi == 1u && w_key.lo != 0u);
+        const int p = ok ? (int)w_key.pos : j;
         if (tid == 0) {
             s_hist[j] = p;
             if (!ok && crank == 0) atomicMin(info, col_base + j + 1);
         }
         if (ok) {
-            const T* u = s_row[par][g.who];
-            const T inv = s_rinv[par][g.who];
+            const T* u = best.row;
+            const T inv = best.rinv;
 #pragma unroll
             for (int k = 0; k < RPT; ++k) {
                 int ps = pos[k];
@@ -300,13 +301,29 @@ __device__ __forceinline__ void leaf_body(T* __restrict__ A, int64_t lda, int m,
                 else if (ps == j) ps = p;
                 pos[k] = ps;
                 if (ps != INT_MAX && ps > j) {
-                    const T l = x[k][j] * inv;
-                    x[k][j] = l;
+                    const T l = x[k][jj] * inv;
+                    x[k][jj] = l;
 #pragma unroll
-                    for (int cc = j + 1; cc < W; ++cc) x[k][cc] -= l * u[cc];
+                    for (int cb = 0; cb < W; cb += GS)
+                        if (cb < live) {
+#pragma unroll
+                            for (int cc = cb; cc < cb + GS; ++cc)
+                                if (cc > jj) x[k][cc] -= l * u[cc];
+                        }
                 }
             }
         }
+    }
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+        T t[GS];
+#pragma unroll
+        for (int c = 0; c < GS; ++c) t[c] = x[k][c];
+#pragma unroll
+        for (int c = 0; c < W - GS; ++c) x[k][c] = x[k][c + GS];
+#pragma unroll
+        for (int c = 0; c < GS; ++c) x[k][W - GS + c] = t[c];
+    }
     }
     cluster.sync();   // every push has landed and been read before any CTA exits
 #pragma unroll
@@ -317,6 +334,14 @@ __device__ __forceinline__ void leaf_body(T* __restrict__ A, int64_t lda, int m,
                 if (c < w) A[(int64_t)pos[k] + (int64_t)c * lda] = x[k][c];
     __syncthreads();
     if (crank == 0 && tid < w) piv[tid] = piv_base + s_hist[tid];
+    if (moved) {
+#pragma unroll
+        for (int k = 0; k < RPT; ++k) {
+            const int row = crank * (kLeafThreads * RPT) + k * kLeafThreads + tid;
+            if (pos[k] != INT_MAX && pos[k] < w) moved[pos[k]] = row;
+            if (pos[k] != INT_MAX && row < w) moved[W + row] = pos[k];
+        }
+    }
     if (tid == 0 && s_fail) atomicMin(info, -1);
 }
 
@@ -324,9 +349,9 @@ template <typename T, int W, int RPT>
 __global__ void __launch_bounds__(kLeafThreads, 1) leaf_lu_kernel(T* __restrict__ A, int64_t lda, int m, int w,
                                                                 int* __restrict__ piv, int piv_base,
                                                                 int* __restrict__ info, int col_base,
-                                                                long wait_limit)
+                                                                long wait_limit, int* __restrict__ moved)
 {
-    leaf_body<T, W, RPT>(A, lda, m, w, piv, piv_base, info, col_base, wait_limit);
+    leaf_body<T, W, RPT>(A, lda, m, w, piv, piv_base, info, col_base, wait_limit, moved);
 }
 
 // The leaves of many systems in one launch: cluster y of the grid factorises
@@ -336,50 +361,177 @@ template <int W, int RPT>
 __global__ void __launch_bounds__(kLeafThreads, 1) leaf_group_kernel(const __grid_constant__ LeafGroup g)
 {
     const LeafRec& r = g.rec[blockIdx.y];
-    leaf_body<float, W, RPT>(r.A, r.lda, r.m, g.w, r.piv, r.piv_base, r.info, r.col_base, g.wait_limit);
+    leaf_body<float, W, RPT>(r.A, r.lda, r.m, g.w, r.piv, r.piv_base, r.info, r.col_base, g.wait_limit, nullptr);
+}
+
+// ------------------------------------------------------------ leaf update
+// The columns of a panel right of a leaf, after the leaf (m x w at A, factors in
+// place, net row movement in moved): row movement, U = L11^-1 times the top
+// rows, and C -= L21 U, in one launch instead of three.  One cluster handles CB
+// columns of all m rows (its CTAs R = 256 RPT rows each): every CTA reads the
+// rows that move to the top and the rows that were there before any CTA of the
+// cluster writes (one cluster barrier), solves for U on its own (32 steps) and
+// updates its rows, each thread RPT rows x CB columns in registers.  FP64-pipe
+// bound: 2 m CB w flops per cluster, 4.2 us for 512 rows x 32 x 32 on one SM.
+constexpr int kUpdThreads = 256;
+template <typename T, int W, int RPT, int CB>
+__global__ void __launch_bounds__(kUpdThreads, RPT == 1 ? 2 : 1) leaf_update_kernel(T* __restrict__ A, int64_t lda, int m, int w,
+                                                                  const int* __restrict__ moved, T* __restrict__ B,
+                                                                  int ncol)
+{
+    constexpr int R = kUpdThreads * RPT;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int crank = (int)cluster.block_rank();
+    const int c0 = blockIdx.y * CB, nc = ncol - c0 < CB ? ncol - c0 : CB;
+    T* __restrict__ Bc = B + (int64_t)c0 * lda;
+    __shared__ __align__(16) T s_u[W][CB + 2];   // rows to be solved, then U
+    __shared__ T s_old[W][CB + 1];               // rows that leave the top
+    __shared__ T s_l[W][W + 1];                  // s_l[k][i] = L11(i, k)
+    __shared__ signed char s_from[R];            // old top row that lands on my row, or -1
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row0 = w + crank * R;              // my first row
+    // every load that waits for nothing: L11, L21 of my rows, my rows
+    for (int t = tid; t < W * W; t += kUpdThreads) {
+        const int i = t % W, k = t / W;
+        s_l[k][i] = (i < w && k < i) ? A[i + (int64_t)k * lda] : (T)0;
+    }
+    // columns of L21 held in registers at a time
+    constexpr int kHold = RPT == 1 ? 16 : 32 / RPT, KC = W < kHold ? W : kHold;
+    T x[RPT][CB], l[RPT][KC];
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+        const int row = row0 + r * kUpdThreads + tid;
+#pragma unroll
+        for (int c = 0; c < CB; ++c) x[r][c] = (row < m && c < nc) ? Bc[row + (int64_t)c * lda] : (T)0;
+#pragma unroll
+        for (int k = 0; k < KC; ++k) l[r][k] = (row < m && k < w) ? A[row + (int64_t)k * lda] : (T)0;
+    }
+    for (int t = tid; t < W * CB; t += kUpdThreads) {
+        const int i = t % W, c = t / W;
+        const bool in = i < w && c < nc;
+        s_u[i][c] = in ? Bc[moved[i] + (int64_t)c * lda] : (T)0;
+        s_old[i][c] = in ? Bc[i + (int64_t)c * lda] : (T)0;
+    }
+    for (int t = tid; t < R; t += kUpdThreads) s_from[t] = -1;
+    __syncthreads();
+    if (tid < w) {
+        const int d = moved[W + tid] - row0;
+        if (d >= 0 && d < R) s_from[d] = (signed char)tid;
+    }
+    // U = L11^-1 (top rows): warp by columns, lane = row
+    {
+        constexpr int kPer = (CB + kUpdThreads / 32 - 1) / (kUpdThreads / 32);
+        T u[kPer];
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const int c = warp * kPer + q;
+            u[q] = lane < W && c < CB ? s_u[lane < W ? lane : 0][c < CB ? c : 0] : (T)0;
+        }
+#pragma unroll 8
+        for (int k = 0; k < W; ++k) {
+            const T lk = lane < W ? s_l[k][lane] : (T)0;
+#pragma unroll
+            for (int q = 0; q < kPer; ++q) u[q] -= lk * __shfl_sync(0xffffffffu, u[q], k);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const int c = warp * kPer + q;
+            if (lane < W && c < CB) s_u[lane][c] = u[q];
+        }
+    }
+    __syncthreads();
+    // rows that arrive from the old top
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+        const int from = s_from[r * kUpdThreads + tid];
+        if (from >= 0) {
+#pragma unroll
+            for (int c = 0; c < CB; ++c) x[r][c] = s_old[from][c];
+        }
+    }
+    cluster.sync();   // every CTA of the cluster has read what it needs of these columns
+    if (crank == 0)
+        for (int t = tid; t < W * CB; t += kUpdThreads) {
+            const int i = t % W, c = t / W;
+            if (i < w && c < nc) Bc[i + (int64_t)c * lda] = s_u[i][c];
+        }
+#pragma unroll 1
+    for (int kb = 0; kb < W; kb += KC) {
+        if (kb > 0) {
+            if (kb >= w) break;
+#pragma unroll
+            for (int r = 0; r < RPT; ++r) {
+                const int row = row0 + r * kUpdThreads + tid;
+#pragma unroll
+                for (int k = 0; k < KC; ++k)
+                    l[r][k] = (row < m && kb + k < w) ? A[row + (int64_t)(kb + k) * lda] : (T)0;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < KC; ++k)
+#pragma unroll
+            for (int c = 0; c < CB; ++c) {
+                const T u = s_u[kb + k][c];
+#pragma unroll
+                for (int r = 0; r < RPT; ++r) x[r][c] -= l[r][k] * u;
+            }
+    }
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+        const int row = row0 + r * kUpdThreads + tid;
+#pragma unroll
+        for (int c = 0; c < CB; ++c)
+            if (row < m && c < nc) Bc[row + (int64_t)c * lda] = x[r][c];
+    }
 }
 
 // ------------------------------------------------------------ row swaps
+// The net movement of npiv <= kMaxSwaps swaps k <-> piv[k] (in order, rows
+// relative to the block top; piv in shared memory, kMaxSwaps entries): 2 npiv
+// (dst, src) pairs, dst -1 where a row stays.  Entry t < npiv follows the
+// content of row t through the sequence, entry npiv + k that of row piv[k]; a
+// row followed twice gives the same pair twice.  About 1.5 us for 256 swaps
+// (chains of one compare and select per swap, four swaps a load).
+__device__ __forceinline__ void collect_moves(const int* piv, int npiv, int* dst, int* src)
+{
+    const int4* p4 = reinterpret_cast<const int4*>(piv);
+    for (int t = threadIdx.x; t < 2 * npiv; t += blockDim.x) {
+        const int row = t < npiv ? t : piv[t - npiv];
+        int at = row;
+#pragma unroll 4
+        for (int k = 0; k + 3 < npiv; k += 4) {
+            const int4 q = p4[k >> 2];
+            at = at == k ? q.x : (at == q.x ? k : at);
+            at = at == k + 1 ? q.y : (at == q.y ? k + 1 : at);
+            at = at == k + 2 ? q.z : (at == q.z ? k + 2 : at);
+            at = at == k + 3 ? q.w : (at == q.w ? k + 3 : at);
+        }
+        for (int k = npiv & ~3; k < npiv; ++k) {
+            const int q = piv[k];
+            at = at == k ? q : (at == q ? k : at);
+        }
+        dst[t] = at == row ? -1 : at;
+        src[t] = row;
+    }
+}
+
 // Applies the swaps row k <-> row piv[k] - row_base (k = 0..npiv-1, in order,
 // rows relative to the block top) to columns [0, ncol1) of A1 and [0, ncol2)
-// of A2.  Every CTA first derives the net movement: each touched row follows
-// its content through the swap sequence, giving at most 2 * npiv (dst, src)
-// pairs; then one warp per column gathers the sources and stores them.
+// of A2.  Every CTA first derives the net movement (collect_moves); then one
+// warp per column gathers the sources and stores them.
 template <typename T>
 __device__ __forceinline__ void laswp_body(T* __restrict__ A1, int ncol1, T* __restrict__ A2, int ncol2, int64_t lda,
                                            const int* __restrict__ piv, int npiv, int row_base, int cta, int ncta)
 {
     constexpr int kPer = 2 * kMaxSwaps / 32;
-    __shared__ int s_piv[kMaxSwaps];
+    __shared__ __align__(16) int s_piv[kMaxSwaps];
     __shared__ int s_dst[2 * kMaxSwaps], s_src[2 * kMaxSwaps];
-    __shared__ int s_count;
     for (int k = threadIdx.x; k < npiv; k += blockDim.x) s_piv[k] = piv[k] - row_base;
-    if (threadIdx.x == 0) s_count = 0;
     __syncthreads();
-    for (int t = threadIdx.x; t < 2 * npiv; t += blockDim.x) {
-        int row = t;
-        bool track = true;
-        if (t >= npiv) {   // a pivot row below the block's first npiv rows, tracked once
-            const int kk = t - npiv;
-            row = s_piv[kk];
-            track = row >= npiv;
-            for (int k = 0; k < kk && track; ++k) track = s_piv[k] != row;
-        }
-        if (!track) continue;
-        int at = row;
-        for (int k = 0; k < npiv; ++k) {
-            const int q = s_piv[k];
-            at = at == k ? q : (at == q ? k : at);
-        }
-        if (at != row) {
-            const int slot = atomicAdd(&s_count, 1);
-            s_dst[slot] = at;
-            s_src[slot] = row;
-        }
-    }
+    collect_moves(s_piv, npiv, s_dst, s_src);
     __syncthreads();
-    const int count = s_count;
-    if (count == 0) return;
+    const int count = 2 * npiv;
     const int lane = threadIdx.x & 31;
     int dst[kPer], src[kPer];
 #pragma unroll
@@ -408,6 +560,18 @@ __global__ void __launch_bounds__(256) laswp_kernel(T* __restrict__ A1, int ncol
                                                     int64_t lda, const int* __restrict__ piv, int npiv, int row_base)
 {
     laswp_body<T>(A1, ncol1, A2, ncol2, lda, piv, npiv, row_base, blockIdx.x, gridDim.x);
+}
+
+// The later leaves' swaps on each leaf's own columns of a panel of w columns in
+// leaves of lw (grid.y: leaf): pivots [max((y + 1) lw, c0), c1) of the panel.
+template <typename T>
+__global__ void __launch_bounds__(256) laswp_panel_kernel(T* __restrict__ A, int64_t lda, int lw, int c0, int c1,
+                                                          const int* __restrict__ piv, int piv_base)
+{
+    const int f = ((int)blockIdx.y + 1) * lw, k0 = f > c0 ? f : c0;
+    if (k0 >= c1) return;
+    laswp_body<T>(A + k0 + (int64_t)blockIdx.y * lw * lda, lw, nullptr, 0, lda, piv + k0, c1 - k0, piv_base + k0,
+                  blockIdx.x, gridDim.x);
 }
 
 __global__ void __launch_bounds__(256) laswp_group_kernel(const __grid_constant__ LaswpGroup g)
@@ -509,55 +673,49 @@ __global__ void __launch_bounds__(128) trsm_group_kernel(const __grid_constant__
     trsm_diag_body<float, false>(r.L, r.ldl, g.b, r.B, r.ldb, r.ncol, blockIdx.x);
 }
 
-// perm[i] = source row of row i after all n pivots (ipiv applied in order),
-// built by one thread in shared memory.
-__global__ void pivots_to_perm_kernel(const int* __restrict__ ipiv, int n, int* __restrict__ perm)
+// perm[i] = source row of row i after all n pivots (ipiv applied in order), in
+// one block: kMaxSwaps pivots at a time, each touched row followed through
+// them by one thread (0.03 ms at n = 6039 where one thread applying the swaps
+// took 0.22 ms).
+__device__ __forceinline__ void perm_body(const int* __restrict__ ipiv, int n, int* __restrict__ perm)
 {
-    extern __shared__ int s_perm[];
-    for (int i = threadIdx.x; i < n; i += blockDim.x) s_perm[i] = i;
-    __syncthreads();
-    if (threadIdx.x == 0)
-        for (int k = 0; k < n; ++k) {
-            const int q = ipiv[k];
-            const int t = s_perm[k];
-            s_perm[k] = s_perm[q];
-            s_perm[q] = t;
-        }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = s_perm[i];
-}
-
-// The same in global memory, for n beyond what shared memory holds.
-__global__ void pivots_to_perm_global_kernel(const int* __restrict__ ipiv, int n, int* __restrict__ perm)
-{
+    __shared__ __align__(16) int s_piv[kMaxSwaps];
+    __shared__ int s_dst[2 * kMaxSwaps], s_src[2 * kMaxSwaps];
     for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = i;
-    __syncthreads();
-    if (threadIdx.x == 0)
-        for (int k = 0; k < n; ++k) {
-            const int q = ipiv[k];
-            const int t = perm[k];
-            perm[k] = perm[q];
-            perm[q] = t;
-        }
-}
-
-// perm from ipiv on stream st (shared-memory kernel where n ints fit)
-cudaError_t launch_pivots_to_perm(cudaStream_t st, const int* ipiv, int64_t n, int* perm)
-{
-    if (n <= 0) return cudaSuccess;
-    int dev = 0, smem_optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    const size_t psmem = (size_t)n * sizeof(int);
-    if (psmem <= (size_t)smem_optin) {
-        cudaError_t e = cudaFuncSetAttribute(pivots_to_perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)psmem);
-        if (e != cudaSuccess) return e;
-        pivots_to_perm_kernel<<<1, 1024, psmem, st>>>(ipiv, (int)n, perm);
-    } else {
-        pivots_to_perm_global_kernel<<<1, 1024, 0, st>>>(ipiv, (int)n, perm);
+    for (int c0 = 0; c0 < n; c0 += kMaxSwaps) {
+        const int np = n - c0 < kMaxSwaps ? n - c0 : kMaxSwaps;
+        __syncthreads();   // perm and the lists of the chunk before are settled
+        for (int k = threadIdx.x; k < np; k += blockDim.x) s_piv[k] = ipiv[c0 + k] - c0;
+        __syncthreads();
+        collect_moves(s_piv, np, s_dst, s_src);
+        __syncthreads();
+        const bool mine = (int)threadIdx.x < 2 * np && s_dst[threadIdx.x] >= 0;
+        const int v = mine ? perm[c0 + s_src[threadIdx.x]] : 0;
+        __syncthreads();
+        if (mine) perm[c0 + s_dst[threadIdx.x]] = v;
     }
-    return cudaGetLastError();
+}
+static_assert(2 * kMaxSwaps <= 1024, "one thread per moved row");
+// The same panel by panel beside the factorisation: one panel's pivots (rows
+// relative to piv_base) applied to perm from its first row on.
+__global__ void __launch_bounds__(512) panel_perm_kernel(const int* __restrict__ piv, int np, int piv_base,
+                                                         int* __restrict__ perm)
+{
+    __shared__ __align__(16) int s_piv[kMaxSwaps];
+    __shared__ int s_dst[2 * kMaxSwaps], s_src[2 * kMaxSwaps];
+    for (int k = threadIdx.x; k < np; k += blockDim.x) s_piv[k] = piv[k] - piv_base;
+    __syncthreads();
+    collect_moves(s_piv, np, s_dst, s_src);
+    __syncthreads();
+    const bool mine = (int)threadIdx.x < 2 * np && s_dst[threadIdx.x] >= 0;
+    const int v = mine ? perm[s_src[threadIdx.x]] : 0;
+    __syncthreads();
+    if (mine) perm[s_dst[threadIdx.x]] = v;
+}
+__global__ void iota_kernel(int* __restrict__ p, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) p[i] = i;
 }
 
 // Y[i, c] = X[perm[i], c]
@@ -576,8 +734,11 @@ template <typename T>
 struct Lu {
     cudaStream_t st;   // the stream the next launches go to
     cudaStream_t main_st, side_st;
+    cudaStream_t aux_st = nullptr;   // the next block column's leaf updates (null: on the main stream)
+    cudaEvent_t ev_leaf = nullptr;
     int* ipiv;    // absolute pivots, device
     int* info;
+    int* moved;   // net row movement of the panel's leaves (64 ints each)
     int cluster;  // largest leaf cluster (16 where the device co-schedules it, else 8)
     long wait_limit = kDefaultWaitLimit;   // try_wait rounds before a leaf gives up on a push
     int min_rpt = 1;        // fewest rows per leaf thread (wider leaves with fewer rows each)
@@ -650,14 +811,51 @@ struct Lu {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         err = cudaLaunchKernelEx(&cfg, leaf_lu_kernel<T, W, RPT>, A, lda, m, w, piv, piv_base, info, col_base,
-                                 wait_limit);
+                                 wait_limit, moved);
         ++launches;
     }
 
-    void leaf(T* A, int64_t lda, int m, int w, int* piv, int piv_base, int col_base)
+    // leaf_update_kernel on the ncol columns at B (their top row level with the
+    // leaf's): rows per thread as few as one cluster allows
+    template <int W, int RPT, int CB>
+    void update_launch(T* A, int64_t lda, int m, int w, T* B, int ncol)
+    {
+        const int R = kUpdThreads * RPT;
+        const int C = (m - w + R - 1) / R;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)C, (unsigned)((ncol + CB - 1) / CB));
+        cfg.blockDim = dim3(kUpdThreads);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)C;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        err = cudaLaunchKernelEx(&cfg, leaf_update_kernel<T, W, RPT, CB>, A, lda, m, w, (const int*)moved, B, ncol);
+        ++launches;
+    }
+    void update(T* A, int64_t lda, int m, int w, int leaf_w, T* B, int ncol)
+    {
+        if (!ok() || ncol <= 0) return;
+        const int rows = m - w;
+        if (leaf_w == 32) {
+            if (rows <= cluster * kUpdThreads) update_launch<32, 1, 16>(A, lda, m, w, B, ncol);
+            else update_launch<32, 2, 16>(A, lda, m, w, B, ncol);
+        } else if (leaf_w == 16) {
+            update_launch<16, 4, 8>(A, lda, m, w, B, ncol);
+        } else {   // leaves of 8: panel_split takes over beyond them
+            update_launch<8, 8, 4>(A, lda, m, w, B, ncol);
+        }
+    }
+
+    // leaf_w: the build's width (that of the panel's first leaf, whose rows need
+    // the most threads)
+    void leaf(T* A, int64_t lda, int m, int w, int* piv, int piv_base, int col_base, int leaf_w)
     {
         if (!ok()) return;
-        switch (leaf_rpt(m)) {
+        switch (kLeafRegs / leaf_w) {
             case 1: leaf_launch<32, 1>(A, lda, m, w, piv, piv_base, col_base); break;
             case 2: leaf_launch<16, 2>(A, lda, m, w, piv, piv_base, col_base); break;
             case 4: leaf_launch<8, 4>(A, lda, m, w, piv, piv_base, col_base); break;
@@ -665,98 +863,163 @@ struct Lu {
         }
     }
 
-    // m x w panel at A; its pivots (relative to the panel top, + piv_base) go to piv[0..w)
-    void panel(T* A, int64_t lda, int m, int w, int* piv, int piv_base, int col_base)
+    // m x w panel at A and the `next` columns to its right (the next block
+    // column): leaf by leaf, factorise, then move, solve and update every column
+    // of the panel right of the leaf in one launch, those of the next block
+    // column in another beside the next leaf.  `ready` (may be null) is waited
+    // for before the next block column is touched.  Pivots go to piv[0..w) (relative to the
+    // panel top, + piv_base); the leaves' own columns still lack the later
+    // leaves' swaps (panel_swaps).  The chain of a 256-column panel is 16
+    // launches; splitting the panel in halves and updating the next block
+    // column after it took 43 launches and 70 us of triangular blocks more.
+    void panel(T* A, int64_t lda, int m, int w, int next, cudaEvent_t ready, int* piv, int piv_base, int col_base)
+    {
+        const int lw = leaf_width(m);
+        int* const moved0 = moved;
+        const bool fork = aux_st && next > 0;
+        const int own = fork ? 0 : next;   // columns beyond the panel that its own updates cover
+        if (ready && ok()) err = cudaStreamWaitEvent(fork ? aux_st : st, ready, 0);
+        for (int o = 0, i = 0; o < w && ok(); o += lw, ++i) {
+            const int wl = w - o < lw ? w - o : lw;
+            T* D = A + o + (int64_t)o * lda;
+            moved = moved0 + 64 * i;
+            leaf(D, lda, m - o, wl, piv + o, piv_base + o, col_base + o, lw);
+            if (m - o <= wl) continue;
+            if (fork && ok()) {   // beside the next leaf
+                err = cudaEventRecord(ev_leaf, main_st);
+                if (ok()) err = cudaStreamWaitEvent(aux_st, ev_leaf, 0);
+                st = aux_st;
+                update(D, lda, m - o, wl, lw, A + o + (int64_t)w * lda, next);
+                st = main_st;
+            }
+            update(D, lda, m - o, wl, lw, D + (int64_t)wl * lda, w - o - wl + own);
+        }
+        if (fork && ok()) {
+            err = cudaEventRecord(ev_leaf, aux_st);
+            if (ok()) err = cudaStreamWaitEvent(main_st, ev_leaf, 0);
+        }
+        moved = moved0;
+    }
+    // The same for panels of more rows than one row per leaf thread can hold
+    // (leaves narrower than 32 columns): the panel split in halves -- factorise
+    // the left one, swap, solve and update the right one, factorise it, swap the
+    // left one -- with the tensor-core products.  Rank-16 updates leaf by leaf
+    // move too much of the panel through L2 there: the 30 000-unknown solve took
+    // 900 ms with them and 745 ms split.
+    void panel_split(T* A, int64_t lda, int m, int w, int* piv, int piv_base, int col_base)
     {
         if (!ok()) return;
         const int lw = leaf_width(m);
         if (w <= lw) {
-            leaf(A, lda, m, w, piv, piv_base, col_base);
+            leaf(A, lda, m, w, piv, piv_base, col_base, lw);
             return;
         }
-        int w1 = w / 2;
-        w1 = (w1 + lw - 1) / lw * lw;
+        int w1 = (w / 2 + lw - 1) / lw * lw;
         if (w1 >= w) w1 = w - lw;
-        panel(A, lda, m, w1, piv, piv_base, col_base);
+        panel_split(A, lda, m, w1, piv, piv_base, col_base);
         laswp(piv, w1, piv_base, A + w1 * lda, w - w1, nullptr, 0, lda);
         trsm_lower(A, lda, w1, A + w1 * lda, lda, w - w1);
         if (m > w1) gemm(m - w1, w - w1, w1, A + w1, lda, A + w1 * lda, lda, A + w1 + w1 * lda, lda);
-        panel(A + w1 + w1 * lda, lda, m - w1, w - w1, piv + w1, piv_base + w1, col_base + w1);
-        // the right half's pivots (rows w1.. of the panel) applied to the left half's columns
+        panel_split(A + w1 + w1 * lda, lda, m - w1, w - w1, piv + w1, piv_base + w1, col_base + w1);
         laswp(piv + w1, w - w1, piv_base + w1, A + w1, w1, nullptr, 0, lda);
+    }
+    // block columns [c, c + nc): the block's swaps, triangular solve and product
+    void apply_block(T* A, int64_t lda, int64_t n, int64_t k, int kb, int64_t c, int nc)
+    {
+        if (nc <= 0 || !ok()) return;
+        laswp(ipiv + k, kb, (int)k, A + k + c * lda, nc, nullptr, 0, lda);
+        trsm_lower(A + k + k * lda, lda, kb, A + k + c * lda, lda, nc);
+        gemm((int)(n - k - kb), nc, kb, A + (k + kb) + k * lda, lda, A + k + c * lda, lda, A + (k + kb) + c * lda, lda);
+    }
+    // the later leaves' swaps on each leaf's own columns of a panel
+    void panel_swaps(T* A, int64_t lda, int m, int w, const int* piv, int piv_base)
+    {
+        const int lw = leaf_width(m);
+        for (int c0 = 0; c0 < w && ok(); c0 += kMaxSwaps) {
+            const int c1 = c0 + kMaxSwaps < w ? c0 + kMaxSwaps : w;
+            const int nleaf = (c1 - 1) / lw;   // leaves with a pivot of [c0, c1) after them
+            if (nleaf == 0) continue;
+            laswp_panel_kernel<T><<<dim3((unsigned)((lw + 7) / 8), (unsigned)nleaf), 256, 0, st>>>(A, lda, lw, c0, c1,
+                                                                                                 piv, piv_base);
+            ++launches;
+            err = cudaGetLastError();
+        }
     }
 
     void use(bool side) { st = side ? side_st : main_st; }
 
-    // Right-looking blocked LU with a look-ahead of one block column.  Block
-    // b's update is split: the main stream swaps, solves and updates block
-    // column b + 1 only, then factorises it as the next panel; the side stream
-    // meanwhile swaps, solves and updates the remaining columns.  The panel is
-    // latency-bound on a few SMs, the trailing GEMM fills the rest.  Events:
-    // panel[b] (block column b factorised; its pivots exist), rest[b] (side
-    // work of block b done -- the main stream waits for it before touching
-    // block column b + 2 or swapping rows of the L columns the side GEMM reads).
-    void factor(T* A, int64_t n, int64_t lda, int nb)
+    // Right-looking blocked LU with a look-ahead of one block column.  The main
+    // stream only factorises panels, each panel's leaves updating the next
+    // block column as they go; the side stream meanwhile applies the panel's
+    // swaps to the columns left of it and swaps, solves and updates the block
+    // columns after the next, first the one the following panel's updates need.
+    // The panel chain is latency-bound on a few SMs, the trailing GEMM fills
+    // the rest.  Events: panel[b] (block column b factorised; its pivots exist),
+    // next[b] (block b applied to block column b + 2).
+    void factor(T* A, int64_t n, int64_t lda, int nb, int* perm)
     {
         use(false);
         set_int_kernel<<<1, 1, 0, st>>>(info, INT_MAX);
-        ++launches;
+        if (n > 0) iota_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(perm, (int)n);
+        launches += 2;
         err = cudaGetLastError();
         const int nblk = (int)((n + nb - 1) / nb);
         if (nblk == 0 || !ok()) return;
-        std::vector<cudaEvent_t> ev_panel(nblk, nullptr), ev_rest(nblk, nullptr);
+        std::vector<cudaEvent_t> ev_panel(nblk, nullptr), ev_next(nblk, nullptr);
+        cudaEvent_t ev_done = nullptr;
+        err = cudaEventCreateWithFlags(&ev_done, cudaEventDisableTiming);
+        if (ok() && aux_st) err = cudaEventCreateWithFlags(&ev_leaf, cudaEventDisableTiming);
         for (int b = 0; b < nblk && ok(); ++b) {
             err = cudaEventCreateWithFlags(&ev_panel[b], cudaEventDisableTiming);
-            if (ok()) err = cudaEventCreateWithFlags(&ev_rest[b], cudaEventDisableTiming);
+            if (ok()) err = cudaEventCreateWithFlags(&ev_next[b], cudaEventDisableTiming);
         }
-        if (ok()) {
-            const int kb0 = (int)(n < nb ? n : nb);
-            panel(A, lda, (int)n, kb0, ipiv, 0, 0);
-            if (ok()) err = cudaEventRecord(ev_panel[0], main_st);
-        }
+        auto width = [&](int64_t k) { return (int)(k >= n ? 0 : n - k < nb ? n - k : nb); };
         for (int b = 0; b < nblk && ok(); ++b) {
-            const int64_t k = (int64_t)b * nb;
-            const int kb = (int)(n - k < nb ? n - k : nb);
-            const int64_t k1 = k + kb;                                  // next block column
-            const int kb1 = (int)(n - k1 < nb ? n - k1 : nb);
-            const int64_t k2 = k1 + kb1;                                // the rest
-            const int nr2 = (int)(n - k2);
+            const int64_t k = (int64_t)b * nb, k1 = k + width(k), k2 = k1 + width(k1), k3 = k2 + width(k2);
+            const int kb = width(k), m = (int)(n - k);
             T* Akk = A + k + k * lda;
-            // main: swaps left of the panel and in the next block column, its
-            // solve and update, then the next panel
             use(false);
-            if (b > 0) err = cudaStreamWaitEvent(main_st, ev_rest[b - 1], 0);
-            laswp(ipiv + k, kb, (int)k, A + k, (int)k, A + k + k1 * lda, kb1, lda);
-            if (kb1 > 0) {
-                trsm_lower(Akk, lda, kb, A + k + k1 * lda, lda, kb1);
-                gemm((int)(n - k1), kb1, kb, A + k1 + k * lda, lda, A + k + k1 * lda, lda, A + k1 + k1 * lda, lda);
-                panel(A + k1 + k1 * lda, lda, (int)(n - k1), kb1, ipiv + k1, (int)k1, (int)k1);
-                if (ok()) err = cudaEventRecord(ev_panel[b + 1], main_st);
+            const cudaEvent_t ready = b > 0 ? ev_next[b - 1] : nullptr;
+            const bool split = leaf_width(m) * min_rpt < 32;
+            if (split)
+                panel_split(Akk, lda, m, kb, ipiv + k, (int)k, (int)k);
+            else
+                panel(Akk, lda, m, kb, width(k1), ready, ipiv + k, (int)k, (int)k);
+            if (ok()) err = cudaEventRecord(ev_panel[b], main_st);
+            if (split) {
+                if (ready && ok()) err = cudaStreamWaitEvent(main_st, ready, 0);
+                apply_block(A, lda, n, k, kb, k1, width(k1));
             }
-            // side: the same for the remaining block columns
             use(true);
-            if (nr2 > 0 && ok()) {
-                err = cudaStreamWaitEvent(side_st, ev_panel[b], 0);
-                laswp(ipiv + k, kb, (int)k, A + k + k2 * lda, nr2, nullptr, 0, lda);
-                trsm_lower(Akk, lda, kb, A + k + k2 * lda, lda, nr2);
-                gemm((int)(n - k1), nr2, kb, A + k1 + k * lda, lda, A + k + k2 * lda, lda, A + k1 + k2 * lda, lda);
+            if (ok()) err = cudaStreamWaitEvent(side_st, ev_panel[b], 0);
+            if (!split) panel_swaps(Akk, lda, m, kb, ipiv + k, (int)k);
+            apply_block(A, lda, n, k, kb, k2, (int)(k3 - k2));
+            if (ok()) err = cudaEventRecord(ev_next[b], side_st);
+            apply_block(A, lda, n, k, kb, k3, (int)(n - k3));
+            if (k > 0) laswp(ipiv + k, kb, (int)k, A + k, (int)k, nullptr, 0, lda);
+            for (int c0 = 0; c0 < kb && ok(); c0 += kMaxSwaps) {
+                const int np = kb - c0 < kMaxSwaps ? kb - c0 : kMaxSwaps;
+                panel_perm_kernel<<<1, 512, 0, st>>>(ipiv + k + c0, np, (int)(k + c0), perm + k + c0);
+                ++launches;
+                err = cudaGetLastError();
             }
-            if (ok()) err = cudaEventRecord(ev_rest[b], side_st);
         }
+        if (ok()) err = cudaEventRecord(ev_done, side_st);
         use(false);
-        if (ok()) err = cudaStreamWaitEvent(main_st, ev_rest[nblk - 1], 0);
+        if (ok()) err = cudaStreamWaitEvent(main_st, ev_done, 0);
         for (int b = 0; b < nblk; ++b) {
             if (ev_panel[b]) cudaEventDestroy(ev_panel[b]);
-            if (ev_rest[b]) cudaEventDestroy(ev_rest[b]);
+            if (ev_next[b]) cudaEventDestroy(ev_next[b]);
         }
+        if (ev_done) cudaEventDestroy(ev_done);
+        if (ev_leaf) cudaEventDestroy(ev_leaf);
+        ev_leaf = nullptr;
     }
 
-    // X (n x nrhs) := A^-1 B with the factors in A; perm: n ints
-    void solve(const T* A, int64_t n, int64_t lda, const T* B, int64_t ldb, int nrhs, T* X, int64_t ldx, int* perm)
+    // X (n x nrhs) := A^-1 B with the factors in A and the factorisation's perm
+    void solve(const T* A, int64_t n, int64_t lda, const T* B, int64_t ldb, int nrhs, T* X, int64_t ldx,
+               const int* perm)
     {
-        if (!ok()) return;
-        err = launch_pivots_to_perm(st, ipiv, n, perm);
-        ++launches;
         if (!ok()) return;
         permute_rows_kernel<T><<<dim3((unsigned)((n + 255) / 256), nrhs), 256, 0, st>>>(B, ldb, perm, (int)n, nrhs, X,
                                                                                         ldx);
@@ -788,6 +1051,12 @@ void allow_wide_clusters()
     cudaFuncSetAttribute(leaf_lu_kernel<T, W, RPT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 
+template <typename T, int W, int RPT, int CB>
+void allow_wide_updates()
+{
+    cudaFuncSetAttribute(leaf_update_kernel<T, W, RPT, CB>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+
 // largest leaf cluster the device co-schedules: 16 CTAs (non-portable) or 8;
 // worked out once per device and precision
 template <typename T>
@@ -807,6 +1076,10 @@ int configure(Lu<T>& lu)
     allow_wide_clusters<T, 16, 2>();
     allow_wide_clusters<T, 8, 4>();
     allow_wide_clusters<T, 4, 8>();
+    allow_wide_updates<T, 32, 1, 16>();
+    allow_wide_updates<T, 32, 2, 16>();
+    allow_wide_updates<T, 16, 4, 8>();
+    allow_wide_updates<T, 8, 8, 4>();
     lu.cluster = 16;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(16);
@@ -835,14 +1108,14 @@ struct LuGraphKey {
     int nrhs, nb;
     const int *ipiv, *perm, *info;
     bool factor, solve;
-    cudaStream_t main, side;
+    cudaStream_t main, side, aux;
     long wait_limit;
     int min_rpt;
     bool same(const LuGraphKey& o) const
     {
         return type == o.type && A == o.A && B == o.B && X == o.X && n == o.n && lda == o.lda && ldb == o.ldb &&
                ldx == o.ldx && nrhs == o.nrhs && nb == o.nb && ipiv == o.ipiv && perm == o.perm && info == o.info &&
-               factor == o.factor && solve == o.solve && main == o.main && side == o.side &&
+               factor == o.factor && solve == o.solve && main == o.main && side == o.side && aux == o.aux &&
                wait_limit == o.wait_limit && min_rpt == o.min_rpt;
     }
 };
@@ -901,7 +1174,7 @@ template <typename T>
 void lu_body(Lu<T>& lu, T* A, int64_t n, int64_t lda, const T* B, int64_t ldb, int nrhs, T* X, int64_t ldx,
              int* perm, int nb, bool factor, bool solve)
 {
-    if (factor) lu.factor(A, n, lda, nb);
+    if (factor) lu.factor(A, n, lda, nb, perm);
     lu.use(false);
     if (solve && nrhs > 0) lu.solve(A, n, lda, B, ldb, nrhs, X, ldx, perm);
 }
@@ -962,9 +1235,11 @@ int lu_factor_solve(const LuStreams& s, T* A, int64_t n, int64_t lda, const T* B
     lu.main_st = s.main;
     // without a side stream the look-ahead degenerates to one in-order stream
     lu.side_st = s.side ? s.side : s.main;
+    lu.aux_st = s.side && s.aux && s.naux > 0 ? s.aux[0] : nullptr;
     lu.use(false);
     lu.ipiv = ipiv;
     lu.info = info;
+    lu.moved = info + 1;
     lu.wait_limit = s.wait_limit > 0 ? s.wait_limit : kDefaultWaitLimit;
     lu.min_rpt = (s.min_leaf_rpt == 2 || s.min_leaf_rpt == 4) ? s.min_leaf_rpt : 1;
     configure(lu);
@@ -980,7 +1255,7 @@ int lu_factor_solve(const LuStreams& s, T* A, int64_t n, int64_t lda, const T* B
                            cudaStreamIsCapturing(s.main, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
     if (cacheable) {
         const LuGraphKey key{(int)sizeof(T), A, B, X, n, lda, ldb, ldx, nrhs, nb, ipiv, perm, info, factor, solve,
-                             lu.main_st, lu.side_st, lu.wait_limit, lu.min_rpt};
+                             lu.main_st, lu.side_st, lu.aux_st, lu.wait_limit, lu.min_rpt};
         entry = s.graphs->find(key);
         if (entry && entry->exec) {   // replay
             if (cudaGraphLaunch(entry->exec, lu.main_st) != cudaSuccess) return LU_CUDA_ERROR;
@@ -1016,7 +1291,7 @@ __global__ void set_ints_kernel(int* p, int n, int v)
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = v;
 }
 
-// perm of every system from its pivots: one CTA per system, in shared memory
+// perm of every system from its pivots: one CTA per system
 struct PermRec {
     const int* ipiv;
     int* perm;
@@ -1028,19 +1303,8 @@ struct PermGroup {
 };
 __global__ void __launch_bounds__(1024) perm_group_kernel(const __grid_constant__ PermGroup g)
 {
-    extern __shared__ int s_perm[];
     const PermRec& r = g.rec[blockIdx.x];
-    for (int i = threadIdx.x; i < r.n; i += blockDim.x) s_perm[i] = i;
-    __syncthreads();
-    if (threadIdx.x == 0)
-        for (int k = 0; k < r.n; ++k) {
-            const int q = r.ipiv[k];
-            const int t = s_perm[k];
-            s_perm[k] = s_perm[q];
-            s_perm[q] = t;
-        }
-    __syncthreads();
-    for (int i = threadIdx.x; i < r.n; i += blockDim.x) r.perm[i] = s_perm[i];
+    perm_body(r.ipiv, r.n, r.perm);
 }
 
 // The blocked right-looking LU of csrc/lu.cu's Lu::factor over many systems
@@ -1370,29 +1634,16 @@ int lu_group_max_rows()
 int lu_pivots_to_perm_group(cudaStream_t st, const std::vector<GroupSystem>& sys, const std::vector<int*>& perms,
                             int64_t* launches)
 {
-    int nmax = 0;
-    for (const auto& y : sys) nmax = y.n_pad > nmax ? y.n_pad : nmax;
-    const size_t smem = (size_t)nmax * sizeof(int);
-    if (cudaFuncSetAttribute(perm_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return LU_CUDA_ERROR;
     PermGroup g{};
     for (size_t p = 0; p <= sys.size(); ++p) {
         if (g.count == kGroupMax || (p == sys.size() && g.count > 0)) {
-            perm_group_kernel<<<(unsigned)g.count, 1024, smem, st>>>(g);
+            perm_group_kernel<<<(unsigned)g.count, 1024, 0, st>>>(g);
             if (launches) ++*launches;
             if (cudaGetLastError() != cudaSuccess) return LU_CUDA_ERROR;
             g.count = 0;
         }
         if (p < sys.size()) g.rec[g.count++] = PermRec{sys[p].ipiv, perms[p], sys[p].n_pad, 0};
     }
-    return LU_OK;
-}
-
-int lu_pivots_to_perm(const LuStreams& s, const int* ipiv, int64_t n, int* perm)
-{
-    if (n <= 0) return LU_OK;
-    if (launch_pivots_to_perm(s.main, ipiv, n, perm) != cudaSuccess) return LU_CUDA_ERROR;
-    if (s.launches) ++*s.launches;
     return LU_OK;
 }
 

@@ -32,7 +32,9 @@ struct LuStreams {
     long wait_limit = 0;     // polls a device wait makes before it gives up (0: kDefaultWaitLimit)
     int min_leaf_rpt = 1;    // fewest rows per leaf thread (1, 2, 4): leaves of 32 / rpt columns
     // grouped factorisations: streams on which the leaf launches of different
-    // cluster sizes run side by side (none: one after the other on main)
+    // cluster sizes run side by side (none: one after the other on main);
+    // single factorisations: the first takes the next block column's leaf
+    // updates (none: on main)
     cudaStream_t* aux = nullptr;
     int naux = 0;
 };
@@ -40,11 +42,17 @@ struct LuStreams {
 // Polls of a device-side wait (a pivot exchange, a chain flag) before the
 // kernel gives up, records the failure in the info word and returns.
 constexpr long kDefaultWaitLimit = 1L << 22;
+// ints behind an lu_factor_solve info pointer: the result, then 64 per leaf of
+// the widest panel (1024 columns in leaves of at least 4)
+constexpr int kLuInfoInts = 1 + 64 * 256;
 
 // Factorise A (n x n, lda, column-major) in place (if factor) and / or solve
 // A X = B with the factors (if solve).  ipiv (n ints), perm (n ints) and info
-// (1 int) are device memory; info ends as INT_MAX when every pivot is
-// non-zero, else the 1-based column of the first zero pivot.  nb: outer block
+// (kLuInfoInts ints, the first the result, the others workspace) are device
+// memory; info ends as INT_MAX when every pivot is non-zero, else the 1-based
+// column of the first zero pivot.  A factorisation also leaves perm: perm[i] =
+// row of the original matrix that the factors' row i came from; a solve alone
+// takes it from there.  nb: outer block
 // width (1..1024).
 // The single-precision variant runs its GEMMs on TF32 tensor cores.
 template <typename T>
@@ -52,7 +60,7 @@ int lu_factor_solve(const LuStreams& s, T* A, int64_t n, int64_t lda, const T* B
                     int64_t ldx, int* ipiv, int* perm, int* info, int nb, bool factor, bool solve);
 
 // x = U^-1 L^-1 P b for one right-hand side with the FP64 factors in A
-// (lda), perm from lu_pivots_to_perm: two ticket-ordered chain launches
+// (lda), perm from lu_factor_solve: two ticket-ordered chain launches
 // (csrc/trsv.cu).  y: n doubles of workspace; sync: lu_chain_sync_ints(n)
 // ints; a dependency wait that runs out sets *info to -1.
 cudaError_t lu_solve_chain_f64(cudaStream_t st, const double* A, int64_t lda, int64_t n, const int* perm,
@@ -64,10 +72,6 @@ cudaError_t lu_solve_chain_f64(cudaStream_t st, const double* A, int64_t lda, in
 cudaError_t lu_chain_timeout_probe(cudaStream_t st, const double* A, int64_t lda, int64_t n, const int* perm,
                                    const double* b, double* y, double* x, int* sync, int* info, long wait_limit);
 size_t lu_chain_sync_ints(int64_t n);
-
-// perm[i] = row of the original matrix that the factorisation's row i came
-// from (the pivots applied in order); perm: n ints, device.
-int lu_pivots_to_perm(const LuStreams& s, const int* ipiv, int64_t n, int* perm);
 
 // One FP32 system of a grouped factorisation: A (n_pad x n_pad, lda), n_pad a
 // multiple of the block width (the caller pads a system with the identity),

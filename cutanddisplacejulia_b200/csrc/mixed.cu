@@ -243,9 +243,7 @@ int mixed_prepare(const LuStreams& ls, const double* A, int64_t lda, int64_t n, 
                                                                                                      A32, ld);
     if (cudaGetLastError() != cudaSuccess) return LU_CUDA_ERROR;
     if (ls.launches) ++*ls.launches;
-    int rc = lu_factor_solve<float>(ls, A32, n, ld, nullptr, 0, 0, nullptr, 0, ipiv, perm, info, nb, true, false);
-    if (rc != LU_OK) return rc;
-    rc = lu_pivots_to_perm(ls, ipiv, n, perm);
+    const int rc = lu_factor_solve<float>(ls, A32, n, ld, nullptr, 0, 0, nullptr, 0, ipiv, perm, info, nb, true, false);
     if (rc != LU_OK || !inverses) return rc;
     const int nblk = (int)((n + kRB - 1) / kRB);
     const size_t smem = (size_t)(kRB * kRB + kRB * (kRB + 1)) * sizeof(float);
