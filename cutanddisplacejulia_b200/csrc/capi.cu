@@ -266,7 +266,7 @@ int td_device(cad_ctx* ctx, const double* X, const double* Y, const double* Z, i
     void* tri;
     if (int r = ensure(ctx, S_TRI, (size_t)N * tri_record_bytes(), &tri)) return r;
     ++ctx->launches;
-    CK(launch_td_setup(P1, P2, P3, N, Dss, Dds, Dn, 1, nu, hs == 1, (TriDev*)tri, ctx->stream));
+    CK(launch_td_setup(P1, P2, P3, N, Dss, Dds, Dn, 1, nu, hs == 1, (TriDev*)tri, ctx->stream, !et.use));
     PairArgs a{};
     a.X = X; a.Y = Y; a.Z = Z; a.M = M; a.tri = (const TriDev*)tri; a.N = N;
     a.tri_chunk = pick_chunk(M, N, out_kind == OUT_SUM);
@@ -347,7 +347,8 @@ int assemble_device(cad_ctx* ctx, const double* normals, const double* mid, cons
     void* tri;
     if (int r = ensure(ctx, S_TRI, (size_t)N * tri_record_bytes(), &tri)) return r;
     ++ctx->launches;
-    CK(launch_td_setup(P1, P2, P3, N, nullptr, nullptr, nullptr, 1, nu, hs == 1, (TriDev*)tri, ctx->stream));
+    CK(launch_td_setup(P1, P2, P3, N, nullptr, nullptr, nullptr, 1, nu, hs == 1, (TriDev*)tri, ctx->stream,
+                       !et.use));
     PairArgs a{};
     a.X = X; a.Y = X + N; a.Z = X + 2 * N; a.M = N; a.tri = (const TriDev*)tri; a.N = N;
     a.tri_chunk = pick_chunk(N, N, false);
@@ -1530,7 +1531,12 @@ static int assemble_fixed_device(cad_ctx* ctx, const double* g, int64_t N, doubl
         PairArgs a{};
         const double* fo = (const double*)fobs;
         a.X = fo; a.Y = fo + nfix; a.Z = fo + 2 * nfix; a.M = nfix;
-        a.tri = (const TriDev*)ctx->buf[S_TRI].p; a.N = N;   // unit-slip records of assemble_device
+        a.tri = (const TriDev*)ctx->buf[S_TRI].p; a.N = N;
+        // unit-slip records again, with their sides: assemble_device leaves
+        // them out where the mesh's edges carry the half-space terms
+        ++ctx->launches;
+        CK(launch_td_setup(g, g + 3 * N, g + 6 * N, N, nullptr, nullptr, nullptr, 1, nu, hs == 1,
+                           (TriDev*)ctx->buf[S_TRI].p, ctx->stream));
         a.tri_chunk = pick_chunk(nfix, N, false);
         a.disp = (double*)fdisp;
         ++ctx->launches;

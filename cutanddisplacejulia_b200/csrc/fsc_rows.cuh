@@ -15,110 +15,111 @@ struct FscRows {
 
 CAD_HD void fsc_rows_setup(double s, double c, double nu, FscRows<double>& k)
 {
-    k.e[0] = (1.0/2.0)*c*(2*nu - 1)*(-c*c)/s;
+    const double is = 1.0 / s, is2 = is * is;
+    k.e[0] = 0.5*c*(2*nu - 1)*(-c*c)*is;
     k.e[1] = -c*(-c*c);
-    k.e[2] = (1.0/2.0)*(2*nu - 1)*(5*nu*(s*s) - 4*nu - 4*(s*s) + 4)/(s*s);
-    k.e[3] = c*(2*nu - 1)*(-c*c)*(-2*nu + (s*s) + 2)/(s*s);
-    k.e[4] = (1.0/4.0)*(2*nu - 1)*(4*(s*s) - 3);
-    k.e[5] = -1.0/4.0*(-8*nu*(s*s) + 6*nu + 5*(s*s*s*s) - 2*(s*s) - 3);
-    k.e[6] = -1.0/2.0*c*(-c*c)*(-2*nu + 2*(s*s) + 1)/s;
-    k.e[7] = (1.0/4.0)*c*s*(3*(s*s) - 7);
-    k.e[8] = (1.0/4.0)*(s*s)*(3*(s*s) - 2);
-    k.e[9] = (1.0/2.0)*c*(2*nu - 1)/s;
+    k.e[2] = 0.5*(2*nu - 1)*(5*nu*(s*s) - 4*nu - 4*(s*s) + 4)*is2;
+    k.e[3] = c*(2*nu - 1)*(-c*c)*(-2*nu + (s*s) + 2)*is2;
+    k.e[4] = 0.25*(2*nu - 1)*(4*(s*s) - 3);
+    k.e[5] = -0.25*(-8*nu*(s*s) + 6*nu + 5*(s*s*s*s) - 2*(s*s) - 3);
+    k.e[6] = -0.5*c*(-c*c)*(-2*nu + 2*(s*s) + 1)*is;
+    k.e[7] = 0.25*c*s*(3*(s*s) - 7);
+    k.e[8] = 0.25*(s*s)*(3*(s*s) - 2);
+    k.e[9] = 0.5*c*(2*nu - 1)*is;
     k.e[10] = -c;
-    k.e[11] = -1.0/2.0*(2*nu - 1)*(nu*(s*s) - 4*nu - 4*(s*s) + 4)/(s*s);
-    k.e[12] = -c*(2*nu - 1)*(2*nu + (s*s) - 2)/(s*s);
-    k.e[13] = (3.0/4.0)*(2*nu - 1);
-    k.e[14] = (3.0/4.0)*(2*nu + (s*s) - 1);
-    k.e[15] = (3.0/4.0)*c*s;
-    k.e[16] = (3.0/4.0)*(s*s);
-    k.e[17] = (1.0/2.0)*c*s*(2*nu - 1);
+    k.e[11] = -0.5*(2*nu - 1)*(nu*(s*s) - 4*nu - 4*(s*s) + 4)*is2;
+    k.e[12] = -c*(2*nu - 1)*(2*nu + (s*s) - 2)*is2;
+    k.e[13] = 0.75*(2*nu - 1);
+    k.e[14] = 0.75*(2*nu + (s*s) - 1);
+    k.e[15] = 0.75*c*s;
+    k.e[16] = 0.75*(s*s);
+    k.e[17] = 0.5*c*s*(2*nu - 1);
     k.e[18] = c*(s*s);
     k.e[19] = 2*nu*(2*nu - 1);
     k.e[20] = c*(-2*nu + (s*s))*(2*nu - 1);
     k.e[21] = (s*s)*(2*nu - 1);
-    k.e[22] = (1.0/4.0)*(s*s)*(-8*nu + 5*(s*s) - 5);
-    k.e[23] = (1.0/2.0)*c*s*(-2*nu + 2*(s*s) - 1);
-    k.e[24] = -1.0/4.0*c*s*(3*(s*s) - 4);
-    k.e[25] = -1.0/4.0*(s*s)*(3*(s*s) + 1);
-    k.e[26] = -1.0/2.0*(2*nu - 1)*(-c*c)/s;
+    k.e[22] = 0.25*(s*s)*(-8*nu + 5*(s*s) - 5);
+    k.e[23] = 0.5*c*s*(-2*nu + 2*(s*s) - 1);
+    k.e[24] = -0.25*c*s*(3*(s*s) - 4);
+    k.e[25] = -0.25*(s*s)*(3*(s*s) + 1);
+    k.e[26] = -0.5*(2*nu - 1)*(-c*c)*is;
     k.e[27] = (-c*c);
-    k.e[28] = (1.0/2.0)*c*(2*nu - 1)*(2*nu + (s*s) - 2)/s;
-    k.e[29] = -1.0/2.0*(2*nu - 1)*(3*nu*(s*s) - 4*nu - 4*(s*s) + 4)/(s*s);
-    k.e[30] = 2*(nu - 1)*(2*nu - 1)*(-c*c)/(s*s);
-    k.e[31] = -1.0/4.0*(2*nu - 1)*(2*(s*s) - 3);
-    k.e[32] = (1.0/4.0)*(-4*nu*(s*s) + 6*nu + (s*s*s*s) + 2*(s*s) - 3);
-    k.e[33] = -1.0/4.0*c*s*(-4*nu + (s*s) + 1);
-    k.e[34] = (1.0/2.0)*(-c*c)*(-2*nu + (s*s) + 1)/s;
-    k.e[35] = -1.0/2.0*c*s*(-c*c);
-    k.e[36] = -1.0/4.0*(s*s)*(2*(s*s) - 3);
-    k.e[37] = -1.0/4.0*c*s*((s*s) + 3);
+    k.e[28] = 0.5*c*(2*nu - 1)*(2*nu + (s*s) - 2)*is;
+    k.e[29] = -0.5*(2*nu - 1)*(3*nu*(s*s) - 4*nu - 4*(s*s) + 4)*is2;
+    k.e[30] = 2*(nu - 1)*(2*nu - 1)*(-c*c)*is2;
+    k.e[31] = -0.25*(2*nu - 1)*(2*(s*s) - 3);
+    k.e[32] = 0.25*(-4*nu*(s*s) + 6*nu + (s*s*s*s) + 2*(s*s) - 3);
+    k.e[33] = -0.25*c*s*(-4*nu + (s*s) + 1);
+    k.e[34] = 0.5*(-c*c)*(-2*nu + (s*s) + 1)*is;
+    k.e[35] = -0.5*c*s*(-c*c);
+    k.e[36] = -0.25*(s*s)*(2*(s*s) - 3);
+    k.e[37] = -0.25*c*s*((s*s) + 3);
     k.e[38] = -s*(-c*c);
-    k.e[39] = (1.0/4.0)*c*s*(-8*nu + 5*(s*s) - 1);
+    k.e[39] = 0.25*c*s*(-8*nu + 5*(s*s) - 1);
     k.e[40] = -(-nu + (s*s))*(-c*c);
-    k.e[41] = (1.0/4.0)*(s*s)*(3*(s*s) - 7);
-    k.e[42] = -1.0/4.0*c*s*(3*(s*s) + 1);
+    k.e[41] = 0.25*(s*s)*(3*(s*s) - 7);
+    k.e[42] = -0.25*c*s*(3*(s*s) + 1);
     k.e[43] = -c*s;
-    k.e[44] = -1.0/4.0*(s*s)*(-4*nu + (s*s) - 1);
-    k.e[45] = -1.0/2.0*c*(-2*nu + (s*s));
-    k.e[46] = -1.0/2.0*(s*s)*(-c*c);
-    k.e[47] = (1.0/4.0)*c*s*(2*(s*s) - 1);
-    k.e[48] = -1.0/4.0*(s*s)*((s*s) + 3);
-    k.e[49] = -1.0/2.0*c*(2*nu - 1)*(4*nu*(s*s) - 2*nu - (s*s) + 2)/s;
-    k.e[50] = -1.0/2.0*(2*nu - 1)*(7*nu*(s*s) - 4*nu - 4*(s*s) + 4)/(s*s);
-    k.e[51] = -2*(2*nu - 1)*(-c*c)*(nu*(s*s) - nu + 1)/(s*s);
-    k.e[52] = (1.0/4.0)*(4*nu*(s*s*s*s) - 16*nu*(s*s) + 6*nu + (s*s*s*s) + 2*(s*s) - 3);
-    k.e[53] = -1.0/4.0*c*s*(4*nu*(s*s) + (s*s) + 1);
-    k.e[54] = (1.0/2.0)*(-c*c)*(2*nu*(s*s) - 2*nu + (s*s) + 1)/s;
-    k.e[55] = -1.0/2.0*(2*nu - 1)/s;
-    k.e[56] = -c*(nu - 1)*(2*nu - 1)/s;
-    k.e[57] = (1.0/4.0)*(4*nu*(s*s) - 6*nu - 3*(s*s) + 3);
-    k.e[58] = -1.0/4.0*c*s*(4*nu - 3);
-    k.e[59] = -1.0/2.0*c*s;
-    k.e[60] = -1.0/2.0*(s*s);
-    k.e[61] = -1.0/4.0*c*s;
-    k.e[62] = -1.0/2.0*s*(2*nu - 1);
+    k.e[44] = -0.25*(s*s)*(-4*nu + (s*s) - 1);
+    k.e[45] = -0.5*c*(-2*nu + (s*s));
+    k.e[46] = -0.5*(s*s)*(-c*c);
+    k.e[47] = 0.25*c*s*(2*(s*s) - 1);
+    k.e[48] = -0.25*(s*s)*((s*s) + 3);
+    k.e[49] = -0.5*c*(2*nu - 1)*(4*nu*(s*s) - 2*nu - (s*s) + 2)*is;
+    k.e[50] = -0.5*(2*nu - 1)*(7*nu*(s*s) - 4*nu - 4*(s*s) + 4)*is2;
+    k.e[51] = -2*(2*nu - 1)*(-c*c)*(nu*(s*s) - nu + 1)*is2;
+    k.e[52] = 0.25*(4*nu*(s*s*s*s) - 16*nu*(s*s) + 6*nu + (s*s*s*s) + 2*(s*s) - 3);
+    k.e[53] = -0.25*c*s*(4*nu*(s*s) + (s*s) + 1);
+    k.e[54] = 0.5*(-c*c)*(2*nu*(s*s) - 2*nu + (s*s) + 1)*is;
+    k.e[55] = -0.5*(2*nu - 1)*is;
+    k.e[56] = -c*(nu - 1)*(2*nu - 1)*is;
+    k.e[57] = 0.25*(4*nu*(s*s) - 6*nu - 3*(s*s) + 3);
+    k.e[58] = -0.25*c*s*(4*nu - 3);
+    k.e[59] = -0.5*c*s;
+    k.e[60] = -0.5*(s*s);
+    k.e[61] = -0.25*c*s;
+    k.e[62] = -0.5*s*(2*nu - 1);
     k.e[63] = -(s*s);
-    k.e[64] = -1.0/2.0*c*s*(2*nu - 1)*(4*nu - 1);
+    k.e[64] = -0.5*c*s*(2*nu - 1)*(4*nu - 1);
     k.e[65] = -2*nu*(2*nu - 1)*(-c*c);
-    k.e[66] = -1.0/2.0*(s*s)*(2*nu - 1);
-    k.e[67] = -1.0/4.0*(s*s)*(4*nu*(s*s) - 12*nu + (s*s) - 1);
-    k.e[68] = (1.0/4.0)*c*s*(4*nu*(s*s) + 4*nu + (s*s) - 2);
-    k.e[69] = -1.0/2.0*s*(2*nu + 1)*(-c*c);
-    k.e[70] = (1.0/2.0)*c*(s*s*s);
-    k.e[71] = (1.0/4.0)*(s*s)*(2*(s*s) - 1);
-    k.e[72] = (1.0/4.0)*c*s*((s*s) + 4);
-    k.e[73] = c*(2*nu - 1)*(2*nu*(s*s) - 2*nu - (s*s) + 2)/(s*s);
-    k.e[74] = -1.0/4.0*(8*nu*(s*s) - 6*nu - 3*(s*s) + 3);
-    k.e[75] = -1.0/2.0*c*(2*nu*(s*s) - 2*nu + 1)/s;
-    k.e[76] = -1.0/4.0*c*s*(4*nu*(s*s) - 12*nu + (s*s) + 1);
-    k.e[77] = -1.0/4.0*(s*s)*(4*nu*(s*s) + (s*s) - 1);
-    k.e[78] = -1.0/2.0*c*(2*nu*(s*s) - 2*nu + (s*s));
+    k.e[66] = -0.5*(s*s)*(2*nu - 1);
+    k.e[67] = -0.25*(s*s)*(4*nu*(s*s) - 12*nu + (s*s) - 1);
+    k.e[68] = 0.25*c*s*(4*nu*(s*s) + 4*nu + (s*s) - 2);
+    k.e[69] = -0.5*s*(2*nu + 1)*(-c*c);
+    k.e[70] = 0.5*c*(s*s*s);
+    k.e[71] = 0.25*(s*s)*(2*(s*s) - 1);
+    k.e[72] = 0.25*c*s*((s*s) + 4);
+    k.e[73] = c*(2*nu - 1)*(2*nu*(s*s) - 2*nu - (s*s) + 2)*is2;
+    k.e[74] = -0.25*(8*nu*(s*s) - 6*nu - 3*(s*s) + 3);
+    k.e[75] = -0.5*c*(2*nu*(s*s) - 2*nu + 1)*is;
+    k.e[76] = -0.25*c*s*(4*nu*(s*s) - 12*nu + (s*s) + 1);
+    k.e[77] = -0.25*(s*s)*(4*nu*(s*s) + (s*s) - 1);
+    k.e[78] = -0.5*c*(2*nu*(s*s) - 2*nu + (s*s));
     k.e[79] = -s;
-    k.e[80] = (1.0/4.0)*c*s*(8*nu - 3);
+    k.e[80] = 0.25*c*s*(8*nu - 3);
     k.e[81] = -nu*(-c*c);
-    k.e[82] = -1.0/2.0*(2*nu - 1)*(-c*c);
+    k.e[82] = -0.5*(2*nu - 1)*(-c*c);
     k.e[83] = -s*(2*nu - 1)*(-c*c);
     k.e[84] = c*s*(2*nu - 1);
-    k.e[85] = -5.0/4.0*c*s*(-c*c);
-    k.e[86] = (1.0/2.0)*(-c*c)*(2*(s*s) - 1);
-    k.e[87] = -1.0/2.0*(2*nu - 1);
+    k.e[85] = -1.25*c*s*(-c*c);
+    k.e[86] = 0.5*(-c*c)*(2*(s*s) - 1);
+    k.e[87] = -0.5*(2*nu - 1);
     k.e[88] = s*(2*nu - 1);
-    k.e[89] = -1.0/2.0;
+    k.e[89] = -0.5;
     k.e[90] = -(s*s*s);
     k.e[91] = -s*(2*nu - 1)*((s*s) - 2);
-    k.e[92] = (1.0/4.0)*c*s*(5*(s*s) - 8);
-    k.e[93] = -1.0/2.0*(s*s)*(2*(s*s) - 3);
-    k.e[94] = (1.0/4.0)*(s*s)*(3*(s*s) - 4);
-    k.e[95] = -1.0/4.0*c*s*(3*(s*s) + 4);
-    k.e[96] = -1.0/2.0*c*(2*nu - 1);
-    k.e[97] = (1.0/4.0)*c*s*(-c*c);
-    k.e[98] = (1.0/4.0)*(s*s)*((s*s) - 3);
-    k.e[99] = (1.0/2.0)*c*(-c*c);
-    k.e[100] = -1.0/4.0*(s*s)*(5*(s*s) - 9);
+    k.e[92] = 0.25*c*s*(5*(s*s) - 8);
+    k.e[93] = -0.5*(s*s)*(2*(s*s) - 3);
+    k.e[94] = 0.25*(s*s)*(3*(s*s) - 4);
+    k.e[95] = -0.25*c*s*(3*(s*s) + 4);
+    k.e[96] = -0.5*c*(2*nu - 1);
+    k.e[97] = 0.25*c*s*(-c*c);
+    k.e[98] = 0.25*(s*s)*((s*s) - 3);
+    k.e[99] = 0.5*c*(-c*c);
+    k.e[100] = -0.25*(s*s)*(5*(s*s) - 9);
     k.e[101] = -c*s*(-c*c);
-    k.e[102] = -1.0/4.0*c*s*(s - 2)*(s + 2);
-    k.e[103] = (1.0/2.0)*s*((s*s) - 2);
+    k.e[102] = -0.25*c*s*(s - 2)*(s + 2);
+    k.e[103] = 0.5*s*((s*s) - 2);
 }
 
 template <typename T>
@@ -128,38 +129,39 @@ struct FscDispRows {
 
 CAD_HD void fsc_rows_setup(double s, double c, double nu, FscDispRows<double>& k)
 {
-    k.d[0] = 2*(nu - 1)*(2*nu - 1)*(-c*c)/(s*s);
-    k.d[1] = (2*nu - 1)*(-c*c)/s;
-    k.d[2] = -1.0/2.0*(-c*c);
-    k.d[3] = -(-c*c)*(-2*nu + (s*s) + 1)/s;
+    const double is = 1.0 / s, is2 = is * is;
+    k.d[0] = 2*(nu - 1)*(2*nu - 1)*(-c*c)*is2;
+    k.d[1] = (2*nu - 1)*(-c*c)*is;
+    k.d[2] = -0.5*(-c*c);
+    k.d[3] = -(-c*c)*(-2*nu + (s*s) + 1)*is;
     k.d[4] = c*s;
-    k.d[5] = -(2*nu - 1)*(3*nu*(s*s) - 2*nu - 2*(s*s) + 2)/(s*s);
-    k.d[6] = c*(2*nu - 1)*(2*nu*(s*s) - 2*nu - (s*s) + 2)/(s*s);
-    k.d[7] = c*(2*nu - 1)/s;
-    k.d[8] = -1.0/2.0*c;
-    k.d[9] = -c*(2*nu*(s*s) - 2*nu + 1)/s;
-    k.d[10] = -1.0/2.0*(2*nu - 1);
-    k.d[11] = (1.0/2.0)*(4*nu*(s*s) - 2*nu - (s*s) + 1);
-    k.d[12] = -1.0/2.0*c*s;
-    k.d[13] = -1.0/2.0*(s*s);
+    k.d[5] = -(2*nu - 1)*(3*nu*(s*s) - 2*nu - 2*(s*s) + 2)*is2;
+    k.d[6] = c*(2*nu - 1)*(2*nu*(s*s) - 2*nu - (s*s) + 2)*is2;
+    k.d[7] = c*(2*nu - 1)*is;
+    k.d[8] = -0.5*c;
+    k.d[9] = -c*(2*nu*(s*s) - 2*nu + 1)*is;
+    k.d[10] = -0.5*(2*nu - 1);
+    k.d[11] = 0.5*(4*nu*(s*s) - 2*nu - (s*s) + 1);
+    k.d[12] = -0.5*c*s;
+    k.d[13] = -0.5*(s*s);
     k.d[14] = c*(2*nu - 1);
     k.d[15] = -c*(-c*c);
     k.d[16] = -(s*s);
-    k.d[17] = -(2*nu - 1)*(nu*(s*s) - 2*nu - 2*(s*s) + 2)/(s*s);
-    k.d[18] = -c*(2*nu - 1)*(2*nu + (s*s) - 2)/(s*s);
-    k.d[19] = -1.0/2.0*(2*nu + (s*s) - 1);
-    k.d[20] = (2*nu - 1)/s;
-    k.d[21] = -1.0/2.0;
+    k.d[17] = -(2*nu - 1)*(nu*(s*s) - 2*nu - 2*(s*s) + 2)*is2;
+    k.d[18] = -c*(2*nu - 1)*(2*nu + (s*s) - 2)*is2;
+    k.d[19] = -0.5*(2*nu + (s*s) - 1);
+    k.d[20] = (2*nu - 1)*is;
+    k.d[21] = -0.5;
     k.d[22] = s*(2*nu - 1);
     k.d[23] = 1 - 2*nu;
-    k.d[24] = (1.0/2.0)*s;
-    k.d[25] = 2*c*(nu - 1)*(2*nu - 1)/s;
+    k.d[24] = 0.5*s;
+    k.d[25] = 2*c*(nu - 1)*(2*nu - 1)*is;
     k.d[26] = 2*c*(nu - 1);
     k.d[27] = c*(-2*nu + (s*s));
-    k.d[28] = -2*(nu - 1)*(2*nu - 1)*(-c*c)/s;
+    k.d[28] = -2*(nu - 1)*(2*nu - 1)*(-c*c)*is;
     k.d[29] = -2*(nu - 1);
     k.d[30] = -2*nu*(-c*c);
-    k.d[31] = -1.0/2.0*c*s*(4*nu - 1);
+    k.d[31] = -0.5*c*s*(4*nu - 1);
     k.d[32] = -2*s*(nu - 1);
     k.d[33] = -s*((s*s) - 2);
 }

@@ -296,11 +296,15 @@ def emit():
     for name, C in (("FscRows", K), ("FscDispRows", KD)):
         L += ["template <typename T>", "struct %s {" % name]
         L += ["    T %s[%d];" % (C.prefix, len(C.order)), "};", ""]
-        L += ["CAD_HD void fsc_rows_setup(double s, double c, double nu, %s<double>& k)" % name, "{"]
+        L += ["CAD_HD void fsc_rows_setup(double s, double c, double nu, %s<double>& k)" % name, "{",
+              "    const double is = 1.0 / s, is2 = is * is;"]
         for co in C.order:
             txt = sp.ccode(sp.factor(co)).replace("(s - 1)*(s + 1)", "(-c*c)")
             for p in (2, 3, 4):
                 txt = txt.replace("pow(s, %d)" % p, "(%s)" % "*".join("s" * p))
+            txt = txt.replace("/(s*s)", "*is2").replace("/s", "*is")
+            txt = txt.replace("(1.0/2.0)", "0.5").replace("1.0/2.0", "0.5").replace("(1.0/4.0)", "0.25").replace(
+                "1.0/4.0", "0.25").replace("(3.0/4.0)", "0.75").replace("3.0/4.0", "0.75").replace("5.0/4.0", "1.25")
             L.append("    k.%s = %s;" % (C.of[sp.expand(co)], txt))
         L += ["}", ""]
     L += ["template <typename R>", "CAD_HD void fsc_rows(const FscRows<R>& k, const FscAcc<R>& a, R z, R e[3][6])", "{",

@@ -1356,8 +1356,10 @@ CAD_HD void pair_net(const TriDev& t, double X, double Y, double Z, double E[6],
     if (HS) td_net<STRAIN, DISP>(t.image, X, Y, Z, t.Dn, t.Dss, t.Dds, t.K8, E, U);
 }
 
+// sides = false leaves the half-space sides unset (their fields come from the
+// mesh's edges).
 CAD_HD void build_triangle(const double a[3], const double b[3], const double c[3], double Dss, double Dds,
-                           double Dn, double nu, bool hs, TriDev& t)
+                           double Dn, double nu, bool hs, TriDev& t, bool sides = true)
 {
     t.Dss = Dss;
     t.Dds = Dds;
@@ -1367,6 +1369,7 @@ CAD_HD void build_triangle(const double a[3], const double b[3], const double c[
     if (!hs) return;
     const double ai[3] = {a[0], a[1], -a[2]}, bi[3] = {b[0], b[1], -b[2]}, ci[3] = {c[0], c[1], -c[2]};
     build_frame(ai, bi, ci, t.image);
+    if (!sides) return;
     build_side(a, b, t.real, t.Dss, t.Dds, t.Dn, nu, t.side[0]);
     build_side(b, c, t.real, t.Dss, t.Dds, t.Dn, nu, t.side[1]);
     build_side(c, a, t.real, t.Dss, t.Dds, t.Dn, nu, t.side[2]);

@@ -30,7 +30,7 @@ namespace cad {
 __global__ void td_setup_kernel(const double* __restrict__ P1, const double* __restrict__ P2,
                                 const double* __restrict__ P3, int64_t N, const double* __restrict__ Dss,
                                 const double* __restrict__ Dds, const double* __restrict__ Dn, int64_t slip_stride,
-                                double nu, int hs, TriDev* __restrict__ out)
+                                double nu, int hs, int sides, TriDev* __restrict__ out)
 {
     const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= N) return;
@@ -39,7 +39,7 @@ __global__ void td_setup_kernel(const double* __restrict__ P1, const double* __r
     const double b[3] = {P2[j], P2[j + N], P2[j + 2 * N]};
     const double c[3] = {P3[j], P3[j + N], P3[j + 2 * N]};
     build_triangle(a, b, c, Dss ? Dss[j * slip_stride] : 1.0, Dds ? Dds[j * slip_stride] : 1.0,
-                   Dn ? Dn[j * slip_stride] : 1.0, nu, hs != 0, t);
+                   Dn ? Dn[j * slip_stride] : 1.0, nu, hs != 0, t, sides != 0);
 }
 
 // ------------------------------------------------ half-space argument check
@@ -640,7 +640,7 @@ cudaError_t launch_assemble_edges(PairArgs a, int out_kind, bool strain, bool di
     }
     if (a.M == 0 || a.N == 0) return cudaSuccess;
     if (E > 0) {
-        edge_setup_kernel<<<(unsigned)((E + 127) / 128), 128, 0, st>>>(edge_pts, E, nu, (FscSide*)edge_rec);
+        edge_setup_kernel<<<(unsigned)((E + 31) / 32), 32, 0, st>>>(edge_pts, E, nu, (FscSide*)edge_rec);
         if (launches) ++*launches;
         if (cudaError_t e = cudaGetLastError()) return e;
     }
@@ -814,7 +814,7 @@ cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, bool full, c
     else
         e = pairs(td_pair_kernel<true, false, true, OUT_SUM, false, false, 1, EDGE_FSC>);
     if (e != cudaSuccess || E == 0) return e;
-    edge_burgers_kernel<<<(unsigned)((E + 63) / 64), 64, 0, st>>>(ed.pts, E, ed.ptr, ed.cnt, ed.sides, a.tri, nu,
+    edge_burgers_kernel<<<(unsigned)((E + 31) / 32), 32, 0, st>>>(ed.pts, E, ed.ptr, ed.cnt, ed.sides, a.tri, nu,
                                                                    (FscSide*)edge_rec);
     if (launches) ++*launches;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -917,12 +917,12 @@ cudaError_t launch_assemble_update(PairArgs a, bool hs, const int* list, int64_t
 
 cudaError_t launch_td_setup(const double* P1, const double* P2, const double* P3, int64_t N, const double* Dss,
                             const double* Dds, const double* Dn, int64_t slip_stride, double nu, bool hs,
-                            TriDev* out, cudaStream_t st)
+                            TriDev* out, cudaStream_t st, bool sides)
 {
     if (N == 0) return cudaSuccess;
-    const int bs = 64;
+    const int bs = 32;   // a thread's chain bounds it: spread over the SMs
     td_setup_kernel<<<(unsigned)((N + bs - 1) / bs), bs, 0, st>>>(P1, P2, P3, N, Dss, Dds, Dn, slip_stride, nu,
-                                                                  hs ? 1 : 0, out);
+                                                                  hs ? 1 : 0, sides ? 1 : 0, out);
     return cudaGetLastError();
 }
 

@@ -112,7 +112,7 @@ size_t tri_record_bytes();
 
 cudaError_t launch_td_setup(const double* P1, const double* P2, const double* P3, int64_t N, const double* Dss,
                             const double* Dds, const double* Dn, int64_t slip_stride, double nu, bool hs,
-                            TriDev* out, cudaStream_t st);
+                            TriDev* out, cudaStream_t st, bool sides = true);   // sides: build_triangle's
 cudaError_t launch_td_pairs(const PairArgs& a, int out, bool hs, bool strain, bool disp, cudaStream_t st);
 // flag |= 1 when an observation z or a vertex z is above 0 (nz set: the
 // observation z is Z - 1e-12 nz); clear: zero the flag first.
