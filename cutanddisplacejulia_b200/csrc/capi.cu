@@ -39,7 +39,7 @@ size_t tri_record_bytes() { return sizeof(TriDev); }
 namespace {
 
 enum Slot {
-    S_OBS, S_GEOM, S_TRI, S_OUT, S_PART, S_DIRS, S_FLAG, S_A, S_B, S_WORK, S_PIV, S_INFO, S_PERM,
+    S_OBS, S_GEOM, S_BATCH, S_TRI, S_OUT, S_PART, S_DIRS, S_FLAG, S_A, S_B, S_WORK, S_PIV, S_INFO, S_PERM,
     S_A32, S_DINV, S_KRYLOV, S_VEC32, S_SYNC, S_TRI32, S_NEAR, S_IR, S_IR32, S_NORMS, S_REL, S_BGEOM, S_BTD, S_MLP,
     S_FIX, S_FOBS, S_FDISP, S_ATA, S_LIST, S_CHAIN, S_LCPJ, S_LCPC, S_LCPV, S_LCPP, S_GEMM, S_LPC_NET, S_LPC_WS, S_LPC_GEOM, S_LPC_TNBR, S_LPC_FEAT, S_LPC_OUT,
     S_LPC_NBR, S_LPC_BLK, S_LPC_MAT, S_LPC_PGEOM, S_BJ_NBR, S_BJ_BLK, S_KWORK, S_A32MV, S_TUNE, S_AT, S_G_A32, S_G_INT, S_G_F32, S_G_F64, S_G_MAPS,
@@ -67,18 +67,21 @@ struct Lane {
     DevBuf buf[L_COUNT];
 };
 constexpr int kLanes = 32;           // cracks of a batch in flight at once
-constexpr int kBatchSweeps = 4;      // refinement sweeps per crack inside the batch graph
+constexpr int kBatchSweeps = 4;      // refinement sweeps per crack before the residuals are read
 constexpr int kGroupBlock = 128;     // block width of the grouped FP32 factorisation (systems padded to it)
 constexpr int kGroupExtraRounds = 3; // rounds of two more grouped sweeps for cracks still above the tolerance
 constexpr int kLeafAux = 4;          // streams for the grouped leaves of different cluster sizes
 
-// The captured graph of the last batched call and what it was captured for.
+// The plan of the last batched call (sizes, settings, workspaces of the
+// context; inputs and results pass through such a workspace too, so any call
+// of the same sizes and settings replays it) and, from its second call on, its
+// captured graph.
 struct BatchGraph {
     cudaGraphExec_t exec = nullptr;
     std::vector<int64_t> offsets;
-    const void* ptrs[9] = {};
+    const void* ptrs[8] = {};
     double params[5] = {};
-    int flags[3] = {};
+    long flags[4] = {};
     int64_t launches = 0;
 };
 
@@ -906,26 +909,11 @@ int batch_body(cad_ctx* ctx, const BatchArgs& b, cudaEvent_t fork)
     return CAD_OK;
 }
 
-int slip_batched(cad_ctx* ctx, int64_t nbatch, const int64_t* offsets, const double* P1, const double* P2,
-                 const double* P3, const double* normals, const double* midpoints, double nu, double G, double lambda,
-                 int hs, const double* T, double* D, double* rel_host)
+// Solves the batch; P1 .. D lie in the context's workspace.
+int slip_batched_ws(cad_ctx* ctx, int64_t nbatch, const int64_t* offsets, const double* P1, const double* P2,
+                    const double* P3, const double* normals, const double* midpoints, double nu, double G,
+                    double lambda, int hs, const double* T, double* D, double* rel_host)
 {
-    if (nbatch == 0) return CAD_OK;
-    if (hs == 1) {   // every crack's vertices and collocation points at or below z = 0
-        void* flag;
-        if (int r = ensure(ctx, S_FLAG, sizeof(int), &flag)) return r;
-        CK(cudaMemsetAsync(flag, 0, sizeof(int), ctx->stream));
-        for (int64_t c = 0; c < nbatch; ++c) {
-            const int64_t o = offsets[c], N = offsets[c + 1] - o;
-            CK(launch_hs_check(midpoints + 3 * o + 2 * N, N, P1 + 3 * o, P2 + 3 * o, P3 + 3 * o, N, (int*)flag,
-                               ctx->stream, normals + 3 * o + 2 * N, false));
-        }
-        ctx->launches += nbatch;
-        int h = 0;
-        CK(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        if (h) return fail(ctx, CAD_ERR_HS_ABOVE_SURFACE, "Half-space solution: Z coordinates must be negative!");
-    }
     // sizes, matrix offsets, lanes (largest cracks first, each to the least
     // loaded lane), issue order (round robin over lanes)
     std::vector<int64_t> aoff((size_t)nbatch + 1, 0), byN((size_t)nbatch);
@@ -997,7 +985,7 @@ int slip_batched(cad_ctx* ctx, int64_t nbatch, const int64_t* offsets, const dou
                 &lane_of, &order, (double*)rel};
     std::vector<CrackRec> crecs;
     std::vector<GroupSystem> gsys;
-    void* ga32 = nullptr;
+    void *ga32 = nullptr, *gint = nullptr, *gf32 = nullptr, *gf64 = nullptr, *gmaps = nullptr;
     if (group) {
         // group buffers: FP32 systems back to back; ints = [every crack's sync
         // words][info per crack][GEMM status][pivots and permutation per
@@ -1020,7 +1008,6 @@ int slip_batched(cad_ctx* ctx, int64_t nbatch, const int64_t* offsets, const dou
             od[c] = nd;
             nd += 2 * np;
         }
-        void *gint, *gf32, *gf64, *gmaps;
         if (int r = ensure(ctx, S_G_A32, na * sizeof(float) + 16, &ga32)) return r;
         if (int r = ensure(ctx, S_G_INT, (ns + (size_t)nbatch + 1 + ni) * sizeof(int), &gint)) return r;
         if (int r = ensure(ctx, S_G_F32, nf * sizeof(float) + 16, &gf32)) return r;
@@ -1055,28 +1042,34 @@ int slip_batched(cad_ctx* ctx, int64_t nbatch, const int64_t* offsets, const dou
         b.gsync = sync_all;
         b.gsync_ints = ns;
     }
-    // the captured graph of an identical earlier call is replayed
+    // a plan seen for the second time is captured, then replayed; the first
+    // call is issued directly (34 ms for 64 cracks of 200 to 1500 elements,
+    // where capture and replay take 50 and the replay alone 32.5)
     BatchGraph& g = ctx->batch;
-    const void* ptrs[9] = {P1, P2, P3, normals, midpoints, T, D, Aall, ga32};
+    const void* ptrs[8] = {P1, Aall, rel, ga32, gint, gf32, gf64, gmaps};
     const double params[5] = {nu, G, lambda, ctx->tol, ctx->near_factor};
-    const int flags[3] = {hs, ctx->assembly, ctx->batch_mode};
-    const bool same = g.exec && g.offsets.size() == (size_t)nbatch + 1 &&
+    const long flags[4] = {hs, ctx->assembly, ctx->batch_mode, ctx->wait_limit};
+    const bool same = g.offsets.size() == (size_t)nbatch + 1 &&
                       std::equal(g.offsets.begin(), g.offsets.end(), offsets) &&
-                      std::equal(ptrs, ptrs + 9, g.ptrs) && std::equal(params, params + 5, g.params) &&
-                      std::equal(flags, flags + 3, g.flags);
+                      std::equal(ptrs, ptrs + 8, g.ptrs) && std::equal(params, params + 5, g.params) &&
+                      std::equal(flags, flags + 4, g.flags);
     cudaEvent_t fork = nullptr;
     CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
     int rc = CAD_OK;
-    if (same) {
+    if (!same) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        g.exec = nullptr;
+        g.offsets.assign(offsets, offsets + nbatch + 1);
+        std::copy(ptrs, ptrs + 8, g.ptrs);
+        std::copy(params, params + 5, g.params);
+        std::copy(flags, flags + 4, g.flags);
+    }
+    if (g.exec) {
         CK(cudaGraphLaunch(g.exec, ctx->stream));
         ctx->launches += g.launches;
-    } else if (ctx->stream == nullptr) {   // the legacy default stream cannot be captured: run directly
+    } else if (!same || ctx->stream == nullptr) {   // the legacy default stream cannot be captured
         rc = batch_body(ctx, b, fork);
     } else {
-        if (g.exec) {
-            cudaGraphExecDestroy(g.exec);
-            g.exec = nullptr;
-        }
         const int64_t l0 = ctx->launches;
         cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed);
         if (e != cudaSuccess) {
@@ -1093,14 +1086,11 @@ int slip_batched(cad_ctx* ctx, int64_t nbatch, const int64_t* offsets, const dou
         }
         if (graph) cudaGraphDestroy(graph);
         if (rc == CAD_OK) {
-            g.offsets.assign(offsets, offsets + nbatch + 1);
-            std::copy(ptrs, ptrs + 9, g.ptrs);
-            std::copy(params, params + 5, g.params);
-            std::copy(flags, flags + 3, g.flags);
             g.launches = ctx->launches - l0;
             e = cudaGraphLaunch(g.exec, ctx->stream);
             if (e != cudaSuccess) rc = cuda_fail(ctx, e, "batched solve: graph launch");
-        } else if (g.exec) {
+        }
+        if (rc != CAD_OK && g.exec) {
             cudaGraphExecDestroy(g.exec);
             g.exec = nullptr;
         }
@@ -1148,6 +1138,46 @@ int slip_batched(cad_ctx* ctx, int64_t nbatch, const int64_t* offsets, const dou
     if (rel_host) std::copy(hrel.begin(), hrel.end(), rel_host);
     if (!converged) return fail(ctx, CAD_ERR_NOT_CONVERGED, "batched solve: a crack did not reach the tolerance");
     return CAD_OK;
+}
+
+int slip_batched(cad_ctx* ctx, int64_t nbatch, const int64_t* offsets, const double* P1, const double* P2,
+                 const double* P3, const double* normals, const double* midpoints, double nu, double G, double lambda,
+                 int hs, const double* T, double* D, double* rel_host)
+{
+    if (nbatch == 0) return CAD_OK;
+    if (hs == 1) {   // every crack's vertices and collocation points at or below z = 0
+        void* flag;
+        if (int r = ensure(ctx, S_FLAG, sizeof(int), &flag)) return r;
+        CK(cudaMemsetAsync(flag, 0, sizeof(int), ctx->stream));
+        for (int64_t c = 0; c < nbatch; ++c) {
+            const int64_t o = offsets[c], N = offsets[c + 1] - o;
+            CK(launch_hs_check(midpoints + 3 * o + 2 * N, N, P1 + 3 * o, P2 + 3 * o, P3 + 3 * o, N, (int*)flag,
+                               ctx->stream, normals + 3 * o + 2 * N, false));
+        }
+        ctx->launches += nbatch;
+        int h = 0;
+        CK(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        if (h) return fail(ctx, CAD_ERR_HS_ABOVE_SURFACE, "Half-space solution: Z coordinates must be negative!");
+    }
+    // The batch runs on copies of its inputs, so that its graph serves every
+    // call of the same sizes. Captured for the caller's pointers it had to be
+    // captured again (17 of 50 ms for 64 cracks of 200 to 1500 elements) for
+    // each new set of arrays; the copies take 0.01 to 0.03 ms.
+    const int64_t words = 3 * offsets[nbatch];
+    void* ws;
+    if (int r = ensure(ctx, S_BATCH, (size_t)(7 * words) * sizeof(double), &ws)) return r;
+    double* w = (double*)ws;
+    const double* in[6] = {P1, P2, P3, normals, midpoints, T};
+    for (int i = 0; i < 6 && words; ++i)
+        CK(cudaMemcpyAsync(w + i * words, in[i], words * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+    double* Dw = w + 6 * words;
+    const int rc = slip_batched_ws(ctx, nbatch, offsets, w, w + words, w + 2 * words, w + 3 * words, w + 4 * words, nu,
+                                   G, lambda, hs, w + 5 * words, Dw, rel_host);
+    if (rc == CAD_ERR_CUDA) return rc;
+    if (words) CK(cudaMemcpyAsync(D, Dw, words * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    return rc;
 }
 
 extern "C" {

@@ -430,9 +430,9 @@ int cad_lpc_install(cad_ctx* ctx, const double* P1, const double* P2, const doub
  * assembly precision (cad_set_assembly) and solved by FP32 LU (TF32
  * updates) with FP64 refinement to the context's tolerance (cad_set_solver),
  * GMRES finishing any crack the refinement leaves.  The cracks run
- * concurrently on 32 stream lanes inside one CUDA graph, captured on the first
- * call with these arguments and replayed by identical calls.  Needs device
- * memory for every crack's 3N_c x 3N_c matrix at once.  rel_residual (host,
+ * concurrently on 32 stream lanes; from the second call in a row with the same
+ * offsets and settings on, whatever the arrays, as one replayed CUDA graph.
+ * Needs device memory for every crack's 3N_c x 3N_c matrix at once.  rel_residual (host,
  * nbatch, may be NULL): each crack's final ||b - A D|| / ||b||. */
 int cad_slip_calculator_batched_dev(cad_ctx* ctx, int64_t nbatch, const int64_t* offsets, const double* P1,
                                     const double* P2, const double* P3, const double* normals,
