@@ -222,6 +222,30 @@ struct EdgeTable {
 // triangles stays on the per-side kernels.
 bool edges_pay(int64_t E, int64_t N) { return 10 * E < 9 * 3 * N; }
 
+// The mesh-edge table of the triangles, on the device (lists: with each edge's
+// sides); count: where its number of edges goes.
+int edge_table(cad_ctx* ctx, const double* P1, const double* P2, const double* P3, int64_t N, bool lists, int* count,
+               EdgeArrays* a)
+{
+    void *pts, *ints;
+    if (int r = ensure(ctx, S_EDGE_PTS, (size_t)18 * N * sizeof(double), &pts)) return r;
+    if (int r = ensure(ctx, S_EDGE_INT, ((size_t)12 * N + edge_work_ints(N)) * sizeof(int), &ints)) return r;
+    int* i = (int*)ints;
+    *a = EdgeArrays{(double*)pts, i, i + 3 * N, i + 6 * N, i + 9 * N, i + 12 * N, count};
+    CK(launch_edge_table(P1, P2, P3, N, *a, lists, ctx->stream, &ctx->launches));
+    return CAD_OK;
+}
+
+// Full-space sums go over the mesh's edges from this many pairs on: about half
+// of a pair's 36 ps is saved (a third for displacements alone), and the edge
+// table costs 40 to 80 us.  Strain at 10 000 x 500 (triangles x points) 252 us
+// over edges and 259 by pairs, 100 x 42 000 178 and 177, 2013 x 3200 209 and
+// 277; displacements alone at 10 000 x 1700 579 and 628.
+bool segments_pay(int64_t M, int64_t N, bool strain)
+{
+    return M >= 256 && M >= (strain ? int64_t(5) << 20 : int64_t(1) << 24) / (N > 0 ? N : 1);
+}
+
 // The half-space argument check and, with et set and shared edges on, the
 // mesh-edge table (lists: with each edge's sides); one read-back for both.
 int hs_check(cad_ctx* ctx, const double* Z, int64_t M, const double* P1, const double* P2, const double* P3,
@@ -234,14 +258,8 @@ int hs_check(cad_ctx* ctx, const double* Z, int64_t M, const double* P1, const d
     CK(launch_hs_check(Z, M, P1, P2, P3, N, (int*)flag, ctx->stream, nullptr, false, et ? (int*)flag + 2 : nullptr));
     // side codes are ints: larger meshes stay on the per-side path
     const bool edges = et && ctx->shared_edges && N > 0 && 3 * N <= INT32_MAX;
-    if (edges) {
-        void *pts, *ints;
-        if (int r = ensure(ctx, S_EDGE_PTS, (size_t)18 * N * sizeof(double), &pts)) return r;
-        if (int r = ensure(ctx, S_EDGE_INT, ((size_t)12 * N + edge_work_ints(N)) * sizeof(int), &ints)) return r;
-        int* i = (int*)ints;
-        et->a = EdgeArrays{(double*)pts, i, i + 3 * N, i + 6 * N, i + 9 * N, i + 12 * N, (int*)flag + 1};
-        CK(launch_edge_table(P1, P2, P3, N, et->a, lists, ctx->stream, &ctx->launches));
-    }
+    if (edges)
+        if (int r = edge_table(ctx, P1, P2, P3, N, lists, (int*)flag + 1, &et->a)) return r;
     int h[3] = {0, 0, 0};
     CK(cudaMemcpyAsync(h, flag, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -308,6 +326,28 @@ int td_device(cad_ctx* ctx, const double* X, const double* Y, const double* Z, i
         CK(cudaEventRecord(ctx->ev[0], ctx->stream));
         CK(launch_td_sum_edges(a, strain == 1, disp == 1, et.full, et.a, et.E, rec, nu, echunk,
                                a.partial + (size_t)nchunk * 9 * M, ctx->stream, &ctx->launches));
+        CK(cudaEventRecord(ctx->ev[1], ctx->stream));
+        ctx->timed[0] = true;
+        const int mask = (strain == 1 ? 0x3f : 0) | (disp == 1 ? 0x1c0 : 0);
+        ++ctx->launches;
+        CK(launch_sum_chunks(a.partial, nchunk + nechunk, M, mask, sum_out, ctx->stream));
+        return CAD_OK;
+    }
+    if (out_kind == OUT_SUM && hs == 0 && edge_kind && ctx->shared_edges && 3 * N <= INT32_MAX &&
+        segments_pay(M, N, strain == 1)) {
+        // nothing is read back (E stays on the device), so the call stays
+        // asynchronous; a mesh without shared edges costs the same as its pairs
+        const int64_t echunk = pick_chunk(M, 3 * N, true), nechunk = (3 * N + echunk - 1) / echunk;
+        void *flag, *rec, *part;
+        if (int r = ensure(ctx, S_FLAG, 3 * sizeof(int), &flag)) return r;
+        if (int r = ensure(ctx, S_EDGE_REC, (size_t)3 * N * segment_record_bytes(), &rec)) return r;
+        if (int r = ensure(ctx, S_PART, (size_t)(nchunk + nechunk) * 9 * M * sizeof(double), &part)) return r;
+        EdgeArrays ed;
+        CK(cudaEventRecord(ctx->ev[0], ctx->stream));
+        if (int r = edge_table(ctx, P1, P2, P3, N, true, (int*)flag, &ed)) return r;
+        a.partial = (double*)part;
+        CK(launch_td_sum_segments(a, strain == 1, disp == 1, ed, rec, nu, nechunk, a.partial + (size_t)nchunk * 9 * M,
+                                  ctx->stream, &ctx->launches));
         CK(cudaEventRecord(ctx->ev[1], ctx->stream));
         ctx->timed[0] = true;
         const int mask = (strain == 1 ? 0x3f : 0) | (disp == 1 ? 0x1c0 : 0);

@@ -1171,6 +1171,86 @@ CAD_HD void build_side_burgers(const double PA[3], const double PB[3], const dou
     side_slip(s, B, s.cs[0]);
 }
 
+// ------------------------------------------- full-space sums over mesh edges
+// A mesh edge PA -> PB with the net Burgers vector B of the triangle sides on
+// it: unit direction t and length, and B in the products a point needs, with k1 = 1 / (4 pi),
+// K8 = 1 / (8 pi (1 - nu)).
+struct SegRec {
+    double PA[3], t[3], len;
+    double b1[3];   // -k1 / 2 B
+    double bK[3];   // -K8 B
+    double c1[3];   // (k1 - 2 K8) / 2 B x t
+    double c2[3];   // (k1 - K8) B x t
+    double pad;
+};
+constexpr int kSegWords = (int)(sizeof(SegRec) / sizeof(double));
+
+CAD_HD void build_segment(const double PA[3], const double PB[3], const double B[3], double K8, SegRec& s)
+{
+    const bool none = B[0] == 0.0 && B[1] == 0.0 && B[2] == 0.0;   // (its sides may have no direction)
+    const double S[3] = {PB[0] - PA[0], PB[1] - PA[1], PB[2] - PA[2]};
+    const double len = norm3_rn(S[0], S[1], S[2]), ka = kInv4Pi - 2.0 * K8;
+    for (int i = 0; i < 3; ++i) {
+        s.PA[i] = PA[i];
+        s.t[i] = none ? (i == 0 ? 1.0 : 0.0) : S[i] / len;
+        s.b1[i] = -0.5 * kInv4Pi * B[i];
+        s.bK[i] = -K8 * B[i];
+    }
+    s.len = none ? 0.0 : len;
+    double c[3];
+    cross3_rn(B, s.t, c);
+    for (int i = 0; i < 3; ++i) {
+        s.c1[i] = 0.5 * ka * c[i];
+        s.c2[i] = (kInv4Pi - K8) * c[i];
+    }
+    s.pad = 0.0;
+}
+
+// Strain of a segment at a point, added into E, and its displacement (but for
+// the solid angles), added into U; EFCS throughout.  With r the point's offset
+// from the segment's line and w = t x r,
+//   grad V = T t - K r,  H = I r r + (3 K - I r.r) t t - K 1 - Q (r t + t r)
+//   strain = -k1 K sym(B w) + (k1 - 2 K8) sym((B x t) grad V) - K8 (B.w) H
+//   displacement = (k1 - K8) V B x t - K8 (B.w) grad V
+template <bool STRAIN, bool DISP>
+CAD_HD void segment_sum(const SegRec& s, double X, double Y, double Z, double E[6], double U[3])
+{
+    const double d[3] = {X - s.PA[0], Y - s.PA[1], Z - s.PA[2]};
+    const double* t = s.t;
+    const double at = d[0] * t[0] + d[1] * t[1] + d[2] * t[2];
+    const double r[3] = {d[0] - at * t[0], d[1] - at * t[1], d[2] - at * t[2]};
+    const double w[3] = {t[1] * r[2] - t[2] * r[1], t[2] * r[0] - t[0] * r[2], t[0] * r[1] - t[1] * r[0]};
+    const double rho2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+    const double sA = -at, sB = s.len - at;
+    const double qA = fmax(rho2 + sA * sA, tiny_square<double>()), qB = fmax(rho2 + sB * sB, tiny_square<double>());
+    const double iA = cad_rsqrt(qA), iB = cad_rsqrt(qB);
+    const SegInt<double> g = seg_integrals<DISP>(qA * iA, iA, qB * iB, iB, sA, sB, rho2);
+    const double be = s.bK[0] * w[0] + s.bK[1] * w[1] + s.bK[2] * w[2];
+    const double gv[3] = {g.T * t[0] - g.K * r[0], g.T * t[1] - g.K * r[1], g.T * t[2] - g.K * r[2]};
+    if (STRAIN) {
+        const double bK = be * g.K, hI = 0.5 * be * g.I, hQ = be * g.Q, tt = 3.0 * bK - be * g.I * rho2;
+        double a[3], b[3], kw[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            a[i] = hI * r[i] - hQ * t[i];
+            b[i] = tt * t[i];
+            kw[i] = g.K * w[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            E[i] += 2.0 * (s.b1[i] * kw[i] + s.c1[i] * gv[i] + r[i] * a[i]) + t[i] * b[i] - bK;
+#pragma unroll
+        for (int k = 3; k < 6; ++k) {
+            const int i = k == 5 ? 1 : 0, j = k == 3 ? 1 : 2;
+            E[k] += s.b1[i] * kw[j] + s.b1[j] * kw[i] + s.c1[i] * gv[j] + s.c1[j] * gv[i] + r[i] * a[j] + r[j] * a[i] +
+                    t[i] * b[j];
+        }
+    }
+    if (DISP)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) U[c] += g.V * s.c2[c] + be * gv[c];
+}
+
 // ------------------------------------------------------------ pair drivers
 // Whether the point lies on a side or a vertex of the triangle or of its
 // mirror image, in its plane (the pair is NaN there).
@@ -1354,6 +1434,37 @@ CAD_HD void pair_net(const TriDev& t, double X, double Y, double Z, double E[6],
     }
     td_net<STRAIN, DISP>(t.real, X, Y, Z, t.Dn, t.Dss, t.Dds, t.K8, E, U);
     if (HS) td_net<STRAIN, DISP>(t.image, X, Y, Z, t.Dn, t.Dss, t.Dds, t.K8, E, U);
+}
+
+// What the full-space sums over mesh edges leave to each triangle: the
+// solid-angle displacement, and NaN where the point lies on one of its sides.
+template <bool STRAIN, bool DISP>
+CAD_HD void pair_angle(const TriDev& t, double X, double Y, double Z, double E[6], double U[3])
+{
+    const Frame& f = t.real;
+    if (DISP) {
+        double x, y, z;
+        to_tdcs(f, X, Y, Z, x, y, z);
+        const double dy[3] = {y - f.p1y, y, y - f.p3y}, dz[3] = {z - f.p1z, z, z - f.p3z};
+        double Rv[3];
+#pragma unroll
+        for (int v = 0; v < 3; ++v) {
+            const double q = x * x + dy[v] * dy[v] + dz[v] * dz[v];
+            Rv[v] = q * cad_rsqrt(q);
+        }
+        if (t.Dn != 0.0 || t.Dss != 0.0 || t.Dds != 0.0) {
+            const double Fi = solid_angle_term(x, dy, dz, Rv);
+            const double bn = t.Dn * Fi, bs = t.Dss * Fi, bd = t.Dds * Fi;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) U[c] += f.Vn[c] * bn + f.Vs[c] * bs + f.Vd[c] * bd;
+        }
+    }
+    if (on_side_or_vertex(f, X, Y, Z)) {
+        if (STRAIN)
+            for (int k = 0; k < 6; ++k) E[k] = qnan<double>();
+        if (DISP)
+            for (int c = 0; c < 3; ++c) U[c] = qnan<double>();
+    }
 }
 
 // sides = false leaves the half-space sides unset (their fields come from the

@@ -141,20 +141,23 @@ __host__ __device__ constexpr int pair_stage(bool hs, int edge, bool one) { retu
 // MINB > 1: compiled for MINB resident blocks per SM (fewer registers per
 // thread, more warps to hide the FP64 latency, some spilling) -- a launch
 // shape the autotuner may pick for the half-space system matrix.
-// EDGE (half space): the staged record is the two frames only.
+// EDGE (half space, but for the full-space sums): the staged record is the
+// two frames only.
 //   EDGE_FSC: the free-surface corrections are left to per-edge work.
 //   OUT_AMAT, OUT_TRAC (strain) and OUT_INF: they come from the per-edge maps
 //   a.fscG (side_map_kernel).  OUT_SUM: they are left out here, and
 //   side_sum_kernel adds each edge's once.
 //   EDGE_FULL: so is the whole strain (real, image and correction), which
 //   depends on the triangles' sides alone; the pair only combines its three
-//   sides' maps (tractions already for OUT_AMAT and OUT_TRAC), or, in
-//   OUT_SUM, marks the points that lie on a side.
+//   sides' maps (tractions already for OUT_AMAT and OUT_TRAC).
+//   EDGE_FULL in full space (OUT_SUM): the solid angle; segment_sum_kernel
+//   adds the rest.
+//   In both, points on a side become NaN.
 template <bool HS, bool STRAIN, bool DISP, int OUT, bool NEAR = false, bool LIST = false, int MINB = 1,
           int EDGE = EDGE_NONE>
 __global__ void __launch_bounds__(kPairThreads, MINB) td_pair_kernel(PairArgs a)
 {
-    static_assert(EDGE == EDGE_NONE || (HS && !LIST && !NEAR &&
+    static_assert(EDGE == EDGE_NONE || (!HS && EDGE == EDGE_FULL && OUT == OUT_SUM) || (HS && !LIST && !NEAR &&
                             (((OUT == OUT_AMAT || OUT == OUT_TRAC) && STRAIN && !DISP) || OUT == OUT_SUM ||
                              OUT == OUT_INF)),
                   "shared edges: HS system matrix, traction or influence fields, or sums only");
@@ -229,15 +232,14 @@ __global__ void __launch_bounds__(kPairThreads, MINB) td_pair_kernel(PairArgs a)
                 }
             continue;
         }
-        if constexpr (OUT == OUT_SUM && (!HS || EDGE != EDGE_NONE)) {
-            if (EDGE == EDGE_FULL && STRAIN && !DISP) {
-                if (pair_on_side(t, X, Y, Z))
-                    for (int k = 0; k < 6; ++k) sumE[k] = qnan<double>();
-            } else {
-                pair_net<HS, STRAIN && EDGE != EDGE_FULL, DISP>(t, X, Y, Z, sumE, sumU);
-                if (EDGE == EDGE_FULL && STRAIN && sumU[0] != sumU[0])
-                    for (int k = 0; k < 6; ++k) sumE[k] = qnan<double>();
-            }
+        if constexpr (OUT == OUT_SUM && !HS && EDGE == EDGE_FULL) {
+            pair_angle<STRAIN, DISP>(t, X, Y, Z, sumE, sumU);
+            continue;
+        } else if constexpr (OUT == OUT_SUM && (!HS || EDGE != EDGE_NONE)) {
+            static_assert(EDGE != EDGE_FULL || DISP, "strain alone leaves the pairs to on_side_kernel");
+            pair_net<HS, STRAIN && EDGE != EDGE_FULL, DISP>(t, X, Y, Z, sumE, sumU);
+            if (EDGE == EDGE_FULL && STRAIN && sumU[0] != sumU[0])
+                for (int k = 0; k < 6; ++k) sumE[k] = qnan<double>();
             continue;
         }
         if (STRAIN) {
@@ -297,6 +299,81 @@ __global__ void __launch_bounds__(kPairThreads, MINB) td_pair_kernel(PairArgs a)
 #pragma unroll
         for (int c = 0; c < 3; ++c) p[(6 + c) * a.M + i] = sumU[c];
     }
+}
+
+// The triangles' share of strain sums whose sides are taken per mesh edge: NaN
+// at points on a side or vertex (HS: or on the mirror image's), 0 elsewhere.
+// A point can be on a side only where its offset from the plane, in unfused
+// arithmetic, is exactly 0; the rest of the test runs only there.  Each thread
+// takes four points: with one, the six values of a plane that every thread
+// reads from shared memory bound it (2013 x 20 000: 129 us, now 37).
+constexpr int kMarkStage = 32, kMarkPts = 4;
+template <bool HS>
+__global__ void __launch_bounds__(kPairThreads) on_side_kernel(PairArgs a)
+{
+    constexpr int F = HS ? 2 : 1;
+    __shared__ __align__(16) double s_plane[kMarkStage][F][6];   // P2, Vn
+    const int64_t i0 = (int64_t)blockIdx.x * (kPairThreads * kMarkPts) + threadIdx.x;
+    double X[kMarkPts], Y[kMarkPts], Z[kMarkPts];
+    bool nan[kMarkPts];
+#pragma unroll
+    for (int q = 0; q < kMarkPts; ++q) {
+        const int64_t i = min(i0 + q * kPairThreads, a.M - 1);
+        X[q] = a.X[i];
+        Y[q] = a.Y[i];
+        Z[q] = a.Z[i];
+        nan[q] = false;
+    }
+    const int64_t j0 = (int64_t)blockIdx.y * a.tri_chunk;
+    const int64_t j1 = min(a.N, j0 + a.tri_chunk);
+    for (int64_t jb = j0; jb < j1; jb += kMarkStage) {
+        const int nt = (int)min((int64_t)kMarkStage, j1 - jb);
+        __syncthreads();
+        for (int w = threadIdx.x; w < nt * F * 6; w += kPairThreads) {
+            const int k = w / (F * 6), f = w / 6 % F, c = w % 6;
+            const Frame& fr = f ? a.tri[jb + k].image : a.tri[jb + k].real;
+            s_plane[k][f][c] = c < 3 ? fr.P2[c] : fr.Vn[c - 3];
+        }
+        __syncthreads();
+#pragma unroll 2
+        for (int k = 0; k < nt; ++k) {
+            unsigned in = 0u;
+#pragma unroll
+            for (int f = 0; f < F; ++f) {
+                const double* p = s_plane[k][f];
+#pragma unroll
+                for (int q = 0; q < kMarkPts; ++q) {
+                    const double x = dot3_rn(p[3], p[4], p[5], sub_rn(X[q], p[0]), sub_rn(Y[q], p[1]), sub_rn(Z[q], p[2]));
+                    in |= x == 0.0 ? 1u << q : 0u;
+                }
+            }
+            if (in) {
+                const TriDev& t = a.tri[jb + k];
+#pragma unroll
+                for (int q = 0; q < kMarkPts; ++q)
+                    if ((in >> q) & 1u)
+                        nan[q] = nan[q] || (HS ? pair_on_side(t, X[q], Y[q], Z[q])
+                                               : on_side_or_vertex(t.real, X[q], Y[q], Z[q]));
+            }
+        }
+    }
+    double* p = a.partial + (int64_t)blockIdx.y * 9 * a.M;
+#pragma unroll
+    for (int q = 0; q < kMarkPts; ++q) {
+        const int64_t i = i0 + q * kPairThreads;
+        if (i < a.M)
+#pragma unroll
+            for (int k = 0; k < 6; ++k) p[k * a.M + i] = nan[q] ? qnan<double>() : 0.0;
+    }
+}
+
+static cudaError_t launch_on_side(const PairArgs& a, bool hs, cudaStream_t st)
+{
+    constexpr int pts = kPairThreads * kMarkPts;
+    const dim3 grid((unsigned)((a.M + pts - 1) / pts), (unsigned)((a.N + a.tri_chunk - 1) / a.tri_chunk));
+    if (hs) on_side_kernel<true><<<grid, kPairThreads, 0, st>>>(a);
+    else on_side_kernel<false><<<grid, kPairThreads, 0, st>>>(a);
+    return cudaGetLastError();
 }
 
 // Adds the per-chunk partial sums in chunk order: out[f][i] = sum_c partial[c][f][i].
@@ -705,18 +782,12 @@ cudaError_t launch_assemble_edges(PairArgs a, int out_kind, bool strain, bool di
     return cudaSuccess;
 }
 
-// Net Burgers vector of each mesh edge: the signed sum over the triangle sides
-// on it (sides[ptr[e] ..] = +-(triangle + 1), sorted here into triangle order,
-// then side order, so the sum does not depend on how the list was filled) of
-// Dn Vn + Dss Vs + Dds Vd, then the edge's record for it.
-__global__ void edge_burgers_kernel(const double* __restrict__ pts, int64_t E, const int* __restrict__ ptr,
-                                    const int* __restrict__ cnt, int* __restrict__ sides,
-                                    const TriDev* __restrict__ tri, double nu, FscSide* __restrict__ out)
+// Net Burgers vector of a mesh edge: the signed sum over the triangle sides on
+// it (list[0 .. n) = +-(triangle + 1), sorted here into triangle order, then
+// side order, so the sum does not depend on how the list was filled) of
+// Dn Vn + Dss Vs + Dds Vd.
+__device__ __forceinline__ void net_burgers(int* __restrict__ list, int n, const TriDev* __restrict__ tri, double B[3])
 {
-    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    int* list = sides + ptr[e];
-    const int n = cnt[e];
     for (int i = 1; i < n; ++i) {
         const int v = list[i];
         int j = i;
@@ -724,19 +795,88 @@ __global__ void edge_burgers_kernel(const double* __restrict__ pts, int64_t E, c
             list[j] = list[j - 1];
         list[j] = v;
     }
-    double B[3] = {0.0, 0.0, 0.0};
+    B[0] = B[1] = B[2] = 0.0;
     for (int k = 0; k < n; ++k) {
         const int c = list[k];
         const TriDev& t = tri[(c > 0 ? c : -c) - 1];
         const double sg = c > 0 ? 1.0 : -1.0;
         const double slip[3] = {t.Dn, t.Dss, t.Dds};
+        if (slip[0] == 0.0 && slip[1] == 0.0 && slip[2] == 0.0) continue;
         const double* axes[3] = {t.real.Vn, t.real.Vs, t.real.Vd};
         for (int m = 0; m < 3; ++m)
             for (int i = 0; i < 3; ++i) B[i] = add_rn(B[i], sg * mul_rn(axes[m][i], slip[m]));
     }
+}
+
+// Each half-space edge's record for its net Burgers vector.
+__global__ void edge_burgers_kernel(const double* __restrict__ pts, int64_t E, const int* __restrict__ ptr,
+                                    const int* __restrict__ cnt, int* __restrict__ sides,
+                                    const TriDev* __restrict__ tri, double nu, FscSide* __restrict__ out)
+{
+    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (e >= E) return;
+    double B[3];
+    net_burgers(sides + ptr[e], cnt[e], tri, B);
     const double PA[3] = {pts[6 * e], pts[6 * e + 1], pts[6 * e + 2]};
     const double PB[3] = {pts[6 * e + 3], pts[6 * e + 4], pts[6 * e + 5]};
     build_side_burgers(PA, PB, B, nu, out[e]);
+}
+
+// Each full-space edge's; the number of edges is read on the device (count).
+__global__ void segment_burgers_kernel(const double* __restrict__ pts, const int* __restrict__ count,
+                                       const int* __restrict__ ptr, const int* __restrict__ cnt,
+                                       int* __restrict__ sides, const TriDev* __restrict__ tri, double K8,
+                                       SegRec* __restrict__ out)
+{
+    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (e >= *count) return;
+    double B[3];
+    net_burgers(sides + ptr[e], cnt[e], tri, B);
+    const double PA[3] = {pts[6 * e], pts[6 * e + 1], pts[6 * e + 2]};
+    const double PB[3] = {pts[6 * e + 3], pts[6 * e + 4], pts[6 * e + 5]};
+    build_segment(PA, PB, B, K8, out[e]);
+}
+
+// partial[(blockIdx.y * 9 + f) M + i] = the full-space strain (f 0-5) and the
+// segments' displacement (f 6-8) at point i of the edges of chunk blockIdx.y of
+// gridDim.y, summed in edge order (kSegStage records staged in shared memory at
+// a time).  FP64 bound, about 160 instructions per (edge, point) against 490 per
+// (triangle, point) side by side: strain of 2013 triangles (3060 edges) at
+// 20 000 points 670 us where the pairs took 1430 (two points per thread: 682).
+constexpr int kSegStage = 16;
+template <bool STRAIN, bool DISP>
+__global__ void __launch_bounds__(kPairThreads) segment_sum_kernel(const SegRec* __restrict__ edges,
+                                                                   const int* __restrict__ count,
+                                                                   const double* __restrict__ X,
+                                                                   const double* __restrict__ Y,
+                                                                   const double* __restrict__ Z, int64_t M,
+                                                                   double* __restrict__ partial)
+{
+    __shared__ __align__(16) double smem[kSegStage * kSegWords];
+    const int64_t i = (int64_t)blockIdx.x * kPairThreads + threadIdx.x;
+    const bool active = i < M;
+    double x = 0.0, y = 0.0, z = 0.0;
+    if (active) { x = X[i]; y = Y[i]; z = Z[i]; }
+    double sE[6] = {}, sU[3] = {};
+    const int64_t E = *count, echunk = (E + gridDim.y - 1) / gridDim.y;
+    const int64_t e0 = min(E, (int64_t)blockIdx.y * echunk), e1 = min(E, e0 + echunk);
+    for (int64_t eb = e0; eb < e1; eb += kSegStage) {
+        const int ne = (int)min((int64_t)kSegStage, e1 - eb);
+        __syncthreads();
+        const double* src = reinterpret_cast<const double*>(edges + eb);
+        for (int w = threadIdx.x; w < ne * kSegWords; w += kPairThreads) smem[w] = src[w];
+        __syncthreads();
+        if (!active) continue;
+#pragma unroll 1
+        for (int k = 0; k < ne; ++k)
+            segment_sum<STRAIN, DISP>(reinterpret_cast<const SegRec*>(smem)[k], x, y, z, sE, sU);
+    }
+    if (!active) return;
+    double* p = partial + (int64_t)blockIdx.y * 9 * M;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) p[k * M + i] = sE[k];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) p[(6 + c) * M + i] = sU[c];
 }
 
 // partial[(blockIdx.y * 9 + f) M + i] = the strain (f 0-5; STRAIN EDGE_FSC: the
@@ -808,9 +948,11 @@ cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, bool full, c
     if (strain && disp)
         e = full ? pairs(td_pair_kernel<true, true, true, OUT_SUM, false, false, 1, EDGE_FULL>)
                  : pairs(td_pair_kernel<true, true, true, OUT_SUM, false, false, 1, EDGE_FSC>);
-    else if (strain)
-        e = full ? pairs(td_pair_kernel<true, true, false, OUT_SUM, false, false, 1, EDGE_FULL>)
-                 : pairs(td_pair_kernel<true, true, false, OUT_SUM, false, false, 1, EDGE_FSC>);
+    else if (strain && full) {
+        e = launch_on_side(a, true, st);
+        if (launches) ++*launches;
+    } else if (strain)
+        e = pairs(td_pair_kernel<true, true, false, OUT_SUM, false, false, 1, EDGE_FSC>);
     else
         e = pairs(td_pair_kernel<true, false, true, OUT_SUM, false, false, 1, EDGE_FSC>);
     if (e != cudaSuccess || E == 0) return e;
@@ -822,6 +964,38 @@ cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, bool full, c
     if (strain) return full ? sums(side_sum_kernel<EDGE_FULL, false>) : sums(side_sum_kernel<EDGE_FSC, false>);
     return sums(side_sum_kernel<EDGE_NONE, true>);
 }
+
+cudaError_t launch_td_sum_segments(PairArgs a, bool strain, bool disp, const EdgeArrays& ed, void* seg_rec, double nu,
+                                   int64_t nechunk, double* edge_partial, cudaStream_t st, int64_t* launches)
+{
+    if (a.M == 0 || a.N == 0 || !(strain || disp)) return cudaSuccess;
+    const size_t psmem = (size_t)pair_words(false, EDGE_FULL) * pair_stage(false, EDGE_FULL, false) * sizeof(double);
+    const unsigned tiles = (unsigned)((a.M + kPairThreads - 1) / kPairThreads);
+    SegRec* rec = (SegRec*)seg_rec;
+    const double K8 = 0.5 * kInv4Pi / (1.0 - nu);
+    segment_burgers_kernel<<<(unsigned)((3 * a.N + 31) / 32), 32, 0, st>>>(ed.pts, ed.count, ed.ptr, ed.cnt, ed.sides,
+                                                                           a.tri, K8, rec);
+    auto pairs = [&](auto kern) -> cudaError_t {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem);
+        if (e != cudaSuccess) return e;
+        kern<<<dim3(tiles, (unsigned)((a.N + a.tri_chunk - 1) / a.tri_chunk)), kPairThreads, psmem, st>>>(a);
+        return cudaGetLastError();
+    };
+    cudaError_t e;
+    if (strain && disp) e = pairs(td_pair_kernel<false, true, true, OUT_SUM, false, false, 1, EDGE_FULL>);
+    else if (strain) e = launch_on_side(a, false, st);
+    else e = pairs(td_pair_kernel<false, false, true, OUT_SUM, false, false, 1, EDGE_FULL>);
+    if (e != cudaSuccess) return e;
+    const dim3 grid(tiles, (unsigned)nechunk);
+    auto sums = [&](auto kern) { kern<<<grid, kPairThreads, 0, st>>>(rec, ed.count, a.X, a.Y, a.Z, a.M, edge_partial); };
+    if (strain && disp) sums(segment_sum_kernel<true, true>);
+    else if (strain) sums(segment_sum_kernel<true, false>);
+    else sums(segment_sum_kernel<false, true>);
+    *launches += 3;
+    return cudaGetLastError();
+}
+
+size_t segment_record_bytes() { return sizeof(SegRec); }
 
 cudaError_t launch_splice_fixed(const double* trac, const double* disp, int64_t N, int64_t nfix, const int* fixrow,
                                 const int* freecol, int64_t nf, bool amat, double* out, int64_t lda, cudaStream_t st)

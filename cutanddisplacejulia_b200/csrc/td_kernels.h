@@ -89,6 +89,14 @@ size_t edge_record_bytes();
 cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, bool full, const EdgeArrays& ed, int64_t E,
                                 void* edge_rec, double nu, int64_t echunk, double* edge_partial, cudaStream_t st, int64_t* launches);
 
+// Full-space sums (OUT_SUM) with the triangles' sides taken once per mesh edge,
+// for the net Burgers vector on it: a.partial as above receives the solid angles
+// (and the NaN of points on a side), edge_partial nechunk x 9 x a.M sums over the
+// edges, whose number stays on the device.  seg_rec: 3 a.N records.
+cudaError_t launch_td_sum_segments(PairArgs a, bool strain, bool disp, const EdgeArrays& ed, void* seg_rec, double nu,
+                                   int64_t nechunk, double* edge_partial, cudaStream_t st, int64_t* launches);
+size_t segment_record_bytes();
+
 // Mixed-precision system matrix: every pair in FP32 (far field), then the
 // pairs of every 128-point tile that has a point within the near radius of
 // the source centroid again in FP64.  near_factor: radius in mean edge lengths.

@@ -156,9 +156,11 @@ int cad_set_lu_block(cad_ctx* ctx, int nb);
  * preconditioned GMRES solvers): 1..63, 0 = the default 30.  Every cycle
  * starts from the FP64 residual b - A x.  No counterpart in the reference. */
 int cad_set_gmres_restart(cad_ctx* ctx, int m);
-/* Half-space work on meshes whose triangles share edges (fewer edges than
- * 0.9 x the triangle sides; other meshes always take the per-side path).
- * 1 (default): the FP64 system matrix and traction influence fields
+/* Work on meshes whose triangles share edges.
+ * 1 (default): in full space the summed evaluations (cad_td_sum_eval*) of
+ * many pairs take each mesh edge once, with the net Burgers vector of the
+ * sides on it; in half space, for fewer edges than 0.9 x the triangle sides
+ * (other meshes always take the per-side path), the FP64 system matrix and traction influence fields
  * (cad_assemble*, cad_slip_calculator*, cad_influence_traction with hs_flag
  * 1) evaluate the free-surface correction of each mesh edge once per
  * collocation point, and the triangles that share the edge reuse it
