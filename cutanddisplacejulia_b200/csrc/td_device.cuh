@@ -639,12 +639,19 @@ CAD_HD void to_adcs(const FscSideT<R>& s, double X, double Y, double Z, R& y1, R
     z = (R)(-Z);
 }
 
+// What the strain's and the displacement's functions of one end share: r, 1 / r,
+// 1 / (r + q), 1 / (r + f z3).
+template <typename R>
+struct FscEnd {
+    R r, ir, ip, iw;
+};
+
 // Adds sg x the values of one end of a side (depth a, point at (y1, y2) from
 // it and at depth z) to the accumulators.  f = +-1 takes the inclined leg's
 // functions along +z3 or -z3 (both ends alike); w = r + f z3 is rho^2 / (r - f
 // z3) where f z3 < 0, so it never cancels.
 template <bool FIRST, typename R>
-CAD_HD void fsc_end(const FscSideT<R>& k, R y1, R y2, R a, R z, R f, R z1, R z3, FscAcc<R>& v)
+CAD_HD void fsc_end(const FscSideT<R>& k, R y1, R y2, R a, R z, R f, R z1, R z3, FscAcc<R>& v, FscEnd<R>& end)
 {
     const R sg = FIRST ? R(-1.0) : R(1.0);
     const R q = z + a;
@@ -655,6 +662,7 @@ CAD_HD void fsc_end(const FscSideT<R>& k, R y1, R y2, R a, R z, R f, R z1, R z3,
     const R den = out ? r + zf : z1 * z1 + y2 * y2, num = out ? R(1.0) : r - zf;
     const R inv = R(1.0) / (p * den);
     const R ip = inv * den, iw = inv * p * num;
+    end = FscEnd<R>{r, ir, ip, iw};
     const R N1 = R(1.0) - R(2.0) * k.nu, hN = R(0.5) * N1;
     const R c1r = y1 * ip, c1i = y2 * ip;                                    // zeta
     const R c2r = c1r * c1r - c1i * c1i, c2i = R(2.0) * c1r * c1i;
@@ -759,8 +767,9 @@ CAD_HD void side_strain_adcs(const FscSideT<R>& s, double X, double Y, double Z,
     const R f = z3A + z3B >= R(0.0) ? R(1.0) : R(-1.0);
     const R z1 = s.c * y1 + s.s * qA;
     FscAcc<R> v;
-    fsc_end<true>(s, y1, y2, s.aA, z, f, z1, z3A, v);
-    fsc_end<false>(s, y1b, y2b, s.aB, z, f, s.c * y1b + s.s * qB, z3B, v);
+    FscEnd<R> eA, eB;
+    fsc_end<true>(s, y1, y2, s.aA, z, f, z1, z3A, v, eA);
+    fsc_end<false>(s, y1b, y2b, s.aB, z, f, s.c * y1b + s.s * qB, z3B, v, eB);
     if (FULL && s.skip != R(0)) {
 #pragma unroll
         for (int k = 0; k < 18; ++k) e[k / 6][k % 6] = R(0.0);
@@ -798,20 +807,6 @@ CAD_HD void adcs_to_efcs(R t[6], R a, R b)
     t[3] = ab * (t11 - t22) + (bb - aa) * t12;
     t[4] = -(a * t13 + b * t23);
     t[5] = a * t23 - b * t13;
-}
-
-// Strain (EFCS) at the point of side s carrying the slip of its mode 0, the
-// real and image segments included, added into E.
-template <typename R>
-CAD_HD void side_strain_sum(const FscSideT<R>& s, double X, double Y, double Z, R E[6])
-{
-    R e[3][6], T[6];
-    side_strain_adcs<true>(s, X, Y, Z, e);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) T[k] = s.cs[0][0] * e[0][k] + s.cs[0][1] * e[1][k] + s.cs[0][2] * e[2][k];
-    adcs_to_efcs(T, s.ea, s.eb);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) E[k] += T[k];
 }
 
 // One side's harmonic correction to the strain, added into E (EFCS).
@@ -908,23 +903,21 @@ CAD_HD void fsc_apply_map(const R (*G)[6], R sign, const FrameT<R>& real, R Dss,
     }
 }
 
-// Adds sg x one end's values to the displacement accumulators; returns r + q
-// and r + f z3 (for the logarithms) and the numerator and denominator of the
-// Burgers function's tangent.
+// Adds sg x one end's values to the displacement accumulators (h: the end's
+// shared values, f their direction).  ff is that of the Burgers function, whose
+// tangent's numerator and denominator are returned.
 template <bool FIRST, typename R>
-CAD_HD void fsc_disp_end(const FscSideT<R>& k, R y1, R y2, R a, R z, R f, FscDispAcc<R>& v, R& p, R& w, R& fn, R& fd)
+CAD_HD void fsc_disp_end(const FscSideT<R>& k, R y1, R y2, R a, R z, R f, R ff, const FscEnd<R>& h, FscDispAcc<R>& v,
+                         R& fn, R& fd)
 {
     const R sg = FIRST ? R(-1.0) : R(1.0);
     const R q = z + a;
-    const R r2 = y1 * y1 + y2 * y2 + q * q;
-    const R ir = cad_rsqrt(r2), r = r2 * ir, ir2 = ir * ir, ir3 = ir2 * ir;
+    const R ir = h.ir, ir2 = ir * ir, ir3 = ir2 * ir;
     const R z1 = k.c * y1 + k.s * q, zf = f * (k.c * q - k.s * y1);
-    p = r + q;
-    w = r + zf;
-    fn = f * y2;
-    fd = f > R(0.0) ? p * k.ct2 - y1 : y1 + p * k.tn2;
-    const R inv = R(1.0) / (p * w);
-    const R ip = inv * w, iw = inv * p;
+    const R p = h.r + q;
+    fn = ff * y2;
+    fd = ff > R(0.0) ? p * k.ct2 - y1 : y1 + p * k.tn2;
+    const R ip = h.ip, iw = h.iw;
     const R N1 = R(1.0) - R(2.0) * k.nu, N2 = R(2.0) * (R(1.0) - k.nu);
     const R c1r = y1 * ip, c1i = y2 * ip;
     const R c2r = c1r * c1r - c1i * c1i, c2i = R(2.0) * c1r * c1i;
@@ -957,24 +950,141 @@ CAD_HD void fsc_disp_end(const FscSideT<R>& k, R y1, R y2, R a, R z, R f, FscDis
 }
 
 // Displacement of a side's correction in ADCS, d[3 component + slip], for a
-// unit ADCS slip along each axis (without K4).  f follows the side of the
-// vertical plane through PA the point lies on, as the reference's choice
-// between beta and beta - pi does: the Burgers function then stays on one
-// branch at both ends, and their difference is one arctangent.
+// unit ADCS slip along each axis (without K4), from the ends' shared values eA,
+// eB (direction f) and chi = int ds / R along the leg.  The Burgers function's
+// own direction follows the side of the vertical plane through PA the point
+// lies on, as the reference's choice between beta and beta - pi does: it then
+// stays on one branch at both ends, and their difference is one arctangent.
+template <typename R>
+CAD_HD void fsc_disp_ends(const FscSideT<R>& s, R y1, R y2, R z, R f, const FscEnd<R>& eA, const FscEnd<R>& eB, R chi,
+                          R d[9])
+{
+    const R ff = y1 >= R(0.0) ? R(-1.0) : R(1.0);
+    FscDispAcc<R> v;
+    R nA, dA, nB, dB;
+    fsc_disp_end<true>(s, y1, y2, s.aA, z, f, ff, eA, v, nA, dA);
+    fsc_disp_end<false>(s, y1 - s.y1B, y2 - s.y2B, s.aB, z, f, ff, eB, v, nB, dB);
+    v.phi = cad_log(eA.ip * ((eB.r + z) + s.aB));
+    v.chi = chi;
+    v.F = R(2.0) * cad_atan2(nB * dA - nA * dB, dA * dB + nA * nB);
+    fsc_disp_rows(s.kd, v, d);
+}
+
+template <typename R>
+CAD_HD FscEnd<R> fsc_end_values(R y1, R y2, R q, R f, R z1, R z3)
+{
+    const R r2 = y1 * y1 + y2 * y2 + q * q;
+    FscEnd<R> e;
+    e.ir = cad_rsqrt(r2);
+    e.r = r2 * e.ir;
+    const R zf = f * z3, p = e.r + q;
+    const bool out = zf >= R(0.0);
+    const R den = out ? e.r + zf : z1 * z1 + y2 * y2, num = out ? R(1.0) : e.r - zf;
+    const R inv = R(1.0) / (p * den);
+    e.ip = inv * den;
+    e.iw = inv * p * num;
+    return e;
+}
+
 template <typename R>
 CAD_HD void fsc_disp_adcs(const FscSideT<R>& s, double X, double Y, double Z, R d[9])
 {
     R y1, y2, z;
     to_adcs(s, X, Y, Z, y1, y2, z);
-    const R f = y1 >= R(0.0) ? R(-1.0) : R(1.0);
-    FscDispAcc<R> v;
-    R pA, wA, nA, dA, pB, wB, nB, dB;
-    fsc_disp_end<true>(s, y1, y2, s.aA, z, f, v, pA, wA, nA, dA);
-    fsc_disp_end<false>(s, y1 - s.y1B, y2 - s.y2B, s.aB, z, f, v, pB, wB, nB, dB);
-    v.phi = cad_log(pB / pA);
-    v.chi = f * cad_log(wB / wA);
-    v.F = R(2.0) * cad_atan2(nB * dA - nA * dB, dA * dB + nA * nB);
-    fsc_disp_rows(s.kd, v, d);
+    const R qA = z + s.aA, qB = z + s.aB;
+    const R y1b = y1 - s.y1B, y2b = y2 - s.y2B;
+    const R z3A = s.c * qA - s.s * y1, z3B = s.c * qB - s.s * y1b;
+    const R f = z3A + z3B >= R(0.0) ? R(1.0) : R(-1.0);
+    const FscEnd<R> eA = fsc_end_values(y1, y2, qA, f, s.c * y1 + s.s * qA, z3A);
+    const FscEnd<R> eB = fsc_end_values(y1b, y2b, qB, f, s.c * y1b + s.s * qB, z3B);
+    fsc_disp_ends(s, y1, y2, z, f, eA, eB, f * cad_log(eA.iw / eB.iw), d);
+}
+
+// Adds a segment's strain and displacement (its axes as in add_segment_adcs)
+// for the Burgers vector (b0, b1, b2) along the ADCS axes to T and u.
+template <bool DISP, typename R>
+CAD_HD void add_segment_net(const SegInt<R>& g, R x, R e, R k1, R K8, R c, R ss, R b0, R b1, R b2, R T[6], R u[3])
+{
+    const SegStrain<R> q = seg_strain(g, x, e, k1, K8);
+    const R bn = c * b0 + ss * b2, bm = b1, bt = c * b2 - ss * b0;
+    const R nn = bn * q.nnn + bm * q.mnn, mm = bn * q.nmm + bm * q.mmm, tt = bn * q.ntt + bm * q.mtt;
+    const R nm = bn * q.nnm + bm * q.mnm, nt = bn * q.nnt + bm * q.mnt + bt * q.tnt;
+    const R mt = bn * q.nmt + bm * q.mmt + bt * q.tmt;
+    const R cc = c * c, s2 = ss * ss, cs = c * ss;
+    T[0] += cc * nn + s2 * tt - R(2.0) * cs * nt;
+    T[1] += mm;
+    T[2] += s2 * nn + cc * tt + R(2.0) * cs * nt;
+    T[3] += c * nm - ss * mt;
+    T[4] += cs * (nn - tt) + (cc - s2) * nt;
+    T[5] += ss * nm + c * mt;
+    if (DISP) {   // as in td_net
+        const R cV = (k1 - K8) * g.V, w = K8 * (bn * e - bm * x);
+        const R un = bm * cV - w * x * g.K, um = -w * e * g.K - bn * cV, ut = w * g.T;
+        u[0] += c * un - ss * ut;
+        u[1] += um;
+        u[2] += ss * un + c * ut;
+    }
+}
+
+// Strain and displacement (EFCS) at the point of side s carrying the slip of its
+// mode 0: the correction and the real and image segments, without the solid
+// angles; added into E and U.
+template <bool DISP, typename R>
+CAD_HD void side_sum_full(const FscSideT<R>& s, double X, double Y, double Z, R E[6], R U[3])
+{
+    R y1, y2, z;
+    to_adcs(s, X, Y, Z, y1, y2, z);
+    const R qA = z + s.aA, qB = z + s.aB;
+    const R y1b = y1 - s.y1B, y2b = y2 - s.y2B;
+    const R z3A = s.c * qA - s.s * y1, z3B = s.c * qB - s.s * y1b;
+    const R f = z3A + z3B >= R(0.0) ? R(1.0) : R(-1.0);
+    const R z1 = s.c * y1 + s.s * qA;
+    const R b0 = s.cs[0][0], b1 = s.cs[0][1], b2 = s.cs[0][2];
+    R T[6] = {R(0.0), R(0.0), R(0.0), R(0.0), R(0.0), R(0.0)}, u[3] = {R(0.0), R(0.0), R(0.0)};
+    SegInt<R> g;
+    FscEnd<R> eA, eB;
+    {
+        FscAcc<R> v;
+        fsc_end<true>(s, y1, y2, s.aA, z, f, z1, z3A, v, eA);
+        fsc_end<false>(s, y1b, y2b, s.aB, z, f, s.c * y1b + s.s * qB, z3B, v, eB);
+        if (s.skip == R(0)) {
+            R e[3][6];
+            fsc_rows(s.ks, v, z, e);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) T[k] = b0 * e[0][k] + b1 * e[1][k] + b2 * e[2][k];
+        }
+        g.K = -f * v.u;
+        g.I = -f * v.v;
+        g.T = v.h0;
+        g.Q = v.c3;
+    }
+    g.V = DISP ? f * cad_log(eA.iw / eB.iw) : R(0.0);
+    const R k1 = R(1.0) - s.nu, K8 = R(0.5);   // 1 / (4 pi) and 1 / (8 pi (1 - nu)) over K4
+    add_segment_net<DISP>(g, z1, y2, k1, K8, s.c, s.s, b0, b1, -b2, T, u);
+    {
+        const R pA = z - s.aA, pB = z - s.aB;   // vertical offsets from the real ends
+        const R x = s.c * y1 - s.s * pA;
+        const R rA2 = fmax(y1 * y1 + y2 * y2 + pA * pA, tiny_square<R>());   // finite at a vertex too
+        const R rB2 = fmax(y1b * y1b + y2b * y2b + pB * pB, tiny_square<R>());
+        const R iA = cad_rsqrt(rA2), iB = cad_rsqrt(rB2);
+        const SegInt<R> h = seg_integrals<DISP>(rA2 * iA, iA, rB2 * iB, iB, -(s.s * y1 + s.c * pA),
+                                                -(s.s * y1b + s.c * pB), x * x + y2 * y2);
+        add_segment_net<DISP>(h, x, y2, k1, K8, s.c, -s.s, b0, b1, b2, T, u);
+    }
+    if (DISP) {
+        if (s.skip == R(0)) {
+            R d[9];
+            fsc_disp_ends(s, y1, y2, z, f, eA, eB, g.V, d);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) u[i] += b0 * d[3 * i] + b1 * d[3 * i + 1] + b2 * d[3 * i + 2];
+        }
+        U[0] += s.ea * u[0] + s.eb * u[1];
+        U[1] += s.eb * u[0] - s.ea * u[1];
+        U[2] -= u[2];
+    }
+    adcs_to_efcs(T, s.ea, s.eb);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) E[k] += T[k];
 }
 
 // One side's harmonic correction to the displacement, added into U (EFCS).
@@ -1436,34 +1546,37 @@ CAD_HD void pair_net(const TriDev& t, double X, double Y, double Z, double E[6],
     if (HS) td_net<STRAIN, DISP>(t.image, X, Y, Z, t.Dn, t.Dss, t.Dds, t.K8, E, U);
 }
 
-// What the full-space sums over mesh edges leave to each triangle: the
-// solid-angle displacement, and NaN where the point lies on one of its sides.
-template <bool STRAIN, bool DISP>
+// -Omega / (4 pi) x the slip of a frame's triangle (EFCS), added into U.
+CAD_HD void add_angle(const Frame& f, double X, double Y, double Z, double Dss, double Dds, double Dn, double U[3])
+{
+    double x, y, z;
+    to_tdcs(f, X, Y, Z, x, y, z);
+    const double dy[3] = {y - f.p1y, y, y - f.p3y}, dz[3] = {z - f.p1z, z, z - f.p3z};
+    double Rv[3];
+#pragma unroll
+    for (int v = 0; v < 3; ++v) {
+        const double q = x * x + dy[v] * dy[v] + dz[v] * dz[v];
+        Rv[v] = q * cad_rsqrt(q);
+    }
+    const double Fi = solid_angle_term(x, dy, dz, Rv);
+    const double bn = Dn * Fi, bs = Dss * Fi, bd = Dds * Fi;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) U[c] += f.Vn[c] * bn + f.Vs[c] * bs + f.Vd[c] * bd;
+}
+
+// What displacement sums over mesh edges leave to each triangle: the solid
+// angles (HS: the mirror image's too), and NaN where the point lies on a side.
+template <bool HS, bool STRAIN>
 CAD_HD void pair_angle(const TriDev& t, double X, double Y, double Z, double E[6], double U[3])
 {
-    const Frame& f = t.real;
-    if (DISP) {
-        double x, y, z;
-        to_tdcs(f, X, Y, Z, x, y, z);
-        const double dy[3] = {y - f.p1y, y, y - f.p3y}, dz[3] = {z - f.p1z, z, z - f.p3z};
-        double Rv[3];
-#pragma unroll
-        for (int v = 0; v < 3; ++v) {
-            const double q = x * x + dy[v] * dy[v] + dz[v] * dz[v];
-            Rv[v] = q * cad_rsqrt(q);
-        }
-        if (t.Dn != 0.0 || t.Dss != 0.0 || t.Dds != 0.0) {
-            const double Fi = solid_angle_term(x, dy, dz, Rv);
-            const double bn = t.Dn * Fi, bs = t.Dss * Fi, bd = t.Dds * Fi;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) U[c] += f.Vn[c] * bn + f.Vs[c] * bs + f.Vd[c] * bd;
-        }
+    if (t.Dn != 0.0 || t.Dss != 0.0 || t.Dds != 0.0) {
+        add_angle(t.real, X, Y, Z, t.Dss, t.Dds, t.Dn, U);
+        if (HS) add_angle(t.image, X, Y, Z, t.Dss, t.Dds, t.Dn, U);
     }
-    if (on_side_or_vertex(f, X, Y, Z)) {
+    if (HS ? pair_on_side(t, X, Y, Z) : on_side_or_vertex(t.real, X, Y, Z)) {
         if (STRAIN)
             for (int k = 0; k < 6; ++k) E[k] = qnan<double>();
-        if (DISP)
-            for (int c = 0; c < 3; ++c) U[c] = qnan<double>();
+        for (int c = 0; c < 3; ++c) U[c] = qnan<double>();
     }
 }
 

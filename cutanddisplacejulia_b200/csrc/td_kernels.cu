@@ -149,10 +149,9 @@ __host__ __device__ constexpr int pair_stage(bool hs, int edge, bool one) { retu
 //   side_sum_kernel adds each edge's once.
 //   EDGE_FULL: so is the whole strain (real, image and correction), which
 //   depends on the triangles' sides alone; the pair only combines its three
-//   sides' maps (tractions already for OUT_AMAT and OUT_TRAC).
-//   EDGE_FULL in full space (OUT_SUM): the solid angle; segment_sum_kernel
-//   adds the rest.
-//   In both, points on a side become NaN.
+//   sides' maps (tractions already for OUT_AMAT and OUT_TRAC).  OUT_SUM (full
+//   space too): the displacement's solid angles; side_sum_kernel or
+//   segment_sum_kernel adds the rest.  Points on a side become NaN.
 template <bool HS, bool STRAIN, bool DISP, int OUT, bool NEAR = false, bool LIST = false, int MINB = 1,
           int EDGE = EDGE_NONE>
 __global__ void __launch_bounds__(kPairThreads, MINB) td_pair_kernel(PairArgs a)
@@ -232,14 +231,12 @@ __global__ void __launch_bounds__(kPairThreads, MINB) td_pair_kernel(PairArgs a)
                 }
             continue;
         }
-        if constexpr (OUT == OUT_SUM && !HS && EDGE == EDGE_FULL) {
-            pair_angle<STRAIN, DISP>(t, X, Y, Z, sumE, sumU);
+        if constexpr (OUT == OUT_SUM && EDGE == EDGE_FULL) {
+            static_assert(DISP, "strain alone leaves the pairs to on_side_kernel");
+            pair_angle<HS, STRAIN>(t, X, Y, Z, sumE, sumU);
             continue;
         } else if constexpr (OUT == OUT_SUM && (!HS || EDGE != EDGE_NONE)) {
-            static_assert(EDGE != EDGE_FULL || DISP, "strain alone leaves the pairs to on_side_kernel");
-            pair_net<HS, STRAIN && EDGE != EDGE_FULL, DISP>(t, X, Y, Z, sumE, sumU);
-            if (EDGE == EDGE_FULL && STRAIN && sumU[0] != sumU[0])
-                for (int k = 0; k < 6; ++k) sumE[k] = qnan<double>();
+            pair_net<HS, STRAIN, DISP>(t, X, Y, Z, sumE, sumU);
             continue;
         }
         if (STRAIN) {
@@ -881,8 +878,12 @@ __global__ void __launch_bounds__(kPairThreads) segment_sum_kernel(const SegRec*
 
 // partial[(blockIdx.y * 9 + f) M + i] = the strain (f 0-5; STRAIN EDGE_FSC: the
 // free-surface correction, EDGE_FULL: all of it) and the correction's
-// displacement (f 6-8) at point i of the edges of chunk blockIdx.y, summed in
-// edge order (8 edge records staged in shared memory at a time).
+// displacement (f 6-8; EDGE_FULL: all but the solid angles) at point i of the edges of chunk blockIdx.y, summed in
+// edge order (8 edge records staged in shared memory at a time).  FP64 bound
+// (68 % of the pipe's rate at two resident blocks; three spill): strain and
+// displacement of 15 150 edges at 10 000 points 14.5 ms, the real and image
+// segments' displacement included, and 2.7 ms for the triangles' solid angles;
+// with the segments' displacement taken side by side the pairs took 7.3.
 template <int STRAIN, bool DISP>
 __global__ void __launch_bounds__(kPairThreads) side_sum_kernel(const FscSide* __restrict__ edges, int64_t E,
                                                                 int64_t echunk, const double* __restrict__ X,
@@ -908,7 +909,10 @@ __global__ void __launch_bounds__(kPairThreads) side_sum_kernel(const FscSide* _
 #pragma unroll 1
         for (int k = 0; k < ne; ++k) {
             const FscSide& s = reinterpret_cast<const FscSide*>(smem)[k];
-            if (STRAIN == EDGE_FULL) side_strain_sum(s, x, y, z, Es[0]);
+            if constexpr (STRAIN == EDGE_FULL) {
+                side_sum_full<DISP>(s, x, y, z, Es[0], Us[0]);
+                continue;
+            }
             if (s.skip != 0.0) continue;
             if (STRAIN == EDGE_FSC) fsc_strain(s, x, y, z, 0.0, 0.0, 1.0, Es);
             if (DISP) fsc_disp(s, x, y, z, 0.0, 0.0, 1.0, Us);
