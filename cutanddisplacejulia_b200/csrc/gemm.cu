@@ -3,10 +3,10 @@
 //
 // * FP64 (the plain FP64 solve, A\b of src/SlipCalculator3D.jl:22): DMMA
 //   tensor-core tiles (mma.sync m8n8k4 f64).  A 128 x 64 block of C per CTA,
-//   4 warps of 64 x 32, three CTAs per SM, k-steps of 16 through a 3-deep
-//   cp.async ring (8-byte copies: any leading dimension and any row offset).
-//   Shared-memory words are XOR-swizzled by row so that every fragment load is
-//   free of bank conflicts.
+//   4 warps of 64 x 32, two CTAs per SM, k-steps of 16 through a 3-deep
+//   cp.async ring (16-byte copies, or 8-byte ones for odd leading dimensions
+//   and offsets).  Shared-memory words are XOR-swizzled by row so that every
+//   fragment load is free of bank conflicts.
 // * FP32 with TF32 tensor cores (the mixed solve's FP32 factorisation):
 //   tcgen05.mma kind::tf32 with operands staged by TMA in 128-byte-swizzled
 //   tiles (the MN-major A in 32-byte swizzle atoms, the only layout MN-major
@@ -34,10 +34,15 @@ namespace {
 // ------------------------------------------------------------------ FP64 DMMA
 // CTA tile BM x BN (128 x 64 for large products, 64 x 32 where the large
 // tiles would not fill the GPU), 4 warps of BM/2 x BN/2 as DMMA tiles of
-// 8 x 8; k-steps of 16; several CTAs per SM (the large tile: three, 72 KB of
-// shared memory each -- 3 stages of unpadded, swizzled tiles) so that the
-// DMMA latency is hidden and one CTA's prologue and epilogue overlap the
-// others' main loops.
+// 8 x 8; k-steps of 16.  One warp per scheduler can keep the DMMA pipe busy
+// (36.4 of 37 TFLOP/s from registers), so what bounds the product is the
+// issue slots and latencies between DMMAs: the fragments of the next four k
+// are loaded and a third of a later stage's copies issued before the DMMAs of
+// the current four, the barrier of a k-step falls among DMMAs whose operands
+// are already in registers, and C's lines are prefetched to L2.  Two CTAs per
+// SM, whose registers hold both fragment sets; three would spill.  8192 x 8192
+// x 256: 29.4 TFLOP/s (26.3 with the copies' predicates and 64-bit products
+// between the DMMAs and single fragments at three CTAs), k = 8192: 33.4 (29.1).
 constexpr int DBK = 16, DSTAGES = 3, DTHREADS = 128;
 constexpr int DLDB = DBK;       // shared row (one n) of the B tile, doubles
 template <int BM, int BN>
@@ -54,11 +59,6 @@ struct DTile {
 // sits at row * ld + (col ^ (4 * (row & 3))).
 __device__ __forceinline__ int swz(int row, int col, int ld) { return row * ld + (col ^ ((row & 3) << 2)); }
 
-__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src, bool pred)
-{
-    // src-size 0 writes zeros (rows or columns outside the operand)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(pred ? 8 : 0) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -97,36 +97,91 @@ __device__ __forceinline__ void dmma16<16>(double& c0, double& c1, double& c2, d
                    "d"(b[0]), "d"(b[1]), "d"(b[2]), "d"(b[3]));
 }
 
-// Stage s of the ring <- k-step kt: the A tile (BM rows x 16 columns, stored
-// k-major: row k holds BM consecutive m) and the B tile (16 rows x BN
-// columns, stored n-major: row n holds 16 consecutive k).
-template <int BM, int BN>
-__device__ __forceinline__ void dgemm_load_stage(double* sA, double* sB, const double* __restrict__ A, int64_t lda,
-                                                 const double* __restrict__ B, int64_t ldb, int m, int n, int k,
-                                                 int m0, int n0, int kt)
-{
-    const int tid = threadIdx.x;
-    const int k0 = kt * DBK;
+// One thread's copies of a k-step into its stage of the ring: the A tile (BM rows
+// x 16 columns, stored k-major: row k holds BM consecutive m) and the B tile (16
+// rows x BN columns, stored n-major: row n holds 16 consecutive k).  VEC: 16-byte
+// copies (operands on 16-byte boundaries, even leading dimensions), else 8-byte.
+// Address arithmetic is what the DMMAs compete with for issue slots, so a copy
+// inside the matrix is a running pointer and nothing else.
+template <int BM, int BN, bool VEC>
+struct DCopy {
+    static constexpr int V = VEC ? 2 : 1;
+    static constexpr int PA = BM / V, KA = DTHREADS / PA, NA = DBK / KA;        // threads along m, k step, copies
+    static constexpr int PB = DBK / V, NSTEP = DTHREADS / PB, NB = BN / NSTEP;  // threads along k, n step, copies
+    static constexpr int NC = NA + NB, NBASE = KA >= 4 ? 1 : 4 / KA;
+    static_assert(NC % 3 == 0, "a third of the copies per sub-step");
+    const double *a, *b;    // my first words of the next k-step to be copied
+    int64_t lda, ldb;
+    int ka, kb, kleft;      // my first k in A and in B, k left from that step on
+    int rows, cols;         // rows and columns of the matrices from my first
+    bool full;              // the tile lies inside the matrices
+    uint32_t da[NBASE], db; // shared byte offsets
+
+    __device__ __forceinline__ void init(const double* A, int64_t lda_, const double* B, int64_t ldb_, int m, int n,
+                                         int k, int m0, int n0)
+    {
+        const int tid = threadIdx.x, mm = V * (tid % PA), nn = tid / PB;
+        lda = lda_;
+        ldb = ldb_;
+        kleft = k;
+        ka = tid / PA;
+        kb = V * (tid % PB);
+        rows = m - m0 - mm;
+        cols = n - n0 - nn;
+        full = m0 + BM <= m && n0 + BN <= n;
+        a = A + (m0 + mm) + (int64_t)ka * lda;
+        b = B + kb + (int64_t)(n0 + nn) * ldb;
 #pragma unroll
-    for (int i = 0; i < (BM * DBK) / DTHREADS; ++i) {
-        const int e = tid + DTHREADS * i;
-        const int kk = e / BM, mm = e % BM;
-        const bool ok = (m0 + mm < m) && (k0 + kk < k);
-        const double* src = ok ? A + (int64_t)(m0 + mm) + (int64_t)(k0 + kk) * lda : A;
-        cp_async8(sm100::smem_addr(sA + swz(kk, mm, BM)), src, ok);
+        for (int q = 0; q < NBASE; ++q) da[q] = 8u * (uint32_t)(ka * BM + (mm ^ (((ka + q * KA) & 3) << 2)));
+        db = 8u * (uint32_t)swz(nn, kb, DLDB);
     }
+    // third q of the copies of the next k-step into the stage at (sA, sB)
+    __device__ __forceinline__ void third(int q, uint32_t sA, uint32_t sB, const double* any) const
+    {
+        const bool in = full && kleft >= DBK;
 #pragma unroll
-    for (int i = 0; i < (BN * DBK) / DTHREADS; ++i) {
-        const int e = tid + DTHREADS * i;
-        const int nn = e / DBK, kk = e % DBK;
-        const bool ok = (n0 + nn < n) && (k0 + kk < k);
-        const double* src = ok ? B + (int64_t)(k0 + kk) + (int64_t)(n0 + nn) * ldb : B;
-        cp_async8(sm100::smem_addr(sB + swz(nn, kk, DLDB)), src, ok);
+        for (int u = 0; u < NC / 3; ++u) {
+            const int c = q * (NC / 3) + u;
+            if (c < NA) {
+                const uint32_t dst = sA + da[c % NBASE] + (uint32_t)(c * KA * BM) * 8u;
+                const double* src = a + (int64_t)(c * KA) * lda;
+                if (in) copy_in(dst, src);
+                else copy_edge(dst, src, any, ka + c * KA < kleft ? rows : 0);
+            } else {
+                const int j = c - NA;
+                const uint32_t dst = sB + db + (uint32_t)(j * NSTEP * DLDB) * 8u;
+                const double* src = b + (int64_t)(j * NSTEP) * ldb;
+                if (in) copy_in(dst, src);
+                else copy_edge(dst, src, any, j * NSTEP < cols ? kleft - kb : 0);
+            }
+        }
     }
-}
+    __device__ __forceinline__ void next()
+    {
+        a += (int64_t)DBK * lda;
+        b += DBK;
+        kleft -= DBK;
+    }
+    static __device__ __forceinline__ void copy_in(uint32_t dst, const double* src)
+    {
+        if (VEC) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+        else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+    }
+    // `left` words are inside the matrix; the rest become zeros
+    static __device__ __forceinline__ void copy_edge(uint32_t dst, const double* src, const double* any, int left)
+    {
+        const int w = left < 0 ? 0 : left < V ? left : V;
+        if (VEC)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(w > 0 ? src : any), "r"(8 * w)
+                         : "memory");
+        else
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(w > 0 ? src : any), "r"(8 * w)
+                         : "memory");
+    }
+};
 
 // MK: k-extent of one DMMA (4: m8n8k4 tiles; 8 or 16: m16n8k8 / m16n8k16)
-template <int MK, int BM, int BN, int MINB>
+template <int MK, int BM, int BN, int MINB, bool VEC>
 __global__ void __launch_bounds__(DTHREADS, MINB) dgemm_sub_kernel(int m, int n, int k, const double* __restrict__ A,
                                                                int64_t lda, const double* __restrict__ B, int64_t ldb,
                                                                double* __restrict__ C, int64_t ldc)
@@ -147,37 +202,74 @@ __global__ void __launch_bounds__(DTHREADS, MINB) dgemm_sub_kernel(int m, int n,
         for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
     const int nk = (k + DBK - 1) / DBK;
+    DCopy<BM, BN, VEC> copy;
+    copy.init(A, lda, B, ldb, m, n, k, m0, n0);
+    const uint32_t uA = sm100::smem_addr(sA), uB = sm100::smem_addr(sB);
+    auto stage_a = [&](int s) { return uA + (uint32_t)(s * TL::STAGE_A) * 8u; };
+    auto stage_b = [&](int s) { return uB + (uint32_t)(s * TL::STAGE_B) * 8u; };
 #pragma unroll
     for (int s = 0; s < DSTAGES - 1; ++s) {
-        if (s < nk)
-            dgemm_load_stage<BM, BN>(sA + s * TL::STAGE_A, sB + s * TL::STAGE_B, A, lda, B, ldb, m, n, k, m0, n0, s);
+        if (s < nk) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) copy.third(q, stage_a(s), stage_b(s), A);
+            copy.next();
+        }
         cp_async_commit();
     }
-    for (int kt = 0; kt < nk; ++kt) {
+    // C's lines on their way to L2 while the products run
+    for (int e = threadIdx.x; e < BN * (BM / 16); e += DTHREADS) {
+        const int col = n0 + e / (BM / 16), r = m0 + (e % (BM / 16)) * 16;
+        if (col < n && r < m) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + (int64_t)col * ldc + r));
+    }
+    if constexpr (MK == 4) {
+        double af[2][MT], bf[2][NT];
+        auto frags = [&](const double* a_s, const double* b_s, int kk, double* fa, double* fb) {
+#pragma unroll
+            for (int i = 0; i < MT; ++i) fa[i] = a_s[swz(kk + t, wm + 8 * i + g, BM)];
+#pragma unroll
+            for (int j = 0; j < NT; ++j) fb[j] = b_s[swz(wn + 8 * j + g, kk + t, DLDB)];
+        };
         cp_async_wait<DSTAGES - 2>();
         __syncthreads();
-        // refill the stage consumed one step ago (every warp is past it)
-        const int kn = kt + DSTAGES - 1;
-        if (kn < nk)
-            dgemm_load_stage<BM, BN>(sA + (kn % DSTAGES) * TL::STAGE_A, sB + (kn % DSTAGES) * TL::STAGE_B, A, lda, B,
-                                     ldb, m, n, k, m0, n0, kn);
-        cp_async_commit();
-        const double* a_s = sA + (kt % DSTAGES) * TL::STAGE_A;
-        const double* b_s = sB + (kt % DSTAGES) * TL::STAGE_B;
-        if constexpr (MK == 4) {
+        frags(sA, sB, 0, af[0], bf[0]);
+        int cur = 0;   // stage of this k-step
+        for (int kt = 0; kt < nk; ++kt) {
+            const int nxt = cur + 1 == DSTAGES ? 0 : cur + 1;
+            const int fill = cur == 0 ? DSTAGES - 1 : cur - 1;   // consumed one step ago, every warp past it
+            const bool more = kt + DSTAGES - 1 < nk;
 #pragma unroll
-            for (int kk = 0; kk < DBK; kk += 4) {
-                double af[MT], bf[NT];
-#pragma unroll
-                for (int i = 0; i < MT; ++i) af[i] = a_s[swz(kk + t, wm + 8 * i + g, BM)];
-#pragma unroll
-                for (int j = 0; j < NT; ++j) bf[j] = b_s[swz(wn + 8 * j + g, kk + t, DLDB)];
+            for (int q = 0; q < 4; ++q) {
+                if (q == 3) {   // this step's last words are in registers: on to the next stage
+                    cp_async_commit();
+                    cp_async_wait<DSTAGES - 2>();
+                    __syncthreads();
+                }
+                const double* a_s = sA + (q == 3 ? nxt : cur) * TL::STAGE_A;
+                const double* b_s = sB + (q == 3 ? nxt : cur) * TL::STAGE_B;
+                frags(a_s, b_s, q == 3 ? 0 : 4 * (q + 1), af[(q + 1) & 1], bf[(q + 1) & 1]);
+                if (q < 3 && more) copy.third(q, stage_a(fill), stage_b(fill), A);
 #pragma unroll
                 for (int i = 0; i < MT; ++i)
 #pragma unroll
-                    for (int j = 0; j < NT; ++j) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+                    for (int j = 0; j < NT; ++j) dmma(acc[i][j][0], acc[i][j][1], af[q & 1][i], bf[q & 1][j]);
             }
-        } else {
+            copy.next();
+            cur = nxt;
+        }
+    } else {
+        for (int kt = 0; kt < nk; ++kt) {
+            cp_async_wait<DSTAGES - 2>();
+            __syncthreads();
+            // refill the stage consumed one step ago (every warp is past it)
+            const int kn = kt + DSTAGES - 1;
+            if (kn < nk) {
+#pragma unroll
+                for (int q = 0; q < 3; ++q) copy.third(q, stage_a(kn % DSTAGES), stage_b(kn % DSTAGES), A);
+                copy.next();
+            }
+            cp_async_commit();
+            const double* a_s = sA + (kt % DSTAGES) * TL::STAGE_A;
+            const double* b_s = sB + (kt % DSTAGES) * TL::STAGE_B;
             // 16-row blocks: acc[2I] holds rows wm + 16I + g, acc[2I + 1]
             // rows wm + 16I + 8 + g (the 8-row layout of the m8n8k4 path)
 #pragma unroll
@@ -517,30 +609,36 @@ bool tma_ok(const float* p, int64_t ld)
 }  // namespace
 
 namespace {
-template <int MK, int BM, int BN, int MINB>
+template <int MK, int BM, int BN, int MINB, bool VEC>
 cudaError_t launch_dgemm_tile(cudaStream_t st, int m, int n, int k, const double* A, int64_t lda, const double* B,
                               int64_t ldb, double* C, int64_t ldc)
 {
     constexpr size_t smem = DTile<BM, BN>::SMEM;
     static std::once_flag once;
     std::call_once(once, [] {
-        cudaFuncSetAttribute(dgemm_sub_kernel<MK, BM, BN, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(dgemm_sub_kernel<MK, BM, BN, MINB, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
-        cudaFuncSetAttribute(dgemm_sub_kernel<MK, BM, BN, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        cudaFuncSetAttribute(dgemm_sub_kernel<MK, BM, BN, MINB, VEC>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             100);
     });
     const dim3 grid((unsigned)((m + BM - 1) / BM), (unsigned)((n + BN - 1) / BN));
-    dgemm_sub_kernel<MK, BM, BN, MINB><<<grid, DTHREADS, smem, st>>>(m, n, k, A, lda, B, ldb, C, ldc);
+    dgemm_sub_kernel<MK, BM, BN, MINB, VEC><<<grid, DTHREADS, smem, st>>>(m, n, k, A, lda, B, ldb, C, ldc);
     return cudaGetLastError();
 }
 
-// the large tile where it gives at least two CTAs per SM, else the small one
+// the large tile where it gives at least two CTAs per SM, else the small one;
+// 16-byte copies where every one of them starts on its boundary
 template <int MK>
 cudaError_t launch_dgemm(cudaStream_t st, int m, int n, int k, const double* A, int64_t lda, const double* B,
                          int64_t ldb, double* C, int64_t ldc)
 {
     const int64_t big = (int64_t)((m + 127) / 128) * ((n + 63) / 64);
-    if (big >= 2 * 148) return launch_dgemm_tile<MK, 128, 64, 3>(st, m, n, k, A, lda, B, ldb, C, ldc);
-    return launch_dgemm_tile<MK, 64, 32, 6>(st, m, n, k, A, lda, B, ldb, C, ldc);
+    const bool vec = !(((uintptr_t)A | (uintptr_t)B) & 15) && !((lda | ldb) & 1);
+    if (big >= 2 * 148)
+        return vec ? launch_dgemm_tile<MK, 128, 64, 2, true>(st, m, n, k, A, lda, B, ldb, C, ldc)
+                   : launch_dgemm_tile<MK, 128, 64, 2, false>(st, m, n, k, A, lda, B, ldb, C, ldc);
+    return vec ? launch_dgemm_tile<MK, 64, 32, 5, true>(st, m, n, k, A, lda, B, ldb, C, ldc)
+               : launch_dgemm_tile<MK, 64, 32, 5, false>(st, m, n, k, A, lda, B, ldb, C, ldc);
 }
 }  // namespace
 
