@@ -49,6 +49,7 @@ enum Slot {
 constexpr int kGmresRestart = 30; // default Krylov dimension of a GMRES cycle
 constexpr int kLuBlock = 256;     // outer block width of the FP64 LU
 constexpr int kLuBlock32 = 512;   // of the FP32 factorisation (its TF32 products gain more from a long k)
+constexpr int64_t kLuWideFrom = 20000;   // and of FP64 ones from this size on (lu_nb)
 constexpr int64_t kStageWords = 32768;   // host calls up to this many doubles in, and out, are staged in one copy each
 constexpr size_t kEdgeMapBytes = size_t(8) << 30;   // cap on the shared-edge free-surface maps of one chunk
 
@@ -149,7 +150,13 @@ struct NvtxRange {
 #define CAD_NVTX_RANGE() NvtxRange nvtx_range_(__func__)
 
 // outer block width of a single-system factorisation
-int lu_nb(const cad_ctx* c, bool fp32) { return c->lu_block > 0 ? c->lu_block : (fp32 ? kLuBlock32 : kLuBlock); }
+// Wide blocks where the FP64 trailing products hide the longer panels: 256 and
+// 512 columns take 167 and 167 ms at n = 18 000, 363 and 357 at 24 000, 681 and
+// 662 at 30 000 (61 and 64 at 12 000).
+int lu_nb(const cad_ctx* c, bool fp32, int64_t n)
+{
+    return c->lu_block > 0 ? c->lu_block : (fp32 || n >= kLuWideFrom ? kLuBlock32 : kLuBlock);
+}
 
 int fail(cad_ctx* c, int code, const std::string& msg)
 {
@@ -511,7 +518,7 @@ int solve_mixed_device(cad_ctx* ctx, int64_t n, const double* A, int64_t lda, do
     ls.naux = kLeafAux;
     ctx->timed[1] = ctx->timed[2] = false;
     int rc = mixed_prepare(ls, A, lda, n, (float*)a32, (float*)dinv, (int*)piv, (int*)perm, (int*)info,
-                           lu_nb(ctx, true));
+                           lu_nb(ctx, true, n));
     if (rc == LU_TOO_LARGE) return fail(ctx, CAD_ERR_ARG, "matrix too large for the dense LU");
     if (rc != LU_OK) return fail(ctx, CAD_ERR_CUDA, "FP32 LU failed (CUDA error)");
     CK(cudaEventRecord(ctx->ev[4], ctx->stream));
@@ -560,7 +567,7 @@ int solve_mixed_device(cad_ctx* ctx, int64_t n, const double* A, int64_t lda, do
         if (int r = ensure(ctx, S_IR32, 2 * (size_t)n * nrhs * sizeof(float), &ir32)) return r;
         if (int r = ensure(ctx, S_NORMS, 2 * (size_t)nrhs * sizeof(double), &norms)) return r;
         X = (double*)ir;
-        IrArgs ia{ls, n, A, lda, B, ldb, (int)nrhs, X, (float*)a32, (int*)piv, (int*)perm, (int*)info, lu_nb(ctx, true),
+        IrArgs ia{ls, n, A, lda, B, ldb, (int)nrhs, X, (float*)a32, (int*)piv, (int*)perm, (int*)info, lu_nb(ctx, true, n),
                   ctx->tol, kIrMaxIter, X + (size_t)n * nrhs, (float*)ir32, (float*)ir32 + (size_t)n * nrhs,
                   (double*)norms};
         IrResult res{};
@@ -752,7 +759,7 @@ int solve_device(cad_ctx* ctx, int64_t n, double* A, int64_t lda, double* B, int
                 if (e != cudaSuccess) return e;
                 lt.min_leaf_rpt = c;
                 return lu_factor_solve<double>(lt, (double*)scratch, n, n, nullptr, 0, 0, nullptr, 0, (int*)piv,
-                                               (int*)perm, (int*)info, lu_nb(ctx, false), true, false) == LU_OK
+                                               (int*)perm, (int*)info, lu_nb(ctx, false, n), true, false) == LU_OK
                            ? cudaSuccess
                            : cudaErrorUnknown;
             });
@@ -763,7 +770,7 @@ int solve_device(cad_ctx* ctx, int64_t n, double* A, int64_t lda, double* B, int
         if (int r = ensure(ctx, S_CHAIN, (size_t)n * sizeof(double) + lu_chain_sync_ints(n) * sizeof(int), &chain))
             return r;
         const int rc = lu_factor_solve<double>(ls, A, n, lda, nullptr, 0, 0, nullptr, 0, (int*)piv, (int*)perm, (int*)info,
-                                         lu_nb(ctx, false), true, false);
+                                         lu_nb(ctx, false, n), true, false);
         if (rc == LU_TOO_LARGE) return fail(ctx, CAD_ERR_ARG, "matrix too large for the dense LU");
         if (rc != LU_OK) return fail(ctx, CAD_ERR_CUDA, "dense LU failed (CUDA error)");
         double* y = (double*)chain;
@@ -775,7 +782,7 @@ int solve_device(cad_ctx* ctx, int64_t n, double* A, int64_t lda, double* B, int
         return CAD_OK;
     }
     const int rc = lu_factor_solve<double>(ls, A, n, lda, B, ldb, (int)nrhs, (double*)work, n, (int*)piv, (int*)perm,
-                                           (int*)info, lu_nb(ctx, false), true, true);
+                                           (int*)info, lu_nb(ctx, false, n), true, true);
     if (rc == LU_TOO_LARGE) return fail(ctx, CAD_ERR_ARG, "matrix too large for the dense LU");
     if (rc != LU_OK) return fail(ctx, CAD_ERR_CUDA, "dense LU failed (CUDA error)");
     CK(cudaMemcpy2DAsync(B, ldb * sizeof(double), work, n * sizeof(double), n * sizeof(double), nrhs,

@@ -70,3 +70,16 @@ def test_lu_repeated_entries_and_singular(cad):
     L, ctx = _lib.load(), _lib.context(0)
     torch.cuda.synchronize()
     assert L.cad_last_error(ctx)
+
+
+@pytest.mark.parametrize("n", [511, 513, 1100, 2100])
+def test_lu_wide_blocks(cad, n):
+    # the block width large systems take
+    from cutanddisplacejulia_b200 import _lib
+    L, ctx = _lib.load(), _lib.context(0)
+    _lib.check(L.cad_set_lu_block(ctx, 512), ctx)
+    try:
+        for nrhs in (1, 3):
+            assert _solve(n, nrhs, 300 + n)[0] < 64 * n * 2.3e-16
+    finally:
+        _lib.check(L.cad_set_lu_block(ctx, 0), ctx)
