@@ -652,17 +652,20 @@ __global__ void __launch_bounds__(256) axpy_group_kernel(const __grid_constant__
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < r.n; i += gridDim.x * blockDim.x) r.x[i] += r.z[i];
 }
 
-// r = b - A x in FP64: thread per row (coalesced down each column), x staged
-// through shared memory, eight column loads in flight per thread into four
-// accumulators (column c to accumulator c % 4, combined in a fixed order);
-// rows past n zero
+// r = b - A x in FP64: 32 rows per block, warp q the columns c with c mod 4 = q
+// (256 bytes of a column per load), x staged through shared memory, eight loads
+// in flight per thread, the four sums combined in a fixed order; rows past n
+// zero.  HBM bound; a thread per row over all columns left the largest cracks'
+// blocks a long tail (64 cracks of 200 to 1500 elements, 2.8 GB: 1.06 ms, now
+// 0.50, 5.6 TB/s).
 __global__ void __launch_bounds__(128) residual_group_kernel(const __grid_constant__ CrackGroup g)
 {
-    __shared__ double s_x[1024];
+    __shared__ double s_x[1024], s_sum[4][32];
     const CrackRec& r = g.rec[blockIdx.y];
-    const int i = blockIdx.x * 128 + threadIdx.x;
-    if ((int)blockIdx.x * 128 >= r.n_pad) return;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    if ((int)blockIdx.x * 32 >= r.n_pad) return;
+    double acc = 0.0;
     for (int c0 = 0; c0 < r.n; c0 += 1024) {
         const int cn = r.n - c0 < 1024 ? r.n - c0 : 1024;
         __syncthreads();
@@ -670,18 +673,21 @@ __global__ void __launch_bounds__(128) residual_group_kernel(const __grid_consta
         __syncthreads();
         if (i < r.n) {
             const double* a = r.A + i + (int64_t)c0 * r.lda;
-            int c = 0;
-            for (; c + 8 <= cn; c += 8) {
+            int c = q;
+            for (; c + 28 < cn; c += 32) {
                 double v[8];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) v[u] = a[(int64_t)(c + u) * r.lda];
+                for (int u = 0; u < 8; ++u) v[u] = a[(int64_t)(c + 4 * u) * r.lda];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) acc[u & 3] = fma(v[u], s_x[c + u], acc[u & 3]);
+                for (int u = 0; u < 8; ++u) acc = fma(v[u], s_x[c + 4 * u], acc);
             }
-            for (; c < cn; ++c) acc[c & 3] = fma(a[(int64_t)c * r.lda], s_x[c], acc[c & 3]);
+            for (; c < cn; c += 4) acc = fma(a[(int64_t)c * r.lda], s_x[c], acc);
         }
     }
-    if (i < r.n_pad) r.r[i] = i < r.n ? r.b[i] - ((acc[0] + acc[1]) + (acc[2] + acc[3])) : 0.0;
+    s_sum[q][lane] = acc;
+    __syncthreads();
+    if (q == 0 && i < r.n_pad)
+        r.r[i] = i < r.n ? r.b[i] - ((s_sum[0][lane] + s_sum[1][lane]) + (s_sum[2][lane] + s_sum[3][lane])) : 0.0;
 }
 
 // rel = ||r|| / ||b|| per crack (fixed-order block reduction)
@@ -754,7 +760,7 @@ int mixed_group_sweeps(const LuStreams& ls, const std::vector<CrackRec>& cracks,
                 axpy_group_kernel<<<dim3((unsigned)((nmax + 255) / 256), g.count), 256, 0, st>>>(g);
             }) ||
             !each_group(cracks, L, [&](const CrackGroup& g, int nmax) {
-                residual_group_kernel<<<dim3((unsigned)((nmax + 127) / 128), g.count), 128, 0, st>>>(g);
+                residual_group_kernel<<<dim3((unsigned)((nmax + 31) / 32), g.count), 128, 0, st>>>(g);
             }))
             return GMRES_CUDA_ERROR;
     }
