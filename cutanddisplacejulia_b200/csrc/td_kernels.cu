@@ -724,8 +724,10 @@ cudaError_t launch_assemble_edges(PairArgs a, int out_kind, bool strain, bool di
     MapKernel ek;
     const bool trac = out_kind != OUT_INF;
     if (trac && full) {
+        // (the maps' loads bound the system matrix of 10 000 triangles: 4.4 ms at
+        // three resident blocks, 4.0 at five)
         pk = out_kind == OUT_TRAC ? td_pair_kernel<true, true, false, OUT_TRAC, false, false, 1, EDGE_FULL>
-                                  : td_pair_kernel<true, true, false, OUT_AMAT, false, false, 1, EDGE_FULL>;
+                                  : td_pair_kernel<true, true, false, OUT_AMAT, false, false, 5, EDGE_FULL>;
         ek = side_map_kernel<EDGE_FULL, false, true>;
     } else if (trac) {
         pk = out_kind == OUT_TRAC ? td_pair_kernel<true, true, false, OUT_TRAC, false, false, 1, EDGE_FSC>
