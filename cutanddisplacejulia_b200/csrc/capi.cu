@@ -1858,6 +1858,9 @@ int cad_gemm_sub_dev(cad_ctx* ctx, int precision, int64_t m, int64_t n, int64_t 
     if (m == 0 || n == 0 || k == 0) return CAD_OK;
     void* st;
     if (int r = ensure(ctx, S_GEMM, sizeof(int), &st)) return r;
+    // the operands may still be read or written by work on the default stream
+    CK(cudaEventRecord(ctx->side_fork, cudaStreamLegacy));
+    CK(cudaStreamWaitEvent(ctx->stream, ctx->side_fork, 0));
     CK(cudaMemsetAsync(st, 0, sizeof(int), ctx->stream));
     if (precision != 1) {
         static const int dmma_k[5] = {0, 0, 4, 8, 16};
