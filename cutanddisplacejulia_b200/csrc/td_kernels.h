@@ -48,7 +48,7 @@ struct PairArgs {
     // resident blocks per SM (1: the full register file; 3 or 4)
     int min_blocks = 1;
     // half-space system matrix with shared-edge free-surface maps: the maps
-    // of this launch's points (18 x M per edge, fsc_edge_kernel) and each
+    // of this launch's points (18 x M per edge, side_map_kernel) and each
     // triangle's three side codes (+-(edge + 1), 0: none); rows are then a
     // block of an Ntot-point system (X, Y, Z, dirs and A or trac start at the
     // block; the output fields keep the system's row stride)

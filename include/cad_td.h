@@ -156,19 +156,20 @@ int cad_set_lu_block(cad_ctx* ctx, int nb);
  * preconditioned GMRES solvers): 1..63, 0 = the default 30.  Every cycle
  * starts from the FP64 residual b - A x.  No counterpart in the reference. */
 int cad_set_gmres_restart(cad_ctx* ctx, int m);
-/* Work on meshes whose triangles share edges.
- * 1 (default): in full space the summed evaluations (cad_td_sum_eval*) of
- * many pairs take each mesh edge once, with the net Burgers vector of the
- * sides on it; in half space, for fewer edges than 0.9 x the triangle sides
- * (other meshes always take the per-side path), the FP64 system matrix and traction influence fields
- * (cad_assemble*, cad_slip_calculator*, cad_influence_traction with hs_flag
- * 1) evaluate the free-surface correction of each mesh edge once per
- * collocation point, and the triangles that share the edge reuse it
- * with the sign of their side's direction, and so do the influence fields
- * (cad_td_inf*, strain and displacement maps per edge); the summed evaluations
- * (cad_td_sum_eval*) evaluate it once per edge for the net Burgers vector of
- * the sides on it.  0: per triangle side, as the reference does.  Same
- * results to rounding.  No counterpart in the reference. */
+/* Work on meshes whose triangles share edges.  1 (default): each mesh edge is
+ * taken once.
+ *   Full space: the summed evaluations (cad_td_sum_eval*) of many pairs, each
+ *   edge with the net Burgers vector of the sides on it.
+ *   Half space, for fewer edges than 0.9 x the triangle sides (other meshes
+ *   take the per-side path): the FP64 system matrix and traction influence
+ *   fields (cad_assemble*, cad_slip_calculator*, cad_influence_traction) and
+ *   the influence fields (cad_td_inf*) from maps of each edge at every point,
+ *   which the triangles that share the edge read with the sign of their side's
+ *   direction; the summed evaluations for the edge's net Burgers vector.  The
+ *   maps are of the whole strain, or of the free-surface correction alone if a
+ *   triangle is exactly horizontal.
+ * 0: per triangle side, as the reference does.  Same results to rounding.  No
+ * counterpart in the reference. */
 int cad_set_shared_edges(cad_ctx* ctx, int enable);
 #define CAD_BATCH_GROUPED 0
 #define CAD_BATCH_LANES 1
