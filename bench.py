@@ -44,19 +44,19 @@ FALG_ASSEMBLY_FS = 2960.0 + 288.0
 # collocation pairs) plus the same traction epilogue.
 FALG_ASSEMBLY_HS = 43867.0 + 288.0
 # DRAM bytes (read + write) of one assembly from the committed ncu captures
-# (profiles/td_pair_kernel_*.md, profiles/fsc_edge_kernel_*.md): (triangles
-# captured, bytes).  Both scale as N^2.  Half space: the shared-edge path's two
-# kernels, fsc_edge_kernel (17.75 MB + 1.0328 GB) and the edge pair kernel
-# built for three blocks per SM (1.0982 GB + 307.38 MB), at 1980 triangles and
-# 3037 edges.
-PAIR_TRAFFIC = {"penny": (2013, 2.49e6 + 233.84e6), "dipping": (1980, 17.75e6 + 1.0328e9 + 1.0982e9 + 307.38e6)}
+# (profiles/td_kernels_edges_and_pairs.md): (triangles captured, bytes).  Both
+# scale as N^2.  Half space: the shared-edge path's two kernels, side_map_kernel
+# (4.80 MB + 380.33 MB) and the combining pair kernel (517.18 MB + 249.88 MB), at
+# 1980 triangles and 3037 edges.
+PAIR_TRAFFIC = {"penny": (2013, 1.04e6 + 231.96e6), "dipping": (1980, 4.80e6 + 380.33e6 + 517.18e6 + 249.88e6)}
 # FP64-pipe activity (fraction of peak, ncu sm__pipe_fp64_cycles_active) of the
 # shared-edge half-space assembly's kernels, from the committed capture at 1980
-# triangles (profiles/fsc_edge_kernel_*.md)
-FP64_PIPE_ACTIVE_HS = {"fsc_edge_kernel": 0.538, "td_pair_kernel_edge": 0.591}
+# triangles (profiles/td_kernels_edges_and_pairs.md); the pair kernel is bound by
+# the maps' bytes
+FP64_PIPE_ACTIVE_HS = {"side_map_kernel": 0.729, "td_pair_kernel_edge": 0.171}
 # share of the step's (serialised) device time taken by the LU panel leaf, from
 # the committed launch list (profiles/launches_penny2013_fp64_and_mixed_step.md)
-DOMINANT_SHARE = {"penny": 0.532}
+DOMINANT_SHARE = {"penny": 0.306}
 SPACING = 0.06          # lattice spacing of the penny crack (~2013 triangles)
 NU, G = 0.25, 1.0
 TRACTION = -1e-3
@@ -569,7 +569,7 @@ def batch_rhs_timing(args, ctx, L, stream, asm_args, nrm, A, dev):
 def run_batch(args, rank, world, local_rank):
     """Many independent cracks (the batching configuration): every crack
     assembled (FP32 far field / FP64 near field) and solved by FP32 LU with
-    FP64 refinement to relative residual 1e-10, all cracks in one captured
+    FP64 refinement to relative residual 1e-10, all cracks in one replayed
     CUDA graph over 32 stream lanes (cad_slip_calculator_batched_dev).  Beside
     it: the plain per-crack FP64 path (assembly + FP64 LU, one crack after the
     other) on the same cracks, and the slip error against it."""
@@ -622,10 +622,10 @@ def run_batch(args, rank, world, local_rank):
 
     with _lib.solver_mode(ctx, "mixed", MIXED_TOL, 400), _lib.assembly_mode(ctx, "mixed", NEAR_FACTOR):
         t0 = time.perf_counter()
-        batched()                                   # captures the batch graph
+        batched()                                   # the plan's first call, issued directly
         torch.cuda.synchronize()
         capture_s = time.perf_counter() - t0
-        for _ in range(max(0, args.warmup - 1)):
+        for _ in range(max(1, args.warmup - 1)):    # the second call captures the batch graph
             batched()
         torch.cuda.synchronize()
         clocks = ClockSampler(local_rank)
@@ -1030,7 +1030,7 @@ def run_c3(args, rank, world, local_rank):
                 "ms_per_step": e2e_ms, "slip_rel_err_vs_fp64_lu": e2e_err,
                 "api": "cad_slip_calculator, solver CAD_SOLVER_GMRES_LEARNED (host C ABI, pinned host buffers)"},
         "gpu_launches": int(launches),
-        "roofline": {"kernel": "fsc_edge_kernel + td_pair_kernel<HS, strain, A-matrix, EDGE> (the step's dominant "
+        "roofline": {"kernel": "side_map_kernel + td_pair_kernel<HS, strain, A-matrix, EDGE> (the step's dominant "
                                "phase: the FP64 shared-edge half-space assembly)",
                      "bound": "fp64", "achieved": asm_tflops, "peak": fp64_peak, "unit": "TFLOP/s",
                      "frac": asm_tflops / fp64_peak,
@@ -1039,13 +1039,14 @@ def run_c3(args, rank, world, local_rank):
                      "falg_per_pair": falg,
                      "traffic": PAIR_TRAFFIC["dipping"][1] * (n / PAIR_TRAFFIC["dipping"][0]) ** 2,
                      "traffic_source": "ncu DRAM bytes (read + write) of the assembly's two kernels at N=%d, "
-                                       "scaled by (N/%d)^2; the edge maps (18 doubles per edge and point) are "
+                                       "scaled by (N/%d)^2; the edge maps (9 doubles per edge and point) are "
                                        "written once and read by the triangles sharing each edge, the rest is "
                                        "the matrix" % (PAIR_TRAFFIC["dipping"][0], PAIR_TRAFFIC["dipping"][0]),
                      "falg_note": "F_alg is the reference's literal count per pair, which evaluates each "
-                                  "side's free-surface correction per triangle and slip mode; the shared-edge "
-                                  "path evaluates it once per edge, so the algorithmic rate exceeds the FP64 "
-                                  "pipe's peak while the pipe itself is about half busy (fp64_pipe_active_ncu)",
+                                  "side's terms per triangle and slip mode from angular dislocations; the "
+                                  "shared-edge path evaluates each edge once, from straight segments and "
+                                  "harmonic functions, so the algorithmic rate exceeds the FP64 pipe's peak "
+                                  "(fp64_pipe_active_ncu is the pipe's own activity)",
                      "fp64_pipe_active_ncu": FP64_PIPE_ACTIVE_HS,
                      "step_share": asm_ms / ms},
         "roofline_gmres": {"kernel": "GMRES(30): FP32 copy of A, one FP32 pass over A per Arnoldi product, "
@@ -1225,7 +1226,7 @@ def run_ours(args, rank, world, local_rank):
         "dominant_kernel": {"name": "leaf_lu_kernel<double, 32, 1>",
                             "share_of_step_ncu": DOMINANT_SHARE.get(args.workload),
                             "bound": "latency: one pivot search and row exchange across a 12-16 CTA cluster per "
-                                     "column (about 1.7 us per column)",
+                                     "column (about 1.3 us per column)",
                             "source": "profiles/launches_penny2013_fp64_and_mixed_step.md",
                             "ncu_full": "profiles/leaf_lu_kernel_penny2013.md",
                             # from that capture (4856 x 32 panel): the panel read once, issue 12.8 %,
@@ -1458,12 +1459,12 @@ def run_tdsum(args, rank, world, local_rank):
                 "h2d_bytes_per_step": (3 * m + 9 * n + 3 * n) * 8, "d2h_bytes_per_step": 9 * m * 8,
                 "api": "cad.TD(..., Strains(), Disps()) with host arrays (cad_td_sum_eval, host C ABI)"},
         "gpu_launches": int(launches),
-        "roofline": {"kernel": "td_pair_kernel<HS, sum, EDGE> + fsc_sum_kernel (shared-edge half-space sums)",
+        "roofline": {"kernel": "side_sum_kernel + td_pair_kernel<HS, sum, EDGE> (shared-edge half-space sums)",
                      "bound": "fp64", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
                      "frac": achieved / peak.value, "falg_per_pair": FALG_SUM_HS,
                      "peak_source": "measured FP64 FMA throughput (cad_fp64_fma_probe, this run)",
                      "falg_note": "the reference's literal count per pair; the shared-edge path evaluates each "
-                                  "edge's free-surface correction once instead of per side and mode",
+                                  "edge's field once instead of per side and mode",
                      "traffic": None},
         "cpu_baseline": cpu,
     }
