@@ -886,17 +886,16 @@ __global__ void __launch_bounds__(kPairThreads) segment_sum_kernel(const SegRec*
 // partial[(blockIdx.y * 9 + f) M + i] = the strain (f 0-5; STRAIN EDGE_FSC: the
 // free-surface correction, EDGE_FULL: all of it) and the correction's
 // displacement (f 6-8; EDGE_FULL: all but the solid angles) at point i of the edges of chunk blockIdx.y, summed in
-// edge order (8 edge records staged in shared memory at a time).  FP64 bound
-// (68 % of the pipe's rate at two resident blocks; three spill): strain and
-// displacement of 15 150 edges at 10 000 points 14.5 ms, the real and image
-// segments' displacement included, and 2.7 ms for the triangles' solid angles;
-// with the segments' displacement taken side by side the pairs took 7.3.
+// edge order (8 edge records staged in shared memory at a time).  FP64 bound;
+// three resident blocks per SM are worth the 128 bytes they spill (strain and
+// displacement of 15 150 edges at 10 000 points, the real and image segments'
+// displacement included: 14.5 ms at two blocks and 66 % of the pipe, 13.6 at
+// three).  The triangles' solid angles take 2.7 ms more; with the segments'
+// displacement taken side by side the pairs took 7.3.
 template <int STRAIN, bool DISP>
-__global__ void __launch_bounds__(kPairThreads) side_sum_kernel(const FscSide* __restrict__ edges, int64_t E,
-                                                                int64_t echunk, const double* __restrict__ X,
-                                                                const double* __restrict__ Y,
-                                                                const double* __restrict__ Z, int64_t M,
-                                                                double* __restrict__ partial)
+__global__ void __launch_bounds__(kPairThreads, STRAIN == EDGE_NONE ? 4 : STRAIN == EDGE_FSC && DISP ? 2 : 3)
+side_sum_kernel(const FscSide* __restrict__ edges, int64_t E, int64_t echunk, const double* __restrict__ X,
+                const double* __restrict__ Y, const double* __restrict__ Z, int64_t M, double* __restrict__ partial)
 {
     extern __shared__ double smem[];
     const int64_t i = (int64_t)blockIdx.x * kPairThreads + threadIdx.x;
