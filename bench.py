@@ -1229,10 +1229,10 @@ def run_ours(args, rank, world, local_rank):
                                      "column (about 1.3 us per column)",
                             "source": "profiles/launches_penny2013_fp64_and_mixed_step.md",
                             "ncu_full": "profiles/leaf_lu_kernel_penny2013.md",
-                            # from that capture (4856 x 32 panel): the panel read once, issue 12.8 %,
-                            # FP64 pipe 2.2 %, DRAM 0.17 % of peak
-                            "ncu_dram_bytes_per_launch": 1.46e6, "ncu_issue_active": 0.128,
-                            "ncu_fp64_pipe": 0.022},
+                            # from that capture (a panel of ten CTAs): the panel read once, issue
+                            # 30.2 %, FP64 pipe 5.0 %, DRAM 0.33 % of peak
+                            "ncu_dram_bytes_per_launch": 1.29e6, "ncu_issue_active": 0.302,
+                            "ncu_fp64_pipe": 0.050},
         "roofline_assembly": {"kernel": "td_pair_kernel<%s, strain, A-matrix>" % ("HS" if hs else "FS"),
                               "bound": "fp64", "achieved": achieved, "peak": fp64_peak_tflops, "unit": "TFLOP/s",
                               "frac": achieved / fp64_peak_tflops,
