@@ -43,7 +43,8 @@ EXPORTS = [
     "cad_assemble_columns_dev", "cad_gemm_sub_dev", "cad_lpc_features_dev", "cad_lpc_set_network",
     "cad_lpc_get_network", "cad_lpc_dataset_add", "cad_lpc_dataset_rows", "cad_lpc_dataset_clear",
     "cad_lpc_dataset_get", "cad_lpc_dataset_set", "cad_lpc_forward_backward", "cad_lpc_train", "cad_lpc_install_dev",
-    "cad_lpc_install", "cad_set_wait_limit", "cad_wait_timeout_probe", "cad_set_gmres_matvec", "cad_set_batch_solve",
+    "cad_lpc_install", "cad_set_wait_limit", "cad_wait_timeout_probe", "cad_leaf_timeout_probe",
+    "cad_set_gmres_matvec", "cad_set_batch_solve",
     "cad_set_lu_block", "cad_set_gmres_restart", "cad_set_shared_edges",
     "cad_set_autotune", "cad_autotune_entries",
 ]
@@ -139,6 +140,7 @@ def load():
     L.cad_autotune_entries.argtypes = [P, ctypes.POINTER(I64)]
     L.cad_autotune_entries.restype = I64
     L.cad_wait_timeout_probe.argtypes = [P, I64]
+    L.cad_leaf_timeout_probe.argtypes = [P, I64]
     L.cad_friction_prepare.argtypes = [P, P, P, P, I64, D, D, D, P, P, INT]
     L.cad_friction_solve.argtypes = [P, I64, P, P, P, P, P, D, INT, P, P, P]
     _lib = L

@@ -1424,6 +1424,29 @@ int cad_wait_timeout_probe(cad_ctx* ctx, int64_t n)
     return CAD_OK;
 }
 
+int cad_leaf_timeout_probe(cad_ctx* ctx, int64_t n)
+{
+    CAD_NVTX_RANGE();
+    if (int r = set_device(ctx)) return r;
+    if (n <= 512 || n > 4096) return fail(ctx, CAD_ERR_ARG, "invalid argument");
+    void *a, *x, *piv, *perm, *info;
+    if (int r = ensure(ctx, S_WORK, (size_t)n * n * sizeof(double), &a)) return r;
+    if (int r = ensure(ctx, S_B, (size_t)n * sizeof(double), &x)) return r;
+    if (int r = ensure(ctx, S_PIV, (size_t)n * sizeof(int), &piv)) return r;
+    if (int r = ensure(ctx, S_PERM, (size_t)n * sizeof(int), &perm)) return r;
+    if (int r = ensure(ctx, S_INFO, kLuInfoInts * sizeof(int), &info)) return r;
+    LuStreams ls{ctx->stream, ctx->side_stream, &ctx->launches, nullptr, ctx->wait_limit};
+    ls.aux = ctx->leaf_aux;
+    ls.naux = kLeafAux;
+    if (lu_leaf_timeout_probe(ls, (double*)a, n, (double*)x, (int*)piv, (int*)perm, (int*)info) != LU_OK)
+        return fail(ctx, CAD_ERR_CUDA, "dense LU failed (CUDA error)");
+    int h = 0;
+    CK(cudaMemcpyAsync(&h, info, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (h < 0) return fail(ctx, CAD_ERR_TIMEOUT, "a device wait ran out (pivot exchange of a leaf)");
+    return CAD_OK;
+}
+
 int cad_last_solve_stats(const cad_ctx* ctx, int* iterations, double* rel_residual)
 {
     if (!ctx) return CAD_ERR_ARG;

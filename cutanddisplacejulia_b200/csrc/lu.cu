@@ -164,7 +164,15 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned mbar, unsigned parity)
 // (1-based, + col_base), or -1 if a wait ran out.  moved (may be null): the net
 // row movement for leaf_update_kernel, moved[c] = panel row now at position c,
 // moved[W + c] = position of the row that was at c (c < w).
-template <typename T, int W, int RPT>
+// A wait that runs out: info becomes -1 and the factors mean nothing.  Every
+// thread still goes through its columns with whatever it took for a payload, so
+// positions may be anything: they are used as addresses, and as pivots, only at
+// the end and only where they are rows of the panel (a test of the position in
+// every column costs another 1 % of a solve).
+// LOSE_PUSH (the timeout probe): from column kLoseFrom on nothing is pushed to
+// CTA 0, whose waits then run out.
+constexpr int kLoseFrom = 5;
+template <typename T, int W, int RPT, bool LOSE_PUSH = false>
 __device__ __forceinline__ void leaf_body(T* __restrict__ A, int64_t lda, int m, int w, int* __restrict__ piv,
                                           int piv_base, int* __restrict__ info, int col_base, long wait_limit,
                                           int* __restrict__ moved)
@@ -218,6 +226,7 @@ __device__ __forceinline__ void leaf_body(T* __restrict__ A, int64_t lda, int m,
     // At group g, x[k][c] is column (g GS + c) mod W; the last g GS are done.
     constexpr int GS = W < 8 ? W : 8;
     static_assert(GS % 4 == 0 && W % GS == 0, "column parity and barrier phase repeat with the group");
+    bool lost = false;   // one of my waits ran out: later ones are not waited for
 #pragma unroll 1
     for (int g0 = 0; g0 < W; g0 += GS) {
     const int live = W - g0;
@@ -263,6 +272,7 @@ __device__ __forceinline__ void leaf_body(T* __restrict__ A, int64_t lda, int m,
             const unsigned bar = smem_u32(&s_bar[par]), slot = smem_u32(&s_pay[par][crank]);
             for (int t = lane; C > 1 && t < C * kPieces; t += 32) {
                 const int q = t / kPieces, pc = t - q * kPieces;
+                if (LOSE_PUSH && j >= kLoseFrom && q == 0) continue;
                 const uint4 v = reinterpret_cast<const uint4*>(&s_mine)[pc];
                 st_async_v4(cluster_map(slot + 16 * pc, (unsigned)q), v.x, v.y, v.z, v.w, cluster_map(bar, (unsigned)q));
             }
@@ -275,13 +285,15 @@ __device__ __forceinline__ void leaf_body(T* __restrict__ A, int64_t lda, int m,
             const unsigned parity = (unsigned)((jj >> 1) & 1);
             long spins = 0;
             while (!mbar_try_wait(bar, parity))
-                if (++spins > (wait_limit >> 2)) {   // a try_wait round may suspend briefly
+                if (lost || ++spins > (wait_limit >> 2)) {   // a try_wait round may suspend briefly
                     s_fail = 1;
+                    lost = true;
                     break;
                 }
         }
         __syncwarp();
-        if (tid == 0 && C > 1 && j + 2 < w) mbar_arrive_expect(smem_u32(&s_bar[par]), col_bytes);
+        // (not while the phase is open: it takes one arrival)
+        if (tid == 0 && C > 1 && j + 2 < w && !lost) mbar_arrive_expect(smem_u32(&s_bar[par]), col_bytes);
         const Key g = lane < C ? s_pay[par][lane].key : Key{0u, 0u, 0xffffffffu, 0u};
         const Payload& best = s_pay[par][warp_key_lane(g)];
         const Key w_key = best.key;
@@ -325,33 +337,37 @@ __device__ __forceinline__ void leaf_body(T* __restrict__ A, int64_t lda, int m,
         for (int c = 0; c < GS; ++c) x[k][W - GS + c] = t[c];
     }
     }
-    cluster.sync();   // every push has landed and been read before any CTA exits
+    cluster.sync();   // every push has been sent, and has landed and been read but where a wait ran out
 #pragma unroll
     for (int k = 0; k < RPT; ++k)
-        if (pos[k] != INT_MAX)
+        if ((unsigned)pos[k] < (unsigned)m)
 #pragma unroll
             for (int c = 0; c < W; ++c)
                 if (c < w) A[(int64_t)pos[k] + (int64_t)c * lda] = x[k][c];
     __syncthreads();
-    if (crank == 0 && tid < w) piv[tid] = piv_base + s_hist[tid];
+    if (crank == 0 && tid < w) piv[tid] = piv_base + ((unsigned)s_hist[tid] < (unsigned)m ? s_hist[tid] : tid);
     if (moved) {
 #pragma unroll
         for (int k = 0; k < RPT; ++k) {
             const int row = crank * (kLeafThreads * RPT) + k * kLeafThreads + tid;
-            if (pos[k] != INT_MAX && pos[k] < w) moved[pos[k]] = row;
-            if (pos[k] != INT_MAX && row < w) moved[W + row] = pos[k];
+            if ((unsigned)pos[k] < (unsigned)w) moved[pos[k]] = row;
+            if ((unsigned)pos[k] < (unsigned)m && row < w) moved[W + row] = pos[k];
         }
     }
-    if (tid == 0 && s_fail) atomicMin(info, -1);
+    if (tid == 0 && s_fail) {
+        atomicMin(info, -1);
+        // pushes still under way to this CTA land before its shared memory goes
+        for (int i = 0; i < 32; ++i) __nanosleep(1000);
+    }
 }
 
-template <typename T, int W, int RPT>
+template <typename T, int W, int RPT, bool LOSE_PUSH = false>
 __global__ void __launch_bounds__(kLeafThreads, 1) leaf_lu_kernel(T* __restrict__ A, int64_t lda, int m, int w,
                                                                 int* __restrict__ piv, int piv_base,
                                                                 int* __restrict__ info, int col_base,
                                                                 long wait_limit, int* __restrict__ moved)
 {
-    leaf_body<T, W, RPT>(A, lda, m, w, piv, piv_base, info, col_base, wait_limit, moved);
+    leaf_body<T, W, RPT, LOSE_PUSH>(A, lda, m, w, piv, piv_base, info, col_base, wait_limit, moved);
 }
 
 // The leaves of many systems in one launch: cluster y of the grid factorises
@@ -373,6 +389,8 @@ __global__ void __launch_bounds__(kLeafThreads, 1) leaf_group_kernel(const __gri
 // cluster writes (one cluster barrier), solves for U on its own (32 steps) and
 // updates its rows, each thread RPT rows x CB columns in registers.  FP64-pipe
 // bound: 2 m CB w flops per cluster, 4.2 us for 512 rows x 32 x 32 on one SM.
+// After a leaf whose wait ran out entries of moved may be unset: one that is no
+// row of the panel is not followed.
 constexpr int kUpdThreads = 256;
 template <typename T, int W, int RPT, int CB>
 __global__ void __launch_bounds__(kUpdThreads, RPT == 1 ? 2 : 1) leaf_update_kernel(T* __restrict__ A, int64_t lda, int m, int w,
@@ -409,7 +427,7 @@ __global__ void __launch_bounds__(kUpdThreads, RPT == 1 ? 2 : 1) leaf_update_ker
     for (int t = tid; t < W * CB; t += kUpdThreads) {
         const int i = t % W, c = t / W;
         const bool in = i < w && c < nc;
-        s_u[i][c] = in ? Bc[moved[i] + (int64_t)c * lda] : (T)0;
+        s_u[i][c] = in ? Bc[min((unsigned)moved[i], (unsigned)m - 1u) + (int64_t)c * lda] : (T)0;
         s_old[i][c] = in ? Bc[i + (int64_t)c * lda] : (T)0;
     }
     for (int t = tid; t < R; t += kUpdThreads) s_from[t] = -1;
@@ -742,6 +760,7 @@ struct Lu {
     int cluster;  // largest leaf cluster (16 where the device co-schedules it, else 8)
     long wait_limit = kDefaultWaitLimit;   // try_wait rounds before a leaf gives up on a push
     int min_rpt = 1;        // fewest rows per leaf thread (wider leaves with fewer rows each)
+    bool lose_push = false; // leaves of the timeout probe
     int64_t launches = 0;   // own kernels launched
     cudaError_t err = cudaSuccess;
 
@@ -810,8 +829,10 @@ struct Lu {
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        err = cudaLaunchKernelEx(&cfg, leaf_lu_kernel<T, W, RPT>, A, lda, m, w, piv, piv_base, info, col_base,
-                                 wait_limit, moved);
+        auto kern = leaf_lu_kernel<T, W, RPT>;
+        if constexpr (sizeof(T) == 8 && W == 32)
+            if (lose_push) kern = leaf_lu_kernel<T, W, RPT, true>;
+        err = cudaLaunchKernelEx(&cfg, kern, A, lda, m, w, piv, piv_base, info, col_base, wait_limit, moved);
         ++launches;
     }
 
@@ -1281,6 +1302,44 @@ int lu_factor_solve(const LuStreams& s, T* A, int64_t n, int64_t lda, const T* B
     if (s.launches) *s.launches += lu.launches;
     if (lu.err != cudaSuccess) return LU_CUDA_ERROR;
     return LU_OK;
+}
+
+// ------------------------------------------------------------ timeout probe
+namespace {
+
+// A[i] in [-1, 1), some digits of i: no structure, no two magnitudes alike
+__global__ void probe_matrix_kernel(double* __restrict__ A, int64_t count)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
+        const unsigned long long z = ((unsigned long long)i + 1) * 0x9e3779b97f4a7c15ull;
+        A[i] = (double)(long long)(z ^ (z << 21)) * 0x1p-63;
+    }
+}
+
+}  // namespace
+
+int lu_leaf_timeout_probe(const LuStreams& s, double* A, int64_t n, double* x, int* ipiv, int* perm, int* info)
+{
+    Lu<double> lu;
+    lu.main_st = s.main;
+    lu.side_st = s.side ? s.side : s.main;
+    lu.aux_st = s.side && s.aux && s.naux > 0 ? s.aux[0] : nullptr;
+    lu.use(false);
+    lu.ipiv = ipiv;
+    lu.info = info;
+    lu.moved = info + 1;
+    lu.wait_limit = s.wait_limit > 0 ? s.wait_limit : kDefaultWaitLimit;
+    configure(lu);
+    lu.lose_push = true;
+    // several CTAs per leaf cluster, of a size every device schedules
+    if (n <= kLeafThreads || n > 8 * kLeafThreads) return LU_TOO_LARGE;
+    probe_matrix_kernel<<<296, 256, 0, s.main>>>(A, n * n);
+    // movement entries no leaf has written are no rows of any panel
+    if (cudaMemsetAsync(lu.moved, 0x7f, (kLuInfoInts - 1) * sizeof(int), s.main) != cudaSuccess) return LU_CUDA_ERROR;
+    ++lu.launches;
+    lu_body(lu, A, n, n, (const double*)A, n, 1, x, n, perm, 256, true, true);
+    if (s.launches) *s.launches += lu.launches;
+    return lu.ok() ? LU_OK : LU_CUDA_ERROR;
 }
 
 // ------------------------------------------------- grouped factorisation

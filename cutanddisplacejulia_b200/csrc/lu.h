@@ -73,6 +73,12 @@ cudaError_t lu_chain_timeout_probe(cudaStream_t st, const double* A, int64_t lda
                                    const double* b, double* y, double* x, int* sync, int* info, long wait_limit);
 size_t lu_chain_sync_ints(int64_t n);
 
+// Timeout probe of the leaves' pivot exchange (512 < n <= 4096): factorises an
+// n x n matrix made in A and solves with it, the leaves' pushes to their first
+// CTA lost from the sixth column on, so that each leaf of several CTAs gives up
+// and info ends as -1.  x: n doubles; ipiv, perm, info as lu_factor_solve.
+int lu_leaf_timeout_probe(const LuStreams& s, double* A, int64_t n, double* x, int* ipiv, int* perm, int* info);
+
 // One FP32 system of a grouped factorisation: A (n_pad x n_pad, lda), n_pad a
 // multiple of the block width (the caller pads a system with the identity),
 // tensor maps 2 map, 2 map + 1 of gemm_group_maps for A in the device array

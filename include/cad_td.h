@@ -187,6 +187,11 @@ int cad_set_wait_limit(cad_ctx* ctx, int64_t polls);
  * sets.  Returns CAD_ERR_TIMEOUT once the waits run out (the kernels end
  * normally; nothing faults or hangs). */
 int cad_wait_timeout_probe(cad_ctx* ctx, int64_t n);
+/* The same for the LU leaves' pivot exchange (512 < n <= 4096): factorises an
+ * n x n matrix of the library's own and solves with it, each leaf's pushes to
+ * its first thread block lost from the sixth column on, so that every leaf of
+ * several blocks gives up.  Returns CAD_ERR_TIMEOUT. */
+int cad_leaf_timeout_probe(cad_ctx* ctx, int64_t n);
 /* Measured FP64 fused-multiply-add throughput of the device (TFLOP/s, 2 flops
  * per FMA), the denominator of the TD kernels' roofline.  No counterpart in
  * the reference (a measurement utility). */
