@@ -84,6 +84,14 @@ struct BatchGraph {
     double params[5] = {};
     long flags[4] = {};
     int64_t launches = 0;
+
+    // the next batch is a plan seen for the first time
+    void drop()
+    {
+        if (exec) cudaGraphExecDestroy(exec);
+        exec = nullptr;
+        offsets.clear();
+    }
 };
 
 }  // namespace
@@ -120,6 +128,7 @@ struct cad_ctx {
     cudaEvent_t side_fork = nullptr, side_join = nullptr;   // work forked onto the side stream
     Tuner tuner;                           // cad_set_autotune
     int shared_edges = 1;                  // cad_set_shared_edges
+    int64_t fail_alloc = 0;                // cad_fail_allocation: allocations until the one that fails (0: none)
     double tol = 1e-10;
     int max_iter = 200;
     bool fric_ready = false;      // cad_friction_prepare: C = inv(A Scl) of fric_N elements in S_LCPC
@@ -176,6 +185,16 @@ int cuda_fail(cad_ctx* c, cudaError_t e, const char* what)
         if (e_ != cudaSuccess) return cuda_fail(ctx, e_, #expr);        \
     } while (0)
 
+// cudaMalloc, or the failure that cad_fail_allocation asked for; a failed one
+// leaves no error behind for the next launch to find
+cudaError_t device_alloc(cad_ctx* ctx, void** p, size_t bytes)
+{
+    const bool fail_now = ctx->fail_alloc > 0 && --ctx->fail_alloc == 0;
+    const cudaError_t e = fail_now ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+
 int ensure(cad_ctx* ctx, Slot s, size_t bytes, void** out)
 {
     DevBuf& b = ctx->buf[s];
@@ -188,7 +207,7 @@ int ensure(cad_ctx* ctx, Slot s, size_t bytes, void** out)
             b.bytes = 0;
         }
         const size_t grown = bytes + bytes / 8;
-        CK(cudaMalloc(&b.p, grown));
+        CK(device_alloc(ctx, &b.p, grown));
         b.bytes = grown;
     }
     *out = b.p;
@@ -827,19 +846,23 @@ bool bad_flag(int f) { return f != 0 && f != 1; }
 
 
 // ------------------------------------------------------------- batched solve
+// The captured plan holds the lanes' addresses, which its key does not name: a
+// buffer that moves takes the plan with it, whatever becomes of the call.
 int lane_ensure(cad_ctx* ctx, Lane& l, LaneSlot slot, size_t bytes, void** out)
 {
     DevBuf& b = l.buf[slot];
     if (bytes == 0) bytes = 16;
     if (b.bytes < bytes) {
         if (b.p) {
+            CK(cudaStreamSynchronize(ctx->stream));
             CK(cudaStreamSynchronize(l.main));
             CK(cudaStreamSynchronize(l.side));
+            ctx->batch.drop();
             CK(cudaFree(b.p));
             b.p = nullptr;
             b.bytes = 0;
         }
-        CK(cudaMalloc(&b.p, bytes));
+        CK(device_alloc(ctx, &b.p, bytes));
         b.bytes = bytes;
     }
     *out = b.p;
@@ -1104,8 +1127,7 @@ int slip_batched_ws(cad_ctx* ctx, int64_t nbatch, const int64_t* offsets, const 
     CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
     int rc = CAD_OK;
     if (!same) {
-        if (g.exec) cudaGraphExecDestroy(g.exec);
-        g.exec = nullptr;
+        g.drop();
         g.offsets.assign(offsets, offsets + nbatch + 1);
         std::copy(ptrs, ptrs + 8, g.ptrs);
         std::copy(params, params + 5, g.params);
@@ -1137,10 +1159,7 @@ int slip_batched_ws(cad_ctx* ctx, int64_t nbatch, const int64_t* offsets, const 
             e = cudaGraphLaunch(g.exec, ctx->stream);
             if (e != cudaSuccess) rc = cuda_fail(ctx, e, "batched solve: graph launch");
         }
-        if (rc != CAD_OK && g.exec) {
-            cudaGraphExecDestroy(g.exec);
-            g.exec = nullptr;
-        }
+        if (rc != CAD_OK) g.drop();
     }
     cudaEventDestroy(fork);
     if (rc != CAD_OK) return rc;
@@ -1394,6 +1413,14 @@ int cad_set_wait_limit(cad_ctx* ctx, int64_t polls)
     if (!ctx) return CAD_ERR_ARG;
     if (polls < 1) return fail(ctx, CAD_ERR_ARG, "invalid argument");
     ctx->wait_limit = (long)polls;
+    return CAD_OK;
+}
+
+int cad_fail_allocation(cad_ctx* ctx, int64_t nth)
+{
+    if (!ctx) return CAD_ERR_ARG;
+    if (nth < 0) return fail(ctx, CAD_ERR_ARG, "invalid argument");
+    ctx->fail_alloc = nth;
     return CAD_OK;
 }
 

@@ -181,6 +181,11 @@ int cad_set_batch_solve(cad_ctx* ctx, int mode);
  * CAD_ERR_TIMEOUT and the context stays usable.  No counterpart in the
  * reference (its waits are CPU thread joins). */
 int cad_set_wait_limit(cad_ctx* ctx, int64_t polls);
+/* Failure injection on the host: the nth allocation of a device workspace from
+ * here on fails as if memory had run out (0: none).  The call that needs it
+ * returns CAD_ERR_OOM or takes a path that needs less; the context stays
+ * usable.  No counterpart in the reference. */
+int cad_fail_allocation(cad_ctx* ctx, int64_t nth);
 /* Exercises that timeout path on an n x n zero system (128 <= n <= 8192): the
  * lower chain of the one-right-hand-side solve is launched with its order
  * counter started past block 0, so every block waits for a flag that no block

@@ -25,3 +25,17 @@ def cad():
     from cutanddisplacejulia_b200 import build
     build.build()
     return cad
+
+
+@pytest.fixture
+def fresh_context(cad, monkeypatch):
+    """A context of the test's own in the process-wide one's place (no
+    workspace grown by earlier tests)."""
+    import ctypes
+
+    from cutanddisplacejulia_b200 import _lib
+    L, h = _lib.load(), ctypes.c_void_p()
+    _lib.check(L.cad_init(0, ctypes.byref(h)), None)
+    monkeypatch.setitem(_lib._ctx, 0, h)
+    yield h
+    L.cad_destroy(h)

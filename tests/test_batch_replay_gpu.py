@@ -1,6 +1,7 @@
-"""GPU test of the batched solve's plan: the first call of a plan is issued
+"""GPU tests of the batched solve's plan: the first call of a plan is issued
 directly, the second captured and later ones replayed, whatever the arrays;
-each call's slip is that of its own inputs, bit for bit."""
+each call's slip is that of its own inputs, bit for bit, also after a larger
+batch moved the lanes' buffers and then ran out of memory."""
 import numpy as np
 import pytest
 
@@ -29,3 +30,38 @@ def test_replays_serve_other_arrays(cad, mode, hs):
     assert not np.array_equal(alone[0][0], alone[1][0])
     for k in (2, 0, 1, 2, 1):        # captured, then replayed
         assert all(np.array_equal(a, b) for a, b in zip(solve(6, *states[k]), alone[k])), k
+
+
+@pytest.mark.parametrize("mode", ["grouped", "lanes_chain"])
+def test_plan_after_a_larger_batch_that_ran_out_of_memory(cad, fresh_context, mode):
+    from cutanddisplacejulia_b200 import _lib, workloads
+    L, ctx = _lib.load(), fresh_context
+    _, _, lam, nu, G = cad.ElasticConstantsCheck(1.0, 0.25)
+
+    def solve(n):
+        cracks, stresses = workloads.crack_batch(seed=5, count=5, n_range=(n, n + 40))
+        bcs = [cad.Stresses(*v) for v in stresses]
+        out, rel = cad.SlipCalculator3D_batched(cracks, nu, G, lam, 0, bcs, tol=1e-10, mode=mode)
+        assert np.all(rel <= 1e-10)
+        return [np.concatenate(r) for r in out]
+
+    want = solve(30)
+    failed = 0
+    try:
+        for nth in range(1, 200):
+            solve(30)
+            solve(30)                        # captured, or replayed
+            _lib.check(L.cad_fail_allocation(ctx, nth), ctx)
+            try:
+                solve(100 + 4 * nth)         # each larger than the one before
+            except cad.CadError as e:
+                assert e.code == _lib.CAD_ERR_OOM
+                failed += 1
+            else:
+                break                        # fewer allocations than nth
+            finally:
+                _lib.check(L.cad_fail_allocation(ctx, 0), ctx)
+            assert all(np.array_equal(a, b) for a, b in zip(solve(30), want)), nth
+    finally:
+        L.cad_fail_allocation(ctx, 0)
+    assert failed > 5
