@@ -1240,7 +1240,9 @@ int slip_batched(cad_ctx* ctx, int64_t nbatch, const int64_t* offsets, const dou
     double* Dw = w + 6 * words;
     const int rc = slip_batched_ws(ctx, nbatch, offsets, w, w + words, w + 2 * words, w + 3 * words, w + 4 * words, nu,
                                    G, lambda, hs, w + 5 * words, Dw, rel_host);
-    if (rc == CAD_ERR_CUDA) return rc;
+    // D is left alone by a call that solved nothing (of a singular crack's batch
+    // the others' slips are handed out)
+    if (rc != CAD_OK && rc != CAD_ERR_NOT_CONVERGED && rc != CAD_ERR_SINGULAR) return rc;
     if (words) CK(cudaMemcpyAsync(D, Dw, words * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return rc;

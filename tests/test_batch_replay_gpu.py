@@ -65,3 +65,37 @@ def test_plan_after_a_larger_batch_that_ran_out_of_memory(cad, fresh_context, mo
     finally:
         L.cad_fail_allocation(ctx, 0)
     assert failed > 5
+
+
+def test_failed_call_leaves_the_slips_alone(cad, fresh_context):
+    import torch
+
+    from cutanddisplacejulia_b200 import _lib, workloads
+    L, ctx = _lib.load(), fresh_context
+    _lib.check(L.cad_set_solver(ctx, _lib.CAD_SOLVER_MIXED, 1e-10, 400), ctx)
+
+    def call(count, n):
+        cracks, _ = workloads.crack_batch(seed=6, count=count, n_range=(n, n + 10))
+        offs = np.concatenate([[0], np.cumsum([len(P[0]) for P in cracks])]).astype(np.int64)
+        args = []
+        for k in range(5):
+            parts = []
+            for P in cracks:
+                nrm, mid = cad.CreateFaceNormalAndMidPoint(*P)
+                parts.append(np.asfortranarray((*P, nrm, mid)[k]).ravel(order="F"))
+            args.append(torch.tensor(np.concatenate(parts), device="cuda"))
+        T = torch.ones(3 * int(offs[-1]), dtype=torch.float64, device="cuda")
+        D = torch.full_like(T, -7.0)
+        torch.cuda.synchronize()
+        rc = L.cad_slip_calculator_batched_dev(ctx, count, offs.ctypes.data, *[a.data_ptr() for a in args], 0.25, 1.0,
+                                               1.0, 0, T.data_ptr(), D.data_ptr(), None)
+        torch.cuda.synchronize()
+        return rc, D
+
+    rc, D = call(4, 30)
+    assert rc == _lib.CAD_OK and not bool((D == -7.0).any())
+    for nth in range(2, 8):          # the first is the copies' own
+        _lib.check(L.cad_fail_allocation(ctx, nth), ctx)
+        rc, D = call(4, 40 + 20 * nth)
+        _lib.check(L.cad_fail_allocation(ctx, 0), ctx)
+        assert rc == _lib.CAD_ERR_OOM and bool((D == -7.0).all()), nth
