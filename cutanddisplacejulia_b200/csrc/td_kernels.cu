@@ -787,9 +787,9 @@ cudaError_t launch_assemble_edges(PairArgs a, int out_kind, bool strain, bool di
 }
 
 // Net Burgers vector of a mesh edge: the signed sum over the triangle sides on
-// it (list[0 .. n) = +-(triangle + 1), sorted here into triangle order, then
-// side order, so the sum does not depend on how the list was filled) of
-// Dn Vn + Dss Vs + Dds Vd.
+// it (list[0 .. n) = +-(triangle + 1), in no fixed order) of Dn Vn + Dss Vs +
+// Dds Vd, the same bits whatever the order.
+// A few sides are sorted into triangle order, then side order, by one thread.
 __device__ __forceinline__ void net_burgers(int* __restrict__ list, int n, const TriDev* __restrict__ tri, double B[3])
 {
     for (int i = 1; i < n; ++i) {
@@ -812,30 +812,129 @@ __device__ __forceinline__ void net_burgers(int* __restrict__ list, int n, const
     }
 }
 
+// Many sides (one patch listed with many slips) are summed by the block without
+// sorting: each term is cut into multiples of three units, the first such that
+// n terms add up exactly in double, each next finer by the bits that are left, so
+// that no order of the additions shows (the reproducible sums of Demmel and
+// Nguyen, 2013).  What is cut off is below n^4 2^-154 of the largest term.
+constexpr int kBurgersThreads = 256, kBurgersWarps = kBurgersThreads / 32;
+__device__ __forceinline__ void side_term(int c, const TriDev* __restrict__ tri, double v[3])
+{
+    const TriDev& t = tri[(c > 0 ? c : -c) - 1];
+    const double sg = c > 0 ? 1.0 : -1.0;
+    const double a = sg * t.Dn, b = sg * t.Dss, d = sg * t.Dds;
+    const bool none = a == 0.0 && b == 0.0 && d == 0.0;   // (its axes may be none)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const double x = dot3_rn(t.real.Vn[i], t.real.Vs[i], t.real.Vd[i], a, b, d);
+        v[i] = none ? 0.0 : x;
+    }
+}
+// (every thread of the block; s_red: 9 kBurgersWarps doubles; B in every thread)
+__device__ __noinline__ void net_burgers_block(const int* __restrict__ list, int n, const TriDev* __restrict__ tri,
+                                               double* s_red, double B[3])
+{
+    constexpr unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double big[3] = {0.0, 0.0, 0.0}, v[3];
+    for (int k = threadIdx.x; k < n; k += kBurgersThreads) {
+        side_term(list[k], tri, v);
+        for (int i = 0; i < 3; ++i) big[i] = fmax(big[i], fabs(v[i]));
+    }
+    __syncthreads();   // s_red is free
+    for (int i = 0; i < 3; ++i) {
+        for (int d = 16; d; d >>= 1) big[i] = fmax(big[i], __shfl_xor_sync(full, big[i], d));
+        if (lane == 0) s_red[3 * warp + i] = big[i];
+    }
+    __syncthreads();
+    for (int w = 0; w < kBurgersWarps; ++w)
+        for (int i = 0; i < 3; ++i) big[i] = fmax(big[i], s_red[3 * w + i]);
+    const int bits = 33 - __clz(n);   // n < 2^(bits - 1)
+    // at[i][q]: a term plus this, less this, is the term in units of its last place
+    double at[3][3], sum[3][3] = {};
+    for (int i = 0; i < 3; ++i)
+        for (int q = 0; q < 3; ++q)
+            at[i][q] = big[i] > 0.0 ? scalbn(1.5, ilogb(big[i]) + 1 + bits + q * (bits - 53)) : 0.0;
+    for (int k = threadIdx.x; k < n; k += kBurgersThreads) {
+        side_term(list[k], tri, v);
+        for (int i = 0; i < 3; ++i)
+            for (int q = 0; q < 3; ++q) {
+                const double u = sub_rn(add_rn(v[i], at[i][q]), at[i][q]);
+                sum[i][q] = add_rn(sum[i][q], u);
+                v[i] = sub_rn(v[i], u);
+            }
+    }
+    __syncthreads();
+    for (int i = 0; i < 3; ++i)
+        for (int q = 0; q < 3; ++q) {
+            for (int d = 16; d; d >>= 1) sum[i][q] = add_rn(sum[i][q], __shfl_xor_sync(full, sum[i][q], d));
+            if (lane == 0) s_red[9 * warp + 3 * i + q] = sum[i][q];
+        }
+    __syncthreads();
+    for (int i = 0; i < 3; ++i) {
+        double t[3] = {0.0, 0.0, 0.0};
+        for (int w = 0; w < kBurgersWarps; ++w)
+            for (int q = 0; q < 3; ++q) t[q] = add_rn(t[q], s_red[9 * w + 3 * i + q]);
+        B[i] = add_rn(t[0], add_rn(t[1], t[2]));
+    }
+}
+
+// The net Burgers vector of edge e = 32 blockIdx.x + lane to each lane of warp 0
+// (none where e >= E); the other warps help with long lists only.  A list goes to
+// the block where one thread's sort of it would take more than some microseconds:
+// sorted by one thread, the five edges of two neighbours listed 100 000 times would
+// take 2.5e9 dependent moves in memory each; at 300 points the whole call takes 3.7 ms.
+constexpr int kSortedSides = 32;
+__device__ __forceinline__ void edge_burgers(int64_t e, int64_t E, const int* __restrict__ ptr,
+                                             const int* __restrict__ cnt, int* __restrict__ sides,
+                                             const TriDev* __restrict__ tri, double B[3])
+{
+    __shared__ int s_first[32], s_n[32];
+    __shared__ double s_red[9 * kBurgersWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    B[0] = B[1] = B[2] = 0.0;
+    int n = 0;
+    if (warp == 0) {
+        const int first = e < E ? ptr[e] : 0;
+        n = e < E ? cnt[e] : 0;
+        s_first[lane] = first;
+        s_n[lane] = n;
+        if (n <= kSortedSides) net_burgers(sides + first, n, tri, B);
+    }
+    if (!__syncthreads_or(n > kSortedSides)) return;
+    for (int q = 0; q < 32; ++q) {
+        if (s_n[q] <= kSortedSides) continue;
+        double S[3];
+        net_burgers_block(sides + s_first[q], s_n[q], tri, s_red, S);
+        if (threadIdx.x == q)
+            for (int i = 0; i < 3; ++i) B[i] = S[i];
+    }
+}
+
 // Each half-space edge's record for its net Burgers vector.
-__global__ void edge_burgers_kernel(const double* __restrict__ pts, int64_t E, const int* __restrict__ ptr,
+__global__ void __launch_bounds__(kBurgersThreads) edge_burgers_kernel(const double* __restrict__ pts, int64_t E, const int* __restrict__ ptr,
                                     const int* __restrict__ cnt, int* __restrict__ sides,
                                     const TriDev* __restrict__ tri, double nu, FscSide* __restrict__ out)
 {
-    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= E) return;
+    const int64_t e = blockIdx.x * (int64_t)32 + (threadIdx.x & 31);
     double B[3];
-    net_burgers(sides + ptr[e], cnt[e], tri, B);
+    edge_burgers(e, E, ptr, cnt, sides, tri, B);
+    if (e >= E || threadIdx.x >= 32) return;
     const double PA[3] = {pts[6 * e], pts[6 * e + 1], pts[6 * e + 2]};
     const double PB[3] = {pts[6 * e + 3], pts[6 * e + 4], pts[6 * e + 5]};
     build_side_burgers(PA, PB, B, nu, out[e]);
 }
 
 // Each full-space edge's; the number of edges is read on the device (count).
-__global__ void segment_burgers_kernel(const double* __restrict__ pts, const int* __restrict__ count,
+__global__ void __launch_bounds__(kBurgersThreads) segment_burgers_kernel(const double* __restrict__ pts, const int* __restrict__ count,
                                        const int* __restrict__ ptr, const int* __restrict__ cnt,
                                        int* __restrict__ sides, const TriDev* __restrict__ tri, double K8,
                                        SegRec* __restrict__ out)
 {
-    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= *count) return;
+    const int64_t e = blockIdx.x * (int64_t)32 + (threadIdx.x & 31), E = *count;
     double B[3];
-    net_burgers(sides + ptr[e], cnt[e], tri, B);
+    edge_burgers(e, E, ptr, cnt, sides, tri, B);
+    if (e >= E || threadIdx.x >= 32) return;
     const double PA[3] = {pts[6 * e], pts[6 * e + 1], pts[6 * e + 2]};
     const double PB[3] = {pts[6 * e + 3], pts[6 * e + 4], pts[6 * e + 5]};
     build_segment(PA, PB, B, K8, out[e]);
@@ -966,7 +1065,7 @@ cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, bool full, c
     else
         e = pairs(td_pair_kernel<true, false, true, OUT_SUM, false, false, 1, EDGE_FSC>);
     if (e != cudaSuccess || E == 0) return e;
-    edge_burgers_kernel<<<(unsigned)((E + 31) / 32), 32, 0, st>>>(ed.pts, E, ed.ptr, ed.cnt, ed.sides, a.tri, nu,
+    edge_burgers_kernel<<<(unsigned)((E + 31) / 32), kBurgersThreads, 0, st>>>(ed.pts, E, ed.ptr, ed.cnt, ed.sides, a.tri, nu,
                                                                    (FscSide*)edge_rec);
     if (launches) ++*launches;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -983,7 +1082,7 @@ cudaError_t launch_td_sum_segments(PairArgs a, bool strain, bool disp, const Edg
     const unsigned tiles = (unsigned)((a.M + kPairThreads - 1) / kPairThreads);
     SegRec* rec = (SegRec*)seg_rec;
     const double K8 = 0.5 * kInv4Pi / (1.0 - nu);
-    segment_burgers_kernel<<<(unsigned)((3 * a.N + 31) / 32), 32, 0, st>>>(ed.pts, ed.count, ed.ptr, ed.cnt, ed.sides,
+    segment_burgers_kernel<<<(unsigned)((3 * a.N + 31) / 32), kBurgersThreads, 0, st>>>(ed.pts, ed.count, ed.ptr, ed.cnt, ed.sides,
                                                                            a.tri, K8, rec);
     auto pairs = [&](auto kern) -> cudaError_t {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem);

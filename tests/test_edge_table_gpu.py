@@ -111,3 +111,38 @@ def test_fields_sums_and_tractions_over_meshes(cad, oracle, name):
     So, Uo = oracle.td_inf(*pts[9:].T, *P, *sl, nu, G, 1, 1, 1)
     assert_parity(got[1][0][:, 9:], So)
     assert_parity(got[1][1][:, 9:], Uo)
+
+
+@pytest.mark.parametrize("hs", [0, 1])
+@pytest.mark.parametrize("k", [31, 32, 33, 100, 3001, 100000])
+def test_one_patch_listed_with_many_slips(cad, oracle, hs, k):
+    """k copies of two neighbours, some with their vertices turned round: their
+    five edges carry up to 2 k sides, and the field is that of the two with the
+    net slips.  The lists are filled in no fixed order; the sums do not show it."""
+    rng = np.random.default_rng(k)
+    v = np.array([[0.0, 0.0, -0.5], [1.0, 0.1, -0.6], [0.2, 0.9, -1.1], [1.1, 1.2, -1.4]])
+    tri = np.array([[0, 1, 2], [1, 3, 2]])
+    which = rng.integers(0, 2, k)
+    turn = rng.integers(0, 3, k)
+    idx = tri[which][np.arange(k)[:, None], (np.arange(3) + turn[:, None]) % 3]
+    P = [v[idx[:, c]] for c in range(3)]
+    sl = rng.uniform(-1e-3, 1e-3, (3, k)) * 10.0 ** rng.uniform(-3, 0, k)
+    sl[:, ::7] = 0.0
+    M = max(300, (5 << 20) // k + 1) if hs == 0 else 300       # full space: over edges from 5 * 2^20 pairs on
+    pts = rng.uniform([-2, -2, -3], [3, 3, -0.01], (M, 3))
+    import math
+    net = np.array([[math.fsum(sl[m][which == t]) for t in range(2)] for m in range(3)])
+
+    def run():
+        S, U = cad.TD(*pts.T, *P, *sl, 0.25, 1.0, 1, 1, hs, cad.Strains(), cad.Disps())
+        return np.stack(list(S)), np.stack(list(U))
+
+    a = run()
+    b = run()
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+    n = 300
+    So, Uo = oracle.td_sum_eval(*pts[:n].T, *[v[tri[:, c]] for c in range(3)], *net, 0.25, 1.0, 1, 1, hs)
+    # a sum of k terms in another order: k eps of the largest patch's field at most, scaled by the slips
+    lost = k * 2.3e-16 * np.abs(sl).sum(1).max() / np.abs(net).max()
+    assert rel_inf_err(a[0][:, :n], So) < 1e-12 + lost
+    assert rel_inf_err(a[1][:, :n], Uo) < 1e-12 + lost
