@@ -282,8 +282,7 @@ int hs_check(cad_ctx* ctx, const double* Z, int64_t M, const double* P1, const d
     ++ctx->launches;
     CK(cudaMemsetAsync(flag, 0, 3 * sizeof(int), ctx->stream));
     CK(launch_hs_check(Z, M, P1, P2, P3, N, (int*)flag, ctx->stream, nullptr, false, et ? (int*)flag + 2 : nullptr));
-    // side codes are ints: larger meshes stay on the per-side path
-    const bool edges = et && ctx->shared_edges && N > 0 && 3 * N <= INT32_MAX;
+    const bool edges = et && ctx->shared_edges && N > 0 && edge_table_fits(N);
     if (edges)
         if (int r = edge_table(ctx, P1, P2, P3, N, lists, (int*)flag + 1, &et->a)) return r;
     int h[3] = {0, 0, 0};
@@ -359,7 +358,7 @@ int td_device(cad_ctx* ctx, const double* X, const double* Y, const double* Z, i
         CK(launch_sum_chunks(a.partial, nchunk + nechunk, M, mask, sum_out, ctx->stream));
         return CAD_OK;
     }
-    if (out_kind == OUT_SUM && hs == 0 && edge_kind && ctx->shared_edges && 3 * N <= INT32_MAX &&
+    if (out_kind == OUT_SUM && hs == 0 && edge_kind && ctx->shared_edges && edge_table_fits(N) &&
         segments_pay(M, N, strain == 1)) {
         // nothing is read back (E stays on the device), so the call stays
         // asynchronous; a mesh without shared edges costs the same as its pairs

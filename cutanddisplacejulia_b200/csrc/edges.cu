@@ -210,14 +210,16 @@ __global__ void __launch_bounds__(kThreads) edge_sides_kernel(const int* __restr
     sides[ptr[e] + atomicAdd(fill + e, 1)] = c > 0 ? t : -t;
 }
 
-unsigned table_slots(int64_t N)
+int64_t table_slots(int64_t N)
 {
-    unsigned t = 64;
-    while ((int64_t)t < 6 * N) t *= 2;
+    int64_t t = 64;
+    while (t < 6 * N) t *= 2;
     return t;
 }
 
 }  // namespace
+
+bool edge_table_fits(int64_t N) { return 6 * N <= int64_t(1) << 31; }
 
 size_t edge_work_ints(int64_t N)
 {
@@ -228,10 +230,11 @@ cudaError_t launch_edge_table(const double* P1, const double* P2, const double* 
                               bool lists, cudaStream_t st, int64_t* launches)
 {
     if (N <= 0) return cudaMemsetAsync(a.count, 0, sizeof(int), st);
-    const unsigned slots = table_slots(N);
+    if (!edge_table_fits(N)) return cudaErrorInvalidValue;
+    const unsigned slots = (unsigned)table_slots(N);
     const unsigned nb = (unsigned)((3 * N + kThreads - 1) / kThreads);
     int* table = a.work;
-    int* rep = table + slots;
+    int* rep = table + (size_t)slots;
     int* number = rep + 3 * N;
     int* fill = number + 3 * N;
     int* block_first = fill + 3 * N;

@@ -21,9 +21,12 @@ struct EdgeArrays {
 };
 
 size_t edge_work_ints(int64_t N);
+// Whether the table of N triangles can be built: its slots (a power of two, at
+// least two per side) are counted in 32 bits.  Larger lists stay per side.
+bool edge_table_fits(int64_t N);
 
 // Fills pts, code and count[0] (and ptr, cnt, sides with lists = true) from
-// the vertex lists (N x 3 column-major).  3 N must fit an int.
+// the vertex lists (N x 3 column-major); edge_table_fits(N).
 cudaError_t launch_edge_table(const double* P1, const double* P2, const double* P3, int64_t N, const EdgeArrays& a,
                               bool lists, cudaStream_t st, int64_t* launches);
 
