@@ -85,7 +85,7 @@ struct FrameT {          // a TD (real or image) in its own coordinate system
 
 template <typename T>
 struct FscSideT {        // one TD side PA -> PB of the free-surface correction
-    T skip;              // 1: the side adds nothing (beta test)
+    T skip;              // 1: the side has no correction (beta test); 2: it carries no slip (build_side_burgers)
     T ea, eb;            // horizontal direction of the side: ADCS y1 = ea X + eb Y, y2 = eb X - ea Y, y3 = -Z
     T PA[3];
     T PAlo[3];           // as P2lo
@@ -1274,11 +1274,13 @@ CAD_HD void build_side(const double PA[3], const double PB[3], const Frame& real
 
 // Side PA -> PB carrying the net Burgers vector B (EFCS) of every triangle side
 // on that mesh edge, as unit mode 0 (evaluate with Dn = 1, Dss = Dds = 0).  The
-// slip coefficients follow build_side's for w = B.
+// slip coefficients follow build_side's for w = B.  skip is 2 where B is zero:
+// the side adds nothing whatever its geometry (it may have no length).
 CAD_HD void build_side_burgers(const double PA[3], const double PB[3], const double B[3], double nu, FscSide& s)
 {
     build_side_geom(PA, PB, nu, s);
     side_slip(s, B, s.cs[0]);
+    if (B[0] == 0.0 && B[1] == 0.0 && B[2] == 0.0) s.skip = 2.0;
 }
 
 // ------------------------------------------- full-space sums over mesh edges

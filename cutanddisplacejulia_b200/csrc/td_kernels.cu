@@ -1015,7 +1015,7 @@ side_sum_kernel(const FscSide* __restrict__ edges, int64_t E, int64_t echunk, co
         for (int k = 0; k < ne; ++k) {
             const FscSide& s = reinterpret_cast<const FscSide*>(smem)[k];
             if constexpr (STRAIN == EDGE_FULL) {
-                side_sum_full<DISP>(s, x, y, z, Es[0], Us[0]);
+                if (s.skip != 2.0) side_sum_full<DISP>(s, x, y, z, Es[0], Us[0]);
                 continue;
             }
             if (s.skip != 0.0) continue;

@@ -146,3 +146,33 @@ def test_one_patch_listed_with_many_slips(cad, oracle, hs, k):
     lost = k * 2.3e-16 * np.abs(sl).sum(1).max() / np.abs(net).max()
     assert rel_inf_err(a[0][:, :n], So) < 1e-12 + lost
     assert rel_inf_err(a[1][:, :n], Uo) < 1e-12 + lost
+
+
+@pytest.mark.parametrize("strain,disp", [(1, 0), (0, 1), (1, 1)])
+def test_degenerate_triangles_without_slip(cad, strain, disp):
+    """Point-like and collinear triangles that carry no slip, repeats and a
+    reversed triangle in a half-space mesh: they add nothing, per edge as per side."""
+    from cutanddisplacejulia_b200 import _lib
+    rng = np.random.default_rng(2)
+    P = [np.concatenate([p, p[:5]]) for p in _strip(60)]       # repeats
+    P[0][7], P[1][7] = P[1][7].copy(), P[0][7].copy()          # reversed
+    P[1][20] = P[0][20]                                        # a side of no length
+    P[1][31] = P[2][31] = P[0][31]                             # a point
+    P[2][44] = 0.5 * (P[0][44] + P[1][44])                     # collinear
+    n = len(P[0])
+    sl = rng.uniform(-1e-3, 1e-3, (3, n))
+    sl[:, [20, 31, 44]] = 0.0
+    sl[:, 50:53] = 0.0                                         # neighbours: an edge without slip
+    pts = rng.uniform([-1, -1, -2], [8, 1, -0.05], (90, 3))
+    L, ctx = _lib.load(), _lib.context(0)
+    got = []
+    for shared in (1, 0):
+        _lib.check(L.cad_set_shared_edges(ctx, shared), ctx)
+        try:
+            S, U = cad.TD(*pts.T, *P, *sl, 0.25, 1.0, disp, strain, 1, cad.Strains(), cad.Disps())
+        finally:
+            _lib.check(L.cad_set_shared_edges(ctx, 1), ctx)
+        got.append([np.stack(list(f)) for f, on in ((S, strain), (U, disp)) if on])
+    for a, b in zip(*got):
+        assert np.isfinite(b).all() and np.isfinite(a).all()
+        assert_parity(a, b)
