@@ -195,6 +195,18 @@ cudaError_t device_alloc(cad_ctx* ctx, void** p, size_t bytes)
     return e;
 }
 
+// The staging buffers of small host calls (kStageWords doubles in, as many out)
+// are there, or could be made.
+bool staging_ready(cad_ctx* ctx)
+{
+    if (ctx->pinned) return true;
+    const bool fail_now = ctx->fail_alloc > 0 && --ctx->fail_alloc == 0;
+    if (!fail_now && cudaMallocHost((void**)&ctx->pinned, 2 * kStageWords * sizeof(double)) == cudaSuccess) return true;
+    cudaGetLastError();
+    ctx->pinned = nullptr;
+    return false;
+}
+
 int ensure(cad_ctx* ctx, Slot s, size_t bytes, void** out)
 {
     DevBuf& b = ctx->buf[s];
@@ -1526,10 +1538,10 @@ static int td_host(cad_ctx* ctx, bool sum_mode, const double* X, const double* Y
     double* g = o + 3 * M;
     double* s = g + 9 * N;
     // small calls: one copy in and one out through pinned memory (nine pageable
-    // copies each way took two thirds of a 16 x 16 call's 165 us)
-    const bool stage_in = in_words <= kStageWords, stage_out = out_words <= kStageWords;
-    if ((stage_in || stage_out) && !ctx->pinned)
-        CK(cudaMallocHost((void**)&ctx->pinned, 2 * kStageWords * sizeof(double)));
+    // copies each way took two thirds of a 16 x 16 call's 165 us); without pinned
+    // memory the copies go as large calls' do
+    const bool small = in_words <= kStageWords || out_words <= kStageWords, staged = small && staging_ready(ctx);
+    const bool stage_in = staged && in_words <= kStageWords, stage_out = staged && out_words <= kStageWords;
     const struct {
         const double* src;
         int64_t n;

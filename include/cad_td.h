@@ -181,8 +181,8 @@ int cad_set_batch_solve(cad_ctx* ctx, int mode);
  * CAD_ERR_TIMEOUT and the context stays usable.  No counterpart in the
  * reference (its waits are CPU thread joins). */
 int cad_set_wait_limit(cad_ctx* ctx, int64_t polls);
-/* Failure injection on the host: the nth allocation of a device workspace from
- * here on fails as if memory had run out (0: none).  The call that needs it
+/* Failure injection on the host: the nth allocation of a device workspace (or of
+ * the pinned staging buffers) from here on fails as if memory had run out (0: none).  The call that needs it
  * returns CAD_ERR_OOM or takes a path that needs less; the context stays
  * usable.  No counterpart in the reference. */
 int cad_fail_allocation(cad_ctx* ctx, int64_t nth);

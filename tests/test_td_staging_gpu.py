@@ -1,6 +1,9 @@
 """GPU tests of the small host calls that move their inputs and their outputs
 in one staged copy each (up to 32,768 doubles): the sizes on both sides of
-each limit against one large, unstaged call."""
+each limit against one large, unstaged call; without pinned memory the same
+results."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -46,3 +49,19 @@ def test_sums_around_the_limits(cad, data, M):
     for part in (run(M), run(M, disp=0) + run(M, strain=0)):
         assert_parity(np.stack(part[:6]), np.stack(whole[:6]))
         assert_parity(np.stack(part[6:]), np.stack(whole[6:]))
+
+
+def test_without_pinned_memory(cad, data, fresh_context):
+    from cutanddisplacejulia_b200 import _lib
+    L = _lib.load()
+    want = _inf(cad, data, OUT)                # with it, in the test's own context
+    other = ctypes.c_void_p()
+    _lib.check(L.cad_init(0, ctypes.byref(other)), None)
+    _lib._ctx[0] = other
+    try:
+        _lib.check(L.cad_fail_allocation(other, 3), other)   # after the inputs' and the outputs' workspaces
+        got = _inf(cad, data, OUT)
+    finally:
+        _lib._ctx[0] = fresh_context
+        L.cad_destroy(other)
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
