@@ -226,6 +226,17 @@ int ensure(cad_ctx* ctx, Slot s, size_t bytes, void** out)
     return CAD_OK;
 }
 
+// Gives a workspace back.
+int release(cad_ctx* ctx, Slot s)
+{
+    DevBuf& b = ctx->buf[s];
+    if (!b.p) return CAD_OK;
+    CK(cudaStreamSynchronize(ctx->stream));
+    CK(cudaFree(b.p));
+    b = DevBuf{};
+    return CAD_OK;
+}
+
 int set_device(cad_ctx* ctx)
 {
     if (!ctx) return CAD_ERR_ARG;
@@ -260,14 +271,20 @@ struct EdgeTable {
 // triangles stays on the per-side kernels.
 bool edges_pay(int64_t E, int64_t N) { return 10 * E < 9 * 3 * N; }
 
+// Its workspaces.
+int edge_table_buffers(cad_ctx* ctx, int64_t N, void** pts, void** ints)
+{
+    if (int r = ensure(ctx, S_EDGE_PTS, (size_t)18 * N * sizeof(double), pts)) return r;
+    return ensure(ctx, S_EDGE_INT, ((size_t)12 * N + edge_work_ints(N)) * sizeof(int), ints);
+}
+
 // The mesh-edge table of the triangles, on the device (lists: with each edge's
 // sides); count: where its number of edges goes.
 int edge_table(cad_ctx* ctx, const double* P1, const double* P2, const double* P3, int64_t N, bool lists, int* count,
                EdgeArrays* a)
 {
     void *pts, *ints;
-    if (int r = ensure(ctx, S_EDGE_PTS, (size_t)18 * N * sizeof(double), &pts)) return r;
-    if (int r = ensure(ctx, S_EDGE_INT, ((size_t)12 * N + edge_work_ints(N)) * sizeof(int), &ints)) return r;
+    if (int r = edge_table_buffers(ctx, N, &pts, &ints)) return r;
     int* i = (int*)ints;
     *a = EdgeArrays{(double*)pts, i, i + 3 * N, i + 6 * N, i + 9 * N, i + 12 * N, count};
     CK(launch_edge_table(P1, P2, P3, N, *a, lists, ctx->stream, &ctx->launches));
@@ -375,22 +392,29 @@ int td_device(cad_ctx* ctx, const double* X, const double* Y, const double* Z, i
         // nothing is read back (E stays on the device), so the call stays
         // asynchronous; a mesh without shared edges costs the same as its pairs
         const int64_t echunk = pick_chunk(M, 3 * N, true), nechunk = (3 * N + echunk - 1) / echunk;
-        void *flag, *rec, *part;
-        if (int r = ensure(ctx, S_FLAG, 3 * sizeof(int), &flag)) return r;
-        if (int r = ensure(ctx, S_EDGE_REC, (size_t)3 * N * segment_record_bytes(), &rec)) return r;
-        if (int r = ensure(ctx, S_PART, (size_t)(nchunk + nechunk) * 9 * M * sizeof(double), &part)) return r;
-        EdgeArrays ed;
-        CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-        if (int r = edge_table(ctx, P1, P2, P3, N, true, (int*)flag, &ed)) return r;
-        a.partial = (double*)part;
-        CK(launch_td_sum_segments(a, strain == 1, disp == 1, ed, rec, nu, nechunk, a.partial + (size_t)nchunk * 9 * M,
-                                  ctx->stream, &ctx->launches));
-        CK(cudaEventRecord(ctx->ev[1], ctx->stream));
-        ctx->timed[0] = true;
-        const int mask = (strain == 1 ? 0x3f : 0) | (disp == 1 ? 0x1c0 : 0);
-        ++ctx->launches;
-        CK(launch_sum_chunks(a.partial, nchunk + nechunk, M, mask, sum_out, ctx->stream));
-        return CAD_OK;
+        void *flag, *rec, *part, *pts, *ints;
+        int r = ensure(ctx, S_FLAG, 3 * sizeof(int), &flag);
+        if (!r) r = ensure(ctx, S_EDGE_REC, (size_t)3 * N * segment_record_bytes(), &rec);
+        if (!r) r = ensure(ctx, S_PART, (size_t)(nchunk + nechunk) * 9 * M * sizeof(double), &part);
+        if (!r) r = edge_table_buffers(ctx, N, &pts, &ints);
+        if (r == CAD_OK) {
+            EdgeArrays ed;
+            CK(cudaEventRecord(ctx->ev[0], ctx->stream));
+            if (int q = edge_table(ctx, P1, P2, P3, N, true, (int*)flag, &ed)) return q;
+            a.partial = (double*)part;
+            CK(launch_td_sum_segments(a, strain == 1, disp == 1, ed, rec, nu, nechunk,
+                                      a.partial + (size_t)nchunk * 9 * M, ctx->stream, &ctx->launches));
+            CK(cudaEventRecord(ctx->ev[1], ctx->stream));
+            ctx->timed[0] = true;
+            const int mask = (strain == 1 ? 0x3f : 0) | (disp == 1 ? 0x1c0 : 0);
+            ++ctx->launches;
+            CK(launch_sum_chunks(a.partial, nchunk + nechunk, M, mask, sum_out, ctx->stream));
+            return CAD_OK;
+        }
+        if (r != CAD_ERR_OOM) return r;
+        // the edges' workspaces do not fit beside the call's arrays: the pairs need less
+        for (Slot s : {S_EDGE_REC, S_PART, S_EDGE_PTS, S_EDGE_INT})
+            if (int q = release(ctx, s)) return q;
     }
     if (out_kind == OUT_SUM) {
         void* part;

@@ -2,6 +2,8 @@
 against the per-triangle sums: meshes with shared, repeated and unshared
 sides, points on vertices, sides and inside elements, zero-slip and
 degenerate triangles, and the sizes at which the edges take over."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -76,3 +78,37 @@ def test_edges_over_sizes(cad, n, M):
     pts = rng.uniform([-2, -2, -3], [34, 34, 1], (M, 3))
     for x, y in zip(_sums(cad, P, sl, pts, True), _sums(cad, P, sl, pts, False)):
         assert_parity(x, y)
+
+
+def test_sums_where_only_the_pairs_fit(cad, fresh_context):
+    """A full-space sum runs over the pairs where the edges' workspaces cannot be
+    had: only the arrays every sum needs are refused."""
+    from cutanddisplacejulia_b200 import _lib
+    L = _lib.load()
+    rng = np.random.default_rng(11)
+    P = _mesh("bent", rng)
+    n = len(P[0])
+    sl = rng.uniform(-1e-3, 1e-3, (3, n))
+    pts = rng.uniform([-2, -2, -3], [5, 5, 1], ((5 << 20) // n + 1, 3))
+    want = _sums(cad, P, sl, pts, False)
+    outcome = []
+    for nth in range(1, 12):
+        h = ctypes.c_void_p()
+        _lib.check(L.cad_init(0, ctypes.byref(h)), None)
+        _lib._ctx[0] = h
+        try:
+            _lib.check(L.cad_fail_allocation(h, nth), h)
+            try:
+                got = _sums(cad, P, sl, pts, True)
+            except cad.CadError as e:
+                assert e.code == _lib.CAD_ERR_OOM
+                outcome.append("refused")
+            else:
+                for x, y in zip(got, want):
+                    assert_parity(x, y)
+                outcome.append("pairs" if all(np.array_equal(x, y) for x, y in zip(got, want)) else "edges")
+        finally:
+            _lib._ctx[0] = fresh_context
+            L.cad_destroy(h)
+    # inputs, outputs, records; then flag, edge records, partial sums, end points, table
+    assert outcome == 3 * ["refused"] + 5 * ["pairs"] + 3 * ["edges"], outcome
