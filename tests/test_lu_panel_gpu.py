@@ -56,9 +56,6 @@ def test_lu_rows_moved_across_the_matrix(cad, n):
 
 
 def test_lu_repeated_entries_and_singular(cad):
-    import torch
-
-    from cutanddisplacejulia_b200 import _lib
     n = 400
     # equal magnitudes everywhere: ties go to the first row, as LAPACK's
     H = np.where(np.random.default_rng(0).random((n, n)) < 0.5, -1.0, 1.0)
@@ -67,9 +64,8 @@ def test_lu_repeated_entries_and_singular(cad):
     S = np.ones((n, n))
     with pytest.raises(cad.CadError):
         cad.solve(S, np.ones(n))
-    L, ctx = _lib.load(), _lib.context(0)
-    torch.cuda.synchronize()
-    assert L.cad_last_error(ctx)
+    # the context solves as before afterwards
+    assert _solve(n, 1, 6)[0] < 64 * n * 2.3e-16
 
 
 @pytest.mark.parametrize("n", [511, 513, 1100, 2100])
@@ -83,3 +79,30 @@ def test_lu_wide_blocks(cad, n):
             assert _solve(n, nrhs, 300 + n)[0] < 64 * n * 2.3e-16
     finally:
         _lib.check(L.cad_set_lu_block(ctx, 0), ctx)
+
+
+@pytest.mark.parametrize("rpt", [2, 4])
+def test_lu_narrow_leaves(cad, tmp_path, rpt):
+    """The leaves of 16 and 8 columns (2 and 4 rows per thread: 1024 and 2048 rows
+    per thread block) that the autotuner may choose, and their update kernels, at
+    remainders of leaves and panels and one to nine blocks per cluster."""
+    from cutanddisplacejulia_b200 import _lib
+    L, ctx = _lib.load(), _lib.context(0)
+    cache = tmp_path / "tune.txt"
+    cache.write_text("".join(f"lu_leaf_f64_n{1 << k} {rpt}\n" for k in range(15)))
+    _lib.check(L.cad_set_autotune(ctx, 2, str(cache).encode()), ctx)     # read, never timed
+    try:
+        sizes = [7, 9, 17, 33, 255, 257, 263, 530, 1023, 1025, 1100, 2049, 2100, 4200] + ([8600] if rpt == 2 else [])
+        for n in sizes:
+            for nrhs in (1, 3):
+                err, A, B, X = _solve(n, nrhs, 500 + n)
+                assert err < 64 * n * 2.3e-16, n
+            if n <= 600:
+                x = np.linalg.solve(A.cpu().numpy(), B.cpu().numpy().T)
+                cond = np.linalg.cond(A.cpu().numpy())
+                assert np.abs(X.cpu().numpy().T - x).max() <= 64 * cond * n * 2.3e-16 * np.abs(x).max(), n
+        import torch
+        rows = torch.arange(1099, -1, -1, device="cuda")
+        assert _solve(1100, 1, 5, rows=rows)[0] < 64 * 1100 * 2.3e-16
+    finally:
+        _lib.check(L.cad_set_autotune(ctx, 0, None), ctx)
