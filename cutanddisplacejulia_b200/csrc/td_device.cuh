@@ -849,12 +849,6 @@ CAD_HD void side_strain_map(const FscSideT<R>& s, double X, double Y, double Z, 
     for (int j = 0; j < 3; ++j) adcs_to_efcs(G[j], s.ea, s.eb);
 }
 
-template <typename R>
-CAD_HD void fsc_strain_map(const FscSideT<R>& s, double X, double Y, double Z, R G[3][6])
-{
-    side_strain_map<false>(s, X, Y, Z, G);
-}
-
 // The whole half-space map of a side as tractions: W[j][r] = traction r
 // (normal, strike, dip) on an element with axes n, ss, ds for a unit Burgers
 // vector along EFCS axis j.  The element's axes are turned into ADCS, where
@@ -1415,7 +1409,7 @@ CAD_HD void sum_side_maps(const double* G, int64_t gq, int64_t ge, const int* co
 }
 
 // Half-space strain with the sides' corrections read from per-edge maps
-// (fsc_strain_map), real and image full-space terms evaluated here.
+// (side_strain_map<false>), real and image full-space terms evaluated here.
 CAD_HD void pair_strain_edges(const TriDev& t, double X, double Y, double Z, const double* G, int64_t gq, int64_t ge,
                               const int* code, double E[3][6])
 {
