@@ -34,26 +34,32 @@ if ROOT not in sys.path:
 
 from cutanddisplacejulia_b200 import dist as cdist  # noqa: E402
 
-# Algorithmic FP64 operations per pair-evaluation of the assembly kernel:
+# The reference's own FP64 operations per pair-evaluation of the assembly:
 # full-space strain of all three unit slip modes (2960, counted with the
 # oracle's counting scalar on this mesh's collocation pairs) plus the strain ->
-# traction epilogue (288 = 3 modes x 96).  Frozen values: kernel-side common
-# subexpressions count as speed-up, not as fewer operations.
+# traction epilogue (288 = 3 modes x 96).  Frozen values, reported as the rate the
+# reference's formulas would need; the rooflines count what the kernels execute.
 FALG_ASSEMBLY_FS = 2960.0 + 288.0
 # Half-space strain of all three unit modes (43867 on the dipping-crack
 # collocation pairs) plus the same traction epilogue.
 FALG_ASSEMBLY_HS = 43867.0 + 288.0
+# FP64 instructions the kernels execute, a thread each (ncu
+# sm__inst_executed_pipe_fp64 x 32 over the threads of whole warps,
+# profiles/td_kernels_edges_and_pairs.md): per pair of the full-space system
+# matrix, per (mesh edge, point) of the half-space traction maps and of the edge
+# sums, per pair of the matrix combined from the maps and of the sums' solid angles
+FP64_INSTR = {"pair_fs": 810.0, "map_hs": 854.0, "pair_from_maps": 128.0, "sum_hs": 1122.0, "angles_hs": 282.0}
 # DRAM bytes (read + write) of one assembly from the committed ncu captures
 # (profiles/td_kernels_edges_and_pairs.md): (triangles captured, bytes).  Both
 # scale as N^2.  Half space: the shared-edge path's two kernels, side_map_kernel
-# (4.80 MB + 380.33 MB) and the combining pair kernel (517.18 MB + 249.88 MB), at
+# (4.75 MB + 380.45 MB) and the combining pair kernel (516.82 MB + 249.50 MB), at
 # 1980 triangles and 3037 edges.
-PAIR_TRAFFIC = {"penny": (2013, 1.04e6 + 231.96e6), "dipping": (1980, 4.80e6 + 380.33e6 + 517.18e6 + 249.88e6)}
+PAIR_TRAFFIC = {"penny": (2013, 1.03e6 + 232.44e6), "dipping": (1980, 4.75e6 + 380.45e6 + 516.82e6 + 249.50e6)}
 # FP64-pipe activity (fraction of peak, ncu sm__pipe_fp64_cycles_active) of the
 # shared-edge half-space assembly's kernels, from the committed capture at 1980
 # triangles (profiles/td_kernels_edges_and_pairs.md); the pair kernel is bound by
 # the maps' bytes
-FP64_PIPE_ACTIVE_HS = {"side_map_kernel": 0.729, "td_pair_kernel_edge": 0.171}
+FP64_PIPE_ACTIVE_HS = {"side_map_kernel": 0.728, "td_pair_kernel_edge": 0.166}
 # share of the step's (serialised) device time taken by the LU panel leaf, from
 # the committed launch list (profiles/launches_penny2013_fp64_and_mixed_step.md)
 DOMINANT_SHARE = {"penny": 0.306}
@@ -88,16 +94,27 @@ WORKLOADS["gemm"] = ("LU trailing-update GEMM TFLOP/s (C -= A B, column-major)",
 METRIC = WORKLOADS["penny"][0]
 
 
+def mesh_edges(P1, P2, P3):
+    """Number of distinct sides of a triangle list, whichever way they run."""
+    import numpy as np
+    V = [np.asarray(p, dtype=np.float64) + 0.0 for p in (P1, P2, P3)]
+    e = np.concatenate([np.stack([V[k], V[(k + 1) % 3]], 1) for k in range(3)])      # sides x ends x 3
+    d = e[:, 0] - e[:, 1]
+    first = np.where(d[:, 0] != 0, d[:, 0], np.where(d[:, 1] != 0, d[:, 1], d[:, 2]))
+    e[first > 0] = e[first > 0][:, ::-1]
+    return len(np.unique(e.reshape(-1, 6), axis=0))
+
+
 def _hbm_peak():
-    """Measured HBM copy bandwidth of this pool's B200s when the peaks file
-    exists, else the earlier measurement on the same pool."""
+    """Measured HBM copy bandwidth of these B200s when the peaks file exists, else
+    an earlier measurement of the same kind."""
     p = os.path.join(ROOT, "MEASURED_PEAKS.json")
     try:
         with open(p) as f:
             v = float(json.load(f)["hbm_gbs"])
         return v, "measured HBM copy bandwidth (MEASURED_PEAKS.json hbm_gbs), of measured"
     except (OSError, KeyError, ValueError, TypeError):
-        return 6650.0, "6.65 TB/s, an earlier copy-bandwidth measurement on this pool (of fallback)"
+        return 6650.0, "6.65 TB/s, an earlier copy-bandwidth measurement on such a GPU (of fallback)"
 
 
 HBM_PEAK_GBS = _hbm_peak()
@@ -998,7 +1015,10 @@ def run_c3(args, rank, world, local_rank):
                "sample": desc + ": assembly %.1f s (scaled), solve %.1f s" % (a_s, s_s)}
 
     falg = FALG_ASSEMBLY_HS
-    asm_tflops = falg * pairs / (asm_ms * 1e-3) / 1e12
+    # executed FP64 instructions of the shared-edge assembly, two flops each
+    edges = mesh_edges(P1, P2, P3)
+    asm_instr = FP64_INSTR["map_hs"] * edges * n + FP64_INSTR["pair_from_maps"] * pairs
+    asm_tflops = 2.0 * asm_instr / (asm_ms * 1e-3) / 1e12 if args.shared_edges else None
     # algorithmic bytes of the solve: the FP32 copy of A (read 8, write 4
     # bytes per entry), one FP32 pass per Arnoldi product, and one FP64 pass
     # per true residual (each restart cycle and the final check)
@@ -1033,20 +1053,24 @@ def run_c3(args, rank, world, local_rank):
         "roofline": {"kernel": "side_map_kernel + td_pair_kernel<HS, strain, A-matrix, EDGE> (the step's dominant "
                                "phase: the FP64 shared-edge half-space assembly)",
                      "bound": "fp64", "achieved": asm_tflops, "peak": fp64_peak, "unit": "TFLOP/s",
-                     "frac": asm_tflops / fp64_peak,
+                     "frac": asm_tflops / fp64_peak if asm_tflops else None,
                      "peak_source": "measured FP64 FMA throughput (cad_fp64_fma_probe, this run); "
                                     "MEASURED_PEAKS.json has no FP64 figure",
-                     "falg_per_pair": falg,
+                     "work": "executed FP64 instructions, two flops each: %d per (mesh edge, point) of the maps, %d "
+                             "per pair (ncu, profiles/td_kernels_edges_and_pairs.md); the pairs are bound by the "
+                             "maps' bytes" % (FP64_INSTR["map_hs"], FP64_INSTR["pair_from_maps"]),
+                     "mesh_edges": edges,
+                     "reference_flops_per_pair": falg,
+                     "reference_flops_rate_tflops": falg * pairs / (asm_ms * 1e-3) / 1e12,
                      "traffic": PAIR_TRAFFIC["dipping"][1] * (n / PAIR_TRAFFIC["dipping"][0]) ** 2,
                      "traffic_source": "ncu DRAM bytes (read + write) of the assembly's two kernels at N=%d, "
                                        "scaled by (N/%d)^2; the edge maps (9 doubles per edge and point) are "
                                        "written once and read by the triangles sharing each edge, the rest is "
                                        "the matrix" % (PAIR_TRAFFIC["dipping"][0], PAIR_TRAFFIC["dipping"][0]),
-                     "falg_note": "F_alg is the reference's literal count per pair, which evaluates each "
-                                  "side's terms per triangle and slip mode from angular dislocations; the "
-                                  "shared-edge path evaluates each edge once, from straight segments and "
-                                  "harmonic functions, so the algorithmic rate exceeds the FP64 pipe's peak "
-                                  "(fp64_pipe_active_ncu is the pipe's own activity)",
+                     "reference_flops_note": "the reference's literal count per pair, which evaluates each side's "
+                                             "terms per triangle and slip mode from angular dislocations; no "
+                                             "roofline: each edge is evaluated once here, from straight segments "
+                                             "and harmonic functions",
                      "fp64_pipe_active_ncu": FP64_PIPE_ACTIVE_HS,
                      "step_share": asm_ms / ms},
         "roofline_gmres": {"kernel": "GMRES(30): FP32 copy of A, one FP32 pass over A per Arnoldi product, "
@@ -1194,7 +1218,10 @@ def run_ours(args, rank, world, local_rank):
     # assembly time per step over the timed region (pair kernel + the two small
     # per-element prep kernels, all on this stream): the launch duration used
     falg = FALG_ASSEMBLY_HS if hs else FALG_ASSEMBLY_FS
-    achieved = falg * pairs / (asm_ms * 1e-3) / 1e12
+    # executed FP64 instructions, two flops each
+    instr = (FP64_INSTR["map_hs"] * mesh_edges(P1, P2, P3) * n + FP64_INSTR["pair_from_maps"] * pairs if hs
+             else FP64_INSTR["pair_fs"] * pairs)
+    achieved = 2.0 * instr / (asm_ms * 1e-3) / 1e12
     lu_flops = (2.0 / 3.0) * n3 ** 3 + 2.0 * n3 * n3
     solve_tflops = lu_flops / (sol_ms * 1e-3) / 1e12
     line = {
@@ -1230,14 +1257,17 @@ def run_ours(args, rank, world, local_rank):
                             "source": "profiles/launches_penny2013_fp64_and_mixed_step.md",
                             "ncu_full": "profiles/leaf_lu_kernel_penny2013.md",
                             # from that capture (a panel of ten CTAs): the panel read once, issue
-                            # 30.2 %, FP64 pipe 5.0 %, DRAM 0.33 % of peak
-                            "ncu_dram_bytes_per_launch": 1.29e6, "ncu_issue_active": 0.302,
+                            # 31.2 %, FP64 pipe 5.0 %, DRAM 0.34 % of peak
+                            "ncu_dram_bytes_per_launch": 1.29e6, "ncu_issue_active": 0.312,
                             "ncu_fp64_pipe": 0.050},
         "roofline_assembly": {"kernel": "td_pair_kernel<%s, strain, A-matrix>" % ("HS" if hs else "FS"),
                               "bound": "fp64", "achieved": achieved, "peak": fp64_peak_tflops, "unit": "TFLOP/s",
                               "frac": achieved / fp64_peak_tflops,
                               "peak_source": "measured FP64 FMA throughput (cad_fp64_fma_probe, this run)",
-                              "falg_per_pair": falg,
+                              "work": "executed FP64 instructions, two flops each (ncu, "
+                                      "profiles/td_kernels_edges_and_pairs.md)",
+                              "reference_flops_per_pair": falg,
+                              "reference_flops_rate_tflops": falg * pairs / (asm_ms * 1e-3) / 1e12,
                               "traffic": PAIR_TRAFFIC[args.workload][1] * (n / PAIR_TRAFFIC[args.workload][0]) ** 2,
                               "traffic_source": "ncu DRAM bytes (read + write) of one launch at "
                                                 "N=%d, scaled by (N/%d)^2" % (PAIR_TRAFFIC[args.workload][0],
@@ -1337,7 +1367,7 @@ def run_gemm(args, rank, world, local_rank):
 
 
 # Half-space strain + displacement per pair, both frozen oracle counts (the
-# summing TD overload evaluates all three slip modes of each).
+# summing TD overload evaluates all three slip modes of each): the reference's.
 FALG_SUM_HS = 43867.0 + 6780.0
 TDSUM_GRID = 100
 
@@ -1361,8 +1391,8 @@ def run_tdsum(args, rank, world, local_rank):
     """The summing TD overload (src/TD.jl:219-410) in half space: strain and
     displacement at the free surface of a slipping dipping crack.  One step =
     one cad_td_sum_eval_dev call on device-resident inputs (the shared-edge
-    path: each mesh edge's free-surface correction once, for the net Burgers
-    vector of its sides); the per-side path and the host API (cad.TD with
+    path: each mesh edge's field once, for the net Burgers vector of its sides,
+    and the triangles' solid angles); the per-side path and the host API (cad.TD with
     Strains/Disps, host arrays) are timed beside it."""
     import numpy as np
     import torch
@@ -1443,7 +1473,8 @@ def run_tdsum(args, rank, world, local_rank):
         cpu = {"value": 300.0 * n / cpu_s, "unit": UNIT, "cores": nthreads, "kind": "port",
                "sample": "oracle HS sums of all %d triangles at 300 seeded grid points (%d threads): %.1f s; "
                          "max rel err of the GPU result there %.2e" % (n, nthreads, cpu_s, err)}
-    achieved = pairs * FALG_SUM_HS / (ms * 1e-3) / 1e12
+    edges = mesh_edges(P1, P2, P3)
+    achieved = 2.0 * (FP64_INSTR["sum_hs"] * edges * m + FP64_INSTR["angles_hs"] * pairs) / (ms * 1e-3) / 1e12
     line = {
         "metric": WORKLOADS["tdsum"][0], "value": cdist.replica_throughput(pairs, ms, world), "unit": UNIT,
         "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,
@@ -1461,10 +1492,13 @@ def run_tdsum(args, rank, world, local_rank):
         "gpu_launches": int(launches),
         "roofline": {"kernel": "side_sum_kernel + td_pair_kernel<HS, sum, EDGE> (shared-edge half-space sums)",
                      "bound": "fp64", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
-                     "frac": achieved / peak.value, "falg_per_pair": FALG_SUM_HS,
+                     "frac": achieved / peak.value, "mesh_edges": edges,
                      "peak_source": "measured FP64 FMA throughput (cad_fp64_fma_probe, this run)",
-                     "falg_note": "the reference's literal count per pair; the shared-edge path evaluates each "
-                                  "edge's field once instead of per side and mode",
+                     "work": "executed FP64 instructions, two flops each: %d per (mesh edge, point), %d per pair (ncu, "
+                             "profiles/td_kernels_edges_and_pairs.md)" % (FP64_INSTR["sum_hs"],
+                                                                          FP64_INSTR["angles_hs"]),
+                     "reference_flops_per_pair": FALG_SUM_HS,
+                     "reference_flops_rate_tflops": pairs * FALG_SUM_HS / (ms * 1e-3) / 1e12,
                      "traffic": None},
         "cpu_baseline": cpu,
     }
