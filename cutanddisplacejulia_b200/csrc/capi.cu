@@ -295,7 +295,12 @@ int edge_table(cad_ctx* ctx, const double* P1, const double* P2, const double* P
 // of a pair's 36 ps is saved (a third for displacements alone), and the edge
 // table costs 40 to 80 us.  Strain at 10 000 x 500 (triangles x points) 252 us
 // over edges and 259 by pairs, 100 x 42 000 178 and 177, 2013 x 3200 209 and
-// 277; displacements alone at 10 000 x 1700 579 and 628.
+// 277; displacements alone at 10 000 x 1700 579 and 628.  The rule looks at pairs
+// alone (E stays on the device), and a mesh without shared sides has twice the
+// edges: at 10 000 x 10 000 strain still takes 3.59 ms over edges and 3.81 by
+// pairs, both fields 5.97 and 6.78, displacements alone 4.34 and 3.50 (with shared
+// sides 1.88 and 3.81, 3.73 and 6.78, 2.90 and 3.50); at 10 000 x 600 strain 0.38
+// and 0.30 (shared 0.26 and 0.30).
 bool segments_pay(int64_t M, int64_t N, bool strain)
 {
     return M >= 256 && M >= (strain ? int64_t(5) << 20 : int64_t(1) << 24) / (N > 0 ? N : 1);
@@ -350,8 +355,9 @@ int td_device(cad_ctx* ctx, const double* X, const double* Y, const double* Z, i
     a.strain = strain_out; a.disp = disp_out;
     const int64_t nchunk = (N + a.tri_chunk - 1) / a.tri_chunk;
     if (et.use && out_kind == OUT_INF) {
-        // per-edge free-surface maps at the points (strain 18, displacement
-        // 9 values), read by the triangles that share each edge
+        // per-edge maps at the points (strain 18, displacement 9 values: of
+        // the whole strain where et.full, else of the correction, and of the
+        // displacement's correction), read by the triangles that share each edge
         void *rec, *gmap;
         if (int r = ensure(ctx, S_EDGE_REC, (size_t)et.E * edge_record_bytes(), &rec)) return r;
         const int64_t per_point =
@@ -368,9 +374,9 @@ int td_device(cad_ctx* ctx, const double* X, const double* Y, const double* Z, i
         return CAD_OK;
     }
     if (et.use) {
-        // real + image terms per triangle chunk, then each mesh edge's
-        // free-surface correction once, for the net Burgers vector of the
-        // sides on it; all partials summed in one fixed order
+        // the triangles' share per triangle chunk, then each mesh edge once, for
+        // the net Burgers vector of the sides on it (launch_td_sum_edges); all
+        // partials summed in one fixed order
         const int64_t echunk = pick_chunk(M, et.E, true);
         const int64_t nechunk = (et.E + echunk - 1) / echunk;
         void *part, *rec;
@@ -390,7 +396,7 @@ int td_device(cad_ctx* ctx, const double* X, const double* Y, const double* Z, i
     if (out_kind == OUT_SUM && hs == 0 && edge_kind && ctx->shared_edges && edge_table_fits(N) &&
         segments_pay(M, N, strain == 1)) {
         // nothing is read back (E stays on the device), so the call stays
-        // asynchronous; a mesh without shared edges costs the same as its pairs
+        // asynchronous, also where the mesh shares no edges (segments_pay)
         const int64_t echunk = pick_chunk(M, 3 * N, true), nechunk = (3 * N + echunk - 1) / echunk;
         void *flag, *rec, *part, *pts, *ints;
         int r = ensure(ctx, S_FLAG, 3 * sizeof(int), &flag);
@@ -472,8 +478,9 @@ int assemble_device(cad_ctx* ctx, const double* normals, const double* mid, cons
         return CAD_OK;
     }
     if (et.use) {
-        // each mesh edge's free-surface map evaluated once, then read by the
-        // (one or two) triangles that share the edge
+        // each mesh edge's map (tractions of the whole strain where et.full, else
+        // the correction's strain) evaluated once, then read by the triangles
+        // that share the edge
         const int64_t E = et.E;
         double* pts = et.a.pts;
         int* codes = et.a.code;
@@ -514,8 +521,8 @@ int assemble_device(cad_ctx* ctx, const double* normals, const double* mid, cons
         return CAD_OK;
     }
     if (out_kind == OUT_AMAT && ctx->tuner.mode != TUNE_OFF) {
-        // triangles per block of the pair kernel (each block stages one
-        // triangle record at a time into shared memory)
+        // triangles per block of the pair kernel (each block stages the records
+        // in shared memory, eight at a time or, in half space, one)
         char key[96];
         std::snprintf(key, sizeof key, "pair_amat_f64_hs%d_N%lld", hs, (long long)tune_class(N));
         PairArgs t = a;
@@ -1148,8 +1155,11 @@ int slip_batched_ws(cad_ctx* ctx, int64_t nbatch, const int64_t* offsets, const 
         b.gsync_ints = ns;
     }
     // a plan seen for the second time is captured, then replayed; the first
-    // call is issued directly (34 ms for 64 cracks of 200 to 1500 elements,
-    // where capture and replay take 50 and the replay alone 32.5)
+    // call is issued directly.  First, second and later calls, ms: 2 cracks of 200
+    // to 400 elements 6.0, 4.6, 1.85; 64 of 50 to 200 6.9, 7.2, 2.07; 16 of 200 to
+    // 1500 17.3, 31.2, 14.5; 64 of them 34.4, 50.2, 30.8; 256 of 200 to 700 31.5,
+    // 40.6, 28.5: the capture pays from the third call on for small cracks, from
+    // the sixth or seventh for large ones.
     BatchGraph& g = ctx->batch;
     const void* ptrs[8] = {P1, Aall, rel, ga32, gint, gf32, gf64, gmaps};
     const double params[5] = {nu, G, lambda, ctx->tol, ctx->near_factor};

@@ -1,17 +1,19 @@
 // Dense LU with partial pivoting and triangular solves (the `A\b` of
 // SlipCalculator3D, src/SlipCalculator3D.jl:22) for sm_100a.
 //
-// Right-looking blocked LU (outer block nb).  Each nb-wide panel is factorised
-// recursively: the left half, then a row swap, a triangular solve and a GEMM
-// update of the right half, then the right half.  The recursion stops at
-// narrow leaves that one thread-block cluster factorises with its rows held in
-// distributed shared memory: per column, every CTA proposes its largest
-// |entry|, the cluster agrees on the pivot through DSMEM, the pivot row and the
-// displaced row are exchanged through DSMEM, and every CTA updates its own rows
-// -- two hardware cluster barriers per column, no global-memory spin.  Rank-nb
-// trailing updates and the intra-panel updates are the library's own tensor-
-// core GEMMs (csrc/gemm.cu: DMMA tiles in FP64; tcgen05 TF32 with TMA-staged
-// operands for the single-precision factorisation).
+// Right-looking blocked LU (outer block nb).  A panel is factorised leaf by leaf:
+// one thread-block cluster factorises up to 32 columns with its rows in registers
+// -- per column every CTA pushes its best row, with its key and reciprocal, into
+// the shared memory of all, waits on its own mbarrier for the others', takes the
+// pivot and updates its rows; no cluster barrier, no global-memory spin -- then
+// one launch moves, solves and updates the panel's columns right of the leaf, and
+// another beside the next leaf those of the next block column.  Panels of more
+// rows than one per leaf thread (8192 with clusters of 16) are split in halves
+// instead: the left one, a row swap, a triangular solve and a GEMM update of the
+// right one, then the right one; so are the grouped factorisation's.  Rank-nb
+// trailing updates are the library's own tensor-core GEMMs (csrc/gemm.cu: DMMA
+// tiles in FP64; tcgen05 TF32 with TMA-staged operands for the single-precision
+// factorisation).
 //
 // Pivot choice is LAPACK's: the first row of largest magnitude; scaling by the
 // reciprocal pivot; ipiv[k] = absolute row swapped with row k.

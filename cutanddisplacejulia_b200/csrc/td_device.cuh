@@ -16,8 +16,9 @@
 // Data layout: everything that depends only on the triangle (frames, angles,
 // per-dislocation constants of every closed-form term, slip rotations) is
 // computed once per triangle by td_setup_kernel into a TriDev record; the pair
-// kernels stage one TriDev at a time in shared memory and every thread of the
-// block (one observation point each) reads it as a broadcast.
+// kernels stage records in shared memory (one, or eight of the small ones, at a
+// time) and every thread of the block (one observation point each) reads each as
+// a broadcast.
 #pragma once
 #include <cfloat>
 #include <cstddef>

@@ -1,9 +1,10 @@
 // TD pair kernels for sm_100a (FP64 CUDA-core work; no tensor-core shape).
 //
 // Work decomposition: one thread per observation point, one block per
-// (128-point tile, chunk of triangles).  The block stages one triangle's
-// precomputed record (TriDev) at a time in shared memory; every thread reads
-// it as a broadcast, evaluates its pair and writes the pair's outputs
+// (128-point tile, chunk of triangles).  The block stages the triangles'
+// precomputed records (TriDev; the full-space and frame-only ones eight at a
+// time) in shared memory; every thread reads each as a broadcast, evaluates its
+// pair and writes the pair's outputs
 // (consecutive threads = consecutive rows of a column-major M x N influence
 // matrix, so every store is coalesced).
 //
@@ -943,8 +944,8 @@ __global__ void __launch_bounds__(kBurgersThreads) segment_burgers_kernel(const 
 // partial[(blockIdx.y * 9 + f) M + i] = the full-space strain (f 0-5) and the
 // segments' displacement (f 6-8) at point i of the edges of chunk blockIdx.y of
 // gridDim.y, summed in edge order (kSegStage records staged in shared memory at
-// a time).  FP64 bound, about 160 instructions per (edge, point) against 490 per
-// (triangle, point) side by side: strain of 2013 triangles (3060 edges) at
+// a time).  FP64 bound, 141 FP64 instructions per (edge, point) against about 490
+// per (triangle, point) side by side: strain of 2013 triangles (3072 edges) at
 // 20 000 points 670 us where the pairs took 1430 (two points per thread: 682).
 constexpr int kSegStage = 16;
 template <bool STRAIN, bool DISP>
@@ -985,11 +986,11 @@ __global__ void __launch_bounds__(kPairThreads) segment_sum_kernel(const SegRec*
 // partial[(blockIdx.y * 9 + f) M + i] = the strain (f 0-5; STRAIN EDGE_FSC: the
 // free-surface correction, EDGE_FULL: all of it) and the correction's
 // displacement (f 6-8; EDGE_FULL: all but the solid angles) at point i of the edges of chunk blockIdx.y, summed in
-// edge order (8 edge records staged in shared memory at a time).  FP64 bound;
-// three resident blocks per SM are worth the 128 bytes they spill (strain and
-// displacement of 15 150 edges at 10 000 points, the real and image segments'
-// displacement included: 14.5 ms at two blocks and 66 % of the pipe, 13.6 at
-// three).  The triangles' solid angles take 2.7 ms more; with the segments'
+// edge order (8 edge records staged in shared memory at a time).  FP64 bound,
+// 1122 FP64 instructions per (edge, point); three resident blocks per SM are worth
+// the spills (208 bytes stored, 208 loaded; strain and displacement of 15 150 edges
+// at 10 000 points, the real and image segments' displacement included: 14.5 ms at
+// two blocks and 66 % of the pipe, 13.6 and 71 % at three).  The triangles' solid angles take 2.7 ms more; with the segments'
 // displacement taken side by side the pairs took 7.3.
 template <int STRAIN, bool DISP>
 __global__ void __launch_bounds__(kPairThreads, STRAIN == EDGE_NONE ? 4 : STRAIN == EDGE_FSC && DISP ? 2 : 3)

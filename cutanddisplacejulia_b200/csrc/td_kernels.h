@@ -47,9 +47,9 @@ struct PairArgs {
     // half-space system matrix: the kernel variant compiled for this many
     // resident blocks per SM (1: the full register file; 3 or 4)
     int min_blocks = 1;
-    // half-space system matrix with shared-edge free-surface maps: the maps
-    // of this launch's points (18 x M per edge, side_map_kernel) and each
-    // triangle's three side codes (+-(edge + 1), 0: none); rows are then a
+    // half-space fields from shared-edge maps: the maps of this launch's points
+    // (edge_map_values x M per edge, side_map_kernel) and each triangle's three
+    // side codes (+-(edge + 1), 0: none); rows are then a
     // block of an Ntot-point system (X, Y, Z, dirs and A or trac start at the
     // block; the output fields keep the system's row stride)
     const double* fscG = nullptr;
@@ -80,11 +80,13 @@ inline int64_t edge_map_values(int out_kind, bool strain, bool disp, bool full)
 }
 size_t edge_record_bytes();
 
-// Half-space sums (OUT_SUM) with the free-surface correction evaluated once
-// per mesh edge for the net Burgers vector of the triangle sides on it:
-// a.partial receives the real + image terms of each triangle chunk (as
-// launch_td_pairs), edge_partial the corrections of each chunk of echunk
-// edges (9 x a.M each).  ed: launch_edge_table's arrays with lists.  a.tri must
+// Half-space sums (OUT_SUM) over the mesh's edges, each for the net Burgers
+// vector of the triangle sides on it.  full (as above), strain asked for: an edge
+// adds its whole strain and all of its displacement but the solid angles
+// (edge_partial, per chunk of echunk edges, 9 x a.M), the triangles the solid
+// angles and the NaN of points on a side (a.partial, per triangle chunk).
+// Otherwise the edges add the free-surface correction alone, the triangles their
+// real + image terms.  ed: launch_edge_table's arrays with lists.  a.tri must
 // hold the records of launch_td_setup (with the triangles' slip).
 cudaError_t launch_td_sum_edges(PairArgs a, bool strain, bool disp, bool full, const EdgeArrays& ed, int64_t E,
                                 void* edge_rec, double nu, int64_t echunk, double* edge_partial, cudaStream_t st, int64_t* launches);
