@@ -285,7 +285,7 @@ struct SegInt {
 template <typename R>
 CAD_HD constexpr R tiny_square()   // its reciprocal's square does not overflow
 {
-    return sizeof(R) == sizeof(double) ? R(1e-140) : R(1e-15);
+    return sizeof(R) == sizeof(double) ? R(1e-140) : R(1e-18);
 }
 
 // Integrals of one side from its end distances (R, 1 / R) and the coordinates
@@ -303,7 +303,10 @@ CAD_HD SegInt<R> seg_integrals(R RA, R iA, R RB, R iB, R sA, R sB, R rho2)
     const bool out = a >= R(0.0);
     // (a point exactly on the side keeps finite integrals: whether its pair is
     // NaN is on_side's decision, triangle by triangle)
-    const R den = out ? Ra + a : (rho2 > tiny_square<R>() ? rho2 : tiny_square<R>()), num = out ? R(1.0) : Ra - a;
+    // (FP32 takes the place of 0 alone: offsets below 1e-9 are the size of a mesh in
+    // very small units, whose field overflows rather than be wrong)
+    const R least = sizeof(R) == sizeof(double) ? tiny_square<R>() : R(0.0);
+    const R den = out ? Ra + a : (rho2 > least ? rho2 : tiny_square<R>()), num = out ? R(1.0) : Ra - a;
     const R wb = Rb + b;
     const R inv = R(1.0) / (den * wb);
     const R iwa = inv * wb * num, iwb = inv * den;   // 1 / (R + s) at both ends

@@ -278,3 +278,34 @@ def test_gmres_restart_setting(cad):
             assert _rel(X, Xo) <= SLIP_TOL
     finally:
         _lib.check(L.cad_set_gmres_restart(ctx, 0), ctx)
+
+
+@pytest.mark.parametrize("hs", [0, 1])
+@pytest.mark.parametrize("k", [-33, -26, -22, 0, 20, 31])
+def test_mixed_assembly_in_other_units(cad, hs, k):
+    """The FP32 far field of a mesh measured in very small or large units: the
+    mixed matrix agrees with the FP64 one of the same mesh (its size 2^k times
+    about 2; single precision's largest and smallest values bound k)."""
+    import torch
+
+    from cutanddisplacejulia_b200 import _lib, workloads
+    L, ctx = _lib.load(), _lib.context(0)
+    P = [p * 2.0 ** k for p in workloads.dipping_rect(seed=3, ntri=240, top_depth=0.1)]
+    n = len(P[0])
+    nrm, mid = cad.CreateFaceNormalAndMidPoint(*P)
+    g = [torch.tensor(np.asfortranarray(a).ravel(order="F"), device="cuda") for a in (nrm, mid, *P)]
+    torch.cuda.synchronize()
+    got = []
+    for mode in (_lib.CAD_ASSEMBLY_MIXED, _lib.CAD_ASSEMBLY_FP64):
+        A = torch.zeros(9 * n * n, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        with _lib.assembly_mode(ctx, "mixed" if mode == _lib.CAD_ASSEMBLY_MIXED else "fp64", 3.0):
+            _lib.check(L.cad_assemble_dev(ctx, *[x.data_ptr() for x in g], n, 0.25, 1.0, 1.0, hs, A.data_ptr(), 3 * n),
+                       ctx)
+        torch.cuda.synchronize()
+        got.append(A * 2.0 ** k)
+    if k < -28:   # beyond single precision's range: not finite rather than wrong
+        assert not bool(torch.isfinite(got[0]).all())
+        return
+    # single precision's rounding through the cancelling sums of three sides
+    assert float(torch.linalg.vector_norm(got[0] - got[1]) / torch.linalg.vector_norm(got[1])) < 1e-6
