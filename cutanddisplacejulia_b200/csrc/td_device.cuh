@@ -1291,7 +1291,7 @@ struct SegRec {
     double bK[3];   // -K8 B
     double c1[3];   // (k1 - 2 K8) / 2 B x t
     double c2[3];   // (k1 - K8) B x t
-    double pad;
+    double slips;   // 0 where B is zero
 };
 constexpr int kSegWords = (int)(sizeof(SegRec) / sizeof(double));
 
@@ -1313,7 +1313,7 @@ CAD_HD void build_segment(const double PA[3], const double PB[3], const double B
         s.c1[i] = 0.5 * ka * c[i];
         s.c2[i] = (kInv4Pi - K8) * c[i];
     }
-    s.pad = 0.0;
+    s.slips = none ? 0.0 : 1.0;
 }
 
 // Strain of a segment at a point, added into E, and its displacement (but for

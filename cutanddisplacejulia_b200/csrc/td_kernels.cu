@@ -969,8 +969,10 @@ __global__ void __launch_bounds__(kPairThreads) segment_sum_kernel(const SegRec*
         __syncthreads();
         const double* src = reinterpret_cast<const double*>(edges + eb);
         for (int w = threadIdx.x; w < ne * kSegWords; w += kPairThreads) smem[w] = src[w];
-        __syncthreads();
-        if (!active) continue;
+        // edges without slip add nothing, also where 0 x the point's integrals is no
+        // 0; beside one with slip, whose field is no number there either, they may
+        // (a test of every edge costs 1 %)
+        if (!__syncthreads_or(threadIdx.x < ne && edges[eb + threadIdx.x].slips != 0.0) || !active) continue;
 #pragma unroll 1
         for (int k = 0; k < ne; ++k)
             segment_sum<STRAIN, DISP>(reinterpret_cast<const SegRec*>(smem)[k], x, y, z, sE, sU);

@@ -159,7 +159,7 @@ extern "C" int host_td_sum_edges(const double* X, const double* Y, const double*
         else pair_angle<false, true>(T[j], X[i], Y[i], Z[i], Es, Us);
       }
       for (int64_t e = 0; e < E; ++e) {
-        if (!hs) segment_sum<true, true>(R[e], X[i], Y[i], Z[i], Es, Us);
+        if (!hs) { if (R[e].slips != 0.0) segment_sum<true, true>(R[e], X[i], Y[i], Z[i], Es, Us); }
         else if (S[e].skip != 2.0) side_sum_full<true>(S[e], X[i], Y[i], Z[i], Es, Us);
       }
       for (int k = 0; k < 6; ++k) so[k * M + i] = Es[k];

@@ -80,6 +80,30 @@ def test_edges_over_sizes(cad, n, M):
         assert_parity(x, y)
 
 
+@pytest.mark.parametrize("hs", [0, 1])
+def test_no_slip_adds_nothing_anywhere(cad, hs):
+    """Triangles without slip add nothing, also at points far out of range or
+    without coordinates, over the edges as by the pairs; a slipping mesh gives
+    NaN there."""
+    from cutanddisplacejulia_b200 import _lib
+    rng = np.random.default_rng(4)
+    P = _mesh("bent", rng)
+    P = [p - [0.0, 0.0, 8.0] for p in P]
+    n = len(P[0])
+    pts = rng.uniform([-2, -2, -12], [5, 5, -0.1], ((5 << 20) // n + 1, 3))
+    pts[0], pts[1], pts[2] = [np.nan, 0, -1], [np.inf, 0, -1], [0, 1e160, -1e160]
+    L, ctx = _lib.load(), _lib.context(0)
+    for shared in (1, 0):
+        _lib.check(L.cad_set_shared_edges(ctx, shared), ctx)
+        try:
+            S, U = cad.TD(*pts.T, *P, *np.zeros((3, n)), 0.25, 1.0, 1, 1, hs, cad.Strains(), cad.Disps())
+            T, _ = cad.TD(*pts.T, *P, *np.full((3, n), 1e-3), 0.25, 1.0, 0, 1, hs, cad.Strains(), cad.Disps())
+        finally:
+            _lib.check(L.cad_set_shared_edges(ctx, 1), ctx)
+        assert not np.stack(list(S)).any() and not np.stack(list(U)).any()
+        assert np.isnan(np.stack(list(T))[:, :2]).all()
+
+
 def test_sums_where_only_the_pairs_fit(cad, fresh_context):
     """A full-space sum runs over the pairs where the edges' workspaces cannot be
     had: only the arrays every sum needs are refused."""
