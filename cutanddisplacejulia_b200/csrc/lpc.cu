@@ -77,7 +77,7 @@ __device__ __forceinline__ bool nearer(double d, int j, double e, int k) { retur
 // nearest so far; a candidate below the last one is inserted by the whole warp,
 // about K (1 + ln(N / K)) times.  With one thread per element 10 000 elements
 // filled 40 SMs, diverging on every insertion: 5.9 ms, now 0.22.  Meshes of fewer than
-// kLpcK elements repeat the farthest neighbour.
+// kLpcK elements repeat the farthest neighbour, lists short of numbers the element.
 constexpr int kKnnWarps = 8;
 __global__ void __launch_bounds__(32 * kKnnWarps) knn_kernel(const double* __restrict__ cen, int64_t N,
                                                              int* __restrict__ nbr)
@@ -127,8 +127,9 @@ __global__ void __launch_bounds__(32 * kKnnWarps) knn_kernel(const double* __res
         }
     }
     const int have = N < kLpcK ? (int)N : kLpcK;
-    const int far = __shfl_sync(full, bi, have - 1);
-    if (live && lane < kLpcK) nbr[i * kLpcK + lane] = lane < have ? bi : far;
+    const int far = __shfl_sync(full, bi, have - 1), mine = lane < have ? bi : far;
+    // (no place in the list for centroids that are not numbers: the element itself instead)
+    if (live && lane < kLpcK) nbr[i * kLpcK + lane] = mine < N ? mine : (int)i;
 }
 
 // X[i, q*7 + c]: offset (3, in i's frame, / h_i), normal (3, in i's frame),

@@ -30,3 +30,38 @@ def test_nearest_by_distance_then_index(cad, n):
     want = np.argsort(d, axis=1, kind="stable")[:, :K]     # stable: ties to the smaller index
     want = np.concatenate([want, np.repeat(want[:, -1:], K - want.shape[1], axis=1)], axis=1)
     assert np.array_equal(nbr.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n", [5, 16, 40, 300])
+def test_elements_without_coordinates_stay_in_range(cad, n):
+    """Centroids that are not numbers are nobody's neighbours; the places they
+    leave in the lists name the element itself."""
+    import torch
+    from cutanddisplacejulia_b200 import _lib
+    L, ctx = _lib.load(), _lib.context(0)
+    rng = np.random.default_rng(n)
+    cen = rng.uniform(-1, 1, (n, 3))
+    bad = np.arange(n) % 3 == 1
+    off = np.array([[0.3, 0, -0.6], [0, 0.6, 0.3], [-0.3, -0.6, 0.3]])
+    V = [cen + o for o in off]
+    V[1][bad, 2] = np.nan
+    P = [torch.from_numpy(np.ascontiguousarray(v.T)).cuda() for v in V]
+    X = torch.empty(n, 7 * K, dtype=torch.float32, device="cuda")
+    nbr = torch.empty(n, K, dtype=torch.int32, device="cuda")
+    h = torch.empty(n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    _lib.check(L.cad_lpc_features_dev(ctx, *[p.data_ptr() for p in P], n, X.data_ptr(), nbr.data_ptr(),
+                                      h.data_ptr()), ctx)
+    torch.cuda.synchronize()
+    got = nbr.cpu().numpy()
+    cen = (V[0] + V[1] + V[2]) / 3
+    good = np.flatnonzero(~bad)
+    for i in range(n):
+        if bad[i]:
+            assert (got[i] == i).all()
+            continue
+        k = min(K, len(good))
+        d = ((cen[good] - cen[i]) ** 2).sum(1)
+        assert set(got[i, :k]) == set(good[np.argsort(d)[:k]])
+        rest = got[i, k:]
+        assert np.isin(rest, [i, got[i, k - 1]]).all()
