@@ -285,9 +285,9 @@ __device__ __forceinline__ void leaf_body(T* __restrict__ A, int64_t lda, int m,
         } else {
             const unsigned bar = smem_u32(&s_bar[par]);
             const unsigned parity = (unsigned)((jj >> 1) & 1);
-            long spins = 0;
+            long spins = lost ? wait_limit : 0;   // (one poll once a wait ran out)
             while (!mbar_try_wait(bar, parity))
-                if (lost || ++spins > (wait_limit >> 2)) {   // a try_wait round may suspend briefly
+                if (++spins > (wait_limit >> 2)) {   // a try_wait round may suspend briefly
                     s_fail = 1;
                     lost = true;
                     break;
